@@ -31,6 +31,33 @@ __host__ __device__ __forceinline__ float hypot_ref(float a, float b) {
     return (float)sqrt(da * da + db * db);
 }
 
+#ifdef __CUDACC__
+// hypot_ref for 1 + c*hypot without the IEEE square root: one third-order
+// Householder step from the hardware estimate of the reciprocal square root
+// (rsqrt.approx; its relative error is below 2^-20 on every upper word, the
+// only one the unit reads, which leaves 2^-58 after the step) and Ziv's
+// rounding test.  The double result r is within kHypotUnits units of its last
+// place of the root, so it rounds to single precision as hypot_ref does unless
+// it lies that close to the midpoint of two neighbouring floats (one sum in
+// 2^25).  `near` is the distance above the lower end of that interval, of the
+// 29 bits below a float's last, modulo 2^32: the result stands if it is above
+// kHypotNear.  2^-400 added to the sum keeps zero off the estimate's pole and
+// is far below a unit of any other; a root below 2^-100 may round differently
+// from hypot_ref's, which 1 + c*hypot does not show.  Infinities give NaN.
+constexpr unsigned kHypotUnits = 8, kHypotNear = 2 * 8 * kHypotUnits;
+__device__ __forceinline__ float hypot_fast(float a, float b, unsigned &near) {
+    const double da = a, db = b;
+    const double s = __fma_rn(da, da, __fma_rn(db, db, 0x1p-400));
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+    const double h = __dmul_rn(s, y);
+    const double e = __fma_rn(-h, y, 1.0);  // s y^2 = 1 - e
+    const double r = __fma_rn(__dmul_rn(h, e), __fma_rn(e, 0.375, 0.5), h);
+    near = (unsigned)__double2loint(r) * 8u + (8u * kHypotUnits - 0x80000000u);
+    return (float)r;
+}
+#endif
+
 #ifdef __CUDA_ARCH__
 #define OF_FMAF(a, b, c) __fmaf_rn(a, b, c)
 #define OF_RCP(x) __frcp_rn(x)
@@ -42,7 +69,7 @@ __host__ __device__ __forceinline__ float hypot_ref(float a, float b) {
 // Hardware reciprocal estimate (PTX rcp.approx), refined below by one Newton
 // step.  On the host the refined form is the plain correctly rounded
 // reciprocal, which satisfies the same contract.
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
 __device__ __forceinline__ float rcp_est(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -67,14 +94,22 @@ __host__ __device__ __forceinline__ float rcp_near_rn(float g) {
 }
 
 // p / g correctly rounded (IEEE division) from y = RN(1/g): q0 = RN(p*y),
-// r = p - q0*g (exact by FMA), q = RN(q0 + r*y) (Markstein).  Valid while
+// r = q0*g - p (exact by FMA), q = RN(q0 - r*y) (Markstein).  Valid while
 // neither the quotient nor p underflows: |p| > 2^-100 with g < 2^24 keeps the
-// quotient above 2^-124; and for p = +0.  markstein_safe says so for p; other
-// p take the plain division.
+// quotient above 2^-124; and for p = +0 or -0 (the residual's sign is chosen
+// so that the quotient keeps p's).  markstein_safe says so for p (it sends -0
+// to the plain division, which agrees); other p take the plain division.
 __host__ __device__ __forceinline__ float markstein(float p, float g, float y) {
     const float q0 = p * y;
-    const float r = OF_FMAF(-q0, g, p);
-    return OF_FMAF(r, y, q0);
+    const float r = OF_FMAF(q0, g, -p);
+    return OF_FMAF(-r, y, q0);
+}
+
+// For a running minimum over numerators: every one is zero or above 2^-100 in
+// magnitude exactly when the minimum of markstein_key is at least kMarksteinKey.
+constexpr unsigned kMarksteinKey = 2u * 0x0d800000u;  // 2^-100
+__host__ __device__ __forceinline__ unsigned markstein_key(float p) {
+    return 2u * (unsigned)__float_as_int_hd(p) - 1u;
 }
 
 __host__ __device__ __forceinline__ bool markstein_safe(float p) {

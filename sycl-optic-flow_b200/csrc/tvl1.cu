@@ -10,9 +10,10 @@
 //   pyr_s[b][2]    pyramid level s of I0 / I1, dense nx_s*ny_s
 //   cc*[b], dv*[b] column coefficients of the warp's bicubic samples of
 //                  (I1, I1x, I1y) at the current level (WarpCoef, 72 B/px)
-//   WR[b]          float4 (I1wx, I1wy, rho_c, |grad I1w|^2) of the current warp
+//   W              float2 planes (I1wx, I1wy) and (rho_c, 1/|grad I1w|^2) of
+//                  the current warp, all pairs of a plane together
 //   U[k][b]        float2 (u1, u2), k = 0..7; Uz[b] upsampled flow
-//   P[k][b]        float4 (p11, p12, p21, p22), k = 0..7
+//   P[k]           float2 planes (p11, p12) and (p21, p22), k = 0..7
 // State buffers 0/1 alternate as the accepted state; 2-4 and 5-7 are two sets
 // of snapshots of the blocked kernel.  Level planes are packed at the start of
 // their level-0-sized buffers.
@@ -38,16 +39,18 @@ namespace oflow {
 
 // ---------------------------------------------------------------- constants
 constexpr int kIterTW = 32, kIterTH = 8, kIterNT = 256;
-// blocked inner iterations: iterations per launch (= halo) and the tile
-// configurations, largest first (tile TW x TH, threads); shared memory is
-// 40 B per region pixel (p 16, (I1wx, I1wy, rho_c, |grad I1w|^2) 16, u 8)
+// blocked inner iterations: iterations per launch (= halo)
 constexpr int kTbK = 4;
-// Inner-iteration configurations of k_tvl1_tb: tile tw x th, nt threads.
+// Inner-iteration configurations of the tiled kernels: the region is 64 x
+// v*nw pixels (the owned tile 4 less on each side), a block has nw warps of v
+// rows each, and mb blocks are resident on an SM (registers: 80 a thread).
 struct TbCfg {
-    int tw, th, nt;
+    int v, nw, mb;
 };
-constexpr TbCfg kTbCfgs[] = {{64, 32, 512}, {64, 16, 256}, {32, 16, 256}, {16, 8, 128}};
+constexpr TbCfg kTbCfgs[] = {{4, 12, 2}, {4, 8, 3}, {2, 12, 2}, {2, 8, 3}};
 constexpr int kTbNumCfgs = 4;
+constexpr int tb_tw() { return 64 - 2 * kTbK; }
+constexpr int tb_th(int c) { return kTbCfgs[c].v * kTbCfgs[c].nw - 2 * kTbK; }
 // Configuration 4: the whole level of a pair in one block (k_tvl1_level), for
 // levels of at most kLvMaxPx pixels.
 constexpr int kLevelCfg = 4;
@@ -58,8 +61,8 @@ constexpr int kNumIterCfgs = 6;
 // tile of a tiled configuration (false for the whole-level ones)
 inline bool cfg_tile(int c, int &tw, int &th) {
     if (c >= 0 && c < kTbNumCfgs) {
-        tw = kTbCfgs[c].tw;
-        th = kTbCfgs[c].th;
+        tw = tb_tw();
+        th = tb_th(c);
         return true;
     }
     return false;
@@ -74,11 +77,6 @@ inline bool cluster_fits(int nx, int ny) {
 constexpr int kLvNT = 1024;
 constexpr int kLvMaxPx = 9216;  // u (8 B) + p (16 B) per pixel: 221,184 B of shared memory
 inline bool level_fits(int nx, int ny) { return (long long)nx * ny <= kLvMaxPx; }
-constexpr size_t tb_smem_bytes(int tw, int th) { return (size_t)(tw + 2 * kTbK) * (th + 2 * kTbK) * 40; }
-// Resident blocks per SM the tiled kernels are compiled for (registers: 64
-// for 512 threads, 85 for fewer), matching what their shared memory allows
-// (64x32: 2, 64x16: 3; the smaller tiles are not limited by it).
-constexpr int tb_min_blocks(int nt) { return nt >= 512 ? 2 : nt >= 256 ? 3 : 6; }
 constexpr int kGaussTW = 64, kGaussTH = 32, kGaussNT = 256, kGaussMaxR = 15;
 constexpr int kIngestNT = 256, kIngestPPT = 8;
 
@@ -170,6 +168,34 @@ __device__ __forceinline__ bool better_min(const NormRec &a, const NormRec &b) {
 constexpr int kStateBufs = 2 + 2 * (kTbK - 1);
 template <typename T> __device__ __forceinline__ T *state_buf(T *b0, T *b1, int k) {
     return b0 + (ptrdiff_t)k * (b1 - b0);
+}
+
+// A float4 per pixel kept as two float2 planes, `plane` elements apart, so
+// that a thread's two neighbouring pixels are one aligned 16-byte access of
+// each plane and a warp's accesses are dense.  p is (p11, p12) and (p21, p22);
+// the warp's data is (I1wx, I1wy) and (rho_c, 1/|grad I1w|^2).
+template <typename F2> struct Quads {
+    F2 *a, *b;
+    __device__ __forceinline__ float4 get(size_t q) const {
+        const float2 u = a[q], v = b[q];
+        return make_float4(u.x, u.y, v.x, v.y);
+    }
+    __device__ __forceinline__ float4 get_ro(size_t q) const {
+        const float2 u = __ldg(a + q), v = __ldg(b + q);
+        return make_float4(u.x, u.y, v.x, v.y);
+    }
+    __device__ __forceinline__ void set(size_t q, float4 v) const {
+        a[q] = make_float2(v.x, v.y);
+        b[q] = make_float2(v.z, v.w);
+    }
+};
+// state buffer k of p, at element offset off
+__device__ __forceinline__ Quads<float2> p_buf(float2 *P, size_t plane, int k, size_t off) {
+    float2 *a = P + (size_t)(2 * k) * plane + off;
+    return Quads<float2>{a, a + plane};
+}
+__device__ __forceinline__ Quads<const float2> w_quads(const float2 *W, size_t plane, size_t off) {
+    return Quads<const float2>{W + off, W + plane + off};
 }
 
 // ---------------------------------------------------------------- ingest
@@ -545,7 +571,7 @@ __global__ void k_cubic_pack(const float *__restrict__ pyr, size_t pyr_stride, i
 // ---------------------------------------------------------------- warping
 // Per warp (tvl1.cpp:197-212): bicubic samples of I1, I1x, I1y at (x+u1,
 // y+u2) with border zeroing, then rho_c and |grad I1w|^2 (tvl1.cpp:202-212),
-// packed as one float4 per pixel.  mode 0: u from U[cur];
+// stored as two float2 planes (Quads).  mode 0: u from U[cur];
 // 1: u from the upsampled Uz (copied into U[cur]); 2: u = 0 (coarsest scale).
 // With first_warp, p is zeroed (tvl1.cpp:190-193).
 enum { kWarpFromU = 0, kWarpFromUz = 1, kWarpZero = 2 };
@@ -559,8 +585,8 @@ enum { kWarpFromU = 0, kWarpFromUz = 1, kWarpZero = 2 };
 // 1024x436 workload at 32 pairs.
 constexpr int kWarpTW = 32, kWarpTH = 8;
 __global__ void __launch_bounds__(kWarpTW * kWarpTH, 6) k_warp(const float *__restrict__ pyr, size_t pyr_stride, WarpCoef wc,
-                       float4 *WR, float2 *U0, float2 *U1, const float2 *Uz, float4 *P0,
-                       float4 *P1, size_t stride, int nx, int ny, int mode, int first_warp,
+                       float2 *W, float2 *U0, float2 *U1, const float2 *Uz, float2 *P, size_t plane,
+                       size_t stride, int nx, int ny, int mode, int first_warp,
                        TvCtrl *ctrl, TbQueue *q, int *left) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -589,7 +615,7 @@ __global__ void __launch_bounds__(kWarpTW * kWarpTH, 6) k_warp(const float *__re
         u = make_float2(0.0f, 0.0f);
         U[p] = u;
     }
-    if (first_warp) (state_buf(P0, P1, cur) + off)[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (first_warp) p_buf(P, plane, cur, off).set(p, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
     const float uu = (float)x + u.x, vv = (float)y + u.y;
     float Iw = 0.0f, Iwx = 0.0f, Iwy = 0.0f;
     BicubicStencil s;
@@ -614,7 +640,8 @@ __global__ void __launch_bounds__(kWarpTW * kWarpTH, 6) k_warp(const float *__re
     }
     const float I0v = __ldg(pyr + (size_t)(2 * b) * pyr_stride + p);
     const float rho_c = (Iw - Iwx * u.x - Iwy * u.y - I0v);
-    WR[off + p] = make_float4(Iwx, Iwy, rho_c, (Iwx * Iwx) + (Iwy * Iwy));
+    W[off + p] = make_float2(Iwx, Iwy);
+    W[plane + off + p] = make_float2(rho_c, rcp_near_rn((Iwx * Iwx) + (Iwy * Iwy)));
 }
 
 // ---------------------------------------------------------------- iteration
@@ -633,31 +660,40 @@ __device__ __forceinline__ float div_border(float a1c, float a1l, float a2c, flo
     return -a1l - a2u;
 }
 
-// TH step (tvl1.cpp:221-245) and u update (:252-265) for one pixel.  wr holds
-// (I1wx, I1wy, rho_c, |grad I1w|^2).  The branches of the reference pick the
+// TH step (tvl1.cpp:221-245) for one pixel: v = u + d.  wr holds (I1wx, I1wy,
+// rho_c, RN(1/|grad I1w|^2)).  The branches of the reference pick the
 // coefficient of (I1wx, I1wy): l_t where rho < -l_t*grad, -l_t where rho >
 // l_t*grad, 0 where the gradient vanishes, else -rho/grad; the products are
 // the reference's, so the result is identical.  The quotient is formed for
-// every pixel (most need it) by Markstein's correction from RN(1/grad), which
-// equals IEEE division inside the ranges rcp_in_range and markstein_safe
-// cover; a pixel that needs the quotient outside them takes the division.
+// every pixel (most need it) by Markstein's correction from the reciprocal
+// k_warp stores, which equals IEEE division while grad is in [1e-10, 2^24)
+// (smaller gradients take d = 0) and |rho| > 2^-100; a pixel that needs the
+// quotient outside that takes the division.  grad itself is formed again
+// from its two factors (three instructions, as many as refining the
+// reciprocal would take, and none of them on the conversion pipe).
+__device__ __forceinline__ float th_grad(float4 wr) { return (wr.x * wr.x) + (wr.y * wr.y); }
+__device__ __forceinline__ float th_rho(float2 u, float4 wr) { return wr.z + (wr.x * u.x + wr.y * u.y); }
+__device__ __forceinline__ float th_coef(float rho, float grad, float quot, float l_t) {
+    const float lg = l_t * grad;
+    return !(rho >= -lg) ? l_t : (rho > lg ? -l_t : (grad < 1E-10f ? 0.0f : quot));
+}
+
+__device__ __forceinline__ float2 th_step(float2 u, float4 wr, float l_t) {
+    const float grad = th_grad(wr), rho = th_rho(u, wr);
+    float q = markstein(-rho, grad, wr.w);
+    if (!(fabsf(rho) > 0x1p-100f && grad < kRcpHi)) q = -rho / grad;
+    const float k = th_coef(rho, grad, q, l_t);
+    return make_float2(u.x + k * wr.x, u.y + k * wr.y);
+}
+
+// TH step and u update (tvl1.cpp:252-265) for one pixel.
 __device__ __forceinline__ float2 th_u_update(float2 u, float4 wr, float4 pc, float4 pl, float4 pu,
                                               bool L, bool R, bool T, bool B, float l_t,
                                               float theta) {
-    const float grad = wr.w;
-    const float rho = wr.z + (wr.x * u.x + wr.y * u.y);
-    const float lg = l_t * grad;
-    const bool c1 = rho >= -lg, c2 = rho > lg, c3 = grad < 1E-10f;
-    const float nrho = -rho;
-    float fi = markstein(nrho, grad, rcp_near_rn(grad));
-    if (c1 && !c2 && !c3 && !(rcp_in_range(grad) && markstein_safe(nrho))) fi = nrho / grad;
-    const float k = !c1 ? l_t : (c2 ? -l_t : fi);
-    const bool flat = c1 && !c2 && c3;  // the reference's d = 0, by selection
-    const float d1 = flat ? 0.0f : k * wr.x, d2 = flat ? 0.0f : k * wr.y;
-    const float v1 = u.x + d1, v2 = u.y + d2;
+    const float2 v = th_step(u, wr, l_t);
     const float div1 = div_border(pc.x, pl.x, pc.y, pu.y, L, R, T, B);
     const float div2 = div_border(pc.z, pl.z, pc.w, pu.w, L, R, T, B);
-    return make_float2(v1 + theta * div1, v2 + theta * div2);
+    return make_float2(v.x + theta * div1, v.y + theta * div2);
 }
 
 // Dual update (tvl1.cpp:268-291) from the forward differences of u(new):
@@ -689,10 +725,51 @@ __device__ __forceinline__ float4 dual_update(float4 po, float f1x, float f1y, f
     return pn;
 }
 
+// What the branch-free forms of the two steps take for granted, kept as
+// running extremes over the pixels and iterations of a thread and checked once
+// per tile: numerators zero or above 2^-100 (key), denominators below 2^24
+// (den), hypots away from the rounding midpoints (near).
+struct FastGuard {
+    unsigned key = ~0u, near = ~0u;
+    float den = 0.0f;
+    __device__ __forceinline__ void add_den(float g) { asm("max.NaN.f32 %0, %0, %1;" : "+f"(den) : "f"(g)); }
+    __device__ __forceinline__ void add_num(float n) { key = umin(key, markstein_key(n)); }
+    __device__ __forceinline__ bool broken() const {
+        return key < kMarksteinKey || near <= kHypotNear || !(den < kRcpHi);
+    }
+};
+
+// The TH step's coefficient and the dual update without branches: the bits of
+// th_step and dual_update while the guard holds.
+__device__ __forceinline__ float th_coef_fast(float2 u, float4 wr, float l_t, FastGuard &fg) {
+    const float grad = th_grad(wr), rho = th_rho(u, wr);
+    fg.add_num(rho);
+    fg.add_den(grad);
+    return th_coef(rho, grad, markstein(-rho, grad, wr.w), l_t);
+}
+
+__device__ __forceinline__ float4 dual_update_fast(float4 po, float f1x, float f1y, float f2x,
+                                                   float f2y, float taut, FastGuard &fg) {
+    unsigned m1, m2;
+    const float h1 = hypot_fast(f1x, f1y, m1), h2 = hypot_fast(f2x, f2y, m2);
+    fg.near = umin(umin(fg.near, m1), m2);
+    const float g1 = 1.0f + taut * h1, g2 = 1.0f + taut * h2;
+    fg.add_den(g1);
+    fg.add_den(g2);
+    const float r1 = rcp_near_rn(g1), r2 = rcp_near_rn(g2);  // g >= 1
+    const float n1 = taut * f1x + po.x, n2 = taut * f1y + po.y;
+    const float n3 = taut * f2x + po.z, n4 = taut * f2y + po.w;
+    fg.key = umin(umin(fg.key, markstein_key(n1)), markstein_key(n2));
+    fg.key = umin(umin(fg.key, markstein_key(n3)), markstein_key(n4));
+    return make_float4(markstein(n1, g1, r1), markstein(n2, g1, r1), markstein(n3, g2, r2),
+                       markstein(n4, g2, r2));
+}
+
 struct IterArgs {
-    const float4 *WR;  // (I1wx, I1wy, rho_c, |grad I1w|^2) per pixel
+    const float2 *W;
     float2 *U0, *U1;
-    float4 *P0, *P1;
+    float2 *P;
+    size_t plane;   // elements of one plane of p and W
     size_t stride;  // elements between pairs
     int nx, ny;
     float l_t, theta, taut, eps2;
@@ -720,9 +797,8 @@ __global__ void __launch_bounds__(NT) k_tvl1_iter(IterArgs a) {
     const size_t off = (size_t)b * a.stride;
     const float2 *__restrict__ Uin = state_buf(a.U0, a.U1, cur) + off;
     float2 *__restrict__ Uout = state_buf(a.U0, a.U1, cur ^ 1) + off;
-    const float4 *__restrict__ Pin = state_buf(a.P0, a.P1, cur) + off;
-    float4 *__restrict__ Pout = state_buf(a.P0, a.P1, cur ^ 1) + off;
-    const float4 *__restrict__ WR = a.WR + off;
+    const Quads<float2> Pin = p_buf(a.P, a.plane, cur, off), Pout = p_buf(a.P, a.plane, cur ^ 1, off);
+    const Quads<const float2> Wq = w_quads(a.W, a.plane, off);
     const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
 
     __shared__ float4 sP[(TH + 2) * (TW + 2)];
@@ -733,7 +809,7 @@ __global__ void __launch_bounds__(NT) k_tvl1_iter(IterArgs a) {
     for (int i = threadIdx.x; i < (TH + 2) * (TW + 2); i += NT) {
         const int x = x0 + i % (TW + 2) - 1, y = y0 + i / (TW + 2) - 1;
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (x >= 0 && x < nx && y >= 0 && y < ny) p = Pin[(size_t)y * nx + x];
+        if (x >= 0 && x < nx && y >= 0 && y < ny) p = Pin.get((size_t)y * nx + x);
         sP[i] = p;
     }
     __syncthreads();
@@ -746,7 +822,7 @@ __global__ void __launch_bounds__(NT) k_tvl1_iter(IterArgs a) {
         const size_t p = (size_t)y * nx + x;
         const float2 u = Uin[p];
         const float4 *c = sP + (ry + 1) * (TW + 2) + (rx + 1);
-        const float2 un = th_u_update(u, WR[p], c[0], c[-1], c[-(TW + 2)], x == 0,
+        const float2 un = th_u_update(u, Wq.get(p), c[0], c[-1], c[-(TW + 2)], x == 0,
                                       x == nx - 1, y == 0, y == ny - 1, a.l_t, a.theta);
         sU[i] = un;
         if (rx < TW && ry < TH) {
@@ -775,7 +851,7 @@ __global__ void __launch_bounds__(NT) k_tvl1_iter(IterArgs a) {
             f2y = ud.y - uc.y;
         }
         const float4 pn = dual_update(sP[(ry + 1) * (TW + 2) + rx + 1], f1x, f1y, f2x, f2y, a.taut);
-        Pout[(size_t)y * nx + x] = pn;
+        Pout.set((size_t)y * nx + x, pn);
     }
 
     // ---- error reduction and loop control (tvl1.cpp:252-265, :216)
@@ -809,21 +885,35 @@ __global__ void __launch_bounds__(NT) k_tvl1_iter(IterArgs a) {
 
 
 // ---------------------------------------------------------------- blocked iterations
-// Up to K inner iterations per launch on a TW x TH tile held in shared memory
-// with a K-pixel halo (the dependency cone of one iteration is one pixel in
-// every direction, so after K iterations the owned tile is exact).  The state
-// is loaded once and stored once per launch, so HBM traffic per iteration
-// drops by about K.  Each iteration's squared change over the owned pixels is
-// kept; the last block of a pair finds the first iteration that meets the
-// stopping rule (tvl1.cpp:216).  When a stop is plausible (kSnapMargin), the
-// owned tile is also stored after each of the first K-1 iterations into a
-// snapshot buffer, so a stop in the middle of the launch accepts that
-// iteration's state; otherwise the next launch re-runs those iterations.
+// Up to K inner iterations per launch on a tile with a K-pixel halo (the
+// dependency cone of one iteration is one pixel in every direction, so after K
+// iterations the owned tile is exact).  The state is loaded once and stored
+// once per launch, so HBM traffic per iteration drops by about K.  Each
+// iteration's squared change over the owned pixels is kept; the last block of
+// a pair finds the first iteration that meets the stopping rule
+// (tvl1.cpp:216).  When a stop is plausible (kSnapMargin), the owned tile is
+// also stored after each of the first K-1 iterations into a snapshot buffer,
+// so a stop in the middle of the launch accepts that iteration's state;
+// otherwise the next launch re-runs those iterations.
+//
+// Measured (32 pairs of 1024x436, the five warp stages of the finest scale):
+// 10.0 ms against 13.05 ms for the form that kept the 72x40 region in shared
+// memory (five 16-byte shared accesses a pixel and iteration, 256 instructions
+// a pixel-iteration).  Here it is about 150 instructions, of which 63 single
+// precision arithmetic, 15 double (the hypots), 11 conversions and estimates,
+// 13 the guard; issue slots are 62 % busy, the rest waits at the block's
+// barriers and for a tile's loads.  Two blocks of 12 warps with 4 rows each
+// (80 registers) beat two of 8 warps with 6 rows (128 registers, fewer warps:
+// 10.6 ms), three of 8 with 4 (64x32 regions, more halo: 10.6 ms) and one of
+// 16 with 4 (12.3 ms).  Skipping the halo rows that no longer reach the owned
+// tile saved 9 % of the arithmetic and cost as much in branches (10.2 ms);
+// waiting for the neighbouring warps' rows only, instead of block barriers,
+// 10.6 ms; the two columns as paired instructions (add/fma .f32x2) 12.2 ms.
 struct TbArgs {
-    const float4 *WR;
+    const float2 *W;
     float2 *U0, *U1;
-    float4 *P0, *P1;
-    size_t stride;
+    float2 *P;
+    size_t plane, stride;
     int nx, ny, max_it;
     float l_t, theta, taut, eps2;
     TvCtrl *ctrl;
@@ -831,132 +921,308 @@ struct TbArgs {
     int max_tiles;
     int *iters;
     int iter_stride, stage;
-    // TMA region loads (k_tvl1_tb): use_tma set when the maps below describe
-    // this level for the launched tile shape; err is set when a load's
-    // bounded wait gives up
-    int use_tma;
-    int *err;
+    int vec;   // two adjacent pixels of a row are 16-byte aligned (even nx and plane size)
+    int *err;  // set when the queue's bounded wait gives up
     // queue form only: size a pair's block of iterations to end where the
     // error's geometric decay predicts its stop (the launch form's fixed
     // schedule needs full blocks)
     int predict;
-    CUtensorMap tmP;  // p: (2 nx, ny, pair, buffer) 8-byte elements
-    CUtensorMap tmU;  // u: (nx, ny, pair, buffer) 8-byte elements
-    CUtensorMap tmW;  // (I1wx, I1wy, rho_c, grad): (2 nx, ny, pair) 8-byte elements
 };
 
-// One blocked iteration j (1-based) over the region.  Phase B (TH + u update)
-// covers [j, RW-j]^2 and phase C (dual update) [j, RW-1-j]^2: exactly the
-// pixels whose values reach the owned tile after K iterations, so no read
-// ever leaves the region.  INTERIOR: no region pixel lies on the image border
-// (no bounds or border tests).
-template <int TW, int TH, int K, int NT, bool INTERIOR>
-__device__ __forceinline__ void tb_iteration(int j, float4 *sP, const float4 *sWR, float2 *sU, int ox, int oy, int nx,
-                                             int ny, float l_t, float theta, float taut,
-                                             double &err) {
-    constexpr int RW = TW + 2 * K, RH = TH + 2 * K;
-    for_rect<NT>(j, RW - j, j, RH - j, [&](int rx, int ry) {
-        const int i = ry * RW + rx;
-        const int x = ox + rx, y = oy + ry;
-        if (!INTERIOR && (x >= nx || y >= ny || x < 0 || y < 0)) return;
-        const float2 u = sU[i];
-        const float2 un = th_u_update(u, sWR[i], sP[i], sP[i - 1], sP[i - RW],
-                                      !INTERIOR && x == 0, !INTERIOR && x == nx - 1,
-                                      !INTERIOR && y == 0, !INTERIOR && y == ny - 1, l_t, theta);
-        sU[i] = un;
-        if (rx >= K && rx < K + TW && ry >= K && ry < K + TH) {
+// Tiles.  The region is 64 pixels wide and V*NW high: a warp owns V rows, a
+// lane two adjacent columns of them, with u and p in its registers for the
+// whole block of iterations.  Left p and right u neighbours come from the
+// lane beside it by shuffle, upper p and lower u neighbours from its own
+// registers, and only the rows between two warps go through shared memory.
+// The warp's data waits in shared memory, each thread's at its own slots.
+// The halo is a whole number of warps above and below and of lanes at each
+// side, so a thread's pixels are owned all or none.
+template <int V_, int NW_> struct RtTile {
+    static constexpr int V = V_, NW = NW_, NT = 32 * NW, K = kTbK;
+    static_assert(K % V == 0, "the halo is whole warps: all rows of a warp are owned or none");
+    static constexpr int RW = 64, RH = V * NW, TW = RW - 2 * K, TH = RH - 2 * K;
+    struct Smem {
+        float4 w[2 * V][NT];    // row v: (I1wx, I1wy) of both columns at [2v], (rho_c, 1/grad) at [2v + 1]
+        float4 pb[NW][32];      // (p12, p22) of both columns of each warp's last row
+        float4 ut[NW][32];      // u of both columns of each warp's first row
+        double err[2][K][NT];   // squared change per thread and iteration, of this tile and the last
+    };
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool ok) {
+    const int n = ok ? 16 : 0;  // 0: zero fill, src is not read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
+// The thread's share of the state: rows of its warp, two columns each.
+template <int V> struct RtState {
+    float2 u[V][2];
+    float4 p[V][2];
+};
+
+// One inner iteration on the registers.  Pixels whose neighbours lie outside
+// the region compute values that no owned pixel sees within K iterations.
+// BORDER: the region touches the image border; the border forms of
+// mask.cpp:63-89 differ from the interior one by neighbours taken as zero and,
+// in the first and last column, by the order of the two additions.  EXACT: the
+// steps with all their branches, for a tile whose guard broke.
+template <typename T, bool BORDER, bool EXACT>
+__device__ __forceinline__ void rt_iteration(RtState<T::V> &s, typename T::Smem &sm, int x, int y0,
+                                             int nx, int ny, float l_t, float theta, float taut,
+                                             FastGuard &fg, double &err) {
+    constexpr int V = T::V;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const bool xl = BORDER && x == 0;
+    // TH step, divergence and u update
+    float4 up = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (wid > 0) up = sm.pb[wid - 1][lane];
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const float l1 = __shfl_up_sync(0xffffffffu, s.p[v][1].x, 1);
+        const float l3 = __shfl_up_sync(0xffffffffu, s.p[v][1].z, 1);
+        const int y = y0 + v;
+        const float4 wa = sm.w[2 * v][tid], wb = sm.w[2 * v + 1][tid];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const float4 pc = s.p[v][c];
+            float a1c = pc.x, a3c = pc.z, a2c = pc.y, a4c = pc.w;
+            float a1l = c ? s.p[v][0].x : l1, a3l = c ? s.p[v][0].z : l3;
+            float a2u = v ? s.p[v ? v - 1 : 0][c].y : (c ? up.z : up.x);
+            float a4u = v ? s.p[v ? v - 1 : 0][c].w : (c ? up.w : up.y);
+            const bool xr = BORDER && x + c == nx - 1;
+            if (BORDER) {
+                if (xl && c == 0) a1l = a3l = 0.0f;
+                if (xr) a1c = a3c = 0.0f;
+                if (y == 0) a2u = a4u = 0.0f;
+                if (y == ny - 1) a2c = a4c = 0.0f;
+            }
+            const float dx1 = a1c - a1l, dx2 = a3c - a3l;
+            float div1 = dx1 + (a2c - a2u), div2 = dx2 + (a4c - a4u);
+            if (BORDER && ((xl && c == 0) || xr)) {
+                div1 = (dx1 + a2c) - a2u;
+                div2 = (dx2 + a4c) - a4u;
+            }
+            const float2 u = s.u[v][c];
+            const float4 w = c ? make_float4(wa.z, wa.w, wb.z, wb.w) : make_float4(wa.x, wa.y, wb.x, wb.y);
+            float2 t;
+            if (EXACT) {
+                t = th_step(u, w, l_t);
+            } else {
+                const float k = th_coef_fast(u, w, l_t, fg);
+                t = make_float2(u.x + k * w.x, u.y + k * w.y);
+            }
+            const float2 un = make_float2(t.x + theta * div1, t.y + theta * div2);
+            s.u[v][c] = un;
             const float e1 = un.x - u.x, e2 = un.y - u.y;
             const float term = e1 * e1 + e2 * e2;
-            err += (double)term;
+            err += (double)(!BORDER || (y < ny && x + c < nx) ? term : 0.0f);
         }
-    });
+    }
+    sm.ut[wid][lane] = make_float4(s.u[0][0].x, s.u[0][0].y, s.u[0][1].x, s.u[0][1].y);
     __syncthreads();
-    for_rect<NT>(j, RW - 1 - j, j, RH - 1 - j, [&](int rx, int ry) {
-        const int i = ry * RW + rx;
-        const int x = ox + rx, y = oy + ry;
-        if (!INTERIOR && (x >= nx || y >= ny || x < 0 || y < 0)) return;
-        const float2 uc = sU[i];
-        float f1x = 0.0f, f2x = 0.0f, f1y = 0.0f, f2y = 0.0f;
-        if (INTERIOR || x < nx - 1) {
-            const float2 ur = sU[i + 1];
-            f1x = ur.x - uc.x;
-            f2x = ur.y - uc.y;
+    // forward gradient of u and dual update
+    float4 dn = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (wid + 1 < T::NW) dn = sm.ut[wid + 1][lane];
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const float rx = __shfl_down_sync(0xffffffffu, s.u[v][0].x, 1);
+        const float ry = __shfl_down_sync(0xffffffffu, s.u[v][0].y, 1);
+        const int y = y0 + v;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const float2 uc = s.u[v][c];
+            const float2 ur = c ? make_float2(rx, ry) : s.u[v][1];
+            const float2 ud = v + 1 < V ? s.u[v + 1 < V ? v + 1 : v][c]
+                                        : (c ? make_float2(dn.z, dn.w) : make_float2(dn.x, dn.y));
+            float f1x = ur.x - uc.x, f2x = ur.y - uc.y, f1y = ud.x - uc.x, f2y = ud.y - uc.y;
+            if (BORDER && x + c == nx - 1) f1x = f2x = 0.0f;
+            if (BORDER && y == ny - 1) f1y = f2y = 0.0f;
+            s.p[v][c] = EXACT ? dual_update(s.p[v][c], f1x, f1y, f2x, f2y, taut)
+                              : dual_update_fast(s.p[v][c], f1x, f1y, f2x, f2y, taut, fg);
         }
-        if (INTERIOR || y < ny - 1) {
-            const float2 ud = sU[i + RW];
-            f1y = ud.x - uc.x;
-            f2y = ud.y - uc.y;
-        }
-        sP[i] = dual_update(sP[i], f1x, f1y, f2x, f2y, taut);
-    });
+    }
+    sm.pb[wid][lane] = make_float4(s.p[V - 1][0].y, s.p[V - 1][0].w, s.p[V - 1][1].y, s.p[V - 1][1].w);
     __syncthreads();
 }
 
-// Per-iteration error sums of one block into its partial slots, then the
-// stopping decision by the last block of the pair to arrive: it finds the
+// Stores the owned pixels of the registers.
+template <typename T>
+__device__ __forceinline__ void rt_store(const RtState<T::V> &s, float2 *__restrict__ Ud,
+                                         const Quads<float2> Pd, int x, int y0, int nx, int ny, int vec) {
+    const int lane = threadIdx.x & 31, r0 = (threadIdx.x >> 5) * T::V;
+    if (lane < T::K / 2 || lane >= 32 - T::K / 2 || x >= nx) return;
+#pragma unroll
+    for (int v = 0; v < T::V; v++) {
+        if (r0 + v < T::K || r0 + v >= T::RH - T::K || y0 + v >= ny) continue;
+        const size_t q = (size_t)(y0 + v) * nx + x;
+        const float4 p0 = s.p[v][0], p1 = s.p[v][1];
+        if (vec) {
+            *reinterpret_cast<float4 *>(Ud + q) =
+                make_float4(s.u[v][0].x, s.u[v][0].y, s.u[v][1].x, s.u[v][1].y);
+            *reinterpret_cast<float4 *>(Pd.a + q) = make_float4(p0.x, p0.y, p1.x, p1.y);
+            *reinterpret_cast<float4 *>(Pd.b + q) = make_float4(p0.z, p0.w, p1.z, p1.w);
+        } else {
+            Ud[q] = s.u[v][0];
+            Pd.set(q, p0);
+            if (x + 1 < nx) {
+                Ud[q + 1] = s.u[v][1];
+                Pd.set(q + 1, p1);
+            }
+        }
+    }
+}
+
+// Two neighbouring float2 at q, past L1; in0, in1: inside the level.
+__device__ __forceinline__ float4 ld_two(const float2 *p, size_t q, int vec, bool in0, bool in1) {
+    if (vec) return in0 ? __ldcg(reinterpret_cast<const float4 *>(p + q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 z = make_float2(0.f, 0.f);
+    const float2 a = in0 ? __ldcg(p + q) : z, b = in1 ? __ldcg(p + q + 1) : z;
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// State of a pair at the start of a block of iterations.
+struct TbStart {
+    int cur, n0, redo, kk;
+    bool snaps;
+};
+
+// One tile of one pair for kk <= K iterations: region in (past L1: other
+// blocks write the state), iterations, snapshot stores and the final store of
+// the owned tile.  Each thread leaves its squared change of iteration j in
+// err[j].  Returns whether the thread's guard broke: the tile is then run
+// again from its untouched input, EXACT.  `issued` runs once the loads are in
+// flight.  The pair and tile come from shared memory and are read again where
+// needed, so that they do not occupy registers during the iterations.
+template <typename T, bool EXACT, typename F>
+__device__ __forceinline__ bool rt_tile(const TbArgs &a, const volatile int *vb, const volatile int *vtile,
+                                        int tiles_x, const TbStart &t, typename T::Smem &sm,
+                                        double (*err)[T::NT], F &&issued) {
+    constexpr int V = T::V, K = T::K;
+    const int nx = a.nx, ny = a.ny;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const auto origin = [&](int &x, int &y0) {
+        const int tile = *vtile, ty = tile / tiles_x, tx = tile - ty * tiles_x;
+        x = tx * T::TW - K + 2 * lane;
+        y0 = ty * T::TH - K + wid * V;
+    };
+    // accepted state in, final state to the other of buffers 0/1, snapshots
+    // after iterations 1..K-1 to the snapshot set not containing the input
+    const auto store = [&](const RtState<V> &s, int k) {
+        int x, y0;
+        origin(x, y0);
+        const size_t off = (size_t)*vb * a.stride;
+        rt_store<T>(s, state_buf(a.U0, a.U1, k) + off, p_buf(a.P, a.plane, k, off), x, y0, nx, ny, a.vec);
+    };
+    int x, y0;
+    origin(x, y0);
+    const size_t off = (size_t)*vb * a.stride;
+    const float2 *__restrict__ Uin = state_buf(a.U0, a.U1, t.cur) + off;
+    const Quads<float2> Pin = p_buf(a.P, a.plane, t.cur, off);
+    const Quads<const float2> Wq = w_quads(a.W, a.plane, off);
+    RtState<V> s;
+    const bool in0 = x >= 0 && x < nx, in1 = x + 1 >= 0 && x + 1 < nx;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const int y = y0 + v;
+        const bool iy = y >= 0 && y < ny, i0 = iy && in0, i1 = iy && in1;
+        const size_t q = (size_t)y * nx + x;
+        if (a.vec) {
+            cp_async16(smem_u32(&sm.w[2 * v][tid]), i0 ? Wq.a + q : Wq.a, i0);
+            cp_async16(smem_u32(&sm.w[2 * v + 1][tid]), i0 ? Wq.b + q : Wq.b, i0);
+        } else {
+            sm.w[2 * v][tid] = ld_two(Wq.a, q, 0, i0, i1);
+            sm.w[2 * v + 1][tid] = ld_two(Wq.b, q, 0, i0, i1);
+        }
+        const float4 pa = ld_two(Pin.a, q, a.vec, i0, i1), pb = ld_two(Pin.b, q, a.vec, i0, i1);
+        const float4 u = ld_two(Uin, q, a.vec, i0, i1);
+        s.p[v][0] = make_float4(pa.x, pa.y, pb.x, pb.y);
+        s.p[v][1] = make_float4(pa.z, pa.w, pb.z, pb.w);
+        s.u[v][0] = make_float2(u.x, u.y);
+        s.u[v][1] = make_float2(u.z, u.w);
+    }
+    issued();
+    sm.pb[wid][lane] = make_float4(s.p[V - 1][0].y, s.p[V - 1][0].w, s.p[V - 1][1].y, s.p[V - 1][1].w);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    // block-uniform: whether the region lies inside the image with a margin of one pixel
+    const int ox = x - 2 * lane, oy = y0 - wid * V;
+    const bool interior = ox >= 1 && oy >= 1 && ox + T::RW <= nx - 1 && oy + T::RH <= ny - 1;
+    FastGuard fg;
+#pragma unroll 1
+    for (int j = 0; j < *(volatile const int *)&t.kk; j++) {
+        double e = 0.0;
+        if (!EXACT && interior)
+            rt_iteration<T, false, false>(s, sm, x, y0, nx, ny, a.l_t, a.theta, a.taut, fg, e);
+        else
+            rt_iteration<T, true, EXACT>(s, sm, x, y0, nx, ny, a.l_t, a.theta, a.taut, fg, e);
+        err[j][tid] = lane >= K / 2 && lane < 32 - K / 2 && wid >= K / V && wid < T::NW - K / V ? e : 0.0;
+        if (t.snaps && j + 1 < t.kk)  // the state a stop after iteration j+1 accepts
+            store(s, (t.cur >= 2 && t.cur < 2 + (K - 1) ? 2 + (K - 1) : 2) + j);
+    }
+    store(s, t.cur == 0 ? 1 : 0);
+    return !EXACT && fg.broken();
+}
+
+template <typename T>
+static __device__ __noinline__ void rt_tile_exact(const TbArgs &a, const volatile int *vb,
+                                                  const volatile int *vtile, int tiles_x, const TbStart &t,
+                                                  typename T::Smem &sm, double (*err)[T::NT]) {
+    rt_tile<T, true>(a, vb, vtile, tiles_x, t, sm, err, [] {});
+}
+
+// Per-iteration error sums of one tile into its partial slots, then the
+// stopping decision by the tile of the pair that arrives last: it finds the
 // first of the kk iterations meeting the stopping rule (tvl1.cpp:216) and
 // accepts the state after that iteration -- the final buffer, or the snapshot
 // written after it (snap >= 0).  Without a snapshot, `redo` makes the next
 // launch re-run exactly that many iterations from the untouched input.  The
 // result is that of one iteration per launch either way.  Partials are summed
 // in a fixed order, so the decision does not depend on block scheduling.
-// Dynamic shared memory the decision may reuse once the tile is stored: K x
-// (NT/32) doubles.  (Static shared memory is kept small: two 64x32 tiles per
-// SM leave it under 512 bytes a block.)
-template <int K, int NT>
-__device__ __forceinline__ bool tb_decide(const TbArgs &a, TvCtrl *ctrl, int b, int tile,
-                                          int ntiles, double wsum, int kk, int fin,
-                                          int snap, int redo, int n0, TbQueue *q, int *left,
-                                          double *scratch) {
-    // The K sums share one block barrier: per warp a fixed shuffle tree, then
-    // thread 0 adds the warps in order (block_sum_double's order, per sum).
-    constexpr int NW = NT / 32;
-    double(*sred)[NW] = reinterpret_cast<double(*)[NW]>(scratch);
-    __shared__ double sE[K];
-    __shared__ int s_last;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// One warp does it, after a block barrier behind every thread's stores and
+// errors, while the block's other warps go on to the next tile: the sums, the
+// fence behind the tile's stores and the arrival would hold up the whole block
+// for about a quarter of a tile's time.
+template <typename T>
+__device__ __forceinline__ void tb_decide(const TbArgs &a, TvCtrl *ctrl, int b, int tile,
+                                          int ntiles, const double (*err)[T::NT], const TbStart &t,
+                                          TbQueue *q, int *left) {
+    constexpr int K = T::K, NW = T::NW;
+    const int lane = threadIdx.x & 31;
+    const int kk = t.kk, redo = t.redo, n0 = t.n0;
+    const int fin = t.cur == 0 ? 1 : 0;
+    const int snap = !t.snaps ? -1 : (t.cur >= 2 && t.cur < 2 + (K - 1)) ? 2 + (K - 1) : 2;
     double *part = a.partials + (size_t)b * a.max_tiles * K;
-    __syncthreads();  // every thread has stored its share of the tile (scratch overlays it)
-    if (lane < K) sred[lane][wid] = wsum;  // the warp sums of tb_tile (lane j: iteration j)
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int j = 0; j < kk; j++) {
-            double r = 0.0;
+    double sum[K];
 #pragma unroll
-            for (int w = 0; w < NW; w++) r += sred[j][w];
-            part[(size_t)tile * K + j] = r;
-        }
+    for (int j = 0; j < K; j++) {
+        double e = 0.0;
+        if (j < kk)
+#pragma unroll
+            for (int i = 0; i < NW; i++) e += err[j][32 * i + lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+        sum[j] = e;
+    }
+    int last = 0;
+    if (lane == 0) {
+#pragma unroll
+        for (int j = 0; j < K; j++)
+            if (j < kk) part[(size_t)tile * K + j] = sum[j];
         __threadfence();
-        const unsigned prev = atomicAdd(&ctrl->arrive, 1u);
-        s_last = (prev == (unsigned)ntiles - 1);
+        last = atomicAdd(&ctrl->arrive, 1u) == (unsigned)ntiles - 1;
     }
-    __syncthreads();
-    if (!s_last) return false;
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
     __threadfence();
-    {
-        double acc[K];
 #pragma unroll
-        for (int j = 0; j < K; j++) acc[j] = 0.0;
-        for (int t = threadIdx.x; t < ntiles; t += NT)
+    for (int j = 0; j < K; j++) {
+        double e = 0.0;
+        if (j < kk)
+            for (int i = lane; i < ntiles; i += 32) e += __ldcg(part + (size_t)i * K + j);
 #pragma unroll
-            for (int j = 0; j < K; j++)
-                if (j < kk) acc[j] += __ldcg(part + (size_t)t * K + j);
-#pragma unroll
-        for (int j = 0; j < K; j++) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_down_sync(0xffffffffu, acc[j], o);
-            if (lane == 0) sred[j][wid] = acc[j];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0)
-            for (int j = 0; j < kk; j++) {
-                double r = 0.0;
-#pragma unroll
-                for (int w = 0; w < NW; w++) r += sred[j][w];
-                sE[j] = r;
-            }
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+        sum[j] = e;
     }
-    if (threadIdx.x == 0) {
+    if (lane == 0) {
         const float npx = (float)(a.nx * a.ny);
         if (redo > 0) {  // the re-run ends exactly at the stopping iteration
             ctrl->n = n0 + redo;
@@ -968,8 +1234,10 @@ __device__ __forceinline__ bool tb_decide(const TbArgs &a, TvCtrl *ctrl, int b, 
         } else {
             int stopj = 0;
             float e_last = INFINITY, e_prev = INFINITY;
-            for (int j = 0; j < kk; j++) {
-                float e = (float)sE[j];
+#pragma unroll
+            for (int j = 0; j < K; j++) {
+                if (j >= kk) break;
+                float e = (float)sum[j];
                 e = e / npx;
                 e_prev = e_last;
                 e_last = e;
@@ -1002,17 +1270,12 @@ __device__ __forceinline__ bool tb_decide(const TbArgs &a, TvCtrl *ctrl, int b, 
             else atomicExch(&q[b].ticket, 0ull);
         }
     }
-    return true;
 }
 
 // Reads the control block of pair b at the start of a block of iterations:
 // the accepted buffer, iterations done, re-run count, and whether snapshots
-// are due (kSnapMargin).  `fresh`: read past L1 (the persistent kernel sees
-// the block change between its tiles).
-struct TbStart {
-    int cur, n0, redo, kk;
-    bool snaps;
-};
+// are due (kSnapMargin), past L1 (the persistent kernel sees the block change
+// between its tiles).
 template <int K>
 __device__ __forceinline__ TbStart tb_start(const TbArgs &a, const TvCtrl *ctrl) {
     TbStart t;
@@ -1044,116 +1307,11 @@ __device__ __forceinline__ TbStart tb_start(const TbArgs &a, const TvCtrl *ctrl)
     return t;
 }
 
-// One tile of one pair for kk <= K iterations: the region in (TMA boxes on
-// `bar` with the given phase parity, or plain loads past L1), the iterations,
-// the snapshot stores and the final store of the owned tile.  The owned
-// pixels' squared change of iteration j is summed over each warp right after
-// the iteration (the fixed shuffle tree tb_decide applies) and lane j keeps
-// the warp's sum in wsum, so no per-iteration accumulator stays live across
-// the iterations.  Returns false if the TMA wait gave up (the error flag is
-// set; the caller leaves).
-template <int TW, int TH, int K, int NT>
-__device__ __forceinline__ bool tb_tile(const TbArgs &a, int b, int tx, int ty, const TbStart &t,
-                                        uint32_t bar, uint32_t parity, float4 *tb_smem,
-                                        double &wsum) {
-    constexpr int RW = TW + 2 * K, RH = TH + 2 * K, RN = RW * RH;
-    float4 *sP = tb_smem;                                  // RN
-    float4 *sWR = sP + RN;                                 // RN
-    float2 *sU = reinterpret_cast<float2 *>(sWR + RN);     // RN
-    const int nx = a.nx, ny = a.ny;
-    const size_t off = (size_t)b * a.stride;
-    const int cur = t.cur, kk = t.kk;
-    // accepted state in, final state to the other of buffers 0/1, snapshots
-    // after iterations 1..K-1 to the snapshot set not containing the input
-    const int fin = cur == 0 ? 1 : 0;
-    const int snap = (cur >= 2 && cur < 2 + (K - 1)) ? 2 + (K - 1) : 2;
-    const float2 *__restrict__ Uin = state_buf(a.U0, a.U1, cur) + off;
-    float2 *__restrict__ Uout = state_buf(a.U0, a.U1, fin) + off;
-    const float4 *__restrict__ Pin = state_buf(a.P0, a.P1, cur) + off;
-    float4 *__restrict__ Pout = state_buf(a.P0, a.P1, fin) + off;
-    const float4 *__restrict__ Wg = a.WR + off;
-    const int ox = tx * TW - K, oy = ty * TH - K;
-    const bool interior = ox >= 1 && oy >= 1 && ox + RW <= nx - 1 && oy + RH <= ny - 1;
-
-    // the region: three TMA boxes (zero outside the level) completing on one
-    // mbarrier, or plain loads where no tensor maps describe the level
-    const uint32_t sbase = smem_u32(tb_smem);
-    if (a.use_tma && (sbase & 127u) == 0) {
-        if (threadIdx.x == 0) {
-            mbar_arrive_expect_tx(bar, (uint32_t)RN * 40u);
-            tma_load_4d(sbase, &a.tmP, 2 * ox, oy, b, cur, bar);
-            tma_load_3d(sbase + RN * 16, &a.tmW, 2 * ox, oy, b, bar);
-            tma_load_4d(sbase + RN * 32, &a.tmU, ox, oy, b, cur, bar);
-        }
-        const bool ok = mbar_wait_bounded(bar, parity);
-        if (__syncthreads_or(!ok)) {
-            // give up this tile: report, let the copies land (bounded), leave
-            // without arriving (the host treats the plan's results as lost)
-            if (threadIdx.x == 0) atomicExch(a.err, 1);
-            mbar_wait_bounded(bar, parity);
-            return false;
-        }
-    } else {
-        for (int i = threadIdx.x; i < RN; i += NT) {
-            const int x = ox + i % RW, y = oy + i / RW;
-            float4 p = make_float4(0.f, 0.f, 0.f, 0.f), w = p;
-            float2 u = make_float2(0.f, 0.f);
-            if (x >= 0 && x < nx && y >= 0 && y < ny) {
-                const size_t q = (size_t)y * nx + x;
-                p = __ldcg(Pin + q);
-                w = Wg[q];
-                u = __ldcg(Uin + q);
-            }
-            sP[i] = p;
-            sWR[i] = w;
-            sU[i] = u;
-        }
-        __syncthreads();
-    }
-
-    // the owned tile is exact after every iteration: store it
-    auto store_owned = [&](float2 *__restrict__ Ud, float4 *__restrict__ Pd) {
-        for (int i = threadIdx.x; i < TW * TH; i += NT) {
-            const int tx2 = i % TW, ty2 = i / TW;
-            const int x = ox + K + tx2, y = oy + K + ty2;
-            if (x >= nx || y >= ny) continue;
-            const int r = (ty2 + K) * RW + tx2 + K;
-            const size_t q = (size_t)y * nx + x;
-            Ud[q] = sU[r];
-            Pd[q] = sP[r];
-        }
-    };
-    wsum = 0.0;
-#pragma unroll
-    for (int j = 0; j < K; j++) {
-        if (j < kk) {  // uniform over the block
-            double e = 0.0;
-            if (interior)
-                tb_iteration<TW, TH, K, NT, true>(j + 1, sP, sWR, sU, ox, oy, nx, ny, a.l_t,
-                                                  a.theta, a.taut, e);
-            else
-                tb_iteration<TW, TH, K, NT, false>(j + 1, sP, sWR, sU, ox, oy, nx, ny, a.l_t,
-                                                   a.theta, a.taut, e);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
-            e = __shfl_sync(0xffffffffu, e, 0);
-            if ((threadIdx.x & 31) == j) wsum = e;
-            if (t.snaps && j + 1 < kk) {  // snapshot: the state a stop after iteration j+1 accepts
-                store_owned(state_buf(a.U0, a.U1, snap + j) + off, state_buf(a.P0, a.P1, snap + j) + off);
-                // the next iteration updates u and p in place: every thread must
-                // have read its share of the snapshot first
-                __syncthreads();
-            }
-        }
-    }
-    store_owned(Uout, Pout);
-    return true;
-}
-
-template <int TW, int TH, int K, int NT>
-__global__ void __launch_bounds__(NT, tb_min_blocks(NT)) k_tvl1_tb(const __grid_constant__ TbArgs a) {
-    extern __shared__ __align__(128) float4 tb_smem[];
-    __shared__ __align__(8) unsigned long long s_bar;
+template <typename T, int MINB>
+__global__ void __launch_bounds__(T::NT, MINB) k_tvl1_tb(const __grid_constant__ TbArgs a) {
+    constexpr int K = T::K;
+    extern __shared__ __align__(128) char rt_smem[];
+    typename T::Smem &sm = *reinterpret_cast<typename T::Smem *>(rt_smem);
     const int b = blockIdx.z;
     TvCtrl *ctrl = a.ctrl + b;
     // The pair's control block changes in this launch only once all of the
@@ -1175,19 +1333,67 @@ __global__ void __launch_bounds__(NT, tb_min_blocks(NT)) k_tvl1_tb(const __grid_
         for (int j = 1; j < K; j++) qk *= q;
         t.snaps = __ldca(&ctrl->last_err) * qk < kSnapMargin * a.eps2;
     }
-    const uint32_t bar = smem_u32(&s_bar);
+    __shared__ int s_b, s_tile;
+    __shared__ TbStart s_t;
     if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
+        s_b = b;
+        s_tile = blockIdx.y * gridDim.x + blockIdx.x;
+        s_t = t;
     }
-    __syncthreads();  // the barrier is initialised before anyone waits on it
-    double wsum;
-    if (!tb_tile<TW, TH, K, NT>(a, b, blockIdx.x, blockIdx.y, t, bar, 0, tb_smem, wsum)) return;
-    const int fin = t.cur == 0 ? 1 : 0;
-    const int snap = (t.cur >= 2 && t.cur < 2 + (K - 1)) ? 2 + (K - 1) : 2;
-    tb_decide<K, NT>(a, ctrl, b, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, wsum,
-                     t.kk, fin, t.snaps ? snap : -1, t.redo, t.n0, nullptr, nullptr,
-                     reinterpret_cast<double *>(tb_smem));
+    __syncthreads();
+    const int tiles_x = gridDim.x;
+    if (__syncthreads_or(rt_tile<T, false>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err[0], [] {}))) {
+        rt_tile_exact<T>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err[0]);
+        __syncthreads();
+    }
+    if (threadIdx.x < 32)
+        tb_decide<T>(a, ctrl, s_b, s_tile, gridDim.x * gridDim.y, sm.err[0], s_t, nullptr, nullptr);
+}
+
+// One warp: the next tile of any pair that has one to hand out, or -1 when
+// every pair stopped.  The pairs are looked at in order, so that the blocks
+// work on as few of them at a time as keep all blocks busy and their state
+// stays in L2 from one block of iterations to the next.
+__device__ __forceinline__ int tb_claim(const TbArgs &a, TbQueue *q, int *left, int ntiles, int B, int first,
+                                        int &tile) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long t0 = 0;
+    for (;;) {
+        for (int k = 0; k < B; k += 32) {
+            const int b = first + k + lane < B ? first + k + lane : first + k + lane - B;
+            bool open = false;
+            if (k + lane < B) {
+                const int stop = *((volatile int *)&a.ctrl[b].stop);
+                const unsigned long long tk = *((volatile unsigned long long *)&q[b].ticket);
+                open = !stop && tk < (unsigned long long)ntiles;
+            }
+            for (unsigned m = __ballot_sync(0xffffffffu, open); m; m &= m - 1) {
+                const int c = __shfl_sync(0xffffffffu, b, __ffs(m) - 1);
+                int got = -1;
+                if (lane == 0) {
+                    const unsigned long long tk = atomicAdd(&q[c].ticket, 1ull);
+                    if (tk < (unsigned long long)ntiles) got = (int)tk;
+                }
+                got = __shfl_sync(0xffffffffu, got, 0);
+                if (got >= 0) {
+                    tile = got;
+                    return c;
+                }
+            }
+        }
+        int more = 1;
+        if (lane == 0) {
+            more = *((volatile int *)left) > 0;
+            if (more && t0 == 0) {
+                t0 = globaltimer();
+            } else if (more && globaltimer() - t0 > kWaitNs) {
+                atomicExch(a.err, 1);  // no work for kWaitNs: give up
+                more = 0;
+            }
+        }
+        if (!__shfl_sync(0xffffffffu, more, 0)) return -1;
+        __nanosleep(128);
+    }
 }
 
 // Persistent form of k_tvl1_tb: one launch runs a whole warp stage of every
@@ -1201,103 +1407,68 @@ __global__ void __launch_bounds__(NT, tb_min_blocks(NT)) k_tvl1_tb(const __grid_
 // tiles, iterations, decisions and bits).  No block waits while it holds an
 // item, so items always finish; a block with nothing to take sleeps briefly,
 // and gives up with the error flag after kWaitNs without finding work.
-template <int TW, int TH, int K, int NT>
-__global__ void __launch_bounds__(NT, tb_min_blocks(NT)) k_tvl1_q(const __grid_constant__ TbArgs a, TbQueue *q,
-                                                  int *left, int tiles_x, int ntiles, int B) {
-    extern __shared__ __align__(128) float4 tb_smem[];
-    __shared__ __align__(8) unsigned long long s_bar;
-    __shared__ int s_b, s_tile;
-    // thread 0 only (in shared memory, not in every thread's registers): the
-    // pair last worked on (first pair to look at), and a tile of that pair's
-    // current block of iterations claimed ahead
-    __shared__ int s_hint, s_ahead;
+template <typename T, int MINB>
+__global__ void __launch_bounds__(T::NT, MINB) k_tvl1_q(const __grid_constant__ TbArgs a, TbQueue *q,
+                                                        int *left, int tiles_x, int ntiles, int B) {
+    constexpr int K = T::K;
+    extern __shared__ __align__(128) char rt_smem[];
+    typename T::Smem &sm = *reinterpret_cast<typename T::Smem *>(rt_smem);
+    // The item worked on, in shared memory rather than in every thread's
+    // registers: s_b, s_tile and s_t; s_ahead: a further tile of the pair's
+    // current block of iterations, claimed while this one's loads are in
+    // flight (that block is not decided before this tile arrives, so the start
+    // state still holds for it), or -1.
+    __shared__ int s_b, s_tile[2], s_ahead[2];
     __shared__ TbStart s_t;
-    const uint32_t bar = smem_u32(&s_bar);
+    volatile int *const v_b = &s_b, *const v_tile = s_tile, *const v_ahead = s_ahead;
     if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-        s_hint = blockIdx.x % B;
-        s_ahead = -1;
+        *v_b = blockIdx.x % B;
+        v_tile[1] = v_ahead[1] = -1;
     }
-    uint32_t parity = 0;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            int hint = s_hint, ahead = s_ahead;
-            int got_b = -1, got_t = 0;
-            if (ahead >= 0) {
-                // claimed while this block held a tile of the same block of
-                // iterations, which therefore had not been decided: the start
-                // state in s_t still holds
-                got_b = hint;
-                got_t = ahead;
-                ahead = -1;
-            } else {
-                unsigned long long t0 = 0;
-                for (;;) {
-                    for (int k = 0; k < B && got_b < 0; k++) {
-                        const int bb = hint + k < B ? hint + k : hint + k - B;
-                        if (*((volatile int *)&a.ctrl[bb].stop)) continue;
-                        if (*((volatile unsigned long long *)&q[bb].ticket) >=
-                            (unsigned long long)ntiles)
-                            continue;
-                        const unsigned long long tk = atomicAdd(&q[bb].ticket, 1ull);
-                        if (tk < (unsigned long long)ntiles) {
-                            got_b = bb;
-                            got_t = (int)tk;
-                        }
+    __syncthreads();
+    for (int it = 0;; it ^= 1) {
+        if (threadIdx.x < 32) {
+            // The last tile's stores reach other SMs before the pair's
+            // decision opens its next block of iterations: the block barrier
+            // behind them, then one thread's device-scope fence before it
+            // arrives (the pattern of a grid-wide barrier).
+            const int prev = v_tile[it ^ 1];
+            if (prev >= 0) tb_decide<T>(a, a.ctrl + *v_b, *v_b, prev, ntiles, sm.err[it ^ 1], s_t, q, left);
+        }
+        if (v_ahead[it ^ 1] < 0) {
+            if (threadIdx.x < 32) {
+                int got_t;
+                const int got_b = tb_claim(a, q, left, ntiles, B, *v_b, got_t);
+                if (threadIdx.x == 0) {
+                    if (got_b >= 0) {
+                        __threadfence();  // the pair's decision and state before its tiles are read
+                        s_t = tb_start<K>(a, a.ctrl + got_b);
                     }
-                    if (got_b >= 0 || *((volatile int *)left) <= 0) break;
-                    if (t0 == 0) {
-                        t0 = globaltimer();
-                    } else if (globaltimer() - t0 > kWaitNs) {
-                        atomicExch(a.err, 1);  // no work for kWaitNs: give up
-                        break;
-                    }
-                    __nanosleep(256);
-                }
-                if (got_b >= 0) {
-                    __threadfence();  // the pair's decision and state before its tiles are read
-                    s_t = tb_start<K>(a, a.ctrl + got_b);
-                    hint = got_b;
+                    *v_b = got_b;
+                    v_tile[it] = got_t;
                 }
             }
-            if (got_b >= 0) {
-                // generic-proxy writes of other blocks, then this block's TMA reads
-                asm volatile("fence.proxy.async.global;\n" ::: "memory");
-                fence_async_smem();  // this block's reads of the last region, then TMA writes
-                // Claim the pair's next tile now; the answer is needed only
-                // after this tile, so the atomic's latency is hidden.  Not
-                // near the end of a block of iterations, where a tile claimed
-                // by a busy block would wait for it while others are idle.
-                if (got_t + 32 < ntiles) {
-                    const unsigned long long tk = atomicAdd(&q[got_b].ticket, 1ull);
-                    ahead = tk < (unsigned long long)ntiles ? (int)tk : -1;
-                }
-            }
-            s_b = got_b;
-            s_tile = got_t;
-            s_hint = hint;
-            s_ahead = ahead;
+        } else if (threadIdx.x == 0) {
+            v_tile[it] = v_ahead[it ^ 1];
         }
         __syncthreads();
-        const int b = s_b;
-        if (b < 0) return;
-        const TbStart t = s_t;
-        const int tile = s_tile;
-        double wsum;
-        if (!tb_tile<TW, TH, K, NT>(a, b, tile % tiles_x, tile / tiles_x, t, bar, parity, tb_smem,
-                                    wsum))
-            return;
-        parity ^= 1u;
-        // The tile's stores reach other SMs before the pair's decision opens
-        // its next block of iterations: the block barrier in tb_decide, then
-        // thread 0's device-scope fence before it arrives (the pattern of a
-        // grid-wide barrier).
-        const int fin = t.cur == 0 ? 1 : 0;
-        const int snap = (t.cur >= 2 && t.cur < 2 + (K - 1)) ? 2 + (K - 1) : 2;
-        tb_decide<K, NT>(a, a.ctrl + b, b, tile, ntiles, wsum, t.kk, fin, t.snaps ? snap : -1,
-                         t.redo, t.n0, q, left, reinterpret_cast<double *>(tb_smem));
-        __syncthreads();  // shared state of this item is dead before the next claim
+        if (*v_b < 0) return;
+        const bool broken = rt_tile<T, false>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err[it], [&] {
+            if (threadIdx.x == 0) {
+                // not near the end of a block of iterations, where a tile
+                // claimed by a busy block would wait for it while others idle
+                int ahead = -1;
+                if (v_tile[it] + 32 < ntiles) {
+                    const unsigned long long tk = atomicAdd(&q[*v_b].ticket, 1ull);
+                    if (tk < (unsigned long long)ntiles) ahead = (int)tk;
+                }
+                v_ahead[it] = ahead;
+            }
+        });
+        if (__syncthreads_or(broken)) {
+            rt_tile_exact<T>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err[it]);
+            __syncthreads();
+        }
     }
 }
 
@@ -1323,13 +1494,12 @@ __global__ void __launch_bounds__(kLvNT) k_tvl1_level(TbArgs a) {
     const int fin = cur == 0 ? 1 : 0;
     const size_t off = (size_t)b * a.stride;
     const float2 *__restrict__ Uin = state_buf(a.U0, a.U1, cur) + off;
-    const float4 *__restrict__ Pin = state_buf(a.P0, a.P1, cur) + off;
+    const Quads<float2> Pin = p_buf(a.P, a.plane, cur, off), Pout = p_buf(a.P, a.plane, fin, off);
     float2 *__restrict__ Uout = state_buf(a.U0, a.U1, fin) + off;
-    float4 *__restrict__ Pout = state_buf(a.P0, a.P1, fin) + off;
-    const float4 *__restrict__ Wg = a.WR + off;
+    const Quads<const float2> Wq = w_quads(a.W, a.plane, off);
     for (int i = tid; i < N; i += kLvNT) {
         sU[i] = Uin[i];
-        sP[i] = Pin[i];
+        sP[i] = Pin.get(i);
     }
     __syncthreads();
     int n = ctrl->n;
@@ -1343,7 +1513,7 @@ __global__ void __launch_bounds__(kLvNT) k_tvl1_level(TbArgs a) {
             const float4 pc = sP[i];
             const float4 pl = x > 0 ? sP[i - 1] : pc;   // unused on the left border
             const float4 pu = y > 0 ? sP[i - nx] : pc;  // unused on the top border
-            const float2 un = th_u_update(u, __ldg(Wg + i), pc, pl, pu, x == 0,
+            const float2 un = th_u_update(u, Wq.get_ro(i), pc, pl, pu, x == 0,
                                           x == nx - 1, y == 0, y == ny - 1, a.l_t, a.theta);
             sU[i] = un;
             const float e1 = un.x - u.x, e2 = un.y - u.y;
@@ -1380,7 +1550,7 @@ __global__ void __launch_bounds__(kLvNT) k_tvl1_level(TbArgs a) {
     }
     for (int i = tid; i < N; i += kLvNT) {
         Uout[i] = sU[i];
-        Pout[i] = sP[i];
+        Pout.set(i, sP[i]);
     }
     if (tid == 0) {
         ctrl->n = n;
@@ -1433,13 +1603,13 @@ __global__ void __cluster_dims__(kClC, 1, 1) __launch_bounds__(NT) k_tvl1_cluste
     const int fin = cur == 0 ? 1 : 0;
     const size_t off = (size_t)b * a.stride;
     const float2 *__restrict__ Uin = state_buf(a.U0, a.U1, cur) + off + (size_t)r0 * nx;
-    const float4 *__restrict__ Pin = state_buf(a.P0, a.P1, cur) + off + (size_t)r0 * nx;
-    const float4 *__restrict__ Wg = a.WR + off + (size_t)r0 * nx;
+    const Quads<float2> Pin = p_buf(a.P, a.plane, cur, off + (size_t)r0 * nx);
+    const Quads<const float2> Wq = w_quads(a.W, a.plane, off + (size_t)r0 * nx);
     const int N = nb * nx;
     for (int i = tid; i < N; i += NT) {
         sU[i] = Uin[i];
-        sP[i] = Pin[i];
-        sW[i] = Wg[i];
+        sP[i] = Pin.get(i);
+        sW[i] = Wq.get(i);
     }
     // the neighbours' rows: p of the band above (its last row), u of the band below (its first)
     const int nb_up = c > 0 ? r0 - (c - 1) * ny / kClC : 0;
@@ -1494,10 +1664,10 @@ __global__ void __cluster_dims__(kClC, 1, 1) __launch_bounds__(NT) k_tvl1_cluste
         done = stop;
     }
     float2 *__restrict__ Uout = state_buf(a.U0, a.U1, fin) + off + (size_t)r0 * nx;
-    float4 *__restrict__ Pout = state_buf(a.P0, a.P1, fin) + off + (size_t)r0 * nx;
+    const Quads<float2> Pout = p_buf(a.P, a.plane, fin, off + (size_t)r0 * nx);
     for (int i = tid; i < N; i += NT) {
         Uout[i] = sU[i];
-        Pout[i] = sP[i];
+        Pout.set(i, sP[i]);
     }
     if (c == 0 && tid == 0) {
         ctrl->n = n;
@@ -1512,7 +1682,7 @@ __global__ void __cluster_dims__(kClC, 1, 1) __launch_bounds__(NT) k_tvl1_cluste
 // sum |rho(u)| with rho linearised at the current warp.  Last block of a pair
 // writes ctrl.energy and, if slot >= 0, energy_out[b * slots + slot].
 constexpr int kEnNT = 256;
-__global__ void __launch_bounds__(kEnNT) k_energy(const float4 *WR, const float2 *U0,
+__global__ void __launch_bounds__(kEnNT) k_energy(const float2 *W, size_t plane, const float2 *U0,
                                                   const float2 *U1, size_t stride, int nx,
                                                   int ny, float lambda, TvCtrl *ctrl,
                                                   double *partials, int max_blocks,
@@ -1530,7 +1700,7 @@ __global__ void __launch_bounds__(kEnNT) k_energy(const float4 *WR, const float2
         if (x < nx - 1) { const float2 r = U[i + 1]; f1x = (double)(r.x - uc.x); f2x = (double)(r.y - uc.y); }
         if (y < ny - 1) { const float2 d = U[i + nx]; f1y = (double)(d.x - uc.x); f2y = (double)(d.y - uc.y); }
         tv += sqrt(f1x * f1x + f1y * f1y) + sqrt(f2x * f2x + f2y * f2y);
-        const float4 w = WR[off + i];
+        const float4 w = w_quads(W, plane, off).get(i);
         const float rho = w.z + (w.x * uc.x + w.y * uc.y);
         data += fabs((double)rho);
     }
@@ -1685,39 +1855,19 @@ bool encode_map8(CUtensorMap *m, void *base, int rank, const cuuint64_t *dims,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor maps of k_tvl1_tb's region loads for tile configuration cfg on a
-// level of nx x ny (planes of N0 elements, B pairs, kStateBufs buffers of u
-// and p).  TMA wants 16-byte row and plane strides, so u (8 bytes a pixel)
-// needs even nx and N0; otherwise the kernel loads the region itself.
-static void tb_maps(TbArgs &ta, int cfg, int nx, int ny, int B, size_t N0, float4 *P0, float2 *U0,
-                    const float4 *WR, int *err) {
-    ta.use_tma = 0;
-    ta.err = err;
-    if (cfg >= kTbNumCfgs || (nx & 1) || (N0 & 1)) return;
-    const cuuint32_t rw = (cuuint32_t)(kTbCfgs[cfg].tw + 2 * kTbK), rh = (cuuint32_t)(kTbCfgs[cfg].th + 2 * kTbK);
-    const cuuint64_t X = (cuuint64_t)nx, Y = (cuuint64_t)ny, NB = (cuuint64_t)B, N = N0;
-    const cuuint64_t dp[4] = {2 * X, Y, NB, (cuuint64_t)kStateBufs}, sp[3] = {16 * X, 16 * N, 16 * N * NB};
-    const cuuint32_t bp[4] = {2 * rw, rh, 1, 1};
-    const cuuint64_t du[4] = {X, Y, NB, (cuuint64_t)kStateBufs}, su[3] = {8 * X, 8 * N, 8 * N * NB};
-    const cuuint32_t bu[4] = {rw, rh, 1, 1};
-    const cuuint64_t dw[3] = {2 * X, Y, NB}, sw[2] = {16 * X, 16 * N};
-    const cuuint32_t bw[3] = {2 * rw, rh, 1};
-    ta.use_tma = encode_map8(&ta.tmP, P0, 4, dp, sp, bp) && encode_map8(&ta.tmU, U0, 4, du, su, bu) &&
-                 encode_map8(&ta.tmW, const_cast<float4 *>(WR), 3, dw, sw, bw);
-}
-
 // A plan needs no repair after a timeout: every warp stage starts with
 // k_warp re-arming each pair's control block and work queue, so the next
 // call runs from a clean state (tested with OFLOW_INJECT_TIMEOUT).
 void TvPlan::check_device_error() {
     if (err_.take())
         throw Error(OFLOW_ERR_TIMEOUT,
-                    "tvl1: a bounded device wait gave up (a tile's TMA load or the work queue)");
+                    "tvl1: a bounded device wait gave up (the work queue)");
 }
 
-template <int TW, int TH, int NT>
-static void tb_launch(dim3 g, cudaStream_t st, const TbArgs &ta) {
-    k_tvl1_tb<TW, TH, kTbK, NT><<<g, NT, tb_smem_bytes(TW, TH), st>>>(ta);
+template <int C> using TbTile = RtTile<kTbCfgs[C].v, kTbCfgs[C].nw>;
+
+template <int C> static void tb_launch(dim3 g, cudaStream_t st, const TbArgs &ta) {
+    k_tvl1_tb<TbTile<C>, kTbCfgs[C].mb><<<g, TbTile<C>::NT, sizeof(typename TbTile<C>::Smem), st>>>(ta);
 }
 
 static void tb_launch_cfg(int cfg, dim3 g, cudaStream_t st, const TbArgs &ta) {
@@ -1739,34 +1889,34 @@ static void tb_launch_cfg(int cfg, dim3 g, cudaStream_t st, const TbArgs &ta) {
         return;
     }
     switch (cfg) {
-        case 0: tb_launch<64, 32, 512>(g, st, ta); break;
-        case 1: tb_launch<64, 16, 256>(g, st, ta); break;
-        case 2: tb_launch<32, 16, 256>(g, st, ta); break;
-        default: tb_launch<16, 8, 128>(g, st, ta); break;
+        case 0: tb_launch<0>(g, st, ta); break;
+        case 1: tb_launch<1>(g, st, ta); break;
+        case 2: tb_launch<2>(g, st, ta); break;
+        default: tb_launch<3>(g, st, ta); break;
     }
 }
 
 // Resident blocks of the persistent kernel per SM, for each tile shape.
-template <int TW, int TH, int NT>
-static int tb_queue_occupancy() {
+template <int C> static int tb_queue_occupancy() {
     static int occ = -1;
     if (occ < 0) {
         int n = 0;
-        OF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tvl1_q<TW, TH, kTbK, NT>, NT,
-                                                              tb_smem_bytes(TW, TH)));
+        OF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tvl1_q<TbTile<C>, kTbCfgs[C].mb>,
+                                                              TbTile<C>::NT,
+                                                              sizeof(typename TbTile<C>::Smem)));
         occ = imax(n, 1);
     }
     return occ;
 }
 
-template <int TW, int TH, int NT>
+template <int C>
 static void tb_launch_q(dim3 g, cudaStream_t st, const TbArgs &ta, TbQueue *q, int *left,
                         int share) {
     const int ntiles = (int)(g.x * g.y);
-    const int slots = imax(1, tb_queue_occupancy<TW, TH, NT>() * kNumSMs / imax(share, 1));
+    const int slots = imax(1, tb_queue_occupancy<C>() * kNumSMs / imax(share, 1));
     const int blocks = imin(ntiles * (int)g.z, slots);
-    k_tvl1_q<TW, TH, kTbK, NT><<<blocks, NT, tb_smem_bytes(TW, TH), st>>>(ta, q, left, (int)g.x,
-                                                                         ntiles, (int)g.z);
+    k_tvl1_q<TbTile<C>, kTbCfgs[C].mb><<<blocks, TbTile<C>::NT, sizeof(typename TbTile<C>::Smem), st>>>(
+        ta, q, left, (int)g.x, ntiles, (int)g.z);
 }
 
 // A whole tiled warp stage as one persistent launch (k_tvl1_q).
@@ -1777,22 +1927,26 @@ static void tb_launch_queue(int cfg, dim3 g, cudaStream_t st, const TbArgs &ta_i
     TbArgs ta = ta_in;
     ta.predict = predict;
     switch (cfg) {
-        case 0: tb_launch_q<64, 32, 512>(g, st, ta, q, left, share); break;
-        case 1: tb_launch_q<64, 16, 256>(g, st, ta, q, left, share); break;
-        case 2: tb_launch_q<32, 16, 256>(g, st, ta, q, left, share); break;
-        default: tb_launch_q<16, 8, 128>(g, st, ta, q, left, share); break;
+        case 0: tb_launch_q<0>(g, st, ta, q, left, share); break;
+        case 1: tb_launch_q<1>(g, st, ta, q, left, share); break;
+        case 2: tb_launch_q<2>(g, st, ta, q, left, share); break;
+        default: tb_launch_q<3>(g, st, ta, q, left, share); break;
     }
 }
 
+template <int C> static void tb_set_smem_attr() {
+    const int n = (int)sizeof(typename TbTile<C>::Smem);
+    OF_CUDA(cudaFuncSetAttribute(k_tvl1_q<TbTile<C>, kTbCfgs[C].mb>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, n));
+    OF_CUDA(cudaFuncSetAttribute(k_tvl1_tb<TbTile<C>, kTbCfgs[C].mb>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, n));
+}
+
 static void tb_set_smem_attrs() {
-    OF_CUDA(cudaFuncSetAttribute(k_tvl1_q<64, 32, kTbK, 512>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tb_smem_bytes(64, 32)));
-    OF_CUDA(cudaFuncSetAttribute(k_tvl1_q<64, 16, kTbK, 256>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tb_smem_bytes(64, 16)));
-    OF_CUDA(cudaFuncSetAttribute(k_tvl1_tb<64, 32, kTbK, 512>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tb_smem_bytes(64, 32)));
-    OF_CUDA(cudaFuncSetAttribute(k_tvl1_tb<64, 16, kTbK, 256>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tb_smem_bytes(64, 16)));
+    tb_set_smem_attr<0>();
+    tb_set_smem_attr<1>();
+    tb_set_smem_attr<2>();
+    tb_set_smem_attr<3>();
     OF_CUDA(cudaFuncSetAttribute(k_tvl1_level, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kLvMaxPx * (int)(sizeof(float4) + sizeof(float2))));
     OF_CUDA(cudaFuncSetAttribute(k_tvl1_cluster<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1813,9 +1967,14 @@ static dim3 tb_grid(int cfg, int nx, int ny, int B) {
     return dim3(div_up(nx, tw), div_up(ny, th), B);
 }
 
-// Largest tile whose grid still gives every SM two blocks; small scales get
-// small tiles (more blocks, shorter per-launch latency).  OFLOW_TB_CFG forces
+// The tile with the least estimated time of a block of K iterations: what one
+// tile takes on an SM of its own, plus what each further tile of the busiest SM
+// adds.  Microseconds measured on single pairs of 160x117 to 1280x720 (first
+// column: 24 / 21 / 17.5 / 16) and on 32 pairs of 1024x436 (second); a large
+// tile wastes less on its halo, small ones use more SMs.  OFLOW_TB_CFG forces
 // one configuration (used to time them against each other).
+constexpr float kTbAlone[kTbNumCfgs] = {24.0f, 21.0f, 17.5f, 16.0f};
+constexpr float kTbMore[kTbNumCfgs] = {12.0f, 7.6f, 6.8f, 4.5f};
 static int tb_pick(int nx, int ny, int B) {
     if (const char *e = getenv("OFLOW_TB_CFG")) {
         const int c = atoi(e);
@@ -1824,9 +1983,17 @@ static int tb_pick(int nx, int ny, int B) {
         if (c == kClusterCfg && cluster_fits(nx, ny)) return c;
     }
     if (level_fits(nx, ny)) return kLevelCfg;
-    for (int c = 0; c < kTbNumCfgs; c++)
-        if (tb_tiles(c, nx, ny) * B >= 2 * kNumSMs) return c;
-    return kTbNumCfgs - 1;
+    int best = 0;
+    float best_t = 1e30f;
+    for (int c = 0; c < kTbNumCfgs; c++) {
+        const long long per_sm = ((long long)tb_tiles(c, nx, ny) * B + kNumSMs - 1) / kNumSMs;
+        const float t = kTbAlone[c] + (float)(per_sm - 1) * kTbMore[c];
+        if (t < best_t) {
+            best_t = t;
+            best = c;
+        }
+    }
+    return best;
 }
 
 // a configuration from a tuning table, if it is valid for this level
@@ -1959,7 +2126,6 @@ void *TvPlan::raw_input(int b, int k) const {
     return ar_.at<char>(o_raw_) + (size_t)(2 * b + k) * N0_ * esz;
 }
 float2 *TvPlan::ubuf(int k) const { return ar_.at<float2>(o_U0_) + (size_t)k * B_ * N0_; }
-float4 *TvPlan::pbuf(int k) const { return ar_.at<float4>(o_P0_) + (size_t)k * B_ * N0_; }
 
 const float *TvPlan::out_u(int b) const { return ar_.at<float>(o_out_) + (size_t)b * N0_; }
 const float *TvPlan::out_v(int b) const { return ar_.at<float>(o_out_) + (size_t)(B_ + b) * N0_; }
@@ -1982,9 +2148,9 @@ void TvPlan::record(cudaStream_t st) {
         wc.dv01 = reinterpret_cast<float4 *>(wc.cc2 + n);
         wc.dv2 = reinterpret_cast<float2 *>(wc.dv01 + n);
     }
-    float4 *WR = ar_.at<float4>(o_WR_);
+    float2 *W = ar_.at<float2>(o_WR_), *P = ar_.at<float2>(o_P0_);
+    const size_t plane = (size_t)B * N0;
     float2 *U0 = ubuf(0), *U1 = ubuf(1), *Uz = ar_.at<float2>(o_Uz_);
-    float4 *P0 = pbuf(0), *P1 = pbuf(1);
     TvCtrl *ctrl = ar_.at<TvCtrl>(o_ctrl_);
     double *part = ar_.at<double>(o_part_);
     NormRec *recs = ar_.at<NormRec>(o_recs_);
@@ -2064,7 +2230,7 @@ void TvPlan::record(cudaStream_t st) {
         }
         k_cubic_pack<<<gr, blk, 0, st>>>(pyr + pyr_off_[s], lp, nx, ny, wc, N0);
         launches_ += 1;
-        IterArgs ia{WR, U0, U1, P0, P1, N0, nx, ny, l_t, prm_.theta, taut, eps2, ctrl, part,
+        IterArgs ia{W, U0, U1, P, plane, N0, nx, ny, l_t, prm_.theta, taut, eps2, ctrl, part,
                     max_blocks_, iters, iter_stride_, 0};
         dim3 ig(div_up(nx, kIterTW), div_up(ny, kIterTH), B);
         const int cfg = tb_cfg_[s];
@@ -2073,16 +2239,17 @@ void TvPlan::record(cudaStream_t st) {
             const int mode = wi > 0 ? kWarpFromU
                                     : (s == s0_ ? (warm_ ? kWarpFromUz : kWarpZero) : kWarpFromUz);
             mark_begin(-1);
-            k_warp<<<wg, wb, 0, st>>>(pyr + pyr_off_[s], lp, wc, WR, U0, U1, Uz, P0, P1,
-                                       N0, nx, ny, mode, wi == 0, ctrl, queue, left);
+            k_warp<<<wg, wb, 0, st>>>(pyr + pyr_off_[s], lp, wc, W, U0, U1, Uz, P, plane, N0,
+                                       nx, ny, mode, wi == 0, ctrl, queue, left);
             mark_end();
             launches_ += 1;
             ia.stage = s * prm_.warps + wi;
             if (!trace_) {
-                TbArgs ta{WR, U0, U1, P0, P1, N0, nx, ny, si_[s], l_t,
+                TbArgs ta{W, U0, U1, P, plane, N0, nx, ny, si_[s], l_t,
                           prm_.theta, taut, eps2, ctrl, part, max_blocks_ / kTbK, iters,
                           iter_stride_, ia.stage};
-                tb_maps(ta, cfg, nx, ny, B, N0, P0, U0, WR, err_.device());
+                ta.vec = (nx & 1) == 0 && (N0 & 1) == 0;
+                ta.err = err_.device();
                 const dim3 tg = tb_grid(cfg, nx, ny, B);
                 mark_begin(s);
                 if (cfg == kLevelCfg || cfg == kClusterCfg || queue_) {
@@ -2111,7 +2278,7 @@ void TvPlan::record(cudaStream_t st) {
                 launches_ += 1;
                 const int slot = (s * prm_.warps + wi) * prm_.max_iterations + it;
                 k_energy<<<dim3(imin(energy_blocks_, div_up(nx * ny, kEnNT * 4)), B), kEnNT, 0,
-                           st>>>(WR, U0, U1, N0, nx, ny, prm_.lambda, ctrl, part, max_blocks_,
+                           st>>>(W, plane, U0, U1, N0, nx, ny, prm_.lambda, ctrl, part, max_blocks_,
                                  energy, energy_slots_, slot, it + 1);
                 launches_ += 1;
             }
@@ -2120,7 +2287,7 @@ void TvPlan::record(cudaStream_t st) {
     // final energy at the finest scale, last warp: in the schedule of a traced
     // plan; otherwise on demand (compute_energy), when statistics are read
     if (trace_) {
-        k_energy<<<dim3(energy_blocks_, B), kEnNT, 0, st>>>(WR, U0, U1, N0, w_, h_, prm_.lambda,
+        k_energy<<<dim3(energy_blocks_, B), kEnNT, 0, st>>>(W, plane, U0, U1, N0, w_, h_, prm_.lambda,
                                                             ctrl, part, max_blocks_, energy,
                                                             energy_slots_, -1, -1);
         launches_ += 1;
@@ -2212,12 +2379,13 @@ void TvPlan::autotune(cudaStream_t st, TuneTable *table, int reps) {
                 // stop); the whole-level kernel is given 2K
                 const bool whole = c == kLevelCfg || c == kClusterCfg;
                 const int iters_run = whole ? 2 * kTbK : kTbK;
-                TbArgs ta{ar_.at<float4>(o_WR_), ubuf(0), ubuf(1), pbuf(0),
-                          pbuf(1), N0,
+                TbArgs ta{ar_.at<float2>(o_WR_), ubuf(0), ubuf(1), ar_.at<float2>(o_P0_),
+                          (size_t)B_ * N0, N0,
                           nx, ny, whole ? iters_run : 1 << 30, l_t, prm_.theta, taut, -1.0f,
                           ctrl, ar_.at<double>(o_part_), max_blocks_ / kTbK, ar_.at<int>(o_iters_),
                           iter_stride_, 0};
-                tb_maps(ta, c, nx, ny, B_, N0, pbuf(0), ubuf(0), ar_.at<float4>(o_WR_), err_.device());
+                ta.vec = (nx & 1) == 0 && (N0 & 1) == 0;
+                ta.err = err_.device();
                 const dim3 tg = tb_grid(c, nx, ny, B_);
                 float ms_min = 1e30f;
                 for (int r = 0; r <= reps; r++) {  // first launch warms up
@@ -2331,7 +2499,7 @@ void TvPlan::run(cudaStream_t st) {
 void TvPlan::compute_energy(cudaStream_t st) {
     if (trace_) return;  // the traced schedule computes it
     k_energy<<<dim3(energy_blocks_, B_), kEnNT, 0, st>>>(
-        ar_.at<float4>(o_WR_), ubuf(0), ubuf(1), N0_, w_, h_, prm_.lambda, ar_.at<TvCtrl>(o_ctrl_),
+        ar_.at<float2>(o_WR_), (size_t)B_ * N0_, ubuf(0), ubuf(1), N0_, w_, h_, prm_.lambda, ar_.at<TvCtrl>(o_ctrl_),
         ar_.at<double>(o_part_), max_blocks_, ar_.at<double>(o_energy_), energy_slots_, 0, -1);
     OF_CUDA(cudaGetLastError());
 }

@@ -165,7 +165,7 @@ class TvPlan {
     const oflow_tvl1_params &params() const { return prm_; }
     size_t device_bytes() const { return ar_.size(); }
     // Throws OFLOW_ERR_TIMEOUT if a kernel of this plan gave up a bounded wait
-    // (a tile's TMA load) since the last check; reads host memory only.
+    // (the work queue) since the last check; reads host memory only.
     void check_device_error();
 
   private:
