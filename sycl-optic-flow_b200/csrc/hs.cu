@@ -6,15 +6,18 @@
 //
 // Layout per pair b (N = w*h at the finest level, levels packed):
 //   raw[b][2] staged frames, pyr_l[b][2] float pyramid (finest = nlevels-1),
-//   D[b] float4 (Ix, Iy, Iz, Ix^2+Iy^2+alpha), dU0/dU1[b] float2 ping-pong
-//   increments, Ua/Ub[b] float2 flow (alternating per level), out[2][b].
+//   D float2 planes (Ix, Iy) and (Iz, Ix^2+Iy^2+alpha) of all pairs, dU0/dU1[b]
+//   float2 ping-pong increments, Ua/Ub[b] float2 flow (alternating per level),
+//   out[2][b].
 // All ping-pong parities are known on the host, so the schedule is static and
 // captured into one CUDA graph.
 //
 // The Jacobi sweeps are temporally blocked: one launch runs up to K sweeps on
-// a TW x TH tile held in shared memory with a K-pixel halo; the halo shrinks
-// by one pixel per sweep, so after K sweeps the owned tile is exact (clamped
+// a tile held in registers with a K-pixel halo; what is exact shrinks by one
+// pixel per sweep, so after K sweeps the owned tile is exact (clamped
 // neighbours at the image border are exact at every sweep).
+#include <cudaTypedefs.h>
+
 #include <cstring>
 
 #include "common.cuh"
@@ -54,7 +57,7 @@ __device__ __forceinline__ float hs_deriv5(float m2, float m1, float p1, float p
 constexpr int kDTW = 32, kDTH = 8;
 __global__ void __launch_bounds__(kDTW *kDTH) k_hs_warp_deriv(
     const float *__restrict__ pyr, size_t lp, int w, int h, const float2 *__restrict__ U,
-    size_t ustride, int zero_flow, float alpha, float4 *D, size_t dstride) {
+    size_t ustride, int zero_flow, float alpha, float2 *D, size_t plane, size_t dstride) {
     constexpr int RW = kDTW + 4, RH = kDTH + 4;
     __shared__ float s0[RH * RW], s1[RH * RW];
     const int b = blockIdx.z;
@@ -83,139 +86,313 @@ __global__ void __launch_bounds__(kDTW *kDTH) k_hs_warp_deriv(
     t1 = hs_deriv5(s1[c - 2 * RW], s1[c - RW], s1[c + RW], s1[c + 2 * RW]);
     const float Iy = (t0 + t1) * 0.5f;
     const float den = Ix * Ix + Iy * Iy + alpha;
-    D[(size_t)b * dstride + (size_t)y * w + x] = make_float4(Ix, Iy, Iz, den);
+    const size_t q = (size_t)b * dstride + (size_t)y * w + x;
+    D[q] = make_float2(Ix, Iy);
+    D[plane + q] = make_float2(Iz, den);
 }
 
-// One Jacobi sweep (solverKernel.cuh:41-153) over cone j of the region:
-// neighbour mean of the increments (clamped at the image border), then
-// frac = (Ix*su + Iy*sv + Iz) / (Ix^2 + Iy^2 + alpha) and the update, in the
-// reference's order.  The division is Markstein's correction from the
-// precomputed reciprocal; operands outside its proven range take the IEEE
-// division.
-template <int RW, int RH, int NT, bool INTERIOR>
-__device__ __forceinline__ void hs_sweep(int j, const float2 *src, float2 *dst, const float4 *sD,
-                                         const float *sR, int x0, int y0, int w, int h) {
-    for_rect<NT>(j, RW - 1 - j, j, RH - 1 - j, [&](int rx, int ry) {
-        const int i = ry * RW + rx;
-        int l = i - 1, r = i + 1, up = i + RW, dn = i - RW;
-        if (!INTERIOR) {
-            const int x = x0 + rx, y = y0 + ry;
-            if (x < 0 || x >= w || y < 0 || y >= h) return;
-            if (x == 0) l = i;
-            if (x == w - 1) r = i;
-            if (y == h - 1) up = i;
-            if (y == 0) dn = i;
-        }
-        const float2 al = src[l], ar = src[r], au = src[up], ad = src[dn];
-        const float su = (al.x + ar.x + au.x + ad.x) * 0.25f;
-        const float sv = (al.y + ar.y + au.y + ad.y) * 0.25f;
-        const float4 d = sD[i];
-        const float p = d.x * su + d.y * sv + d.z;
-        float frac = markstein(p, d.w, sR[i]);
-        if (!(rcp_in_range(d.w) && markstein_safe(p))) frac = p / d.w;
-        dst[i] = make_float2(su - d.x * frac, sv - d.y * frac);
-    });
-}
-
-// Region loads of k_hs_jacobi by TMA: D as (2w, h, pair) and the incoming
-// increments as (w, h, pair), 8-byte elements, zero fill outside the level
-// (pixels outside are never read by a sweep).  use = 0: plain loads.
-struct HsTma {
-    int use;
-    int *err;  // set when a bounded wait gives up
-    CUtensorMap tD, tIn;
+// Jacobi tiles: the region is 64 pixels wide and V*NW high, a warp owns V rows
+// and a lane two adjacent columns of them, with the increments and D in
+// registers for all sweeps of the launch.  Left and right neighbours come by
+// shuffle, upper and lower ones from the thread's own registers, and only the
+// first and last row of a warp goes through shared memory.  A sweep is 33
+// instructions a pixel (19 of them the arithmetic, two shuffles, two the
+// division's guard) and issue-bound while it runs.  64 pairs of 320x240, 200
+// sweeps: 3.73 ms with D and the increments in shared memory (seven accesses a
+// pixel), 2.52 ms here with 48x48 tiles and 8 sweeps a launch; without the
+// fetch of the next tile's data during the sweeps 3.1 ms, with border tests in
+// every pixel of a border region 2.7 ms.
+//
+// The division by Ix^2+Iy^2+alpha is Markstein's correction from the
+// reciprocal, formed once per launch.  What that takes for granted (numerators
+// zero or above 2^-100, denominators in [2^-40, 2^24)) is kept as a running
+// minimum; a block that breaks it runs its tile again from the untouched input
+// with IEEE divisions.
+template <int V_, int NW_, int K_> struct HsTile {
+    static constexpr int V = V_, NW = NW_, K = K_, NT = 32 * NW;
+    static constexpr int RW = 64, RH = V * NW, TW = RW - 2 * K, TH = RH - 2 * K;
 };
 
-// K Jacobi sweeps (solverKernel.cuh:41-153) on a tile with a KH-pixel halo.
-// sweeps <= KH.  first: increments start at 0 (flow.cu:168-171).  last: add
-// the increment to the flow (AddKernel, addKernel.cuh:28-36) instead of
-// storing it.
-template <int TW, int TH, int KH, int NT>
-__global__ void __launch_bounds__(NT) k_hs_jacobi(const float4 *__restrict__ D, size_t dstride,
-                                                  const float2 *__restrict__ dUin,
-                                                  float2 *dUout, float2 *U, size_t stride,
-                                                  int w, int h, int sweeps, int first, int last,
-                                                  const __grid_constant__ HsTma tma) {
-    constexpr int RW = TW + 2 * KH, RH = TH + 2 * KH, RN = RW * RH;
-    extern __shared__ __align__(128) float4 smem[];
-    float4 *sD = smem;                                   // RN
-    float2 *sA = reinterpret_cast<float2 *>(sD + RN);    // RN
-    float2 *sB = sA + RN;                                // RN
-    float *sR = reinterpret_cast<float *>(sB + RN);      // RN
-    const int b = blockIdx.z;
-    const float4 *Db = D + (size_t)b * dstride;
-    const float2 *In = dUin + (size_t)b * stride;
-    const int x0 = blockIdx.x * TW - KH, y0 = blockIdx.y * TH - KH;
-    const uint32_t sbase = smem_u32(smem);
-    if (tma.use && (sbase & 127u) == 0) {
-        __shared__ __align__(8) unsigned long long s_bar;
-        const uint32_t bar = smem_u32(&s_bar);
-        if (threadIdx.x == 0) {
-            mbar_init(bar, 1);
-            fence_mbar_init();
-            mbar_arrive_expect_tx(bar, (uint32_t)RN * (first ? 16u : 24u));
-            tma_load_3d(sbase, &tma.tD, 2 * x0, y0, b, bar);
-            if (!first) tma_load_3d(sbase + RN * 16, &tma.tIn, x0, y0, b, bar);
-        }
-        if (first)
-            for (int i = threadIdx.x; i < RN; i += NT) sA[i] = make_float2(0.f, 0.f);
-        __syncthreads();  // the barrier is initialised before anyone waits on it
-        const bool ok = mbar_wait_bounded(bar, 0);
-        if (__syncthreads_or(!ok)) {
-            // report, let the copies land (bounded), leave; the host drops
-            // the plan's results
-            if (threadIdx.x == 0) atomicExch(tma.err, 1);
-            mbar_wait_bounded(bar, 0);
-            return;
-        }
-    } else {
-        for (int i = threadIdx.x; i < RN; i += NT) {
-            const int x = x0 + i % RW, y = y0 + i / RW;
-            float4 d = make_float4(0.f, 0.f, 0.f, 1.f);
-            float2 a = make_float2(0.f, 0.f);
-            if (x >= 0 && x < w && y >= 0 && y < h) {
-                const size_t p = (size_t)y * w + x;
-                d = Db[p];
-                if (!first) a = In[p];
-            }
-            sD[i] = d;
-            sA[i] = a;
-        }
-    }
-    __syncthreads();
-    // RN(1 / (Ix^2 + Iy^2 + alpha)) per region pixel, constant over the sweeps:
-    // the quotient below is then Markstein's exact form (exact_math.cuh)
-    for (int i = threadIdx.x; i < RN; i += NT) sR[i] = rcp_near_rn(sD[i].w);
-    __syncthreads();
-    // Sweep j (1-based) updates [j, RW-1-j] x [j, RH-1-j]: exactly the cells
-    // whose values can still reach the owned tile, so no read leaves the
-    // region.  A region inside the image with a one-pixel margin takes the
-    // path without image-border tests.
-    const bool interior = x0 >= 0 && y0 >= 0 && x0 + RW <= w && y0 + RH <= h;
-    float2 *src = sA, *dst = sB;
+template <int V> struct HsState {
+    float2 a[V][2];           // increments
+    float ix[V][2], iy[V][2], iz[V][2], den[V][2], rcp[V][2];
+};
+
+struct HsJacobiArgs {
+    const float2 *D;
+    size_t plane, dstride;    // elements between D's planes, between pairs
+    const float2 *in;         // increments before (ignored when first), after
+    float2 *out, *U;          // U: the flow, updated by the last launch
+    size_t stride;
+    int w, h, sweeps, first, last;
+    int vec;                  // two neighbouring pixels are 16-byte aligned
+    int tiles_x, tiles_y, tiles;  // tiles: of all pairs
+    int tma;                  // the maps below describe the level
+    int *err;                 // set when a bounded wait gives up
+    CUtensorMap m0, m1, mi;   // D's planes, the increments: (w, h, pair), 8-byte elements
+};
+
+// Where a region meets the image border (all but odd and the lanes' x are
+// uniform over the warp).  The first image row is the first of a warp (the halo
+// is whole warps), so it only replaces the row from the warp above.
+struct HsEdge {
+    bool left, right, odd;  // this lane's column 0 is the first, column 1 the last; column 0 is the last (odd widths)
+    int bottom;             // the warp's row that is the last of the image (else out of its rows)
+};
+
+// One sweep (solverKernel.cuh:41-153): neighbour mean of the increments
+// (clamped at the image border), frac = (Ix*su + Iy*sv + Iz) / den and the
+// update, in the reference's order.  above / below: the neighbouring warps'
+// rows.
+// EDGE: 0 the region lies inside the image; 1 it meets its top, left or (at an
+// even width) right border; 2 any border.
+template <typename T, int EDGE, bool EXACT>
+__device__ __forceinline__ void hs_sweep(HsState<T::V> &s, float4 above, float4 below, const HsEdge &e,
+                                         unsigned &key) {
+    constexpr int V = T::V;
+    float2 dn[2] = {make_float2(above.x, above.y), make_float2(above.z, above.w)};  // y - 1, before the sweep
 #pragma unroll
-    for (int j = 1; j <= KH; j++) {
-        if (j > sweeps) break;
-        if (interior)
-            hs_sweep<RW, RH, NT, true>(j, src, dst, sD, sR, x0, y0, w, h);
-        else
-            hs_sweep<RW, RH, NT, false>(j, src, dst, sD, sR, x0, y0, w, h);
-        __syncthreads();
-        float2 *t = src;
-        src = dst;
-        dst = t;
+    for (int v = 0; v < V; v++) {
+        const float2 c0 = s.a[v][0], c1 = s.a[v][1];
+        float2 l, r, m = c1;  // left of column 0, right of column 1, right of column 0
+        l.x = __shfl_up_sync(0xffffffffu, c1.x, 1);
+        l.y = __shfl_up_sync(0xffffffffu, c1.y, 1);
+        r.x = __shfl_down_sync(0xffffffffu, c0.x, 1);
+        r.y = __shfl_down_sync(0xffffffffu, c0.y, 1);
+        float2 up0 = v + 1 < V ? s.a[v + 1 < V ? v + 1 : v][0] : make_float2(below.x, below.y);
+        float2 up1 = v + 1 < V ? s.a[v + 1 < V ? v + 1 : v][1] : make_float2(below.z, below.w);
+        if (EDGE) {
+            if (e.left) l = c0;
+            if (e.right) r = c1;
+        }
+        if (EDGE == 2) {
+            if (e.odd) m = c0;
+            if (e.bottom == v) {
+                up0 = c0;
+                up1 = c1;
+            }
+        }
+        float p[2];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const float2 al = c ? c0 : l, ar = c ? r : m, au = c ? up1 : up0, ad = dn[c];
+            const float su = (al.x + ar.x + au.x + ad.x) * 0.25f;
+            const float sv = (al.y + ar.y + au.y + ad.y) * 0.25f;
+            p[c] = s.ix[v][c] * su + s.iy[v][c] * sv + s.iz[v][c];
+            const float frac = EXACT ? p[c] / s.den[v][c] : markstein(p[c], s.den[v][c], s.rcp[v][c]);
+            s.a[v][c] = make_float2(su - s.ix[v][c] * frac, sv - s.iy[v][c] * frac);
+        }
+        if (!EXACT) key = umin(umin(key, markstein_key(p[0])), markstein_key(p[1]));
+        dn[0] = c0;
+        dn[1] = c1;
     }
-    for (int i = threadIdx.x; i < TW * TH; i += NT) {
-        const int tx = i % TW, ty = i / TW;
-        const int x = x0 + KH + tx, y = y0 + KH + ty;
-        if (x >= w || y >= h) continue;
-        const float2 a = src[(ty + KH) * RW + tx + KH];
-        const size_t p = (size_t)b * stride + (size_t)y * w + x;
-        if (last) {
-            const float2 u = U[p];
-            U[p] = make_float2(u.x + a.x, u.y + a.y);
+}
+
+// Sweep j of a tile: the warps' first and last rows exchanged through
+// alternating buffers (one barrier a sweep), then the sweep.
+template <typename T, int EDGE, bool EXACT, typename F>
+__device__ __forceinline__ void hs_step(HsState<T::V> &s, int j, float4 (*sRow)[2][T::NW][32], bool top,
+                                        const HsEdge &e, unsigned &key, F &&taken) {
+    constexpr int V = T::V, NW = T::NW;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float4(*row)[NW][32] = sRow[j & 1];
+    const float4 first = make_float4(s.a[0][0].x, s.a[0][0].y, s.a[0][1].x, s.a[0][1].y);
+    row[0][wid][lane] = first;
+    row[1][wid][lane] = make_float4(s.a[V - 1][0].x, s.a[V - 1][0].y, s.a[V - 1][1].x, s.a[V - 1][1].y);
+    __syncthreads();
+    if (j == 0) taken();
+    float4 above = row[1][wid > 0 ? wid - 1 : 0][lane];
+    const float4 below = row[0][wid + 1 < NW ? wid + 1 : wid][lane];
+    if (EDGE && top) above = first;
+    hs_sweep<T, EDGE, EXACT>(s, above, below, e, key);
+}
+
+// Two neighbouring float2 at q; in0, in1: inside the level.
+__device__ __forceinline__ float4 hs_ld_two(const float2 *p, size_t q, int vec, bool in0, bool in1) {
+    if (vec) return in0 ? *reinterpret_cast<const float4 *>(p + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 z = make_float2(0.f, 0.f);
+    const float2 a = in0 ? p[q] : z, b = in1 ? p[q + 1] : z;
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Pair, region origin and the thread's first pixel of a tile.
+struct HsAt {
+    int b, ox, oy, x, y0;
+};
+template <typename T> __device__ __forceinline__ HsAt hs_at(const HsJacobiArgs &a, int tile) {
+    HsAt t;
+    const int row = tile / a.tiles_x;
+    t.b = row / a.tiles_y;
+    t.ox = (tile - row * a.tiles_x) * T::TW - T::K;
+    t.oy = (row - t.b * a.tiles_y) * T::TH - T::K;
+    t.x = t.ox + 2 * (threadIdx.x & 31);
+    t.y0 = t.oy + (threadIdx.x >> 5) * T::V;
+    return t;
+}
+
+// A tile's data in shared memory: D's planes and the increments of the region.
+template <typename T> struct HsSmem {
+    float2 d0[T::RH][T::RW], d1[T::RH][T::RW], in[T::RH][T::RW];
+};
+
+// Brings a tile's region into shared memory: by one thread's TMA boxes (zero
+// outside the level), completing on `bar`, or by every thread's loads.
+template <typename T>
+__device__ __forceinline__ void hs_fetch_tma(const HsJacobiArgs &a, int tile, HsSmem<T> &sm, uint32_t bar) {
+    const HsAt t = hs_at<T>(a, tile);
+    mbar_arrive_expect_tx(bar, (uint32_t)(T::RH * T::RW * 8) * (a.first ? 2u : 3u));
+    tma_load_3d(smem_u32(&sm.d0), &a.m0, t.ox, t.oy, t.b, bar);
+    tma_load_3d(smem_u32(&sm.d1), &a.m1, t.ox, t.oy, t.b, bar);
+    if (!a.first) tma_load_3d(smem_u32(&sm.in), &a.mi, t.ox, t.oy, t.b, bar);
+}
+template <typename T>
+__device__ __forceinline__ void hs_fetch(const HsJacobiArgs &a, int tile, HsSmem<T> &sm) {
+    const HsAt t = hs_at<T>(a, tile);
+    const float2 *D0 = a.D + (size_t)t.b * a.dstride, *D1 = D0 + a.plane, *In = a.in + (size_t)t.b * a.stride;
+    const float2 z = make_float2(0.f, 0.f);
+    for (int i = threadIdx.x; i < T::RH * T::RW; i += T::NT) {
+        const int rx = i % T::RW, ry = i / T::RW, x = t.ox + rx, y = t.oy + ry;
+        const bool in = x >= 0 && x < a.w && y >= 0 && y < a.h;
+        const size_t q = (size_t)y * a.w + x;
+        sm.d0[ry][rx] = in ? D0[q] : z;
+        sm.d1[ry][rx] = in ? D1[q] : z;
+        if (!a.first) sm.in[ry][rx] = in ? In[q] : z;
+    }
+}
+
+// Up to K sweeps of one tile whose data is in shared memory; once every thread
+// has taken its share into registers, `taken` runs.  first: increments start at 0
+// (flow.cu:168-171); last: add the increment to the flow (AddKernel,
+// addKernel.cuh:28-36) instead of storing it.  Returns whether the guard broke
+// (nothing is stored then).
+template <typename T, bool EXACT, typename F>
+__device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const HsSmem<T> &sm,
+                                        float4 (*sRow)[2][T::NW][32], F &&taken) {
+    constexpr int V = T::V, K = T::K, NW = T::NW;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, w = a.w, h = a.h;
+    const HsAt t = hs_at<T>(a, tile);
+    const int x = t.x, y0 = t.y0;
+    HsState<V> s;
+    unsigned key = ~0u;
+    const bool in0 = x >= 0 && x < w, in1 = x + 1 >= 0 && x + 1 < w;
+    bool broken = false;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const bool iy = y0 + v >= 0 && y0 + v < h;
+        const int r = wid * V + v;
+        const float4 d0 = *reinterpret_cast<const float4 *>(&sm.d0[r][2 * lane]);
+        const float4 d1 = *reinterpret_cast<const float4 *>(&sm.d1[r][2 * lane]);
+        const float4 u = a.first ? make_float4(0.f, 0.f, 0.f, 0.f)
+                                 : *reinterpret_cast<const float4 *>(&sm.in[r][2 * lane]);
+        s.a[v][0] = make_float2(u.x, u.y);
+        s.a[v][1] = make_float2(u.z, u.w);
+        s.ix[v][0] = d0.x; s.iy[v][0] = d0.y; s.iz[v][0] = d1.x; s.den[v][0] = iy && in0 ? d1.y : 1.0f;
+        s.ix[v][1] = d0.z; s.iy[v][1] = d0.w; s.iz[v][1] = d1.z; s.den[v][1] = iy && in1 ? d1.w : 1.0f;
+    }
+#pragma unroll
+    for (int v = 0; v < V; v++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            s.rcp[v][c] = rcp_near_rn(s.den[v][c]);
+            broken |= !rcp_in_range(s.den[v][c]);
+        }
+    const bool interior = t.ox >= 1 && t.oy >= 1 && t.ox + T::RW <= w - 1 && t.oy + T::RH <= h - 1;
+    const HsEdge e{x == 0, x + 1 == w - 1, x == w - 1, h - 1 - y0};
+    const bool top = y0 == 0;
+    if (EXACT) {
+#pragma unroll 1
+        for (int j = 0; j < a.sweeps; j++) hs_step<T, 2, true>(s, j, sRow, top, e, key, taken);
+    } else if (a.sweeps != K) {
+#pragma unroll 1
+        for (int j = 0; j < a.sweeps; j++) hs_step<T, 2, false>(s, j, sRow, top, e, key, taken);
+    } else if (interior) {
+        // unrolled, so that old and new increments swap registers instead of being copied
+#pragma unroll 4
+        for (int j = 0; j < K; j++) hs_step<T, 0, false>(s, j, sRow, top, e, key, taken);
+    } else if (t.oy + T::RH <= h - 1 && (w & 1) == 0) {
+#pragma unroll 2
+        for (int j = 0; j < K; j++) hs_step<T, 1, false>(s, j, sRow, top, e, key, taken);
+    } else {
+#pragma unroll 2
+        for (int j = 0; j < K; j++) hs_step<T, 2, false>(s, j, sRow, top, e, key, taken);
+    }
+    // (also: every warp has read the rows before the next tile writes them)
+    if (__syncthreads_or(!EXACT && (broken || key < kMarksteinKey))) return true;
+    if (lane < K / 2 || lane >= 32 - K / 2 || wid < K / V || wid >= NW - K / V || x >= w) return false;
+    float2 *Out = (a.last ? a.U : a.out) + (size_t)t.b * a.stride;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        if (y0 + v >= h) break;
+        const size_t q = (size_t)(y0 + v) * w + x;
+        float2 r0 = s.a[v][0], r1 = s.a[v][1];
+        if (a.last) {
+            const float4 u = hs_ld_two(Out, q, a.vec, true, in1);
+            r0 = make_float2(u.x + r0.x, u.y + r0.y);
+            r1 = make_float2(u.z + r1.x, u.w + r1.y);
+        }
+        if (a.vec) {
+            *reinterpret_cast<float4 *>(Out + q) = make_float4(r0.x, r0.y, r1.x, r1.y);
         } else {
-            dUout[p] = a;
+            Out[q] = r0;
+            if (in1) Out[q + 1] = r1;
+        }
+    }
+    return false;
+}
+
+// Resident blocks walk the tiles of all pairs; a tile's data is brought to
+// shared memory (TMA, where the level's strides allow it) while the block's
+// previous tile is in the registers.
+template <typename T, int MINB>
+__global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant__ HsJacobiArgs a) {
+    extern __shared__ __align__(128) char hs_dyn[];
+    HsSmem<T> &sm = *reinterpret_cast<HsSmem<T> *>(hs_dyn);
+    __shared__ float4 sRow[2][2][T::NW][32];
+    __shared__ __align__(8) unsigned long long s_bar;
+    const uint32_t bar = smem_u32(&s_bar);
+    uint32_t parity = 0;
+    if (a.tma && threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        fence_mbar_init();
+        hs_fetch_tma<T>(a, blockIdx.x, sm, bar);
+    }
+    __syncthreads();  // the barrier is initialised before anyone waits on it
+    for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
+        const int next = tile + gridDim.x;
+        if (a.tma) {
+            const bool ok = mbar_wait_bounded(bar, parity);
+            parity ^= 1u;
+            if (__syncthreads_or(!ok)) {
+                // report, let the copies land (bounded), leave; the host drops
+                // the plan's results
+                if (threadIdx.x == 0) atomicExch(a.err, 1);
+                mbar_wait_bounded(bar, parity ^ 1u);
+                return;
+            }
+        } else {
+            hs_fetch<T>(a, tile, sm);
+            __syncthreads();
+        }
+        const auto fetch_next = [&] {
+            if (a.tma && next < a.tiles && threadIdx.x == 0) {
+                fence_async_smem();  // the block's reads of this tile, then the copies of the next
+                hs_fetch_tma<T>(a, next, sm, bar);
+            }
+        };
+        if (hs_tile<T, false>(a, tile, sm, sRow, fetch_next)) {
+            // again from the untouched input, then the next tile's copies again
+            if (a.tma && next < a.tiles) {
+                const bool ok = mbar_wait_bounded(bar, parity);
+                parity ^= 1u;
+                if (__syncthreads_or(!ok)) {
+                    if (threadIdx.x == 0) atomicExch(a.err, 1);
+                    mbar_wait_bounded(bar, parity ^ 1u);
+                    return;
+                }
+            }
+            hs_fetch<T>(a, tile, sm);
+            __syncthreads();
+            hs_tile<T, true>(a, tile, sm, sRow, fetch_next);
         }
     }
 }
@@ -345,86 +522,131 @@ void launch_split2(const float2 *U, size_t stride, int N, float *out, int B, cud
 }
 
 // ================================================================ host plan
-constexpr int kJTW = 32, kJTH = 16, kJK = 4, kJNT = 256;
-
-// Jacobi configurations: tile tw x th, up to k sweeps per launch (halo k),
-// nt threads; 36 B of shared memory per region pixel (D 16, two u buffers,
-// the reciprocal of the denominator).
+// Jacobi configurations: the region is 64 x v*nw pixels with a k-pixel halo, nw
+// warps, mb blocks resident on an SM.
 struct HsJCfg {
-    int tw, th, k, nt;
+    int v, nw, k, mb;
 };
-constexpr HsJCfg kHsCfgs[] = {{32, 16, 4, 256}, {32, 16, 8, 256}, {64, 32, 8, 512},
-                              {64, 16, 4, 256}, {32, 32, 16, 512}, {64, 32, 4, 512}};
+constexpr HsJCfg kHsCfgs[] = {{4, 16, 4, 1}, {4, 8, 4, 2}, {4, 16, 8, 1}, {2, 12, 4, 2}, {4, 16, 16, 1}, {2, 16, 8, 2}};
 constexpr int kHsNumCfgs = 6;
-constexpr size_t hs_smem(const HsJCfg &c) { return (size_t)(c.tw + 2 * c.k) * (c.th + 2 * c.k) * 36; }
+template <int C> using HsCfgTile = HsTile<kHsCfgs[C].v, kHsCfgs[C].nw, kHsCfgs[C].k>;
 
-template <int TW, int TH, int KH, int NT>
-static void hs_jacobi_launch(dim3 g, cudaStream_t st, const float4 *D, size_t dstride,
-                             const float2 *in, float2 *out, float2 *U, size_t stride, int w,
-                             int h, int sweeps, int first, int last, const HsTma &tma) {
-    const size_t smem = (size_t)(TW + 2 * KH) * (TH + 2 * KH) * 36;
-    k_hs_jacobi<TW, TH, KH, NT><<<g, NT, smem, st>>>(D, dstride, in, out, U, stride, w, h, sweeps,
-                                                     first, last, tma);
+template <int C> constexpr int hs_smem() { return (int)sizeof(HsSmem<HsCfgTile<C>>); }
+
+// cuTensorMapEncodeTiled, looked up in the driver once (null if unavailable).
+static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+    }();
+    return fn;
 }
 
-static void hs_jacobi_cfg(int c, dim3 g, cudaStream_t st, const float4 *D, size_t dstride,
-                          const float2 *in, float2 *out, float2 *U, size_t stride, int w, int h,
-                          int sweeps, int first, int last, const HsTma &t) {
+// A tiled map of 8-byte elements, zero fill outside; dims innermost first,
+// byte strides of dims 1..rank-1.
+static bool encode_map8(CUtensorMap *m, void *base, int rank, const cuuint64_t *dims,
+                 const cuuint64_t *strides, const cuuint32_t *box) {
+    const PFN_cuTensorMapEncodeTiled_v12000 fn = tensor_map_encoder();
+    if (!fn) return false;
+    const cuuint32_t es[5] = {1, 1, 1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, (cuuint32_t)rank, base, dims, strides, box, es,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Tensor maps of the regions of configuration c.  TMA wants 16-byte strides
+// (even w and pair stride); otherwise, or without err, the kernel loads the
+// regions itself.
+static void hs_maps(HsJacobiArgs &a, int c, int B, int *err) {
+    a.err = err;
+    a.tma = 0;
+    if (!a.vec || !err) return;
+    const cuuint32_t box[3] = {64, (cuuint32_t)(kHsCfgs[c].v * kHsCfgs[c].nw), 1};
+    const cuuint64_t dims[3] = {(cuuint64_t)a.w, (cuuint64_t)a.h, (cuuint64_t)B};
+    const cuuint64_t sd[2] = {8 * (cuuint64_t)a.w, 8 * (cuuint64_t)a.dstride};
+    const cuuint64_t si[2] = {8 * (cuuint64_t)a.w, 8 * (cuuint64_t)a.stride};
+    a.tma = encode_map8(&a.m0, const_cast<float2 *>(a.D), 3, dims, sd, box) &&
+            encode_map8(&a.m1, const_cast<float2 *>(a.D + a.plane), 3, dims, sd, box) &&
+            encode_map8(&a.mi, const_cast<float2 *>(a.in), 3, dims, si, box);
+}
+
+template <int C> static void hs_jacobi_launch(int B, cudaStream_t st, const HsJacobiArgs &a) {
+    using T = HsCfgTile<C>;
+    HsJacobiArgs t = a;
+    t.tiles_x = div_up(a.w, T::TW);
+    t.tiles_y = div_up(a.h, T::TH);
+    t.tiles = t.tiles_x * t.tiles_y * B;
+    k_hs_jacobi<T, kHsCfgs[C].mb><<<imin(t.tiles, kHsCfgs[C].mb * kNumSMs), T::NT, hs_smem<C>(), st>>>(t);
+}
+
+template <int C> static void hs_set_smem_attr() {
+    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<HsCfgTile<C>, kHsCfgs[C].mb>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, hs_smem<C>()));
+}
+static void hs_set_smem_attrs() {
+    hs_set_smem_attr<0>();
+    hs_set_smem_attr<1>();
+    hs_set_smem_attr<2>();
+    hs_set_smem_attr<3>();
+    hs_set_smem_attr<4>();
+    hs_set_smem_attr<5>();
+}
+
+static void hs_jacobi_cfg(int c, int B, cudaStream_t st, const HsJacobiArgs &a) {
     switch (c) {
-        case 1: hs_jacobi_launch<32, 16, 8, 256>(g, st, D, dstride, in, out, U, stride, w, h, sweeps, first, last, t); break;
-        case 2: hs_jacobi_launch<64, 32, 8, 512>(g, st, D, dstride, in, out, U, stride, w, h, sweeps, first, last, t); break;
-        case 3: hs_jacobi_launch<64, 16, 4, 256>(g, st, D, dstride, in, out, U, stride, w, h, sweeps, first, last, t); break;
-        case 4: hs_jacobi_launch<32, 32, 16, 512>(g, st, D, dstride, in, out, U, stride, w, h, sweeps, first, last, t); break;
-        case 5: hs_jacobi_launch<64, 32, 4, 512>(g, st, D, dstride, in, out, U, stride, w, h, sweeps, first, last, t); break;
-        default: hs_jacobi_launch<32, 16, 4, 256>(g, st, D, dstride, in, out, U, stride, w, h, sweeps, first, last, t); break;
+        case 1: hs_jacobi_launch<1>(B, st, a); break;
+        case 2: hs_jacobi_launch<2>(B, st, a); break;
+        case 3: hs_jacobi_launch<3>(B, st, a); break;
+        case 4: hs_jacobi_launch<4>(B, st, a); break;
+        case 5: hs_jacobi_launch<5>(B, st, a); break;
+        default: hs_jacobi_launch<0>(B, st, a); break;
     }
 }
 
-// Tensor maps of the Jacobi region loads for configuration c on a level of
-// w x h (pairs N apart, B pairs) reading increments from `in`.  TMA wants
-// 16-byte strides: even w and N, else the kernel loads the region itself.
-static HsTma hs_tma(int c, const float4 *D, const float2 *in, int w, int h, size_t N, int B,
-                    int *err) {
-    HsTma t;
-    memset(&t, 0, sizeof(t));
-    t.err = err;
-    if ((w & 1) || (N & 1) || err == nullptr) return t;
-    const HsJCfg &jc = kHsCfgs[c];
-    const cuuint32_t rw = (cuuint32_t)(jc.tw + 2 * jc.k), rh = (cuuint32_t)(jc.th + 2 * jc.k);
-    const cuuint64_t dd[3] = {2 * (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)B};
-    const cuuint64_t sd[2] = {16 * (cuuint64_t)w, 16 * (cuuint64_t)N};
-    const cuuint32_t bd[3] = {2 * rw, rh, 1};
-    const cuuint64_t di[3] = {(cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)B};
-    const cuuint64_t si[2] = {8 * (cuuint64_t)w, 8 * (cuuint64_t)N};
-    const cuuint32_t bi[3] = {rw, rh, 1};
-    t.use = encode_map8(&t.tD, const_cast<float4 *>(D), 3, dd, sd, bd) &&
-            encode_map8(&t.tIn, const_cast<float2 *>(in), 3, di, si, bi);
-    return t;
+// All sweeps of one warp: from zero increments to the flow updated.
+static void hs_sweeps(int cfg, int B, cudaStream_t st, const float2 *D, size_t plane, float2 *const dU[2],
+                      float2 *U, size_t stride, int w, int h, int sweeps, bool update, int *err) {
+    const int K = kHsCfgs[cfg].k;
+    for (int done = 0, cur = 0; done < sweeps; cur ^= 1) {
+        const int k = imin(K, sweeps - done);
+        HsJacobiArgs a;
+        memset(&a, 0, sizeof(a));
+        a.D = D;
+        a.plane = plane;
+        a.dstride = a.stride = stride;
+        a.in = dU[cur];
+        a.out = dU[cur ^ 1];
+        a.U = U;
+        a.w = w;
+        a.h = h;
+        a.sweeps = k;
+        a.first = done == 0;
+        a.last = update && done + k == sweeps;
+        a.vec = (w & 1) == 0 && (stride & 1) == 0;
+        hs_maps(a, cfg, B, err);
+        hs_jacobi_cfg(cfg, B, st, a);
+        done += k;
+    }
 }
 
-static void hs_set_smem_attrs() {
-    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<32, 16, 4, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)hs_smem(kHsCfgs[0])));
-    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<32, 16, 8, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)hs_smem(kHsCfgs[1])));
-    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<64, 32, 8, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)hs_smem(kHsCfgs[2])));
-    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<64, 16, 4, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)hs_smem(kHsCfgs[3])));
-    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<32, 32, 16, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)hs_smem(kHsCfgs[4])));
-    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<64, 32, 4, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)hs_smem(kHsCfgs[5])));
-}
-
-// OFLOW_HS_CFG forces one configuration (used to test and time them); else
-// configuration 0 unless the tuning table has the level
-static int hs_pick() {
+// The configuration of a level; OFLOW_HS_CFG forces one (used to test and time
+// them), and a plan's tuning table comes before it.  A level whose 48x16 tiles
+// all fit on the GPU at once is bound by the launches' latency: small tiles of 8
+// sweeps (150 sweeps of a single 160x120, 80x60 or 40x30 level: 0.12 ms against
+// 0.16 with 48x48 tiles, 0.15 to 0.22 with 4 sweeps a launch).  Larger work takes
+// 48x48 tiles of 8 sweeps (64 pairs of 320x240, 200 sweeps: 2.7 ms against 3.1 to
+// 3.7).
+static int hs_pick(int w, int h, int B) {
     if (const char *e = getenv("OFLOW_HS_CFG")) {
         const int c = atoi(e);
         if (c >= 0 && c < kHsNumCfgs) return c;
     }
-    return 0;
+    const long long small = (long long)div_up(w, 48) * div_up(h, 16) * B;
+    return small <= 2 * kNumSMs ? 5 : 2;
 }
 
 HsPlan::HsPlan(int w, int h, int B, int dtype, const oflow_hs_params &prm, const TuneTable *tuned)
@@ -471,7 +693,7 @@ HsPlan::HsPlan(int w, int h, int B, int dtype, const oflow_hs_params &prm, const
     for (int l = 0; l < L_; l++) {
         const auto it = tuned ? tuned->find(tune_key(W_[l], H_[l], B, kTuneHs)) : TuneTable::const_iterator();
         const bool ok = tuned && it != tuned->end() && it->second >= 0 && it->second < kHsNumCfgs;
-        jcfg_[l] = ok ? it->second : hs_pick();
+        jcfg_[l] = ok ? it->second : hs_pick(W_[l], H_[l], B);
     }
 }
 
@@ -492,7 +714,7 @@ void HsPlan::bind_own_out(int b) {
 void HsPlan::record(cudaStream_t st) {
     const int B = B_;
     float *pyr = ar_.at<float>(o_pyr_);
-    float4 *D = ar_.at<float4>(o_D_);
+    float2 *D = ar_.at<float2>(o_D_);
     float2 *dU[2] = {ar_.at<float2>(o_dU0_), ar_.at<float2>(o_dU1_)};
     float2 *Ubuf[2] = {ar_.at<float2>(o_Ua_), ar_.at<float2>(o_Ub_)};
     const int top = L_ - 1;
@@ -509,25 +731,15 @@ void HsPlan::record(cudaStream_t st) {
     int ub = 0;  // Ubuf index holding the flow of the current level
     OF_CUDA(cudaMemsetAsync(Ubuf[ub], 0, B * N_ * 8, st));
     for (int l = 0; l < L_; l++) {
-        const HsJCfg &jc = kHsCfgs[jcfg_[l]];
         const int lw = W_[l], lh = H_[l];
         const size_t lp = (size_t)lw * lh;
         for (int wi = 0; wi < prm_.nwarp; wi++) {
             dim3 dg(div_up(lw, kDTW), div_up(lh, kDTH), B);
             k_hs_warp_deriv<<<dg, dim3(kDTW, kDTH), 0, st>>>(pyr + pyr_off_[l], lp, lw, lh,
-                                                             Ubuf[ub], N_, 0, prm_.alpha, D, N_);
-            dim3 jg(div_up(lw, jc.tw), div_up(lh, jc.th), B);
-            int done = 0, cur = 0;
-            if (prm_.nsolver == 0) continue;  // du = 0: the flow is unchanged
-            while (done < prm_.nsolver) {
-                const int k = imin(jc.k, prm_.nsolver - done);
-                const bool first = done == 0, last = done + k == prm_.nsolver;
-                const HsTma tm = hs_tma(jcfg_[l], D, dU[cur], lw, lh, N_, B, err_.device());
-                hs_jacobi_cfg(jcfg_[l], jg, st, D, N_, dU[cur], dU[cur ^ 1], Ubuf[ub], N_, lw, lh, k,
-                              first, last, tm);
-                cur ^= 1;
-                done += k;
-            }
+                                                             Ubuf[ub], N_, 0, prm_.alpha, D, B * N_, N_);
+            // with no sweeps du = 0: the flow is unchanged
+            hs_sweeps(jcfg_[l], B, st, D, B * N_, dU, Ubuf[ub], N_, lw, lh, prm_.nsolver, true,
+                      err_.device());
         }
         if (l != top) {
             const float sx = (float)W_[l + 1] / (float)lw;
@@ -547,38 +759,28 @@ void HsPlan::run(cudaStream_t st) {
     graph_.launch(st);
 }
 
-// Best of `reps` timed runs of 16 sweeps (in launches of the configuration's
+// Best of `reps` timed runs of 48 sweeps (in launches of the configuration's
 // depth) per configuration and level.  The sweep has no data-dependent control
 // flow, so the derivative buffer the last solve left is fine input at every
 // level size; the runs write only the du scratch, never the flow or outputs.
 void HsPlan::autotune(cudaStream_t st, TuneTable *table, int reps) {
-    float4 *D = ar_.at<float4>(o_D_);
+    float2 *D = ar_.at<float2>(o_D_);
     float2 *dU[2] = {ar_.at<float2>(o_dU0_), ar_.at<float2>(o_dU1_)};
     float2 *U = ar_.at<float2>(o_Ua_);
     cudaEvent_t e0, e1;
     OF_CUDA(cudaEventCreate(&e0));
     OF_CUDA(cudaEventCreate(&e1));
-    constexpr int kSweeps = 16;
+    constexpr int kSweeps = 48;
     try {
         for (int l = 0; l < L_; l++) {
             const int lw = W_[l], lh = H_[l];
             float best = 1e30f;
             int best_c = jcfg_[l];
             for (int c = 0; c < kHsNumCfgs; c++) {
-                const HsJCfg &jc = kHsCfgs[c];
-                dim3 jg(div_up(lw, jc.tw), div_up(lh, jc.th), B_);
                 float ms_min = 1e30f;
                 for (int r = 0; r <= reps; r++) {  // the first round warms up
                     OF_CUDA(cudaEventRecord(e0, st));
-                    int done = 0, cur = 0;
-                    while (done < kSweeps) {
-                        const int k = imin(jc.k, kSweeps - done);
-                        const HsTma tm = hs_tma(c, D, dU[cur], lw, lh, N_, B_, err_.device());
-                        hs_jacobi_cfg(c, jg, st, D, N_, dU[cur], dU[cur ^ 1], U, N_, lw, lh, k,
-                                      done == 0, 0, tm);
-                        cur ^= 1;
-                        done += k;
-                    }
+                    hs_sweeps(c, B_, st, D, B_ * N_, dU, U, N_, lw, lh, kSweeps, false, err_.device());
                     OF_CUDA(cudaEventRecord(e1, st));
                     OF_CUDA(cudaEventSynchronize(e1));
                     float ms = 0.0f;
@@ -601,6 +803,10 @@ void HsPlan::autotune(cudaStream_t st, TuneTable *table, int reps) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     graph_.reset();  // the next run captures the new configurations
+}
+
+void HsPlan::check_device_error() {
+    if (err_.take()) throw Error(OFLOW_ERR_TIMEOUT, "hs: a Jacobi tile's TMA load gave up its bounded wait");
 }
 
 // ================================================================ caller scratch
@@ -635,15 +841,10 @@ size_t hs_scratch_bytes(int w, int h, int nlevels) {
     return off;
 }
 
-void HsPlan::check_device_error() {
-    if (err_.take()) throw Error(OFLOW_ERR_TIMEOUT, "hs: a Jacobi tile's TMA load gave up its bounded wait");
-}
-
 void hs_enqueue_into(void *scratch, const float *I0, const float *I1, int w, int h, int pitch,
                      const oflow_hs_params &prm, float *u, float *v, int out_pitch,
                      cudaStream_t st) {
-    HsTma no_tma;  // this path loads its regions with plain instructions
-    memset(&no_tma, 0, sizeof(no_tma));
+    hs_set_smem_attrs();
     const int L = prm.nlevels;
     int Wl[16], Hl[16];
     Wl[L - 1] = w;
@@ -661,7 +862,7 @@ void hs_enqueue_into(void *scratch, const float *I0, const float *I1, int w, int
     size_t off = 0;
     char *base = static_cast<char *>(scratch);
     float *pyr = reinterpret_cast<float *>(base + hs_carve(off, acc * 4));
-    float4 *D = reinterpret_cast<float4 *>(base + hs_carve(off, N * 16));
+    float2 *D = reinterpret_cast<float2 *>(base + hs_carve(off, N * 16));
     float2 *dU[2];
     dU[0] = reinterpret_cast<float2 *>(base + hs_carve(off, N * 8));
     dU[1] = reinterpret_cast<float2 *>(base + hs_carve(off, N * 8));
@@ -681,24 +882,15 @@ void hs_enqueue_into(void *scratch, const float *I0, const float *I1, int w, int
     }
     int ub = 0;
     OF_CUDA(cudaMemsetAsync(Ubuf[ub], 0, N * 8, st));  // the flow starts at zero
-    const size_t smem = (size_t)(kJTW + 2 * kJK) * (kJTH + 2 * kJK) * 36;
     for (int l = 0; l < L; l++) {
         const int lw = Wl[l], lh = Hl[l];
         const size_t lp = (size_t)lw * lh;
         for (int wi = 0; wi < prm.nwarp; wi++) {
             dim3 dg(div_up(lw, kDTW), div_up(lh, kDTH), 1);
             k_hs_warp_deriv<<<dg, dim3(kDTW, kDTH), 0, st>>>(pyr + pyr_off[l], lp, lw, lh,
-                                                             Ubuf[ub], N, 0, prm.alpha, D, N);
-            dim3 jg(div_up(lw, kJTW), div_up(lh, kJTH), 1);
-            int done = 0, cur = 0;
-            while (done < prm.nsolver) {
-                const int k = imin(kJK, prm.nsolver - done);
-                k_hs_jacobi<kJTW, kJTH, kJK, kJNT><<<jg, kJNT, smem, st>>>(
-                    D, N, dU[cur], dU[cur ^ 1], Ubuf[ub], N, lw, lh, k, done == 0,
-                    done + k == prm.nsolver, no_tma);
-                cur ^= 1;
-                done += k;
-            }
+                                                             Ubuf[ub], N, 0, prm.alpha, D, N, N);
+            hs_sweeps(hs_pick(lw, lh, 1), 1, st, D, N, dU, Ubuf[ub], N, lw, lh, prm.nsolver, true,
+                      nullptr);
         }
         if (l != top) {
             const float sx = (float)Wl[l + 1] / (float)lw;

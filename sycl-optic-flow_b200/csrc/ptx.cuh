@@ -15,6 +15,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Asynchronous 16-byte copy to shared memory (waited for by cp.async.wait_all).
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool ok) {
+    const int n = ok ? 16 : 0;  // 0: zero fill, src is not read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
 __device__ __forceinline__ unsigned long long globaltimer() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

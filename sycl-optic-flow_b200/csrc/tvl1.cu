@@ -30,7 +30,6 @@
 #include "tvl1.hpp"
 
 #include <cooperative_groups.h>
-#include <cudaTypedefs.h>
 
 #include <cmath>
 #include <cstring>
@@ -949,11 +948,6 @@ template <int V_, int NW_> struct RtTile {
     };
 };
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool ok) {
-    const int n = ok ? 16 : 0;  // 0: zero fill, src is not read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
-}
-
 // The thread's share of the state: rows of its warp, two columns each.
 template <int V> struct RtState {
     float2 u[V][2];
@@ -1830,31 +1824,6 @@ int launch_zoom_out(const float *src, size_t sstride, int nx, int ny, float *T, 
 }
 
 // ================================================================ host plan
-// cuTensorMapEncodeTiled, looked up in the driver once (null if unavailable).
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }();
-    return fn;
-}
-
-// A tiled map of 8-byte elements, zero fill outside; dims innermost first,
-// byte strides of dims 1..rank-1.
-bool encode_map8(CUtensorMap *m, void *base, int rank, const cuuint64_t *dims,
-                 const cuuint64_t *strides, const cuuint32_t *box) {
-    const PFN_cuTensorMapEncodeTiled_v12000 fn = tensor_map_encoder();
-    if (!fn) return false;
-    const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, (cuuint32_t)rank, base, dims, strides, box, es,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // A plan needs no repair after a timeout: every warp stage starts with
 // k_warp re-arming each pair's control block and work queue, so the next
 // call runs from a clean state (tested with OFLOW_INJECT_TIMEOUT).

@@ -3,8 +3,6 @@
 // iterations, output split).
 #pragma once
 
-#include <cuda.h>
-
 #include <map>
 #include <tuple>
 
@@ -45,12 +43,6 @@ void launch_resample(const float *src, size_t sstride, int nx, int ny, float *ds
 int launch_zoom_out(const float *src, size_t sstride, int nx, int ny, float *T, float *dst,
                     size_t dstride, int nxx, int nyy, float zfactor, const GaussTaps &t,
                     int planes, cudaStream_t st);
-
-// A tiled TMA map of 8-byte elements with zero fill outside (dims innermost
-// first, byte strides of dims 1..rank-1, box per dim); false if the driver
-// refuses it (the caller then loads with plain instructions).
-bool encode_map8(CUtensorMap *m, void *base, int rank, const cuuint64_t *dims,
-                 const cuuint64_t *strides, const cuuint32_t *box);
 
 // Column coefficients of the warp's bicubic samples at one level, per texel
 // of every pair: (c3, c2) of I1, I1x and I1y in double, and (v2 - v0, v1) of
