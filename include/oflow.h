@@ -155,8 +155,8 @@ oflow_status oflow_tvl1_batch_profile(oflow_ctx *ctx, int n, const oflow_image *
  * inner-iteration configuration at every scale on the device and keeps the
  * fastest for plans of this size and batch: 0 = 56x40 tiles, 1 = 56x24,
  * 2 = 56x16, 3 = 56x8 (up to 4 iterations per launch), 4 = the whole level of
- * a pair in one block, 5 = the whole level in row bands over a cluster of 8
- * blocks (4 and 5 where the level fits shared memory).
+ * a pair in the registers of one block, 5 = in row bands over a cluster of up to
+ * 16 blocks (4 and 5 where the level fits).
  * cfg_per_scale (OFLOW_MAX_SCALES ints, may be NULL) receives the choice per
  * scale, -1 past the last scale.  The table lives in the context; it can be
  * saved to / loaded from a text file (lines: solver width height batch config)

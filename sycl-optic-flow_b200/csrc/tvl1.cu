@@ -33,6 +33,9 @@
 
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 namespace oflow {
 
@@ -50,11 +53,9 @@ constexpr TbCfg kTbCfgs[] = {{4, 12, 2}, {4, 8, 3}, {2, 12, 2}, {2, 8, 3}};
 constexpr int kTbNumCfgs = 4;
 constexpr int tb_tw() { return 64 - 2 * kTbK; }
 constexpr int tb_th(int c) { return kTbCfgs[c].v * kTbCfgs[c].nw - 2 * kTbK; }
-// Configuration 4: the whole level of a pair in one block (k_tvl1_level), for
-// levels of at most kLvMaxPx pixels.
+// Configurations 4 and 5: the whole level of a pair resident in one block or in
+// a cluster of blocks (k_tvl1_res).
 constexpr int kLevelCfg = 4;
-// Configuration 5: the whole level of a pair in row bands over a cluster of
-// kClC blocks (k_tvl1_cluster), for levels whose band fits shared memory.
 constexpr int kClusterCfg = 5;
 constexpr int kNumIterCfgs = 6;
 // tile of a tiled configuration (false for the whole-level ones)
@@ -66,16 +67,21 @@ inline bool cfg_tile(int c, int &tw, int &th) {
     }
     return false;
 }
-constexpr int kClC = 8;
-constexpr size_t kClMaxSmem = 200 * 1024;
-__host__ __device__ inline int cl_band_rows(int ny) { return (ny + kClC - 1) / kClC; }
-// u (8 B), p (16 B) and the warp data (16 B) of a band in shared memory
-inline bool cluster_fits(int nx, int ny) {
-    return ny >= 2 * kClC && (size_t)cl_band_rows(ny) * nx * 40 <= kClMaxSmem;
+// How a level of nx x ny is cut for k_tvl1_res: C blocks of wx x wy warps, a
+// thread with cpl columns of v rows.  false: it does not fit.
+struct ResCut {
+    int cpl, v, C, wx, wy;
+};
+constexpr int kResWarps = 16, kResBlocks = 16;
+constexpr int kResForms[][2] = {{1, 1}, {2, 1}, {2, 2}};  // (cpl, v)
+inline bool res_cut(int nx, int ny, int cpl, int v, int C, ResCut &r) {
+    r.cpl = cpl;
+    r.v = v;
+    r.C = C;
+    r.wx = div_up(nx, 32 * cpl);
+    r.wy = div_up(div_up(ny, v), C);
+    return r.wx * r.wy <= kResWarps;
 }
-constexpr int kLvNT = 1024;
-constexpr int kLvMaxPx = 9216;  // u (8 B) + p (16 B) per pixel: 221,184 B of shared memory
-inline bool level_fits(int nx, int ny) { return (long long)nx * ny <= kLvMaxPx; }
 constexpr int kGaussTW = 64, kGaussTH = 32, kGaussNT = 256, kGaussMaxR = 15;
 constexpr int kIngestNT = 256, kIngestPPT = 8;
 
@@ -1466,208 +1472,281 @@ __global__ void __launch_bounds__(T::NT, MINB) k_tvl1_q(const __grid_constant__ 
     }
 }
 
-// ---------------------------------------------------------------- whole level per block
-// A level small enough for shared memory (u and p, 24 B per pixel) runs a
-// whole warp stage in one launch: one block per pair, the inner iterations one
-// after another separated by block barriers, the squared change of each
-// summed in the block (per-thread double, fixed tree) and the stopping rule
-// (tvl1.cpp:216) applied after each iteration.  No halo is recomputed and the
-// state never leaves shared memory between iterations; I1wx, I1wy and rho_c
-// come through the cache.  The per-pixel arithmetic is th_u_update and
-// dual_update, as in the tiled kernels.
-__global__ void __launch_bounds__(kLvNT) k_tvl1_level(TbArgs a) {
-    extern __shared__ float4 lv_smem[];
-    __shared__ double sred[kLvNT / 32];
-    __shared__ int s_stop;
-    const int nx = a.nx, ny = a.ny, N = nx * ny;
-    float4 *sP = lv_smem;
-    float2 *sU = reinterpret_cast<float2 *>(sP + N);
-    const int b = blockIdx.x, tid = threadIdx.x;
-    TvCtrl *ctrl = a.ctrl + b;
-    const int cur = ctrl->cur;
-    const int fin = cur == 0 ? 1 : 0;
-    const size_t off = (size_t)b * a.stride;
-    const float2 *__restrict__ Uin = state_buf(a.U0, a.U1, cur) + off;
-    const Quads<float2> Pin = p_buf(a.P, a.plane, cur, off), Pout = p_buf(a.P, a.plane, fin, off);
-    float2 *__restrict__ Uout = state_buf(a.U0, a.U1, fin) + off;
-    const Quads<const float2> Wq = w_quads(a.W, a.plane, off);
-    for (int i = tid; i < N; i += kLvNT) {
-        sU[i] = Uin[i];
-        sP[i] = Pin.get(i);
-    }
-    __syncthreads();
-    int n = ctrl->n;
-    bool done = n >= a.max_it;
-    while (!done) {
-        // TH + u update; only the pixel's own u is read, so in place
-        double err = 0.0;
-        for (int i = tid; i < N; i += kLvNT) {
-            const int y = i / nx, x = i - y * nx;
-            const float2 u = sU[i];
-            const float4 pc = sP[i];
-            const float4 pl = x > 0 ? sP[i - 1] : pc;   // unused on the left border
-            const float4 pu = y > 0 ? sP[i - nx] : pc;  // unused on the top border
-            const float2 un = th_u_update(u, Wq.get_ro(i), pc, pl, pu, x == 0,
-                                          x == nx - 1, y == 0, y == ny - 1, a.l_t, a.theta);
-            sU[i] = un;
-            const float e1 = un.x - u.x, e2 = un.y - u.y;
-            const float term = e1 * e1 + e2 * e2;
-            err += (double)term;
-        }
-        __syncthreads();
-        // dual update; only the pixel's own p is read, so in place
-        for (int i = tid; i < N; i += kLvNT) {
-            const int y = i / nx, x = i - y * nx;
-            const float2 uc = sU[i];
-            float f1x = 0.0f, f2x = 0.0f, f1y = 0.0f, f2y = 0.0f;
-            if (x < nx - 1) {
-                const float2 ur = sU[i + 1];
-                f1x = ur.x - uc.x;
-                f2x = ur.y - uc.y;
-            }
-            if (y < ny - 1) {
-                const float2 ud = sU[i + nx];
-                f1y = ud.x - uc.x;
-                f2y = ud.y - uc.y;
-            }
-            sP[i] = dual_update(sP[i], f1x, f1y, f2x, f2y, a.taut);
-        }
-        const double tot = block_sum_double<kLvNT>(err, sred);  // barrier inside
-        n++;
-        if (tid == 0) {
-            float e = (float)tot;
-            e = e / (float)(nx * ny);
-            s_stop = !(e > a.eps2) || n >= a.max_it;
-        }
-        __syncthreads();
-        done = s_stop != 0;
-    }
-    for (int i = tid; i < N; i += kLvNT) {
-        Uout[i] = sU[i];
-        Pout.set(i, sP[i]);
-    }
-    if (tid == 0) {
-        ctrl->n = n;
-        ctrl->cur = fin;
-        ctrl->stop = 1;
-        a.iters[(size_t)b * a.iter_stride + a.stage] = n;
-    }
-}
+// ---------------------------------------------------------------- whole level resident
+// A small level stays in the registers of a cluster of C blocks (one cluster
+// per pair; C = 1 to 16) for a whole warp stage.  The level is cut into row
+// bands, one per block; a warp owns V rows of 32*CPL columns, a lane CPL
+// adjacent columns, with u, p and the warp's data in its registers.  Nothing is
+// recomputed: before each half of an iteration the edges the other half needs
+// (p right and down, u left and up) have been written to the reader's shared
+// memory -- the block's own, or for the rows between two bands the neighbouring
+// block's, by remote stores -- and one barrier (of the cluster, where C > 1)
+// makes them visible.
+//
+// These levels are bound by the latency of an iteration: a warp's instructions,
+// of which one starts every two to four cycles, and two barriers.  So a thread
+// gets as few pixels as the level's size allows (res_pick), and the sums and
+// the stopping decision (tvl1.cpp:216) are left to a warp of their own: it adds
+// the block's squared changes during the dual update, sends the sum to every
+// block, and decides from all of them during the first half of the next
+// iteration, which is dropped if the level had stopped (u is kept for that).
+// Every block adds the same sums in the same order, so all decide alike.  The
+// steps are the branch-free ones; a stage whose guard broke anywhere in the
+// cluster is run again, EXACT, from its untouched input.
+//
+// p11 of the last column and p12 of the last row are zero throughout (their
+// numerators are), so the border forms of mask.cpp:63-89 only differ by a
+// neighbour of zero before the first column and row, which the edge slots
+// hold, and in the first and last column by the order of the additions.
+//
+// Measured, microseconds of an iteration (here; a cluster of 8 blocks with the
+// state in shared memory; one such block of 1024 threads): 20x15 0.73, 2.1, 4.9;
+// 41x30 1.35, 2.4, 5.0; 81x59 1.8, 3.7, 5.4; 161x117 2.4, 6.0 (5.5 tiled).
+constexpr int kResMaxC = kResBlocks, kResMaxNW = kResWarps;
+struct ResArgs {
+    TbArgs t;
+    int wx, wy;  // warps of a block across the level's width, and down its band
+};
+template <int CPL, int V> struct ResSmem {
+    float2 pr[kResMaxNW + 1][V];            // (p11, p21) of each warp's last column, from [1]; [0] is zero
+    float2 ul[kResMaxNW + 1][V];            // u of each warp's first column
+    float2 pd[2 * kResMaxNW + 1][CPL][32];  // (p12, p22) of each warp's last row, the band above's before them
+    float2 uu[2 * kResMaxNW + 1][CPL][32];  // u of each warp's first row, the band below's after them
+                                            // (the last row of both: written by warps without a reader)
+    double err[kResMaxNW][32];              // squared change per thread
+    double part[kResMaxC];                  // and per block
+    int stop, broken[kResMaxC];
+};
 
-// ---------------------------------------------------------------- level per cluster
-// A level split into row bands over a cluster of kClC blocks, one cluster per
-// pair: for levels that one block runs too slowly and tiles leave most SMs
-// idle.  Each block keeps its band's u, p and warp data in shared memory and reads the one
-// neighbouring row it needs -- p of the row above its band, u of the row below
-// it -- from the adjacent block's shared memory (distributed shared memory).
-// Per inner iteration the cluster synchronises twice: after the TH step and u
-// update (u new everywhere, the bands' squared-change sums posted) and after
-// the dual update (p new everywhere).  Every block adds the bands' sums in rank
-// order from the others' shared memory, so all take the same stopping decision
-// (tvl1.cpp:216) and run the same number of cluster barriers.  The per-pixel
-// arithmetic is th_u_update and dual_update, as in the tiled kernels.
-// (ly, x) of pixel i + NT from that of pixel i in rows of nx pixels.
-template <int NT>
-__device__ __forceinline__ void cl_step(int &ly, int &x, int nx) {
-    ly += NT / nx;
-    x += NT % nx;
-    if (x >= nx) {
-        x -= nx;
-        ly += 1;
-    }
-}
-
-template <int NT>
-__global__ void __cluster_dims__(kClC, 1, 1) __launch_bounds__(NT) k_tvl1_cluster(TbArgs a) {
+template <int CPL, int V, bool CL, bool EXACT>
+__device__ __forceinline__ bool res_stage(const ResArgs &ra, ResSmem<CPL, V> &sm, int &n_out) {
     namespace cg = cooperative_groups;
+    using Row = float2[CPL][32];
+    const TbArgs &a = ra.t;
     cg::cluster_group cluster = cg::this_cluster();
-    const int c = (int)cluster.block_rank();
-    extern __shared__ float4 cl_smem[];
-    __shared__ double sred[NT / 32];
-    __shared__ double s_part;
-    const int nx = a.nx, ny = a.ny, tid = threadIdx.x;
-    const int r0 = c * ny / kClC, r1 = (c + 1) * ny / kClC, nb = r1 - r0;
-    const size_t cap = (size_t)cl_band_rows(ny) * nx;
-    float4 *sP = cl_smem;
-    float4 *sW = sP + cap;
-    float2 *sU = reinterpret_cast<float2 *>(sW + cap);
+    const int C = CL ? (int)gridDim.x : 1, rank = CL ? (int)cluster.block_rank() : 0;
+    const auto sync = [&] {
+        if (CL)
+            cluster.sync();
+        else
+            __syncthreads();
+    };
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int NX = ra.wx, NY = ra.wy, NW = NX * NY;
+    const int wy = wid / NX, wx = wid - wy * NX;
+    const int nx = a.nx, ny = a.ny;
     const int b = blockIdx.y;
     TvCtrl *ctrl = a.ctrl + b;
-    const int cur = *((volatile int *)&ctrl->cur);
-    const int fin = cur == 0 ? 1 : 0;
-    const size_t off = (size_t)b * a.stride;
-    const float2 *__restrict__ Uin = state_buf(a.U0, a.U1, cur) + off + (size_t)r0 * nx;
-    const Quads<float2> Pin = p_buf(a.P, a.plane, cur, off + (size_t)r0 * nx);
-    const Quads<const float2> Wq = w_quads(a.W, a.plane, off + (size_t)r0 * nx);
-    const int N = nb * nx;
-    for (int i = tid; i < N; i += NT) {
-        sU[i] = Uin[i];
-        sP[i] = Pin.get(i);
-        sW[i] = Wq.get(i);
-    }
-    // the neighbours' rows: p of the band above (its last row), u of the band below (its first)
-    const int nb_up = c > 0 ? r0 - (c - 1) * ny / kClC : 0;
-    const float4 *upP = c > 0 ? cluster.map_shared_rank(sP, c - 1) + (size_t)(nb_up - 1) * nx : nullptr;
-    const float2 *dnU = c + 1 < kClC ? cluster.map_shared_rank(sU, c + 1) : nullptr;
-    cluster.sync();
     int n = *((volatile int *)&ctrl->n);
-    bool done = n >= a.max_it;
-    const int ly0 = tid / nx, x0 = tid - ly0 * nx;  // band row and column of pixel tid
-    while (!done) {
-        double err = 0.0;
-        for (int i = tid, ly = ly0, x = x0; i < N; i += NT, cl_step<NT>(ly, x, nx)) {
-            const int y = r0 + ly;
-            const float2 u = sU[i];
-            const float4 pc = sP[i];
-            const float4 pl = x > 0 ? sP[i - 1] : pc;  // unused on the left border
-            const float4 pu = y == 0 ? pc : (ly > 0 ? sP[i - nx] : upP[x]);  // unused on the top border
-            const float2 un = th_u_update(u, sW[i], pc, pl, pu, x == 0, x == nx - 1, y == 0,
-                                          y == ny - 1, a.l_t, a.theta);
-            sU[i] = un;
-            const float e1 = un.x - u.x, e2 = un.y - u.y;
-            const float term = e1 * e1 + e2 * e2;
-            err += (double)term;
-        }
-        const double bs = block_sum_double<NT>(err, sred);
-        if (tid == 0) s_part = bs;
-        cluster.sync();  // u new in every band, the bands' sums posted
-        double tot = 0.0;
+    const float npx = (float)(nx * ny);
+    if (wid == NW) {  // the warp that sums and decides
+        sync();
+        sync();
+        while (n < a.max_it) {
+            sync();  // squared changes of iteration n + 1
+            if (sm.stop) break;
+            double e = 0.0;
+            for (int i = 0; i < NW; i++) e += sm.err[i][lane];
 #pragma unroll
-        for (int k = 0; k < kClC; k++) tot += *cluster.map_shared_rank(&s_part, k);
-        n++;
-        float e = (float)tot;
-        e = e / (float)(nx * ny);
-        const bool stop = !(e > a.eps2) || n >= a.max_it;
-        for (int i = tid, ly = ly0, x = x0; i < N; i += NT, cl_step<NT>(ly, x, nx)) {
-            const int y = r0 + ly;
-            const float2 uc = sU[i];
-            float f1x = 0.0f, f2x = 0.0f, f1y = 0.0f, f2y = 0.0f;
-            if (x < nx - 1) {
-                const float2 ur = sU[i + 1];
-                f1x = ur.x - uc.x;
-                f2x = ur.y - uc.y;
+            for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+            if (CL) {
+                if (lane < C) *cluster.map_shared_rank(&sm.part[rank], lane) = e;
             }
-            if (y < ny - 1) {
-                const float2 ud = ly + 1 < nb ? sU[i + nx] : dnU[x];
-                f1y = ud.x - uc.x;
-                f2y = ud.y - uc.y;
+            sync();
+            n++;
+            if (CL) {
+                e = 0.0;
+                for (int k = 0; k < C; k++) e += sm.part[k];
             }
-            sP[i] = dual_update(sP[i], f1x, f1y, f2x, f2y, a.taut);
+            float m = (float)e;
+            m = m / npx;
+            if (lane == 0) sm.stop = !(m > a.eps2);
         }
-        cluster.sync();  // p new in every band; the sums may be overwritten
-        done = stop;
+    } else {
+        const int x = (wx * 32 + lane) * CPL, y0 = (rank * NY + wy) * V;
+        const int cur = *((volatile int *)&ctrl->cur), fin = cur == 0 ? 1 : 0;
+        const size_t off = (size_t)b * a.stride;
+        float2 u[V][CPL], ub[V][CPL];
+        float4 p[V][CPL], w[V][CPL];
+        float own[V][CPL], fx[CPL], fy[V];  // 1, or 0 where the pixel / its difference does not exist
+        FastGuard fg;
+        {
+            const float2 *__restrict__ Uin = state_buf(a.U0, a.U1, cur) + off;
+            const Quads<float2> Pin = p_buf(a.P, a.plane, cur, off);
+            const Quads<const float2> Wq = w_quads(a.W, a.plane, off);
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                fy[v] = y0 + v < ny - 1 ? 1.0f : 0.0f;
+#pragma unroll
+                for (int c = 0; c < CPL; c++) {
+                    const bool in = y0 + v < ny && x + c < nx;
+                    const size_t q = (size_t)(y0 + v) * nx + x + c;
+                    p[v][c] = in ? Pin.get(q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    w[v][c] = in ? Wq.get(q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    u[v][c] = in ? Uin[q] : make_float2(0.f, 0.f);
+                    own[v][c] = in ? 1.0f : 0.0f;
+                    fx[c] = x + c < nx - 1 ? 1.0f : 0.0f;
+                }
+            }
+        }
+        // where this warp's edges go: the rows of pd below it, the rows of uu above it
+        Row *pd_to = &sm.pd[NX + wid], *uu_to = &sm.uu[wid];
+        if (CL && wy == NY - 1)
+            pd_to = rank + 1 < C ? cluster.map_shared_rank(&sm.pd[wx], rank + 1) : &sm.pd[2 * kResMaxNW];
+        if (CL && wy == 0)
+            uu_to = rank > 0 ? cluster.map_shared_rank(&sm.uu[NW + wx], rank - 1) : &sm.uu[2 * kResMaxNW];
+        const float2 *const pr_from = sm.pr[wx > 0 ? wid : 0];  // of the warp to the left
+        const bool ul_right = wx + 1 < NX;
+        const auto post_p = [&] {
+            if (lane == 31)
+#pragma unroll
+                for (int v = 0; v < V; v++) sm.pr[wid + 1][v] = make_float2(p[v][CPL - 1].x, p[v][CPL - 1].z);
+#pragma unroll
+            for (int c = 0; c < CPL; c++) (*pd_to)[c][lane] = make_float2(p[V - 1][c].y, p[V - 1][c].w);
+        };
+        sync();  // (CL: every block of the cluster runs before its memory is written)
+        post_p();
+        sync();
+        while (n < a.max_it) {
+            // TH step, divergence and u update
+            double err = 0.0;
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                float l1 = __shfl_up_sync(0xffffffffu, p[v][CPL - 1].x, 1);
+                float l3 = __shfl_up_sync(0xffffffffu, p[v][CPL - 1].z, 1);
+                if (lane == 0) {
+                    l1 = pr_from[v].x;
+                    l3 = pr_from[v].y;
+                }
+#pragma unroll
+                for (int c = 0; c < CPL; c++) {
+                    const float4 pc = p[v][c];
+                    const float2 up = v ? make_float2(p[v ? v - 1 : 0][c].y, p[v ? v - 1 : 0][c].w) : sm.pd[wid][c][lane];
+                    const float a1l = c ? p[v][c ? c - 1 : 0].x : l1, a3l = c ? p[v][c ? c - 1 : 0].z : l3;
+                    const float dx1 = pc.x - a1l, dx2 = pc.z - a3l;
+                    float div1 = dx1 + (pc.y - up.x), div2 = dx2 + (pc.w - up.y);
+                    if (x + c == 0 || x + c == nx - 1) {
+                        div1 = (dx1 + pc.y) - up.x;
+                        div2 = (dx2 + pc.w) - up.y;
+                    }
+                    const float2 uo = u[v][c];
+                    ub[v][c] = uo;
+                    float2 t;
+                    if (EXACT) {
+                        t = th_step(uo, w[v][c], a.l_t);
+                    } else {
+                        const float k = th_coef_fast(uo, w[v][c], a.l_t, fg);
+                        t = make_float2(uo.x + k * w[v][c].x, uo.y + k * w[v][c].y);
+                    }
+                    const float2 un = make_float2(t.x + a.theta * div1, t.y + a.theta * div2);
+                    u[v][c] = un;
+                    const float e1 = un.x - uo.x, e2 = un.y - uo.y;
+                    const float term = e1 * e1 + e2 * e2;
+                    err += (double)(EXACT ? (own[v][c] != 0.0f ? term : 0.0f) : term * own[v][c]);
+                }
+            }
+            if (lane == 0)
+#pragma unroll
+                for (int v = 0; v < V; v++) sm.ul[wid][v] = u[v][0];
+#pragma unroll
+            for (int c = 0; c < CPL; c++) (*uu_to)[c][lane] = u[0][c];
+            sm.err[wid][lane] = err;
+            sync();
+            if (sm.stop) {  // iteration n was the last
+#pragma unroll
+                for (int v = 0; v < V; v++)
+#pragma unroll
+                    for (int c = 0; c < CPL; c++) u[v][c] = ub[v][c];
+                break;
+            }
+            // dual update from the forward differences of u
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                float2 r;
+                r.x = __shfl_down_sync(0xffffffffu, u[v][0].x, 1);
+                r.y = __shfl_down_sync(0xffffffffu, u[v][0].y, 1);
+                if (lane == 31 && ul_right) r = sm.ul[wid + 1][v];
+#pragma unroll
+                for (int c = 0; c < CPL; c++) {
+                    const float2 uc = u[v][c], ur = c + 1 < CPL ? u[v][c + 1 < CPL ? c + 1 : c] : r;
+                    const float2 ud = v + 1 < V ? u[v + 1 < V ? v + 1 : v][c] : sm.uu[wid + NX][c][lane];
+                    float f1x = ur.x - uc.x, f2x = ur.y - uc.y, f1y = ud.x - uc.x, f2y = ud.y - uc.y;
+                    if (EXACT) {
+                        if (fx[c] == 0.0f) f1x = f2x = 0.0f;
+                        if (fy[v] == 0.0f) f1y = f2y = 0.0f;
+                        p[v][c] = dual_update(p[v][c], f1x, f1y, f2x, f2y, a.taut);
+                    } else {  // (an infinite or NaN difference breaks the guard)
+                        f1x *= fx[c];
+                        f2x *= fx[c];
+                        f1y *= fy[v];
+                        f2y *= fy[v];
+                        p[v][c] = dual_update_fast(p[v][c], f1x, f1y, f2x, f2y, a.taut, fg);
+                    }
+                }
+            }
+            post_p();
+            sync();
+            n++;
+        }
+        if (!EXACT) {
+            // the cluster agrees on whether a guard broke; a pixel outside the
+            // level holds values that no pixel inside sees
+            const bool bad = y0 < ny && x < nx && fg.broken();
+            if (__any_sync(0xffffffffu, bad) && lane < C)
+                *(CL ? cluster.map_shared_rank(&sm.broken[rank], lane) : &sm.broken[0]) = 1;
+        } else {
+            n_out = n;
+        }
+        if (!EXACT) sync();
+        int any = 0;
+        if (!EXACT)
+            for (int k = 0; k < C; k++) any |= sm.broken[k];
+        if (any) return false;
+        float2 *__restrict__ Uout = state_buf(a.U0, a.U1, fin) + off;
+        const Quads<float2> Pout = p_buf(a.P, a.plane, fin, off);
+#pragma unroll
+        for (int v = 0; v < V; v++)
+#pragma unroll
+            for (int c = 0; c < CPL; c++)
+                if (y0 + v < ny && x + c < nx) {
+                    const size_t q = (size_t)(y0 + v) * nx + x + c;
+                    Uout[q] = u[v][c];
+                    Pout.set(q, p[v][c]);
+                }
+        n_out = n;
+        return true;
     }
-    float2 *__restrict__ Uout = state_buf(a.U0, a.U1, fin) + off + (size_t)r0 * nx;
-    const Quads<float2> Pout = p_buf(a.P, a.plane, fin, off + (size_t)r0 * nx);
-    for (int i = tid; i < N; i += NT) {
-        Uout[i] = sU[i];
-        Pout.set(i, sP[i]);
+    n_out = n;
+    if (EXACT) return true;
+    sync();
+    int any = 0;
+    for (int k = 0; k < C; k++) any |= sm.broken[k];
+    return !any;
+}
+
+template <int CPL, int V, bool CL>
+__global__ void __launch_bounds__(32 * (kResMaxNW + 1)) k_tvl1_res(const __grid_constant__ ResArgs ra) {
+    __shared__ ResSmem<CPL, V> sm;
+    // edges that no warp writes (before the first column and band, below the last band) read as zero
+    const float2 z = make_float2(0.f, 0.f);
+    for (int i = threadIdx.x; i < (2 * kResMaxNW + 1) * CPL * 32; i += blockDim.x)
+        (&sm.pd[0][0][0])[i] = (&sm.uu[0][0][0])[i] = z;
+    if (threadIdx.x < V) sm.pr[0][threadIdx.x] = z;
+    if (threadIdx.x < kResMaxC) sm.broken[threadIdx.x] = 0;
+    if (threadIdx.x == 0) sm.stop = 0;
+    int n;
+    if (!res_stage<CPL, V, CL, false>(ra, sm, n)) {
+        __syncthreads();  // (everyone has left the first run's last barrier before its flags change)
+        if (threadIdx.x == 0) sm.stop = 0;
+        res_stage<CPL, V, CL, true>(ra, sm, n);
     }
-    if (c == 0 && tid == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const TbArgs &a = ra.t;
+        TvCtrl *ctrl = a.ctrl + blockIdx.y;
         ctrl->n = n;
-        ctrl->cur = fin;
+        ctrl->cur = ctrl->cur == 0 ? 1 : 0;
         ctrl->stop = 1;
-        a.iters[(size_t)b * a.iter_stride + a.stage] = n;
+        a.iters[(size_t)blockIdx.y * a.iter_stride + a.stage] = n;
     }
 }
 
@@ -1839,22 +1918,93 @@ template <int C> static void tb_launch(dim3 g, cudaStream_t st, const TbArgs &ta
     k_tvl1_tb<TbTile<C>, kTbCfgs[C].mb><<<g, TbTile<C>::NT, sizeof(typename TbTile<C>::Smem), st>>>(ta);
 }
 
-static void tb_launch_cfg(int cfg, dim3 g, cudaStream_t st, const TbArgs &ta) {
-    if (cfg == kClusterCfg) {
-        // 256 threads where they cover a band in one pass, else 512 (1024
-        // threads leave one block per SM: 32 clusters of 8 then take two
-        // waves, and the 128x55 level took 1.6 ms instead of 0.95)
-        const int band = cl_band_rows(ta.ny) * ta.nx;
-        const size_t smem = (size_t)band * (2 * sizeof(float4) + sizeof(float2));
-        if (band <= 256)
-            k_tvl1_cluster<256><<<dim3(kClC, g.z), 256, smem, st>>>(ta);
-        else
-            k_tvl1_cluster<512><<<dim3(kClC, g.z), 512, smem, st>>>(ta);
-        return;
+// Launch configuration of a cut for B pairs; at: its cluster attribute.
+static cudaLaunchConfig_t res_config(const ResCut &r, int B, cudaLaunchAttribute &at) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(r.C, B);
+    lc.blockDim = dim3(32 * (r.wx * r.wy + 1));
+    at = cudaLaunchAttribute{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = r.C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    lc.attrs = &at;
+    lc.numAttrs = r.C > 1 ? 1 : 0;
+    return lc;
+}
+using ResKernel = void (*)(ResArgs);
+static ResKernel res_kernel(const ResCut &r) {
+    if (r.cpl == 1) return r.C > 1 ? k_tvl1_res<1, 1, true> : k_tvl1_res<1, 1, false>;
+    if (r.v == 1) return r.C > 1 ? k_tvl1_res<2, 1, true> : k_tvl1_res<2, 1, false>;
+    return r.C > 1 ? k_tvl1_res<2, 2, true> : k_tvl1_res<2, 2, false>;
+}
+
+// Pairs that run at the same time in this cut (0: the device takes no such cluster).
+static int res_active(const ResCut &r) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, int, int, int>, int> seen;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(r.cpl, r.v, r.C, r.wx * r.wy);
+    const auto it = seen.find(key);
+    if (it != seen.end()) return it->second;
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t lc = res_config(r, 1, at);
+    int n = 0;
+    if (r.C > 1) {
+        if (cudaOccupancyMaxActiveClusters(&n, (const void *)res_kernel(r), &lc) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+    } else {
+        OF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void *)res_kernel(r), (int)lc.blockDim.x, 0));
+        n *= kNumSMs;
     }
-    if (cfg == kLevelCfg) {
-        const size_t smem = (size_t)ta.nx * ta.ny * (sizeof(float4) + sizeof(float2));
-        k_tvl1_level<<<g.z, kLvNT, smem, st>>>(ta);
+    return seen[key] = n;
+}
+
+// Microseconds of an iteration of a cut, for B pairs: the barriers of a cluster
+// of that size, and the arithmetic of the warps that share an SM; times the
+// waves of clusters.  Measured on single pairs of 161x117 and 640x480 and their
+// coarser levels (within 10 % for levels of 20x15 to 161x117); several clusters
+// at a time take longer for their barriers (32 pairs of 256x109: 1.4 times).
+static float res_time(const ResCut &r, int B) {
+    constexpr float kSync[] = {0.45f, 1.10f, 1.12f, 1.20f, 1.42f};  // C = 1, 2, 4, 8, 16
+    int k = 0;
+    while ((1 << k) < r.C) k++;
+    const float per_warp = r.cpl == 1 ? 0.020f : r.v == 1 ? 0.043f : 0.075f;
+    const float t = kSync[k] + per_warp * (float)(r.wx * r.wy) + (r.v == 2 ? 0.1f : 0.0f);
+    const int active = res_active(r);
+    return active ? t * (B > 1 ? 1.4f : 1.0f) * (float)div_up(B, active) : 1e30f;
+}
+
+// The cut of a level for B pairs with clusters of at most max_c blocks: of those
+// that fit, the fastest.  OFLOW_RES=cpl,v,C forces one (used to test and time
+// them).
+static bool res_pick(int nx, int ny, int B, int max_c, ResCut &best) {
+    int fc = 0, fv = 0, fC = 0;
+    const char *env = getenv("OFLOW_RES");
+    if (env && sscanf(env, "%d,%d,%d", &fc, &fv, &fC) != 3) fC = 0;
+    bool found = false, forced = false;
+    for (const auto &f : kResForms)
+        for (int C = 1; C <= max_c; C *= 2) {
+            ResCut r;
+            if (!res_cut(nx, ny, f[0], f[1], C, r)) continue;
+            const bool asked = f[0] == fc && f[1] == fv && C == fC;
+            if (!found || asked || (!forced && res_time(r, B) < res_time(best, B))) best = r;
+            found = true;
+            forced = forced || asked;
+        }
+    return found;
+}
+
+static void tb_launch_cfg(int cfg, dim3 g, cudaStream_t st, const TbArgs &ta) {
+    if (cfg == kLevelCfg || cfg == kClusterCfg) {
+        ResCut r;
+        if (!res_pick(ta.nx, ta.ny, (int)g.z, cfg == kClusterCfg ? kResBlocks : 1, r))
+            throw Error(OFLOW_ERR_UNSUPPORTED, "tvl1: level too large for the resident kernel");
+        cudaLaunchAttribute at;
+        cudaLaunchConfig_t lc = res_config(r, (int)g.z, at);
+        lc.stream = st;
+        OF_CUDA(cudaLaunchKernelEx(&lc, res_kernel(r), ResArgs{ta, r.wx, r.wy}));
         return;
     }
     switch (cfg) {
@@ -1916,12 +2066,10 @@ static void tb_set_smem_attrs() {
     tb_set_smem_attr<1>();
     tb_set_smem_attr<2>();
     tb_set_smem_attr<3>();
-    OF_CUDA(cudaFuncSetAttribute(k_tvl1_level, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kLvMaxPx * (int)(sizeof(float4) + sizeof(float2))));
-    OF_CUDA(cudaFuncSetAttribute(k_tvl1_cluster<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kClMaxSmem));
-    OF_CUDA(cudaFuncSetAttribute(k_tvl1_cluster<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kClMaxSmem));
+    // clusters of 16 blocks
+    OF_CUDA(cudaFuncSetAttribute(k_tvl1_res<1, 1, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    OF_CUDA(cudaFuncSetAttribute(k_tvl1_res<2, 1, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    OF_CUDA(cudaFuncSetAttribute(k_tvl1_res<2, 2, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
 }
 
 static int tb_tiles(int cfg, int nx, int ny) {
@@ -1936,22 +2084,28 @@ static dim3 tb_grid(int cfg, int nx, int ny, int B) {
     return dim3(div_up(nx, tw), div_up(ny, th), B);
 }
 
-// The tile with the least estimated time of a block of K iterations: what one
-// tile takes on an SM of its own, plus what each further tile of the busiest SM
-// adds.  Microseconds measured on single pairs of 160x117 to 1280x720 (first
-// column: 24 / 21 / 17.5 / 16) and on 32 pairs of 1024x436 (second); a large
-// tile wastes less on its halo, small ones use more SMs.  OFLOW_TB_CFG forces
-// one configuration (used to time them against each other).
+// A level that fits is kept resident while that is faster than tiles; else the
+// tile with the least estimated time of a block of K iterations: what one tile
+// takes on an SM of its own, plus what each further tile of the busiest SM adds.
+// Microseconds measured on single pairs of 160x117 to 1280x720 (kTbAlone) and on
+// 32 pairs of 1024x436 (kTbMore); a large tile wastes less on its halo, small
+// ones use more SMs.  OFLOW_TB_CFG forces one configuration (used to test and
+// time them).  In the launch form (OFLOW_TB_QUEUE=0) levels above kTiledPx run
+// tiled.
+constexpr long long kTiledPx = 9216;
 constexpr float kTbAlone[kTbNumCfgs] = {24.0f, 21.0f, 17.5f, 16.0f};
 constexpr float kTbMore[kTbNumCfgs] = {12.0f, 7.6f, 6.8f, 4.5f};
-static int tb_pick(int nx, int ny, int B) {
+static bool res_fits(int nx, int ny, int max_c) {
+    ResCut r;
+    return res_pick(nx, ny, 1, max_c, r);
+}
+static int tb_pick(int nx, int ny, int B, bool tiles) {
     if (const char *e = getenv("OFLOW_TB_CFG")) {
         const int c = atoi(e);
         if (c >= 0 && c < kTbNumCfgs) return c;
-        if (c == kLevelCfg && level_fits(nx, ny)) return c;
-        if (c == kClusterCfg && cluster_fits(nx, ny)) return c;
+        if (c == kLevelCfg && res_fits(nx, ny, 1)) return c;
+        if (c == kClusterCfg && res_fits(nx, ny, kResBlocks)) return c;
     }
-    if (level_fits(nx, ny)) return kLevelCfg;
     int best = 0;
     float best_t = 1e30f;
     for (int c = 0; c < kTbNumCfgs; c++) {
@@ -1962,13 +2116,17 @@ static int tb_pick(int nx, int ny, int B) {
             best = c;
         }
     }
+    ResCut r;
+    if (!(tiles && (long long)nx * ny > kTiledPx) && res_pick(nx, ny, B, kResBlocks, r) &&
+        kTbK * res_time(r, B) < best_t)
+        return kClusterCfg;
     return best;
 }
 
 // a configuration from a tuning table, if it is valid for this level
 static bool cfg_valid(int c, int nx, int ny) {
-    return (c >= 0 && c < kTbNumCfgs) || (c == kLevelCfg && level_fits(nx, ny)) ||
-           (c == kClusterCfg && cluster_fits(nx, ny));
+    return (c >= 0 && c < kTbNumCfgs) || (c == kLevelCfg && res_fits(nx, ny, 1)) ||
+           (c == kClusterCfg && res_fits(nx, ny, kResBlocks));
 }
 
 TvPlan::TvPlan(int w, int h, int B, int dtype, const oflow_tvl1_params &prm, bool trace,
@@ -2001,14 +2159,18 @@ TvPlan::TvPlan(int w, int h, int B, int dtype, const oflow_tvl1_params &prm, boo
         si_[s] = prm.max_iterations;
     }
 
+    tb_set_smem_attrs();
     const size_t N0 = (size_t)w * h;
     N0_ = N0;
+    // OFLOW_TB_QUEUE=0 runs the tiled stages as one launch per block of K
+    // iterations (k_tvl1_tb) instead of the persistent work queue (k_tvl1_q)
+    if (const char *e = getenv("OFLOW_TB_QUEUE")) queue_off_env_ = atoi(e) == 0;
     iter_blocks_ = div_up(w, kIterTW) * div_up(h, kIterTH);
     for (int s = 0; s < ns_; s++) {
         const auto it = tuned ? tuned->find(tune_key(nx_[s], ny_[s], B)) : TuneTable::const_iterator();
         tb_cfg_[s] = (tuned && it != tuned->end() && cfg_valid(it->second, nx_[s], ny_[s]))
                          ? it->second
-                         : tb_pick(nx_[s], ny_[s], B);
+                         : tb_pick(nx_[s], ny_[s], B, queue_off_env_);
         for (int c = 0; c < kNumIterCfgs; c++)  // any configuration may run while tuning
             iter_blocks_ = imax(iter_blocks_, tb_tiles(c, nx_[s], ny_[s]) * kTbK);
     }
@@ -2055,9 +2217,6 @@ TvPlan::TvPlan(int w, int h, int B, int dtype, const oflow_tvl1_params &prm, boo
                        cudaMemcpyHostToDevice));
     OF_CUDA(cudaMemset(ar_.at<char>(o_ctrl_), 0, B * sizeof(TvCtrl)));
     OF_CUDA(cudaMemset(ar_.at<char>(o_queue_), 0, B * sizeof(TbQueue)));
-    // OFLOW_TB_QUEUE=0 runs the tiled stages as one launch per block of K
-    // iterations (k_tvl1_tb) instead of the persistent work queue (k_tvl1_q)
-    if (const char *e = getenv("OFLOW_TB_QUEUE")) queue_off_env_ = atoi(e) == 0;
     queue_ = !queue_off_env_;
     // The queue form sizes each block of iterations to end at the stop its
     // error decay predicts and drops the snapshots of a shortened block (2,
@@ -2066,7 +2225,6 @@ TvPlan::TvPlan(int w, int h, int B, int dtype, const oflow_tvl1_params &prm, boo
     if (const char *e = getenv("OFLOW_TB_PREDICT")) predict_ = atoi(e);
     // scales above a warm start's first scale never record a count
     OF_CUDA(cudaMemset(ar_.at<char>(o_iters_), 0, (size_t)B * iter_stride_ * 4));
-    tb_set_smem_attrs();
 }
 
 void TvPlan::bind_frame(int b, int k, const void *p, int pitch) {
