@@ -875,10 +875,38 @@ oflow_status oflow_lk(oflow_ctx *ctx, const oflow_image *frames, int iframe,
             pl = ctx->lk.back().get();
         }
         const cudaStream_t st = ctx->stream();
-        for (int k = 0; k < T; k++) stage_image(frames[k], pl->ring_slot(k), 1, st);
-        pl->run(iframe, st);
-        unstage_plane(pl->out_u(), w, h, out->u, out->pitch, out->location, st);
-        unstage_plane(pl->out_v(), w, h, out->v, out->pitch, out->location, st);
+        // Device frames and flows in place, the others through the plan's buffers;
+        // so are device flows that overlap a frame or start off a float's boundary.
+        FrameRef ring[9];
+        OutRef o{pl->out_u(), pl->out_v(), w};
+        if (out->location == OFLOW_DEVICE) {
+            const long long op = out->pitch ? out->pitch : w;
+            const size_t obytes = ((size_t)op * (h - 1) + w) * sizeof(float);
+            auto apart = [&](const float *f) {
+                const uintptr_t f0 = reinterpret_cast<uintptr_t>(f);
+                bool ok = f0 % alignof(float) == 0;
+                for (int k = 0; k < T; k++) {
+                    const uintptr_t a0 = reinterpret_cast<uintptr_t>(frames[k].data);
+                    const size_t fp = frames[k].pitch ? frames[k].pitch : w;
+                    ok = ok && (f0 + obytes <= a0 || a0 + fp * (h - 1) + w <= f0);
+                }
+                return ok;
+            };
+            if (apart(out->u) && apart(out->v)) o = OutRef{out->u, out->v, op};
+        }
+        for (int k = 0; k < T; k++) {
+            if (frames[k].location == OFLOW_DEVICE) {
+                ring[k] = FrameRef{frames[k].data, frames[k].pitch ? frames[k].pitch : w};
+            } else {
+                stage_image(frames[k], pl->ring_slot(k), 1, st);
+                ring[k] = FrameRef{pl->ring_slot(k), w};
+            }
+        }
+        pl->run(ring, iframe, o, st);
+        if (o.u == pl->out_u()) {
+            unstage_plane(pl->out_u(), w, h, out->u, out->pitch, out->location, st);
+            unstage_plane(pl->out_v(), w, h, out->v, out->pitch, out->location, st);
+        }
         finish(ctx, out->location == OFLOW_DEVICE);
     });
 }

@@ -420,16 +420,30 @@ __device__ __forceinline__ float2 bilinear2(const float2 *__restrict__ src, int 
     return r;
 }
 
+// Two pixels of a row a thread; rx = w/nw and ry = h/nh come from the host
+// (one IEEE division either way).
 __global__ void k_upscale2(const float2 *__restrict__ src, size_t sstride, int w, int h,
-                           float2 *dst, size_t dstride, int nw, int nh, float sx, float sy) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+                           float2 *dst, size_t dstride, int nw, int nh, float sx, float sy, float rx, float ry) {
+    const int x = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= nw || y >= nh) return;
-    const float rx = (float)w / (float)nw, ry = (float)h / (float)nh;
-    const float fx = ((float)x + 0.5f) * rx - 0.5f;
+    const float2 *s = src + (size_t)blockIdx.z * sstride;
+    float2 *d = dst + (size_t)blockIdx.z * dstride + (size_t)y * nw + x;
     const float fy = ((float)y + 0.5f) * ry - 0.5f;
-    const float2 r = bilinear2(src + (size_t)blockIdx.z * sstride, w, h, fx, fy);
-    dst[(size_t)blockIdx.z * dstride + (size_t)y * nw + x] = make_float2(r.x * sx, r.y * sy);
+    const float2 a = bilinear2(s, w, h, ((float)x + 0.5f) * rx - 0.5f, fy);
+    const float2 ra = make_float2(a.x * sx, a.y * sy);
+    if (x + 1 >= nw) {
+        d[0] = ra;
+        return;
+    }
+    const float2 b = bilinear2(s, w, h, ((float)(x + 1) + 0.5f) * rx - 0.5f, fy);
+    const float2 rb = make_float2(b.x * sx, b.y * sy);
+    if (reinterpret_cast<uintptr_t>(d) % 16 == 0) {
+        *reinterpret_cast<float4 *>(d) = make_float4(ra.x, ra.y, rb.x, rb.y);
+    } else {
+        d[0] = ra;
+        d[1] = rb;
+    }
 }
 
 __global__ void k_split2(const float2 *__restrict__ U, size_t stride, int N, float *ou, float *ov,
@@ -445,8 +459,9 @@ __global__ void k_split2(const float2 *__restrict__ U, size_t stride, int N, flo
 void launch_upscale2(const float2 *src, size_t sstride, int w, int h, float2 *dst,
                      size_t dstride, int nw, int nh, float sx, float sy, int B,
                      cudaStream_t st) {
-    dim3 blk(32, 8), g(div_up(nw, 32), div_up(nh, 8), B);
-    k_upscale2<<<g, blk, 0, st>>>(src, sstride, w, h, dst, dstride, nw, nh, sx, sy);
+    dim3 blk(32, 8), g(div_up(nw, 64), div_up(nh, 8), B);
+    k_upscale2<<<g, blk, 0, st>>>(src, sstride, w, h, dst, dstride, nw, nh, sx, sy, (float)w / (float)nw,
+                                  (float)h / (float)nh);
 }
 
 // Each thread converts four consecutive pixels of a row; rows whose source and destination allow it move them as one vector.

@@ -15,8 +15,8 @@
 
 namespace oflow {
 
-constexpr int kLTW = 32, kLTH = 8, kLNT = kLTW * kLTH;
-constexpr int kLMaxC = 4, kLMaxF = 4, kLMaxT = 9;
+constexpr int kLTile = 32;  // pixels a side of a block's tile
+constexpr int kLMaxC = 4, kLMaxT = 9;
 
 struct LkTaps {
     float fs[9];
@@ -46,81 +46,163 @@ int lk_taps(int spac, int temp, float *fs, float *ft) {
     return 0;
 }
 
-// Window sums in the reference order and the closed-form 2x2 solve
-// (kernels.cu:150-179).  gx/gy/gt: region planes of width RW.
-__device__ __forceinline__ void lk_window_solve(const float *gx, const float *gy, const float *gt,
-                                                int RW, int cidx, int c, float &vx, float &vy) {
-    float sxx = 0.0f, sxy = 0.0f, syy = 0.0f, sxt = 0.0f, syt = 0.0f;
-    for (int ii = -c; ii <= c; ii++) {
-        const int row = cidx + ii * RW;
-        for (int jj = -c; jj <= c; jj++) {
-            const int q = row + jj;
-            const float ix = gx[q], iy = gy[q], it = gt[q];
-            sxx += ix * ix;
-            sxy += ix * iy;
-            syy += iy * iy;
-            sxt += ix * it;
-            syt += iy * it;
+// Window sums and the closed-form 2x2 solve (kernels.cu:150-179) of 2 x PY
+// pixels: two columns from col (even), rows of centres from row.  gx/gy/gt are
+// region planes of RW columns in shared memory, the window of pixel (0, 0)
+// starting at (row, col).  Each window element is loaded and its five products
+// formed once for all pixels whose window holds it; each pixel still adds them
+// in the reference's row-major order.
+//
+// The additions are 5 (2C+1)^2 a pixel and cannot be shared (a prefix sum or a
+// separable box would round differently); eight pixels a thread leave 30
+// multiplications and 9 shared loads a pixel at C = 2, where four in one column
+// took 50 and 30.
+template <int C, int PY>
+__device__ __forceinline__ void lk_window_solve(const float *gx, const float *gy, const float *gt, int RW,
+                                                int row, int col, float (&vx)[PY][2], float (&vy)[PY][2]) {
+    float sxx[PY][2], sxy[PY][2], syy[PY][2], sxt[PY][2], syt[PY][2];
+#pragma unroll
+    for (int k = 0; k < PY; k++)
+#pragma unroll
+        for (int m = 0; m < 2; m++) sxx[k][m] = sxy[k][m] = syy[k][m] = sxt[k][m] = syt[k][m] = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 2 * C + PY; r++) {
+        const int at = (row + r) * RW + col;
+        float ix[2 * C + 2], iy[2 * C + 2], it[2 * C + 2];
+#pragma unroll
+        for (int j = 0; j < C + 1; j++) {
+            const float2 a = *reinterpret_cast<const float2 *>(gx + at + 2 * j);
+            const float2 b = *reinterpret_cast<const float2 *>(gy + at + 2 * j);
+            const float2 t = *reinterpret_cast<const float2 *>(gt + at + 2 * j);
+            ix[2 * j] = a.x; ix[2 * j + 1] = a.y;
+            iy[2 * j] = b.x; iy[2 * j + 1] = b.y;
+            it[2 * j] = t.x; it[2 * j + 1] = t.y;
+        }
+#pragma unroll
+        for (int j = 0; j < 2 * C + 2; j++) {
+            const float pxx = ix[j] * ix[j], pxy = ix[j] * iy[j], pyy = iy[j] * iy[j], pxt = ix[j] * it[j],
+                        pyt = iy[j] * it[j];
+#pragma unroll
+            for (int k = 0; k < PY; k++)
+#pragma unroll
+                for (int m = 0; m < 2; m++)
+                    if (r - k >= 0 && r - k <= 2 * C && j - m >= 0 && j - m <= 2 * C) {
+                        sxx[k][m] += pxx;
+                        sxy[k][m] += pxy;
+                        syy[k][m] += pyy;
+                        sxt[k][m] += pxt;
+                        syt[k][m] += pyt;
+                    }
         }
     }
-    const float det = (sxx * syy - sxy * sxy);
-    vx = 0.0f;
-    vy = 0.0f;
-    if (det != 0.0f) {
-        vx = 1.0f / det * (syy * (-sxt) + (-sxy) * (-syt));
-        vy = 1.0f / det * ((-sxy) * (-sxt) + sxx * (-syt));
-    }
+#pragma unroll
+    for (int k = 0; k < PY; k++)
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const float det = (sxx[k][m] * syy[k][m] - sxy[k][m] * sxy[k][m]);
+            vx[k][m] = 0.0f;
+            vy[k][m] = 0.0f;
+            if (det != 0.0f) {
+                const float inv = 1.0f / det;
+                vx[k][m] = inv * (syy[k][m] * (-sxt[k][m]) + (-sxy[k][m]) * (-syt[k][m]));
+                vy[k][m] = inv * ((-sxy[k][m]) * (-sxt[k][m]) + sxx[k][m] * (-syt[k][m]));
+            }
+        }
 }
 
-// Single step over a ring of T uint8 frames (slot k at ring + k*N); the newest
-// frame is in slot iframe % T.  One kernel: spatial FIR of the oldest frame,
-// temporal FIR over the ring, window sums and solve.  Pixels closer than the
-// window radius to the border get 0.
-__global__ void __launch_bounds__(kLNT) k_lk_step(const uint8_t *__restrict__ ring, int T,
-                                                  int iframe, int nx, int ny, const __grid_constant__ LkTaps taps,
-                                                  int c, float *Vx, float *Vy) {
-    constexpr int RWm = kLTW + 2 * kLMaxC, RHm = kLTH + 2 * kLMaxC;
-    constexpr int FWm = RWm + 2 * kLMaxF, FHm = RHm + 2 * kLMaxF;
-    __shared__ float sf[FWm * FHm];
-    __shared__ float gx[RWm * RHm], gy[RWm * RHm], gt[RWm * RHm];
-    const int fc = (taps.ns - 1) / 2;
-    const int RW = kLTW + 2 * c, RH = kLTH + 2 * c;
-    const int FW = RW + 2 * fc, FH = RH + 2 * fc;
-    const size_t N = (size_t)nx * ny;
-    const uint8_t *old = ring + (size_t)((iframe + 1) % T) * N;
-    const int fx0 = blockIdx.x * kLTW - c - fc, fy0 = blockIdx.y * kLTH - c - fc;
-    for (int i = threadIdx.x; i < FW * FH; i += kLNT) {
-        const int x = fx0 + i % FW, y = fy0 + i / FW;
-        sf[i] = (x >= 0 && x < nx && y >= 0 && y < ny) ? (float)old[(size_t)y * nx + x] : 0.0f;
-    }
+// Visits the RW x RH region with NT threads, rows by warps, without divisions
+// for the first 32 columns.
+template <int NT, int RW, int RH, typename F> __device__ __forceinline__ void for_region(F &&f) {
+    constexpr int NWARP = NT / 32, X = RW - 32;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll 4
+    for (int ry = wid; ry < RH; ry += NWARP) f(lane, ry);
+    if (X > 0)
+        for (int i = threadIdx.x; i < X * RH; i += NT) f(32 + i % imax(X, 1), i / imax(X, 1));
+}
+
+// Single step over T uint8 frames in temporal order (src[0] the oldest), read
+// where they lie.  One kernel: spatial FIR of the oldest frame, temporal FIR,
+// window sums and solve.  Pixels closer than the window radius to the border
+// get 0.  The five frames of a 1280x720 step used to be copied into the plan and
+// the flow out of it (31 of 96 us), and the sums ran one pixel a thread (65 us);
+// with eight pixels a thread the whole step takes 28 us.
+struct LkStep {
+    const uint8_t *src[kLMaxT];
+    long long pitch[kLMaxT];
+    int T, nx, ny;
+    LkTaps taps;
+    float *u, *v;
+    long long out_pitch;
+};
+template <int C, int NS, int PY>
+__global__ void __launch_bounds__(kLTile *kLTile / (2 * PY)) k_lk_step(const __grid_constant__ LkStep a) {
+    constexpr int NT = kLTile * kLTile / (2 * PY), F = (NS - 1) / 2;
+    constexpr int RW = kLTile + 2 * C, FW = RW + 2 * F;
+    __shared__ float sf[FW * FW];
+    __shared__ __align__(8) float gx[RW * RW], gy[RW * RW], gt[RW * RW];
+    const int nx = a.nx, ny = a.ny;
+    const int x0 = blockIdx.x * kLTile - C, y0 = blockIdx.y * kLTile - C;
+    const uint8_t *old = a.src[0];
+    for_region<NT, FW, FW>([&](int rx, int ry) {
+        const int x = x0 - F + rx, y = y0 - F + ry;
+        sf[ry * FW + rx] = (x >= 0 && x < nx && y >= 0 && y < ny) ? (float)__ldg(old + (size_t)y * a.pitch[0] + x) : 0.0f;
+    });
     __syncthreads();
-    for (int i = threadIdx.x; i < RW * RH; i += kLNT) {
-        const int rx = i % RW, ry = i / RW;
-        const int x = fx0 + fc + rx, y = fy0 + fc + ry;
-        if (x < 0 || x >= nx || y < 0 || y >= ny) continue;
-        const float *f = sf + (ry + fc) * FW + (rx + fc);
+    for_region<NT, RW, RW>([&](int rx, int ry) {
+        const int x = x0 + rx, y = y0 + ry;
+        if (x < 0 || x >= nx || y < 0 || y >= ny) {
+            // read only by the sums of border pixels, whose results are not used
+            gx[ry * RW + rx] = gy[ry * RW + rx] = gt[ry * RW + rx] = 0.0f;
+            return;
+        }
+        const float *f = sf + (ry + F) * FW + rx + F;
         float ax = 0.0f, ay = 0.0f;
-        for (int k = 0; k < taps.ns; k++) {
-            const int xx = x + k - fc, yy = y + k - fc;
-            if (xx >= 0 && xx < nx) ax += f[k - fc] * taps.fs[k];
-            if (yy >= 0 && yy < ny) ay += f[(k - fc) * FW] * taps.fs[k];
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            const int xx = x + k - F, yy = y + k - F;
+            if (xx >= 0 && xx < nx) ax += f[k - F] * a.taps.fs[k];
+            if (yy >= 0 && yy < ny) ay += f[(k - F) * FW] * a.taps.fs[k];
         }
         float at = 0.0f;
-        for (int fr = 0; fr < T; fr++)
-            at += taps.ft[fr] * (float)ring[(size_t)((fr + iframe + 1) % T) * N + (size_t)y * nx + x];
-        gx[i] = ax;
-        gy[i] = ay;
-        gt[i] = at;
-    }
+        for (int k = 0; k < a.T; k++) at += a.taps.ft[k] * (float)__ldg(a.src[k] + (size_t)y * a.pitch[k] + x);
+        gx[ry * RW + rx] = ax;
+        gy[ry * RW + rx] = ay;
+        gt[ry * RW + rx] = at;
+    });
     __syncthreads();
-    const int x = blockIdx.x * kLTW + threadIdx.x % kLTW, y = blockIdx.y * kLTH + threadIdx.x / kLTW;
-    if (x >= nx || y >= ny) return;
-    float vx = 0.0f, vy = 0.0f;
-    if (x >= c && y >= c && x < nx - c && y < ny - c)
-        lk_window_solve(gx, gy, gt, RW, (threadIdx.x / kLTW + c) * RW + threadIdx.x % kLTW + c, c,
-                        vx, vy);
-    Vx[(size_t)y * nx + x] = vx;
-    Vy[(size_t)y * nx + x] = vy;
+    const int tx = 2 * (threadIdx.x % (kLTile / 2)), ty = (threadIdx.x / (kLTile / 2)) * PY;
+    const int x = blockIdx.x * kLTile + tx, yb = blockIdx.y * kLTile + ty;
+    if (x >= nx || yb >= ny) return;
+    float dx[PY][2], dy[PY][2];
+    lk_window_solve<C, PY>(gx, gy, gt, RW, ty, tx, dx, dy);
+#pragma unroll
+    for (int k = 0; k < PY; k++)
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const int xx = x + m, y = yb + k;
+            if (xx >= nx || y >= ny) continue;
+            const bool in = xx >= C && y >= C && xx < nx - C && y < ny - C;
+            a.u[(size_t)y * a.out_pitch + xx] = in ? dx[k][m] : 0.0f;
+            a.v[(size_t)y * a.out_pitch + xx] = in ? dy[k][m] : 0.0f;
+        }
+}
+
+template <int C, int NS> static void lk_step_launch(const LkStep &a, cudaStream_t st) {
+    const dim3 g(div_up(a.nx, kLTile), div_up(a.ny, kLTile));
+    if ((size_t)g.x * g.y > 4 * (size_t)kNumSMs)
+        k_lk_step<C, NS, 4><<<g, kLTile * kLTile / 8, 0, st>>>(a);
+    else
+        k_lk_step<C, NS, 1><<<g, kLTile * kLTile / 2, 0, st>>>(a);
+}
+template <int C> static void lk_step_launch_c(const LkStep &a, cudaStream_t st) {
+    switch (a.taps.ns) {
+        case 1: lk_step_launch<C, 1>(a, st); break;
+        case 3: lk_step_launch<C, 3>(a, st); break;
+        case 5: lk_step_launch<C, 5>(a, st); break;
+        case 7: lk_step_launch<C, 7>(a, st); break;
+        default: lk_step_launch<C, 9>(a, st); break;
+    }
 }
 
 // Spatial FIR (zero padding by dropped taps) of a float plane -> float2 (Ix, Iy),
@@ -153,8 +235,62 @@ __global__ void k_lk_grad(const float *__restrict__ src, size_t sstride, int nx,
     G[(size_t)blockIdx.z * gstride + (size_t)y * nx + x] = make_float2(ax, ay);
 }
 
+// The same for rows of whole aligned quads: four pixels a thread, the vertical
+// taps and the results as vectors (64 pairs of 640x480 and two coarser levels:
+// 109 -> 67 us).  Quads whose taps leave the image take k_lk_grad's sums.
+template <int NS>
+__global__ void k_lk_grad4(const float *__restrict__ src, size_t sstride, int nx, int ny,
+                           const __grid_constant__ LkTaps taps, float2 *G, size_t gstride) {
+    constexpr int FC = (NS - 1) / 2;
+    const int x = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int y = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= nx || y >= ny) return;
+    const float *f = src + (size_t)blockIdx.z * sstride;
+    float ax[4] = {0.0f, 0.0f, 0.0f, 0.0f}, ay[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (x >= FC && x + 3 < nx - FC && y >= FC && y < ny - FC) {
+        const float *row = f + (size_t)y * nx + x - FC, *col = f + (size_t)(y - FC) * nx + x;
+        float r[4 + 2 * FC];
+#pragma unroll
+        for (int k = 0; k < 4 + 2 * FC; k++) r[k] = __ldg(row + k);
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            const float4 c = __ldg(reinterpret_cast<const float4 *>(col + (size_t)k * nx));
+            const float cc[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                ax[m] += r[m + k] * taps.fs[k];
+                ay[m] += cc[m] * taps.fs[k];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+            for (int k = 0; k < NS; k++) {
+                const int xx = x + m + k - FC, yy = y + k - FC;
+                if (xx >= 0 && xx < nx) ax[m] += __ldg(f + (size_t)y * nx + xx) * taps.fs[k];
+                if (yy >= 0 && yy < ny) ay[m] += __ldg(f + (size_t)yy * nx + x + m) * taps.fs[k];
+            }
+    }
+    float4 *o = reinterpret_cast<float4 *>(G + (size_t)blockIdx.z * gstride + (size_t)y * nx + x);
+    o[0] = make_float4(ax[0], ay[0], ax[1], ay[1]);
+    o[1] = make_float4(ax[2], ay[2], ax[3], ay[3]);
+}
+
 static void launch_lk_grad(dim3 g, dim3 blk, cudaStream_t st, const float *src, size_t sstride,
                            int nx, int ny, const LkTaps &taps, float2 *G, size_t gstride) {
+    // planes start at multiples of sstride / gstride elements of 256-byte aligned buffers
+    if (nx % 4 == 0 && sstride % 4 == 0 && gstride % 2 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0) {
+        const dim3 g4(div_up(nx, 32 * 4), g.y, g.z);
+        switch (taps.ns) {
+            case 1: k_lk_grad4<1><<<g4, blk, 0, st>>>(src, sstride, nx, ny, taps, G, gstride); break;
+            case 3: k_lk_grad4<3><<<g4, blk, 0, st>>>(src, sstride, nx, ny, taps, G, gstride); break;
+            case 5: k_lk_grad4<5><<<g4, blk, 0, st>>>(src, sstride, nx, ny, taps, G, gstride); break;
+            case 7: k_lk_grad4<7><<<g4, blk, 0, st>>>(src, sstride, nx, ny, taps, G, gstride); break;
+            default: k_lk_grad4<9><<<g4, blk, 0, st>>>(src, sstride, nx, ny, taps, G, gstride); break;
+        }
+        return;
+    }
     switch (taps.ns) {
         case 1: k_lk_grad<1><<<g, blk, 0, st>>>(src, sstride, nx, ny, taps, G, gstride); break;
         case 3: k_lk_grad<3><<<g, blk, 0, st>>>(src, sstride, nx, ny, taps, G, gstride); break;
@@ -164,118 +300,152 @@ static void launch_lk_grad(dim3 g, dim3 blk, cudaStream_t st, const float *src, 
     }
 }
 
-// Window sums and the 2x2 solve of P vertically adjacent pixels (column cidx,
-// rows of centres crow .. crow+P-1 in shared memory): each window element is
-// loaded and its five products formed once for every pixel whose window holds
-// it; each pixel still adds them in the reference's row-major order
-// (kernels.cu:150-179), so its sums are those of lk_window_solve.
-template <int C, int P>
-__device__ __forceinline__ void lk_window_solve_p(const float *gx, const float *gy, const float *gt,
-                                                  int RW, int top, float (&vx)[P], float (&vy)[P]) {
-    float sxx[P], sxy[P], syy[P], sxt[P], syt[P];
+// It, Ix, Iy of up to M pixels of a region into its shared planes: the flows of
+// all of them are loaded first, then all their samples of I1 (bilinear,
+// clamp-to-edge; the few whose taps leave the image go through
+// bilinear_clamped afterwards), so that a thread's gathers are in flight
+// together.  on[m] false: no such pixel.
+template <int M>
+__device__ __forceinline__ void lk_warp_pixels(const int (&rx)[M], const int (&ry)[M], const bool (&on)[M], int x0, int y0,
+                                               int RW, const float *__restrict__ I0, const float *__restrict__ I1,
+                                               const float2 *__restrict__ G, const float2 *__restrict__ U, int nx,
+                                               int ny, float *gx, float *gy, float *gt) {
+    int q[M], base[M];
+    bool in[M], easy[M];
+    float2 u[M], g[M];
+    float i0[M], xf[M], yf[M], v00[M], v10[M], v01[M], v11[M];
 #pragma unroll
-    for (int k = 0; k < P; k++) sxx[k] = sxy[k] = syy[k] = sxt[k] = syt[k] = 0.0f;
-#pragma unroll
-    for (int r = 0; r < 2 * C + P; r++) {
-        const int row = top + r * RW;
-#pragma unroll
-        for (int jj = 0; jj <= 2 * C; jj++) {
-            const float ix = gx[row + jj], iy = gy[row + jj], it = gt[row + jj];
-            const float pxx = ix * ix, pxy = ix * iy, pyy = iy * iy, pxt = ix * it, pyt = iy * it;
-#pragma unroll
-            for (int k = 0; k < P; k++)
-                if (r - k >= 0 && r - k <= 2 * C) {
-                    sxx[k] += pxx;
-                    sxy[k] += pxy;
-                    syy[k] += pyy;
-                    sxt[k] += pxt;
-                    syt[k] += pyt;
-                }
-        }
+    for (int m = 0; m < M; m++) {
+        const int x = x0 + rx[m], y = y0 + ry[m];
+        in[m] = on[m] && x >= 0 && x < nx && y >= 0 && y < ny;
+        q[m] = in[m] ? y * nx + x : 0;
+        u[m] = U[q[m]];
+        xf[m] = (float)x;
+        yf[m] = (float)y;
     }
 #pragma unroll
-    for (int k = 0; k < P; k++) {
-        const float det = (sxx[k] * syy[k] - sxy[k] * sxy[k]);
-        vx[k] = 0.0f;
-        vy[k] = 0.0f;
-        if (det != 0.0f) {
-            vx[k] = 1.0f / det * (syy[k] * (-sxt[k]) + (-sxy[k]) * (-syt[k]));
-            vy[k] = 1.0f / det * ((-sxy[k]) * (-sxt[k]) + sxx[k] * (-syt[k]));
+    for (int m = 0; m < M; m++) {
+        g[m] = G[q[m]];
+        i0[m] = __ldg(I0 + q[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        xf[m] += u[m].x;
+        yf[m] += u[m].y;
+        easy[m] = xf[m] >= 0.0f && yf[m] >= 0.0f && xf[m] < (float)(nx - 1) && yf[m] < (float)(ny - 1);
+        base[m] = easy[m] ? (int)yf[m] * nx + (int)xf[m] : 0;  // (nonnegative: truncation is floor)
+        const float *p = I1 + base[m];
+        v00[m] = __ldg(p);
+        v10[m] = __ldg(p + 1);
+        v01[m] = __ldg(p + nx);
+        v11[m] = __ldg(p + nx + 1);
+    }
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        const float fx = xf[m] - (float)(int)xf[m], fy = yf[m] - (float)(int)yf[m];
+        const float ex = 1.0f - fx, ey = 1.0f - fy;
+        const float top = ex * v00[m] + fx * v10[m];
+        const float bot = ex * v01[m] + fx * v11[m];
+        float w = ey * top + fy * bot;
+        if (!easy[m]) w = bilinear_clamped(I1, nx, ny, xf[m], yf[m]);
+        float it = 0.0f;
+        it += -1.0f * i0[m];
+        it += 1.0f * w;
+        if (on[m]) {
+            // outside the image: read only by the sums of border pixels, whose results are not used
+            const int i = ry[m] * RW + rx[m];
+            gx[i] = in[m] ? g[m].x : 0.0f;
+            gy[i] = in[m] ? g[m].y : 0.0f;
+            gt[i] = in[m] ? it : 0.0f;
         }
     }
 }
 
 // One refinement of pyramidal LK: warp I1 by the current flow (bilinear,
 // clamp-to-edge), It = 0 + (-1)*I0 + 1*I1w, window solve, Uout = Uin + d.
-// Tile 32 x kPTH with the window radius C as halo; a thread solves PP
-// vertically adjacent pixels (lk_window_solve_p): 4 when a launch has tiles
-// enough to fill the GPU (the elements of eight window rows loaded and
-// multiplied once for four pixels: 29.0k against 28.0k pairs/s on 64 pairs of
-// 640x480), else 2 (twice the threads: 9.7k against 9.2k pairs/s for one
-// pair).  (Window sums read from precomputed product planes measured slower:
-// 18.2k against 21.4k pairs/s batched; five loads per window element instead
-// of three bound the LSU pipe.)
-constexpr int kPTW = 32, kPTH = 32;
-template <int C, int PP>
-__global__ void __launch_bounds__(kPTW * kPTH / PP) k_pyrlk_iter(const float *__restrict__ pyr, size_t lp,
-                                                                 const float2 *__restrict__ G, size_t gstride,
-                                                                 const float2 *__restrict__ Uin,
-                                                                 float2 *Uout, size_t ustride, int nx,
-                                                                 int ny) {
-    constexpr int kPNT = kPTW * kPTH / PP;
-    constexpr int RW = kPTW + 2 * C, RH = kPTH + 2 * C;
-    __shared__ float gx[RW * RH], gy[RW * RH], gt[RW * RH];
+// Tile 32 x 32 with the window radius C as halo; a thread solves two columns of
+// PY rows (lk_window_solve): 4 when a launch has tiles enough to fill the GPU,
+// else 1 (four times the threads).  64 pairs of 640x480, three levels of three
+// refinements at C = 2: 1.05 ms of launches (1.24 with one pixel a thread and
+// its gathers one after the other); issue slots 79 % used, the additions bound it.
+template <int C, int PY>
+__global__ void __launch_bounds__(kLTile *kLTile / (2 * PY)) k_pyrlk_iter(
+    const float *__restrict__ pyr, size_t lp, const float2 *__restrict__ G, size_t gstride,
+    const float2 *__restrict__ Uin, float2 *Uout, size_t ustride, int nx, int ny,
+    const OutRef *__restrict__ outs) {
+    constexpr int NT = kLTile * kLTile / (2 * PY), RW = kLTile + 2 * C;
+    __shared__ __align__(8) float gx[RW * RW], gy[RW * RW], gt[RW * RW];
     const int b = blockIdx.z;
     const float *I0 = pyr + (size_t)(2 * b) * lp;
     const float *I1 = pyr + (size_t)(2 * b + 1) * lp;
     const float2 *Gb = G + (size_t)b * gstride;
     const float2 *Ub = Uin + (size_t)b * ustride;
-    const int x0 = blockIdx.x * kPTW - C, y0 = blockIdx.y * kPTH - C;
-    for (int i = threadIdx.x; i < RW * RH; i += kPNT) {
-        const int x = x0 + i % RW, y = y0 + i / RW;
-        if (x < 0 || x >= nx || y < 0 || y >= ny) {
-            // read only by the sums of border pixels, whose results are not used
-            gx[i] = gy[i] = gt[i] = 0.0f;
-            continue;
+    const int x0 = blockIdx.x * kLTile - C, y0 = blockIdx.y * kLTile - C;
+    {
+        // rows by warps, three at a time, then the columns beyond the 32nd
+        constexpr int M = 3, NWARP = NT / 32, X = RW - 32;
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        int rx[M], ry[M];
+        bool on[M];
+#pragma unroll 1
+        for (int r = wid; r < RW; r += M * NWARP) {
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                rx[m] = lane;
+                ry[m] = r + m * NWARP;
+                on[m] = ry[m] < RW;
+            }
+            lk_warp_pixels<M>(rx, ry, on, x0, y0, RW, I0, I1, Gb, Ub, nx, ny, gx, gy, gt);
         }
-        const size_t p = (size_t)y * nx + x;
-        const float2 u = Ub[p];
-        const float w = bilinear_clamped(I1, nx, ny, (float)x + u.x, (float)y + u.y);
-        float it = 0.0f;
-        it += -1.0f * __ldg(I0 + p);
-        it += 1.0f * w;
-        const float2 g = Gb[p];
-        gx[i] = g.x;
-        gy[i] = g.y;
-        gt[i] = it;
+        if (X > 0)
+#pragma unroll 1
+            for (int i = threadIdx.x; i < X * RW; i += M * NT) {
+#pragma unroll
+                for (int m = 0; m < M; m++) {
+                    const int k = i + m * NT;
+                    on[m] = k < X * RW;
+                    rx[m] = 32 + k % imax(X, 1);
+                    ry[m] = k / imax(X, 1);
+                }
+                lk_warp_pixels<M>(rx, ry, on, x0, y0, RW, I0, I1, Gb, Ub, nx, ny, gx, gy, gt);
+            }
     }
     __syncthreads();
-    const int tx = threadIdx.x % kPTW, ty = (threadIdx.x / kPTW) * PP;
-    const int x = blockIdx.x * kPTW + tx, yb = blockIdx.y * kPTH + ty;
+    const int tx = 2 * (threadIdx.x % (kLTile / 2)), ty = (threadIdx.x / (kLTile / 2)) * PY;
+    const int x = blockIdx.x * kLTile + tx, yb = blockIdx.y * kLTile + ty;
     if (x >= nx || yb >= ny) return;
-    float dx[PP], dy[PP];
-    // top-left of the first pixel's window: row ty, column tx of the region
-    lk_window_solve_p<C, PP>(gx, gy, gt, RW, ty * RW + tx, dx, dy);
+    float dx[PY][2], dy[PY][2];
+    lk_window_solve<C, PY>(gx, gy, gt, RW, ty, tx, dx, dy);
+    OutRef o{nullptr, nullptr, 0};
+    if (outs) o = outs[b];
 #pragma unroll
-    for (int k = 0; k < PP; k++) {
-        const int y = yb + k;
-        if (y >= ny) break;
-        const bool in = x >= C && y >= C && x < nx - C && y < ny - C;
-        const size_t q = (size_t)y * nx + x;
-        const float2 u = Ub[q];
-        Uout[(size_t)b * ustride + q] = make_float2(u.x + (in ? dx[k] : 0.0f), u.y + (in ? dy[k] : 0.0f));
-    }
+    for (int k = 0; k < PY; k++)
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const int xx = x + m, y = yb + k;
+            if (xx >= nx || y >= ny) continue;
+            const bool in = xx >= C && y >= C && xx < nx - C && y < ny - C;
+            const size_t q = (size_t)y * nx + xx;
+            const float2 u = Ub[q];
+            const float2 r = make_float2(u.x + (in ? dx[k][m] : 0.0f), u.y + (in ? dy[k][m] : 0.0f));
+            if (outs) {  // the solve's last refinement writes the caller's planes
+                o.u[(size_t)y * o.pitch + xx] = r.x;
+                o.v[(size_t)y * o.pitch + xx] = r.y;
+            } else {
+                Uout[(size_t)b * ustride + q] = r;
+            }
+        }
 }
 
 static void launch_pyrlk_iter(int c, dim3 g, cudaStream_t st, const float *pyr, size_t lp,
                               const float2 *G, size_t gstride, const float2 *Uin, float2 *Uout,
-                              size_t ustride, int nx, int ny) {
+                              size_t ustride, int nx, int ny, const OutRef *outs) {
     const bool wide = (size_t)g.x * g.y * g.z > 4 * (size_t)kNumSMs;
 #define OF_PYRLK(C)                                                                                  \
     if (wide)                                                                                        \
-        k_pyrlk_iter<C, 4><<<g, kPTW * kPTH / 4, 0, st>>>(pyr, lp, G, gstride, Uin, Uout, ustride, nx, ny); \
+        k_pyrlk_iter<C, 4><<<g, kLTile * kLTile / 8, 0, st>>>(pyr, lp, G, gstride, Uin, Uout, ustride, nx, ny, outs); \
     else                                                                                             \
-        k_pyrlk_iter<C, 2><<<g, kPTW * kPTH / 2, 0, st>>>(pyr, lp, G, gstride, Uin, Uout, ustride, nx, ny);
+        k_pyrlk_iter<C, 1><<<g, kLTile * kLTile / 2, 0, st>>>(pyr, lp, G, gstride, Uin, Uout, ustride, nx, ny, outs);
     switch (c) {
         case 0: OF_PYRLK(0) break;
         case 1: OF_PYRLK(1) break;
@@ -309,15 +479,30 @@ LkPlan::LkPlan(int w, int h, const oflow_lk_params &prm) : w_(w), h_(h), prm_(pr
 }
 
 uint8_t *LkPlan::ring_slot(int k) const { return ar_.at<uint8_t>(o_ring_) + (size_t)k * N_; }
-const float *LkPlan::out_u() const { return ar_.at<float>(o_out_); }
-const float *LkPlan::out_v() const { return ar_.at<float>(o_out_) + N_; }
+float *LkPlan::out_u() const { return ar_.at<float>(o_out_); }
+float *LkPlan::out_v() const { return ar_.at<float>(o_out_) + N_; }
 
-void LkPlan::run(int iframe, cudaStream_t st) {
-    const LkTaps taps = make_lk_taps(prm_.spac, prm_.temp);
-    dim3 g(div_up(w_, kLTW), div_up(h_, kLTH));
-    float *o = ar_.at<float>(o_out_);
-    k_lk_step<<<g, kLNT, 0, st>>>(ar_.at<uint8_t>(o_ring_), prm_.temp, iframe, w_, h_, taps,
-                                  (prm_.window - 1) / 2, o, o + N_);
+void LkPlan::run(const FrameRef *ring, int iframe, const OutRef &out, cudaStream_t st) {
+    LkStep a{};
+    a.T = prm_.temp;
+    for (int k = 0; k < a.T; k++) {  // temporal order: the slot after the newest frame's is the oldest
+        const FrameRef &f = ring[(k + iframe + 1) % a.T];
+        a.src[k] = static_cast<const uint8_t *>(f.p);
+        a.pitch[k] = f.pitch;
+    }
+    a.nx = w_;
+    a.ny = h_;
+    a.taps = make_lk_taps(prm_.spac, prm_.temp);
+    a.u = out.u;
+    a.v = out.v;
+    a.out_pitch = out.pitch;
+    switch ((prm_.window - 1) / 2) {
+        case 0: lk_step_launch_c<0>(a, st); break;
+        case 1: lk_step_launch_c<1>(a, st); break;
+        case 2: lk_step_launch_c<2>(a, st); break;
+        case 3: lk_step_launch_c<3>(a, st); break;
+        default: lk_step_launch_c<4>(a, st); break;
+    }
     OF_CUDA(cudaGetLastError());
 }
 
@@ -404,9 +589,11 @@ void PyrLkPlan::record(cudaStream_t st) {
         dim3 blk(32, 8), g(div_up(lw, 32), div_up(lh, 8), B);
         // Ix, Iy of I0: plane 2b of the level, so a stride of two planes
         launch_lk_grad(g, blk, st, pyr + pyr_off_[l], 2 * lp, lw, lh, taps, G, N_);
-        dim3 ig(div_up(lw, kPTW), div_up(lh, kPTH), B);
+        dim3 ig(div_up(lw, kLTile), div_up(lh, kLTile), B);
         for (int r = 0; r < prm_.iters; r++) {
-            launch_pyrlk_iter(c, ig, st, pyr + pyr_off_[l], lp, G, N_, U[cur], U[cur ^ 1], N_, lw, lh);
+            const bool end = l == 0 && r + 1 == prm_.iters;
+            launch_pyrlk_iter(c, ig, st, pyr + pyr_off_[l], lp, G, N_, U[cur], U[cur ^ 1], N_, lw, lh,
+                              end ? io_.outs() : nullptr);
             cur ^= 1;
         }
         if (l > 0) {
@@ -416,7 +603,7 @@ void PyrLkPlan::record(cudaStream_t st) {
             cur ^= 1;
         }
     }
-    launch_split_tab(U[cur], N_, w_, h_, io_.outs(), B, st);
+    if (prm_.iters == 0) launch_split_tab(U[cur], N_, w_, h_, io_.outs(), B, st);
     OF_CUDA(cudaGetLastError());
 }
 

@@ -14,9 +14,11 @@ class LkPlan {
   public:
     LkPlan(int w, int h, const oflow_lk_params &prm);
     uint8_t *ring_slot(int k) const;  // dense w*h uint8 plane of ring slot k
-    const float *out_u() const;
-    const float *out_v() const;
-    void run(int iframe, cudaStream_t st);
+    float *out_u() const;
+    float *out_v() const;
+    // ring: the slots' frames (device, uint8, pitch in bytes), the newest in
+    // slot iframe % temp; out: where the flow goes (device)
+    void run(const FrameRef *ring, int iframe, const OutRef &out, cudaStream_t st);
     int width() const { return w_; }
     int height() const { return h_; }
     const oflow_lk_params &params() const { return prm_; }
