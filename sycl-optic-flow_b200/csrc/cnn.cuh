@@ -32,13 +32,30 @@ inline int conv_out(int n, int stride) { return stride == 1 ? n : (n + 1) / 2; }
 
 // forward: x bf16 [N,H,W,C], w bf16 [K,3,3,C], bias f32 [K] -> y [N,P,Q,K]
 // (bf16, or f32 when y_f32); relu applies max(0, .).  With err (a device int)
-// the tcgen05 kernel runs where the shape allows (C % 16 == 0, K <= 128) and
-// sets *err if one of its bounded waits gave up; otherwise, and without err,
-// the mma.sync kernel runs.
+// the tcgen05 kernel runs where the shape allows (C % 16 == 0, K <= 128) on the
+// packed weights and sets *err if one of its bounded waits gave up; otherwise,
+// and without err, the mma.sync kernel runs.
 void conv_forward(const ConvDims &d, const __nv_bfloat16 *x, const __nv_bfloat16 *w,
                   const float *bias, void *y, bool y_f32, bool relu, cudaStream_t st,
-                  int *err = nullptr);
-// the tcgen05 form alone; false (nothing launched) when the shape is outside it.
+                  int *err = nullptr, const __nv_bfloat16 *packed = nullptr);
+// Weights packed for the tcgen05 kernels (16-byte aligned; conv_packed_size
+// elements for either direction with C % 16 == 0): several layers in one launch.
+struct ConvPack {
+    struct Job {
+        const __nv_bfloat16 *w;  // [K][3][3][C], 16-byte aligned
+        __nv_bfloat16 *dst;
+        int K, C, backward;      // backward: for the backward-data product
+    };
+    int n = 0;
+    Job job[20];
+    void add(const __nv_bfloat16 *w, __nv_bfloat16 *dst, int K, int C, bool backward) {
+        job[n++] = Job{w, dst, K, C, backward ? 1 : 0};
+    }
+};
+size_t conv_packed_size(int K, int C);
+void conv_pack_weights(const ConvPack &a, cudaStream_t st);
+// the tcgen05 form alone, on packed weights; false (nothing launched) when the
+// shape is outside it.
 // ldy: elements between output rows (0: K); accumulate: y += (f32 output
 // only); bias may be null.  A negative d.stride (-2) reads the input dilated
 // by 2, the gather of a stride-2 layer's backward-data product.
@@ -46,9 +63,8 @@ bool conv_forward_umma(const ConvDims &d, const __nv_bfloat16 *x, const __nv_bfl
                        const float *bias, void *y, bool y_f32, bool relu, int *err, cudaStream_t st,
                        int ldy = 0, bool accumulate = false);
 // backward-data on the tcgen05 kernel: the ReLU-masked gradient rounded to
-// bf16 and the rotated, transposed weights go to `scratch`
-// (conv_backward_data_umma_scratch bytes), then the product runs as forward
-// convolutions of at most 128 output channels each; a K that is not a
+// bf16 goes to `scratch` (conv_backward_data_umma_scratch bytes), then the
+// product runs on weights packed for it as forward convolutions of at most 128 output channels each; a K that is not a
 // multiple of 16 is padded to one (zero channels, zero weights).  false
 // (nothing launched) when K is not a multiple of 8, C not one of 16, or gin is
 // not 16-byte aligned.

@@ -3,19 +3,44 @@
 // FP32 accumulate in tensor memory).
 //
 //   out[m][k] = bias[k] + sum_{tap, c} x[n][p*st+r-1][q*st+s-1][c] * w[k][tap][c]
-//   m = (n, p, q) flattened (NHWC), tap = 3r + s
+//   m = (n, p, q) (NHWC), tap = 3r + s
 //
-// One CTA (4 warps) owns 128 consecutive output pixels and all NP (= K padded
-// to a multiple of 16) output channels.  The reduction runs over stages of one
-// tap x CK channels: every thread gathers its pixel's CK channels of the tap
-// (16-byte cp.async, zero-filled outside the image) and a share of the
-// weights into shared memory in the no-swizzle K-major layout of the UMMA
-// descriptors (8-row x 16-byte core matrices); thread 0 then issues CK/16
-// MMAs of 128 x NP x 16 and commits them to the stage's mbarrier.  Four stage
-// buffers with a prefetch distance of two let the gathers of stage s+2 and the
-// MMAs of stage s+1 run while stage s computes.  The epilogue reads the
-// accumulator back with tcgen05.ld (warp w holds TMEM lanes 32w..32w+31, one
-// pixel per thread), adds the bias, applies the ReLU and stores bf16 or f32.
+// A CTA owns a rectangle of output pixels, NACC accumulators of 128 of them
+// (8 columns x 16 rows each), and all NP (= K padded to a multiple of 16)
+// output channels.  The input pixels of all taps, with their halo, are copied
+// to shared memory once (16-byte cp.async, zero-filled outside the image), as
+// planes of 8 channels: 16 bytes a pixel, pixels of a row next to each other.
+// Eight neighbouring pixels of a plane are then one 8-row x 16-byte core matrix
+// of the no-swizzle K-major layout wherever they start, rows of the image are
+// the descriptor's stride (SBO), planes its other stride (LBO), and a tap is
+// an offset of the descriptor's start address.  Only the weights stream.  They
+// are packed once (conv_pack_weights) to the order in which the stages of one
+// tap x 8 kcs channels take them, so that a stage is one bulk copy; the copies
+// run as many stages ahead as there are buffers.  One thread issues the MMAs of
+// 128 x NP x 16 of a stage and commits them to the mbarrier that frees its buffer.
+// Taps come in order and channels in order within a tap, whatever the tile.
+//
+//   stride 1    the region is the tile and one pixel around it
+//   stride 2    even and odd columns of a region row lie apart, so that a tap's
+//               every second pixel are neighbours; every second row is the SBO
+//   dilated     (backward-data of stride 2) the four parities of an output pixel
+//               are the four accumulators; a tap has whole sources in exactly one
+//
+// Gathering every tap of 128 flat pixels anew moved nine times the input, and the
+// weights once per 128 pixels, through L1 and L2 with the tensor pipe idle, and the
+// dilated form multiplied 36 taps by zeros for its 9.  16 images, on the device:
+//
+//   128x55  160 -> 64    204 -> 52 us       128x55   64 -> 64    92 -> 23 us
+//   256x109  32 -> 32     84 -> 31 us       64x28   224 -> 96    73 -> 30 us
+//   512x218  16 -> 32 s2  50 -> 38 us       256x109  32 -> 64 s2 47 -> 24 us
+//
+// What is left: an MMA with N = 64 reads 6 KB of shared memory (48 cycles, three
+// times its multiplication), and a CTA loads, multiplies and stores one after the
+// other, covered only by the other CTAs of the SM.
+//
+// The epilogue reads the accumulators back with tcgen05.ld (warp w holds TMEM
+// lanes 32 (w % 4) ..., one pixel per thread), adds the bias, applies the ReLU
+// and stores bf16 or f32.
 //
 // Every wait on an mbarrier is bounded (kWaitNs of %globaltimer); when one
 // gives up, the kernel sets *err, waits (bounded) for its own copies, frees
@@ -32,10 +57,10 @@
 namespace oflow {
 namespace {
 
-constexpr int kUmBM = 128;       // output pixels per CTA (UMMA M)
-constexpr int kUmNT = 128;       // threads per CTA
-constexpr int kUmStages = 4;     // shared-memory stage buffers
-constexpr int kUmAhead = 2;      // stages gathered ahead of the one being multiplied
+constexpr int kUmBM = 128;       // rows of a tile (UMMA M)
+constexpr int kUmNT = 128;       // threads per CTA of the backward-weight kernel
+constexpr int kUmStages = 4;     // stage buffers of the backward-weight kernel
+constexpr int kWgAhead = 2;      // its stages gathered ahead of the one being multiplied
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
     const int n = valid ? 16 : 0;  // 0 bytes read: the destination is zero-filled
@@ -94,31 +119,106 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-template <int NP> __host__ __device__ constexpr uint32_t tmem_cols() { return NP <= 32 ? 32 : NP <= 64 ? 64 : NP <= 128 ? 128 : 256; }
+// tensor-memory columns of N accumulator columns (a power of two, at least 32)
+template <int N> __host__ __device__ constexpr uint32_t tmem_cols() {
+    return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : N <= 256 ? 256 : 512;
+}
 
-template <int NP, int CK> __host__ __device__ constexpr int um_stage_bytes() { return (kUmBM + NP) * CK * 2; }
+// True in one thread of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(p));
+    return p != 0;
+}
 
-template <int NP, int CK>
-__global__ void __launch_bounds__(kUmNT) k_conv_fwd_umma(ConvDims d, const __nv_bfloat16 *__restrict__ x,
-                                                         const __nv_bfloat16 *__restrict__ w,
-                                                         const float *__restrict__ bias, void *y,
-                                                         int flags, int ldy, int *err) {
-    static_assert(NP % 16 == 0 && NP >= 16 && NP <= 256, "UMMA M=128 needs N = 16..256, step 16");
-    static_assert(CK == 16 || CK == 32, "stage depth is 16 or 32 channels");
-    constexpr int A_BYTES = kUmBM * CK * 2;
-    constexpr int STAGE = um_stage_bytes<NP, CK>();
-    constexpr uint32_t TCOLS = tmem_cols<NP>();
+enum UmMode { kUmStride1 = 0, kUmStride2 = 1, kUmDilated = 2 };
+
+// Geometry of a CTA's tile: NACC accumulators of 128 pixels, output rectangle
+// TW x TH, input region RW x RH (stored RW pixels a row, a plane of PX pixels;
+// PX is odd so that the planes of one pixel fall into different banks), SBO in
+// pixels.
+template <int MODE, int MT> struct UmTile {
+    static constexpr int NACC = MODE == kUmDilated ? 4 : MT;
+    static constexpr int TW = MODE == kUmDilated ? 16 : 8 * MT, TH = MODE == kUmDilated ? 32 : 16;
+    static constexpr int RW = MODE == kUmStride1 ? 8 * MT + 2 : MODE == kUmStride2 ? 16 * MT + 1 : 9;
+    static constexpr int RH = MODE == kUmStride1 ? 18 : MODE == kUmStride2 ? 33 : 17;
+    static constexpr int PX = (RW * RH) | 1;
+    static constexpr int ROW = MODE == kUmStride2 ? 2 * RW : RW;
+    static constexpr int NT = NACC == 1 ? 128 : 256;
+};
+
+constexpr int kUmMaxBufs = 16;  // weight buffers of the forward kernel at most
+
+// Bytes of one weight stage: kcs planes of 8 channels, NP rows of 16 bytes.
+__host__ __device__ constexpr int um_wstage(int np, int kcs) { return kcs * np * 16; }
+
+// The MMAs of one weight stage for accumulators t0 .. t1 - 1 (t0 + 1 when
+// DILATED); straight code, since a loop with addresses to compute issues one in
+// 110 cycles.
+template <int NP, int NACC, bool DILATED, int PX, int KCS>
+__device__ __forceinline__ void um_issue(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, int t0, int nacc,
+                                         bool first) {
+#pragma unroll
+    for (int t = 0; t < (DILATED ? 1 : NACC); t++) {
+        if (!DILATED && t >= nacc) break;
+        const uint32_t acc = tmem + (uint32_t)((DILATED ? t0 : t) * NP);
+#pragma unroll
+        for (int j = 0; j < KCS / 2; j++)
+            umma_bf16(acc, ad + (uint32_t)(8 * t + 2 * j * PX), bd + (uint32_t)(2 * j * NP), idesc,
+                      j == 0 && first ? 0u : 1u);
+    }
+}
+
+// w: packed weights.  kcs: planes of 8 channels a weight stage (2, 4 or 8);
+// bufs: weight buffers; cr: channels of the region held at a time (all of them
+// unless they don't fit); 8 kcs divides cr and C.
+template <int NP, int MODE, int MT>
+__global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
+    k_conv_fwd_umma(ConvDims d, const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
+                    const float *__restrict__ bias, void *y, int flags, int ldy, int kcs, int bufs, int cr, int *err) {
+    static_assert(NP % 16 == 0 && NP >= 16 && NP <= 128, "UMMA M=128 needs N a multiple of 16");
+    using T = UmTile<MODE, MT>;
+    constexpr int NT = T::NT, RW = T::RW, PX = T::PX;
+    constexpr uint32_t TCOLS = tmem_cols<T::NACC * NP>();
     constexpr uint32_t IDESC = umma_idesc_bf16(kUmBM, NP);
     extern __shared__ __align__(1024) uint8_t um_smem[];
-    __shared__ __align__(8) uint64_t mbar[kUmStages];
+    __shared__ __align__(8) uint64_t mbar[2 * kUmMaxBufs + 1];  // landed, freed; the region has landed
     __shared__ uint32_t tmem_base;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int M = d.N * d.P * d.Q;
-    const int m0 = blockIdx.x * kUmBM;
-    const int nchunk = d.C / CK;
-    const int nst = 9 * nchunk;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
+    const int gx = div_up(d.Q, T::TW), gy = div_up(d.P, T::TH);
+    const int q0 = (blockIdx.x % gx) * T::TW, p0 = (blockIdx.x / gx) % gy * T::TH, n = blockIdx.x / (gx * gy);
+    const int wstage = um_wstage(NP, kcs);
+    const uint32_t sreg = smem_u32(um_smem), sring = sreg + (uint32_t)(cr / 8) * (PX * 16);
+    const int nst = 9 * (d.C / 8 / kcs), per_reg = 9 * (cr / 8 / kcs);
+    // accumulators with a column inside the image
+    const int nacc = MODE == kUmDilated ? 4 : imin(MT, div_up(d.Q - q0, 8));
+    const uint32_t full = smem_u32(mbar), freed = full + 8 * kUmMaxBufs, regbar = freed + 8 * kUmMaxBufs;
 
+    // first input row and column of the region
+    const int y0 = MODE == kUmStride1 ? p0 - 1 : MODE == kUmStride2 ? 2 * p0 - 1 : p0 / 2;
+    const int x0 = MODE == kUmStride1 ? q0 - 1 : MODE == kUmStride2 ? 2 * q0 - 1 : q0 / 2;
+    const __nv_bfloat16 *xn = x + (size_t)n * d.H * d.W * d.C;
+    // lanes run over the channel planes of a pixel first: whole sectors
+    auto load_region = [&](int c0) {
+        const int nk = cr / 8;
+        const uint32_t magic = 0xFFFFFFFFu / (uint32_t)nk + 1u;  // exact quotients below 2^16
+        for (int e = tid - 32; e < RW * T::RH * nk; e += NT - 32) {
+            const int px = (int)__umulhi((uint32_t)e, magic), kc = e - px * nk;
+            const int ry = px / RW, rx = px % RW, yy = y0 + ry, xx = x0 + rx;
+            const bool ok = (unsigned)yy < (unsigned)d.H && (unsigned)xx < (unsigned)d.W;
+            const int pos = MODE == kUmStride2 ? ry * RW + (rx >> 1) + (rx & 1 ? 8 * MT + 1 : 0) : px;
+            cp_async16(sreg + (uint32_t)(kc * PX + pos) * 16,
+                       ok ? xn + ((size_t)yy * d.W + xx) * d.C + c0 + kc * 8 : x, ok);
+        }
+    };
+
+    if (warp > 0) load_region(0);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                          smem_u32(&tmem_base)),
@@ -127,155 +227,194 @@ __global__ void __launch_bounds__(kUmNT) k_conv_fwd_umma(ConvDims d, const __nv_
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        for (int i = 0; i < kUmStages; i++) mbar_init(smem_u32(&mbar[i]), 1);
+        for (int i = 0; i < bufs; i++) {
+            mbar_init(full + 8 * i, 1);
+            mbar_init(freed + 8 * i, 1);
+        }
+        mbar_init(regbar, NT - 32);
         fence_mbar_init();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
-
-    // this thread gathers output pixel m0 + tid
-    const int m = m0 + tid;
-    const bool mval = m < M;
-    int pn = 0, pp = 0, pq = 0;
-    if (mval) {
-        pq = m % d.Q;
-        const int t = m / d.Q;
-        pp = t % d.P;
-        pn = t / d.P;
-    }
-    const uint32_t sbase = smem_u32(um_smem);
-
-    auto gather = [&](int s) {
-        const int buf = s % kUmStages;
-        const int tap = s / nchunk, c0 = (s % nchunk) * CK;
-        int yy, xx;
-        bool ok;
-        if (d.stride > 0) {
-            yy = pp * d.stride + tap / 3 - 1;
-            xx = pq * d.stride + tap % 3 - 1;
-            ok = mval && yy >= 0 && yy < d.H && xx >= 0 && xx < d.W;
-        } else {
-            // input dilated by 2 (the backward-data product of a stride-2
-            // layer): output (p, q) reads input ((p + r - 1)/2, (q + s - 1)/2)
-            // where both are whole
-            const int y2 = pp + tap / 3 - 1, x2 = pq + tap % 3 - 1;
-            yy = y2 >> 1;
-            xx = x2 >> 1;
-            ok = mval && ((y2 | x2) & 1) == 0 && y2 >= 0 && x2 >= 0 && yy < d.H && xx < d.W;
-        }
-        const __nv_bfloat16 *src = ok ? x + (((size_t)pn * d.H + yy) * d.W + xx) * d.C + c0 : x;
-        const uint32_t a = sbase + buf * STAGE;
-#pragma unroll
-        for (int kc = 0; kc < CK / 8; kc++) cp_async16(a + kc * (kUmBM * 16) + tid * 16, src + kc * 8, ok);
-        const uint32_t b = a + A_BYTES;
-        for (int e = tid; e < NP * (CK / 8); e += kUmNT) {
-            const int n = e % NP, kc = e / NP;
-            const bool okb = n < d.K;
-            const __nv_bfloat16 *ws = okb ? w + ((size_t)n * 9 + tap) * d.C + c0 + kc * 8 : w;
-            cp_async16(b + kc * (NP * 16) + n * 16, ws, okb);
-        }
-    };
-
-    // one cp.async group per stage (empty past the last), so waiting until
-    // kUmAhead groups are pending means stage s has landed
     bool timed_out = false;
-#pragma unroll 1
-    for (int s = 0; s < kUmAhead; s++) {
-        if (s < nst) gather(s);
+
+    if (warp > 0) {
+        // thread 32 fetches the weights: stages follow one another by channels of
+        // the region, taps, regions (counters, since a division a stage would cost
+        // more than its MMAs)
+        int issued = 0, fbuf = 0, fkc = 0, ftap = 0;
+        const __nv_bfloat16 *src = w, *reg0 = w;
+        auto fetch = [&]() {
+            mbar_arrive_expect_tx(full + 8 * fbuf, (uint32_t)wstage);
+            bulk_load(sring + (uint32_t)(fbuf * wstage), src, (uint32_t)wstage, full + 8 * fbuf);
+            issued++;
+            if (++fbuf == bufs) fbuf = 0;
+            src += wstage / 2;
+            fkc += kcs;
+            if (fkc == cr / 8) {
+                fkc = 0;
+                src += (size_t)(d.C - cr) * NP;
+                if (++ftap == 9) {
+                    ftap = 0;
+                    src = reg0 += (size_t)cr * NP;
+                }
+            }
+        };
+        if (tid == 32)
+            while (issued < imin(bufs, nst)) fetch();
         cp_async_commit();
-    }
-#pragma unroll 1
-    for (int s = 0; s < nst; s++) {
-        const int sl = s + kUmAhead;
-        if (sl < nst) {
-            // buffer sl % 4 last held stage sl - 4 = s - 2, committed two stages ago
-            if (sl >= kUmStages && !timed_out) {
-                const int so = sl - kUmStages;
-                if (!mbar_wait_bounded(smem_u32(&mbar[so % kUmStages]), (so / kUmStages) & 1))
-                    timed_out = true;
-            }
-            gather(sl);
-        }
-        cp_async_commit();  // one group per stage (possibly empty)
-        cp_async_wait<kUmAhead>();
+        cp_async_wait<0>();
         fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const int buf = s % kUmStages;
-            const uint32_t a = sbase + buf * STAGE, b = a + A_BYTES;
-#pragma unroll
-            for (int j = 0; j < CK / 16; j++) {
-                const uint64_t ad = umma_desc(a + 2 * j * (kUmBM * 16), kUmBM * 16, 128);
-                const uint64_t bd = umma_desc(b + 2 * j * (NP * 16), NP * 16, 128);
-                umma_bf16(tmem, ad, bd, IDESC, (s > 0 || j > 0) ? 1u : 0u);
+        mbar_arrive(regbar);
+        int buf = 0, ph = 0, left = per_reg, c0 = 0;  // stage s: its buffer is freed for the (ph + 1)-th time
+        // with several regions every thread follows the phases
+        if (tid == 32 || per_reg < nst)
+#pragma unroll 1
+            for (int s = 0; s < nst; s++) {
+                if (!mbar_wait_bounded(freed + 8 * buf, ph)) {
+                    timed_out = true;
+                    break;
+                }
+                if (tid == 32 && issued < nst) fetch();
+                if (--left == 0 && s + 1 < nst) {  // the region's MMAs are done: the next channels replace it
+                    left = per_reg;
+                    load_region(c0 += cr);
+                    cp_async_commit();
+                    cp_async_wait<0>();
+                    fence_async_smem();
+                    mbar_arrive(regbar);
+                }
+                if (++buf == bufs) {
+                    buf = 0;
+                    ph ^= 1;
+                }
             }
-            umma_commit(smem_u32(&mbar[buf]));
+        if (timed_out && tid == 32)  // its own copies in flight
+            for (int s = imax(0, issued - bufs); s < issued; s++)
+                mbar_wait_bounded(full + 8 * (s % bufs), (uint32_t)(s / bufs) & 1u);
+    } else {
+        // the whole warp follows the stages, so that addresses and descriptors are
+        // uniform; one thread issues
+        const bool issuer = elect_one();
+        const uint64_t adesc = umma_desc(0, PX * 16, T::ROW * 16), bdesc = umma_desc(0, NP * 16, 128);
+        int tap = 0, kc0 = 0, buf = 0, ph = 0;
+#pragma unroll 1
+        for (int s = 0; s < nst; s++) {
+            if ((tap == 0 && kc0 == 0 && !mbar_wait_bounded(regbar, (uint32_t)(s / per_reg) & 1u)) ||
+                !mbar_wait_bounded(full + 8 * buf, ph)) {
+                timed_out = true;
+                break;
+            }
+            tc_fence_after();
+            const int r = tap / 3, sx = tap % 3;
+            // the tap's first pixel in the region, its accumulator, and whether
+            // that holds anything yet
+            int off, t0 = 0;
+            bool first = s == 0;
+            if (MODE == kUmStride1) {
+                off = r * RW + sx;
+            } else if (MODE == kUmStride2) {
+                off = r * RW + (sx == 1 ? 8 * MT + 1 : sx >> 1);
+            } else {
+                off = (r >> 1) * RW + (sx >> 1);
+                t0 = (r != 1 ? 2 : 0) + (sx != 1 ? 1 : 0);
+                first = s < per_reg && kc0 == 0 && r < 2 && sx < 2;
+            }
+            const uint64_t ad = adesc + ((sreg >> 4) + (uint32_t)(kc0 * PX + off));
+            const uint64_t bd = bdesc + ((sring + (uint32_t)(buf * wstage)) >> 4);
+            if (issuer) {
+                constexpr bool DIL = MODE == kUmDilated;
+                switch (kcs) {
+                    case 2: um_issue<NP, T::NACC, DIL, PX, 2>(tmem, ad, bd, IDESC, t0, nacc, first); break;
+                    case 4: um_issue<NP, T::NACC, DIL, PX, 4>(tmem, ad, bd, IDESC, t0, nacc, first); break;
+                    case 6: um_issue<NP, T::NACC, DIL, PX, 6>(tmem, ad, bd, IDESC, t0, nacc, first); break;
+                    case 8: um_issue<NP, T::NACC, DIL, PX, 8>(tmem, ad, bd, IDESC, t0, nacc, first); break;
+                    case 10: um_issue<NP, T::NACC, DIL, PX, 10>(tmem, ad, bd, IDESC, t0, nacc, first); break;
+                    default: um_issue<NP, T::NACC, DIL, PX, 14>(tmem, ad, bd, IDESC, t0, nacc, first); break;
+                }
+                umma_commit(freed + 8 * buf);
+            }
+            __syncwarp();
+            kc0 += kcs;
+            if (kc0 == cr / 8) {
+                kc0 = 0;
+                if (++tap == 9) tap = 0;
+            }
+            // the last commit tracks every MMA of this CTA
+            if (s == nst - 1 && !mbar_wait_bounded(freed + 8 * buf, ph)) timed_out = true;
+            if (++buf == bufs) {
+                buf = 0;
+                ph ^= 1;
+            }
         }
     }
-    // the last commit tracks every MMA of this CTA
-    {
-        const int sL = nst - 1;
-        if (!timed_out && !mbar_wait_bounded(smem_u32(&mbar[sL % kUmStages]), (sL / kUmStages) & 1))
-            timed_out = true;
-    }
-    cp_async_wait<0>();
     // block-uniform from here: tcgen05.ld is warp-collective
     timed_out = __syncthreads_or(timed_out);
     if (timed_out && tid == 0) atomicOr(err, 1);
     tc_fence_after();
     if (!timed_out) {
-        const int mo = m0 + warp * 32 + lane;
+        const int row = (warp & 3) * 32 + lane;
         const bool relu = flags & 1, f32 = flags & 2, accum = flags & 4;
         const int ld = ldy > 0 ? ldy : d.K;  // elements between output rows
         const bool vec = d.K % 8 == 0 && ld % 8 == 0;  // rows of y start on 16-byte boundaries
 #pragma unroll 1
-        for (int c0 = 0; c0 < NP; c0 += 16) {
-            uint32_t r[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
-            if (mo >= M) continue;
-            float v[16];
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const int col = c0 + j;
-                float t = __uint_as_float(r[j]) + ((bias && col < d.K) ? bias[col] : 0.0f);
-                v[j] = relu ? fmaxf(t, 0.0f) : t;
+        for (int t = warp >> 2; t < nacc; t += NT / 128) {
+            int p = p0 + (row >> 3), q = q0 + 8 * t + (row & 7);
+            if (MODE == kUmDilated) {
+                p = p0 + 2 * (row >> 3) + (t >> 1);
+                q = q0 + 2 * (row & 7) + (t & 1);
             }
-            if (f32) {
-                float *o = static_cast<float *>(y) + (size_t)mo * ld + c0;
-                if (accum) {  // each output element belongs to one thread
+            const bool inside = p < d.P && q < d.Q;
+            const size_t mo = ((size_t)n * d.P + p) * d.Q + q;
+#pragma unroll 1
+            for (int c0 = 0; c0 < NP; c0 += 16) {
+                uint32_t r[16];
+                tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(t * NP + c0), r);
+                if (!inside) continue;
+                float v[16];
 #pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (c0 + j < d.K) o[j] += v[j];
-                    continue;
+                for (int j = 0; j < 16; j++) {
+                    const int col = c0 + j;
+                    float f = __uint_as_float(r[j]) + ((bias && col < d.K) ? bias[col] : 0.0f);
+                    v[j] = relu ? fmaxf(f, 0.0f) : f;
                 }
+                if (f32) {
+                    float *o = static_cast<float *>(y) + mo * ld + c0;
 #pragma unroll
-                for (int j = 0; j < 16; j += 4)
-                    if (vec && c0 + j + 3 < d.K)
-                        *reinterpret_cast<float4 *>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    else
-                        for (int e = 0; e < 4; e++)
-                            if (c0 + j + e < d.K) o[j + e] = v[j + e];
-            } else {
-                __nv_bfloat16 *o = static_cast<__nv_bfloat16 *>(y) + (size_t)mo * ld + c0;
+                    for (int j = 0; j < 16; j += 4)
+                        if (vec && c0 + j + 3 < d.K) {
+                            float4 *o4 = reinterpret_cast<float4 *>(o + j);
+                            float4 f = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                            if (accum) {  // each output element belongs to one thread
+                                const float4 g = *o4;
+                                f = make_float4(g.x + f.x, g.y + f.y, g.z + f.z, g.w + f.w);
+                            }
+                            *o4 = f;
+                        } else {
+                            for (int e = 0; e < 4; e++)
+                                if (c0 + j + e < d.K) o[j + e] = accum ? o[j + e] + v[j + e] : v[j + e];
+                        }
+                } else {
+                    __nv_bfloat16 *o = static_cast<__nv_bfloat16 *>(y) + mo * ld + c0;
 #pragma unroll
-                for (int j = 0; j < 16; j += 8) {
-                    if (vec && c0 + j + 7 < d.K) {
-                        uint4 pk;
-                        __nv_bfloat162 h0 = __floats2bfloat162_rn(v[j], v[j + 1]);
-                        __nv_bfloat162 h1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
-                        __nv_bfloat162 h2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]);
-                        __nv_bfloat162 h3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-                        pk.x = *reinterpret_cast<uint32_t *>(&h0);
-                        pk.y = *reinterpret_cast<uint32_t *>(&h1);
-                        pk.z = *reinterpret_cast<uint32_t *>(&h2);
-                        pk.w = *reinterpret_cast<uint32_t *>(&h3);
-                        *reinterpret_cast<uint4 *>(o + j) = pk;
-                    } else {
-                        for (int e = 0; e < 8; e++)
-                            if (c0 + j + e < d.K) o[j + e] = __float2bfloat16(v[j + e]);
+                    for (int j = 0; j < 16; j += 8) {
+                        if (vec && c0 + j + 7 < d.K) {
+                            uint4 pk;
+                            __nv_bfloat162 h0 = __floats2bfloat162_rn(v[j], v[j + 1]);
+                            __nv_bfloat162 h1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
+                            __nv_bfloat162 h2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]);
+                            __nv_bfloat162 h3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
+                            pk.x = *reinterpret_cast<uint32_t *>(&h0);
+                            pk.y = *reinterpret_cast<uint32_t *>(&h1);
+                            pk.z = *reinterpret_cast<uint32_t *>(&h2);
+                            pk.w = *reinterpret_cast<uint32_t *>(&h3);
+                            *reinterpret_cast<uint4 *>(o + j) = pk;
+                        } else {
+                            for (int e = 0; e < 8; e++)
+                                if (c0 + j + e < d.K) o[j + e] = __float2bfloat16(v[j + e]);
+                        }
                     }
                 }
             }
@@ -288,26 +427,85 @@ __global__ void __launch_bounds__(kUmNT) k_conv_fwd_umma(ConvDims d, const __nv_
                      : "memory");
 }
 
-template <int NP, int CK>
-void launch_umma(const ConvDims &d, const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *bias,
-                 void *y, int flags, int ldy, int *err, cudaStream_t st) {
-    constexpr int smem = kUmStages * um_stage_bytes<NP, CK>();
-    OF_CUDA(cudaFuncSetAttribute(k_conv_fwd_umma<NP, CK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 smem));
-    const int M = d.N * d.P * d.Q;
-    k_conv_fwd_umma<NP, CK><<<div_up(M, kUmBM), kUmNT, smem, st>>>(d, x, w, bias, y, flags, ldy, err);
+// What one forward launch gets.
+struct UmCall {
+    const ConvDims &d;
+    const __nv_bfloat16 *x, *w;
+    const float *bias;
+    void *y;
+    int flags, ldy, *err;
+    cudaStream_t st;
+};
+
+// Planes of 8 channels a weight stage, and its buffers: the deepest stage of at
+// most 12 KB, and 16 KB of buffers or two.  Stages of 4 KB take 61 us where those of
+// 10 take 52 (16 x 128x55, 160 -> 64 channels), and 32 KB of buffers cost resident
+// CTAs (35 us for 30.5 at 32 -> 32).
+int um_kcs(int C, int np) {
+    int kcs = 2;
+    for (int k : {4, 6, 8, 10, 14})
+        if (C / 8 % k == 0 && um_wstage(np, k) <= 12 * 1024) kcs = k;
+    return kcs;
+}
+int um_bufs(int C, int np) { return imax(2, imin(kUmMaxBufs, 16 * 1024 / um_wstage(np, um_kcs(C, np)))); }
+
+constexpr int kUmSmemMax = 227 * 1024 - 1024;
+
+template <int MODE, int MT> int um_tiles(const ConvDims &d) {
+    using T = UmTile<MODE, MT>;
+    return div_up(d.Q, T::TW) * div_up(d.P, T::TH) * d.N;
 }
 
-template <int CK>
-bool dispatch_np(int np, const ConvDims &d, const __nv_bfloat16 *x, const __nv_bfloat16 *w,
-                 const float *bias, void *y, int flags, int ldy, int *err, cudaStream_t st) {
+template <int MODE, int MT> int um_smem(int np, int C, int cr) {
+    return cr / 8 * UmTile<MODE, MT>::PX * 16 + um_bufs(C, np) * um_wstage(np, um_kcs(C, np));
+}
+
+template <int NP, int MODE, int MT> void launch_um(const UmCall &c) {
+    const int kcs = um_kcs(c.d.C, NP), nk = c.d.C / 8;
+    int cr = c.d.C;  // fewer channels a region where it would not fit
+    while (um_smem<MODE, MT>(NP, c.d.C, cr) > kUmSmemMax) {
+        cr -= 8 * kcs;
+        while (nk % (cr / 8) != 0) cr -= 8 * kcs;
+    }
+    const int smem = um_smem<MODE, MT>(NP, c.d.C, cr);
+    OF_CUDA(cudaFuncSetAttribute(k_conv_fwd_umma<NP, MODE, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_conv_fwd_umma<NP, MODE, MT><<<um_tiles<MODE, MT>(c.d), UmTile<MODE, MT>::NT, smem, c.st>>>(
+        c.d, c.x, c.w, c.bias, c.y, c.flags, c.ldy, kcs, um_bufs(c.d.C, NP), cr, c.err);
+}
+
+// Wide tiles (half or less of a narrow one's halo) where the layer has few output
+// channels, so that the region and not the multiplication takes the time, and
+// tiles enough for two CTAs an SM that leave room for each other: 16 images of
+// 256x109, 32 -> 32 channels, 30.5 us with four accumulators and 36.2 with one;
+// 512x218 to half size, 16 -> 32, 38 and 41 with two and one.  With 64 output
+// channels narrow tiles, of which more fit an SM, are the faster ones: 16 x 128x55,
+// 64 -> 64, 26.3 us with two accumulators and 23.3 with one.
+template <int NP, int MODE, int MT> bool um_wide(const ConvDims &d) {
+    return um_smem<MODE, MT>(NP, d.C, d.C) <= 113 * 1024 && um_tiles<MODE, MT>(d) >= 2 * kNumSMs;
+}
+
+template <int NP> void launch_umma(const UmCall &c) {
+    if (c.d.stride == 1) {
+        if constexpr (NP <= 32)
+            if (um_wide<NP, kUmStride1, 4>(c.d)) return launch_um<NP, kUmStride1, 4>(c);
+        launch_um<NP, kUmStride1, 1>(c);
+    } else if (c.d.stride == 2) {
+        if constexpr (NP <= 32)
+            if (um_wide<NP, kUmStride2, 2>(c.d)) return launch_um<NP, kUmStride2, 2>(c);
+        launch_um<NP, kUmStride2, 1>(c);
+    } else {
+        launch_um<NP, kUmDilated, 1>(c);
+    }
+}
+
+bool dispatch_np(int np, const UmCall &c) {
     switch (np) {
-        case 16: launch_umma<16, CK>(d, x, w, bias, y, flags, ldy, err, st); return true;
-        case 32: launch_umma<32, CK>(d, x, w, bias, y, flags, ldy, err, st); return true;
-        case 48: launch_umma<48, CK>(d, x, w, bias, y, flags, ldy, err, st); return true;
-        case 64: launch_umma<64, CK>(d, x, w, bias, y, flags, ldy, err, st); return true;
-        case 96: launch_umma<96, CK>(d, x, w, bias, y, flags, ldy, err, st); return true;
-        case 128: launch_umma<128, CK>(d, x, w, bias, y, flags, ldy, err, st); return true;
+        case 16: launch_umma<16>(c); return true;
+        case 32: launch_umma<32>(c); return true;
+        case 48: launch_umma<48>(c); return true;
+        case 64: launch_umma<64>(c); return true;
+        case 96: launch_umma<96>(c); return true;
+        case 128: launch_umma<128>(c); return true;
         default: return false;
     }
 }
@@ -425,16 +623,16 @@ __global__ void __launch_bounds__(kUmNT) k_conv_wgrad_mn(ConvDims d, const __nv_
     };
 
     // one cp.async group per stage (empty past the last), so waiting until
-    // kUmAhead groups are pending means stage s has landed
+    // kWgAhead groups are pending means stage s has landed
     bool timed_out = false;
 #pragma unroll 1
-    for (int s = 0; s < kUmAhead; s++) {
+    for (int s = 0; s < kWgAhead; s++) {
         if (s < nst) gather(s);
         cp_async_commit();
     }
 #pragma unroll 1
     for (int s = 0; s < nst; s++) {
-        const int sl = s + kUmAhead;
+        const int sl = s + kWgAhead;
         if (sl < nst) {
             // buffer sl % 4 last held stage sl - 4 = s - 2, committed two stages ago
             if (sl >= kUmStages && !timed_out) {
@@ -445,7 +643,7 @@ __global__ void __launch_bounds__(kUmNT) k_conv_wgrad_mn(ConvDims d, const __nv_
             gather(sl);
         }
         cp_async_commit();
-        cp_async_wait<kUmAhead>();
+        cp_async_wait<kWgAhead>();
         fence_async_smem();
         __syncthreads();
         if (tid == 0) {
@@ -538,12 +736,11 @@ constexpr int kBiasBlocks = 4 * kNumSMs;
 constexpr int kBiasFinalNT = 256;
 
 // Scratch of the backward products, in bytes from its start: the masked bf16
-// gradient, the rotated weights (each rounded up to 64 elements, 128-byte
-// aligned), then the bias partial sums (kBiasBlocks x K floats).
+// gradient (rounded up to 64 elements), then the bias partial sums
+// (kBiasBlocks x K floats).
 size_t bwd_scratch_part(const ConvDims &d) {
     const size_t kp = (size_t)(d.K + 15) / 16 * 16;  // gradient channels padded to 16
-    const size_t g = (size_t)d.N * d.P * d.Q * kp, wt = kp * 9 * d.C;
-    return ((g + 63) / 64 * 64 + (wt + 63) / 64 * 64) * sizeof(__nv_bfloat16);
+    return ((size_t)d.N * d.P * d.Q * kp + 63) / 64 * 64 * sizeof(__nv_bfloat16);
 }
 
 __global__ void __launch_bounds__(256) k_mask_bias(const float *__restrict__ g,
@@ -606,15 +803,32 @@ __global__ void __launch_bounds__(kBiasFinalNT) k_bias_final(const float *__rest
     if (threadIdx.x == 0) gb[k] = (float)r;
 }
 
-// wt[c][tap][k] = w[k][8 - tap][c]: the weights of the backward-data product
-// seen as a forward convolution (rotated taps, input and output channels
-// exchanged), with Kp >= K input channels (zero for k >= K)
-__global__ void k_flip_weights(const __nv_bfloat16 *__restrict__ w, int K, int Kp, int C,
-                               __nv_bfloat16 *wt) {
-    const int n = Kp * 9 * C;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int k = i % Kp, tap = (i / Kp) % 9, c = i / (9 * Kp);
-        wt[i] = k < K ? w[((size_t)k * 9 + (8 - tap)) * C + c] : __float2bfloat16(0.0f);
+// Weights in the order of the forward kernel's stages: one 16-byte unit a
+// thread, dst[tap][plane of 8 input channels][output channel][8].  Forward:
+// w[k][tap][c]; output channels padded to 16 (zeros).  Backward-data seen as a
+// forward convolution: rotated taps, input and output channels exchanged, output
+// channels in groups of at most 128 one after the other, input channels padded
+// to 16 (zeros).
+__global__ void k_pack_weights(const __grid_constant__ ConvPack a) {
+    const ConvPack::Job &J = a.job[blockIdx.y];
+    const int outs = J.backward ? J.C : (J.K + 15) / 16 * 16, planes = (J.backward ? (J.K + 15) / 16 * 16 : J.C) / 8;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < outs * planes * 9; i += gridDim.x * blockDim.x) {
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (J.backward) {
+            const int g = i / (128 * 9 * planes), np = imin(128, outs - 128 * g), e = i - g * (128 * 9 * planes);
+            const int c = 128 * g + e % np, pl = (e / np) % planes, tap = e / (np * planes);
+            __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int k = 8 * pl + q;
+                h[q] = k < J.K ? J.w[((size_t)k * 9 + (8 - tap)) * J.C + c] : __float2bfloat16(0.0f);
+            }
+            v = *reinterpret_cast<const uint4 *>(h);
+        } else {
+            const int k = i % outs, pl = (i / outs) % planes, tap = i / (outs * planes);
+            if (k < J.K) v = *reinterpret_cast<const uint4 *>(J.w + ((size_t)k * 9 + tap) * J.C + 8 * pl);
+        }
+        reinterpret_cast<uint4 *>(J.dst)[i] = v;
     }
 }
 
@@ -637,6 +851,12 @@ __global__ void k_mask_pad_bf16(const float *__restrict__ g, const __nv_bfloat16
 
 }  // namespace
 
+size_t conv_packed_size(int K, int C) { return (size_t)(K + 15) / 16 * 16 * 9 * C; }
+
+void conv_pack_weights(const ConvPack &a, cudaStream_t st) {
+    if (a.n > 0) k_pack_weights<<<dim3(32, a.n), 256, 0, st>>>(a);
+}
+
 bool conv_forward_umma(const ConvDims &d, const __nv_bfloat16 *x, const __nv_bfloat16 *w,
                        const float *bias, void *y, bool y_f32, bool relu, int *err, cudaStream_t st,
                        int ldy, bool accumulate) {
@@ -647,8 +867,7 @@ bool conv_forward_umma(const ConvDims &d, const __nv_bfloat16 *x, const __nv_bfl
     if (!a16(x) || !a16(w) || !a16(y)) return false;
     const int np = (d.K + 15) / 16 * 16;
     const int flags = (relu ? 1 : 0) | (y_f32 ? 2 : 0) | (accumulate ? 4 : 0);
-    if (d.C % 32 == 0) return dispatch_np<32>(np, d, x, w, bias, y, flags, ldy, err, st);
-    return dispatch_np<16>(np, d, x, w, bias, y, flags, ldy, err, st);
+    return dispatch_np(np, UmCall{d, x, w, bias, y, flags, ldy, err, st});
 }
 
 bool conv_backward_weight_umma(const ConvDims &d, const float *g, const __nv_bfloat16 *y_act,
@@ -704,18 +923,16 @@ bool conv_backward_data_umma(const ConvDims &d, const float *g, const __nv_bfloa
     const int M = d.N * d.P * d.Q;
     const size_t ng = (size_t)M * Kp;
     __nv_bfloat16 *gb = static_cast<__nv_bfloat16 *>(scratch);
-    __nv_bfloat16 *wt = gb + (ng + 63) / 64 * 64;  // 128-byte aligned
     if (Kp != d.K)
         k_mask_pad_bf16<<<imin((int)((ng + 255) / 256), 4096), 256, 0, st>>>(g, y_act, M, d.K, Kp, gb);
     else if (!g_masked)
         k_mask_bf16<<<imin((int)((ng + 255) / 256), 4096), 256, 0, st>>>(g, y_act, gb, ng);
-    k_flip_weights<<<imin(div_up(Kp * 9 * d.C, 256), 1024), 256, 0, st>>>(w, d.K, Kp, d.C, wt);
     // the product as a forward convolution over the output gradient: input
     // (N, P, Q, Kp), output (N, H, W, C); stride 2 layers read a dilated input
     ConvDims t{d.N, d.P, d.Q, Kp, d.H, d.W, 0, d.stride == 1 ? 1 : -2};
     for (int c0 = 0; c0 < d.C; c0 += 128) {  // at most 128 output channels a launch
         t.K = imin(128, d.C - c0);
-        if (!conv_forward_umma(t, gb, wt + (size_t)c0 * 9 * Kp, nullptr, gin + c0, true, false, err,
+        if (!conv_forward_umma(t, gb, w + (size_t)c0 * 9 * Kp, nullptr, gin + c0, true, false, err,
                                st, d.C, accumulate))
             return false;
     }

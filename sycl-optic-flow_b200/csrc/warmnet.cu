@@ -54,6 +54,8 @@ WarmNet::WarmNet(int w, int h, int B) : w_(w), h_(h), B_(B) {
         off += (size_t)kLayers[l].cout * 9 * kLayers[l].cin;
         boff_[l] = off;
         off += kLayers[l].cout;
+        pkoff_[l] = npk_;
+        npk_ += conv_packed_size(kLayers[l].cout, kLayers[l].cin);
     }
     np_ = off;
     // activation sizes (pixels) per tensor
@@ -73,6 +75,8 @@ WarmNet::WarmNet(int w, int h, int B) : w_(w), h_(h), B_(B) {
     o_gout_ = ar_.reserve(p3 * 8 * 4);
     o_p_ = ar_.reserve(np_ * 4);
     o_pb_ = ar_.reserve(np_ * 2);
+    o_pkf_ = ar_.reserve(npk_ * 2);
+    o_pkb_ = ar_.reserve(npk_ * 2);
     o_gp_ = ar_.reserve(np_ * 4);
     o_m_ = ar_.reserve(np_ * 4);
     o_v_ = ar_.reserve(np_ * 4);
@@ -88,15 +92,29 @@ WarmNet::WarmNet(int w, int h, int B) : w_(w), h_(h), B_(B) {
     OF_CUDA(cudaMemset(ar_.at<char>(o_v_), 0, np_ * 4));
     OF_CUDA(cudaMemset(ar_.at<char>(o_p_), 0, np_ * 4));
     OF_CUDA(cudaMemset(ar_.at<char>(o_pb_), 0, np_ * 2));
+    OF_CUDA(cudaMemset(ar_.at<char>(o_pkf_), 0, npk_ * 2));
+    OF_CUDA(cudaMemset(ar_.at<char>(o_pkb_), 0, npk_ * 2));
 }
 
 void WarmNet::set_params(const float *host, cudaStream_t st) {
     OF_CUDA(cudaMemcpyAsync(ar_.at<float>(o_p_), host, np_ * 4, cudaMemcpyHostToDevice, st));
     cnn_f32_to_bf16(ar_.at<float>(o_p_), ar_.at<__nv_bfloat16>(o_pb_), np_, st);
+    pack(st);
     OF_CUDA(cudaStreamSynchronize(st));
     step_ = 0;
     OF_CUDA(cudaMemsetAsync(ar_.at<char>(o_m_), 0, np_ * 4, st));
     OF_CUDA(cudaMemsetAsync(ar_.at<char>(o_v_), 0, np_ * 4, st));
+}
+
+void WarmNet::pack(cudaStream_t st) {
+    // layer 0 has no backward-data product
+    ConvPack a;
+    const __nv_bfloat16 *W = ar_.at<__nv_bfloat16>(o_pb_);
+    for (int l = 0; l < 10; l++) {
+        a.add(W + woff_[l], ar_.at<__nv_bfloat16>(o_pkf_) + pkoff_[l], kLayers[l].cout, kLayers[l].cin, false);
+        if (l > 0) a.add(W + woff_[l], ar_.at<__nv_bfloat16>(o_pkb_) + pkoff_[l], kLayers[l].cout, kLayers[l].cin, true);
+    }
+    conv_pack_weights(a, st);
 }
 
 void WarmNet::get_params(float *host, cudaStream_t st) const {
@@ -116,6 +134,7 @@ ConvDims WarmNet::dims(int l) const {
 void WarmNet::forward(const void *frames, int dtype, size_t pair_stride, cudaStream_t st) {
     auto A = [&](int t) { return ar_.at<__nv_bfloat16>(aoff_[t]); };
     const __nv_bfloat16 *W = ar_.at<__nv_bfloat16>(o_pb_);
+    const __nv_bfloat16 *PK = ar_.at<__nv_bfloat16>(o_pkf_);
     const float *P = ar_.at<float>(o_p_);
     cnn_input(frames, dtype, w_, h_, B_, pair_stride, A(0), st);
     // tensors: 0 x0, 1 c1, 2 c2, 3 c3, 4 c4, 5 c5, 6 c6, 7 c7, 8 cat1, 9 c8, 10 cat2, 11 c9
@@ -129,10 +148,10 @@ void WarmNet::forward(const void *frames, int dtype, size_t pair_stride, cudaStr
         const ConvDims d = dims(l);
         if (l < 9)
             conv_forward(d, A(src[l]), W + woff_[l], P + boff_[l], A(dst[l]), false, kLayers[l].relu, st,
-                         ar_.at<int>(o_err_));
+                         ar_.at<int>(o_err_), PK + pkoff_[l]);
         else
             conv_forward(d, A(src[l]), W + woff_[l], P + boff_[l], ar_.at<float>(o_out_), true, false,
-                         st, ar_.at<int>(o_err_));
+                         st, ar_.at<int>(o_err_), PK + pkoff_[l]);
     }
 }
 
@@ -142,6 +161,7 @@ double WarmNet::train_step(const void *frames, int dtype, size_t pair_stride, co
     auto A = [&](int t) { return ar_.at<__nv_bfloat16>(aoff_[t]); };
     auto G = [&](int t) { return ar_.at<float>(goff_[t]); };
     const __nv_bfloat16 *W = ar_.at<__nv_bfloat16>(o_pb_);
+    const __nv_bfloat16 *PKB = ar_.at<__nv_bfloat16>(o_pkb_);
     float *gp = ar_.at<float>(o_gp_);
     const int M3 = B_ * hs_[3] * ws_[3];
     flow_loss(ar_.at<float>(o_out_), 8, target, M3, ar_.at<float>(o_gout_), ar_.at<double>(o_loss_), st);
@@ -157,7 +177,7 @@ double WarmNet::train_step(const void *frames, int dtype, size_t pair_stride, co
         if (!wg) conv_backward_weight(d, g, yact, A(x_t), gp + woff_[l], gp + boff_[l], st);
         // the tensor-core backward-weight product left the masked bf16
         // gradient at the start of the shared scratch
-        if (gin && (bwd_mma_ || !conv_backward_data_umma(d, g, yact, W + woff_[l], gin, acc,
+        if (gin && (bwd_mma_ || !conv_backward_data_umma(d, g, yact, PKB + pkoff_[l], gin, acc,
                                                           ar_.at<char>(o_bwd_), ar_.at<int>(o_err_), st,
                                                           wg)))
             conv_backward_data(d, g, yact, W + woff_[l], gin, acc, st);
@@ -180,6 +200,7 @@ double WarmNet::train_step(const void *frames, int dtype, size_t pair_stride, co
     adam_step(ar_.at<float>(o_p_), gp, ar_.at<float>(o_m_), ar_.at<float>(o_v_), np_, lr, 0.9f,
               0.999f, 1e-8f, step_, st);
     cnn_f32_to_bf16(ar_.at<float>(o_p_), ar_.at<__nv_bfloat16>(o_pb_), np_, st);
+    pack(st);
     double loss = 0.0;
     OF_CUDA(cudaMemcpyAsync(&loss, ar_.at<double>(o_loss_), 8, cudaMemcpyDeviceToHost, st));
     OF_CUDA(cudaStreamSynchronize(st));

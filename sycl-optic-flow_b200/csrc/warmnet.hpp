@@ -37,14 +37,15 @@ class WarmNet {
 
   private:
     ConvDims dims(int l) const;
+    void pack(cudaStream_t st);  // the bf16 weights for the tensor-core kernels
     int w_, h_, B_;
     int hs_[6] = {}, ws_[6] = {};
-    size_t woff_[10] = {}, boff_[10] = {};
+    size_t woff_[10] = {}, boff_[10] = {}, pkoff_[10] = {};
     size_t np_ = 0;
     Arena ar_;
     size_t aoff_[12] = {}, goff_[12] = {}, gsize_[12] = {};
     size_t o_out_ = 0, o_gout_ = 0, o_p_ = 0, o_pb_ = 0, o_gp_ = 0, o_m_ = 0, o_v_ = 0,
-           o_loss_ = 0, o_err_ = 0, o_bwd_ = 0;
+           o_loss_ = 0, o_err_ = 0, o_bwd_ = 0, o_pkf_ = 0, o_pkb_ = 0, npk_ = 0;
     bool bwd_mma_ = false;  // backward products on the mma.sync kernel only
     int step_ = 0;
 };
