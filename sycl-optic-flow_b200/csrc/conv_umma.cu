@@ -58,9 +58,6 @@ namespace oflow {
 namespace {
 
 constexpr int kUmBM = 128;       // rows of a tile (UMMA M)
-constexpr int kUmNT = 128;       // threads per CTA of the backward-weight kernel
-constexpr int kUmStages = 4;     // stage buffers of the backward-weight kernel
-constexpr int kWgAhead = 2;      // its stages gathered ahead of the one being multiplied
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
     const int n = valid ? 16 : 0;  // 0 bytes read: the destination is zero-filled
@@ -512,206 +509,215 @@ bool dispatch_np(int np, const UmCall &c) {
 
 // Backward-weight product on the tensor cores:
 //   gw[k][tap][c] = sum_m x[pixel(m, tap)][c] * g[m][k]
-// as D = A B with the rows of D the (tap, c) pairs of the layer (9C rows, in
-// 128-row UMMA tiles, row = tap * C + c), its columns the output channels k
-// (K rounded up to 16 = KP) and the reduction over output pixels m, 32 per
-// stage.  Both operands are read in the layout they have in memory and
-// staged MN-major (no swizzle): a core matrix is 8 reduction rows (pixels) of
-// 16 bytes, each 16 bytes being 8 consecutive (tap, c) rows of A -- the
-// channels c..c+7 of one input pixel -- or 8 consecutive output channels of B
-// -- g[m][k..k+7].  So every gather is one 16-byte cp.async of NHWC memory,
-// with no transposition.  In a stage, core matrices along the reduction are
-// 128 bytes apart (LBO) and groups of 8 rows 512 bytes apart (SBO); tile t of
-// A starts t * 8 KB into the stage.  A CTA owns up to kWgMT tiles of rows
-// (gridDim.x runs over groups of tiles), shares each stage's gradient tile
-// between them, reduces a range of pixels (gridDim.y splits the pixels) and
-// adds its rows to gw with atomics.  Pipeline, commits and bounded waits as in
-// the forward kernel.
-constexpr int kWgMT = 4;       // row tiles a CTA at most
-constexpr int kWgPix = 32;     // pixels a stage
-constexpr int kWgTile = kUmBM * kWgPix * 2;  // bytes of one row tile a stage
+// as D = A B with rows of D (tap column, c), one accumulator per tap row, columns
+// the output channels k (K rounded up to 16 = KP), and the reduction over output
+// pixels m in tiles of 8 columns x 16 rows.  Both operands stay in the layout they
+// have in memory, MN-major (no swizzle): a core matrix is 8 reduction rows (8
+// neighbouring pixels) of 16 bytes (8 channels).  A tile of x is kept as planes of
+// 16 bytes a pixel, one per 8 channels and tap column -- the columns' planes hold
+// the same image shifted, so that planes are the M groups at one distance (SBO) and
+// image rows the reduction groups at another (LBO) -- and a tap row is an offset
+// of the start address: three times the image in shared memory for nine taps.
+//
+// A CTA takes the three tap columns of at most 5 channel groups (15 of the 16 M
+// groups; the rest of the 128 rows is read from whatever follows and ignored)
+// and every gridDim.y-th pixel tile, and adds its rows to gw with atomics.  Warps
+// 1 to 7 load tiles (16-byte cp.async, zeros outside) into two or three buffers; a
+// thread of warp 0 issues a tile's 24 MMAs and commits them to the mbarrier that
+// frees the buffer.  Bounded waits as in the forward kernel.
+//
+// Gathering each of the nine taps on its own, behind a block barrier per 32 pixels,
+// took 181 us for 160 -> 64 channels of 16 images of 128x55 where this takes 57;
+// 78 and 37 us for 32 -> 32 of 256x109, 59 and 41 for 224 -> 96 of 64x28, 48 and 38
+// for 16 -> 32 of 512x218 to half size.  What is left is the tiles' way from L2
+// (some 50 KB a tile and CTA, 4 TB/s).
+constexpr int kWgNT = 256;
+constexpr int kWgGroups = 5;  // channel groups of 8 a CTA at most
 
-template <int KP>
-__global__ void __launch_bounds__(kUmNT) k_conv_wgrad_mn(ConvDims d, const __nv_bfloat16 *__restrict__ gb,
-                                                         const __nv_bfloat16 *__restrict__ x, float *gw,
-                                                         int ntg, int pix_per_cta, uint32_t tcols, int *err) {
+// Geometry: input rows of a tile, pixels of a plane of x and of g (one more than
+// they hold, so that planes fall into different banks).
+template <int STRIDE> struct WgTile {
+    static constexpr int RH = STRIDE == 1 ? 18 : 33;
+    static constexpr int PXA = RH * 8 + 1, PXB = 129;
+};
+
+template <int KP, int STRIDE>
+__global__ void __launch_bounds__(kWgNT) k_conv_wgrad_mn(ConvDims d, const __nv_bfloat16 *__restrict__ gb,
+                                                         const __nv_bfloat16 *__restrict__ x, float *gw, int groups,
+                                                         int bufs, int *err) {
     static_assert(KP % 16 == 0 && KP >= 16 && KP <= 128, "N = 16..128, step 16");
+    using T = WgTile<STRIDE>;
     constexpr uint32_t IDESC = umma_idesc_bf16(kUmBM, KP) | (1u << 15) | (1u << 16);  // A, B MN-major
-    constexpr int B_BYTES = KP * kWgPix * 2;
+    constexpr uint32_t TCOLS = tmem_cols<3 * KP>();
     extern __shared__ __align__(1024) uint8_t um_smem[];
-    __shared__ __align__(8) uint64_t mbar[kUmStages];
+    __shared__ __align__(8) uint64_t mbar[6];  // landed, freed
     __shared__ uint32_t tmem_base;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int M = d.N * d.P * d.Q;
-    const int rows = 9 * d.C;
-    const int tiles = div_up(rows, kUmBM);
-    const int t0 = blockIdx.x * ntg;                 // first row tile of this CTA
-    const int nt = imin(ntg, tiles - t0);            // row tiles of this CTA
-    const int stage_bytes = ntg * kWgTile + B_BYTES;
-    const int m_lo = blockIdx.y * pix_per_cta;
-    const int m_hi = imin(M, m_lo + pix_per_cta);
-    const int nst = m_hi > m_lo ? div_up(m_hi - m_lo, kWgPix) : 0;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
+    const int kc0 = blockIdx.x * groups, planes = 3 * imin(groups, d.C / 8 - kc0);
+    const int gx = div_up(d.Q, 8), gy = div_up(d.P, 16), tiles = gx * gy * d.N;
+    const int nt = div_up(tiles - (int)blockIdx.y, (int)gridDim.y);
+    const uint32_t a_bytes = (uint32_t)(3 * groups * T::PXA * 16), stage = a_bytes + KP / 8 * T::PXB * 16;
+    const uint32_t sbase = smem_u32(um_smem);
+    const uint32_t full = smem_u32(mbar), freed = full + 24;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                          smem_u32(&tmem_base)),
-                     "r"(tcols)
+                     "r"(TCOLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        for (int i = 0; i < kUmStages; i++) mbar_init(smem_u32(&mbar[i]), 1);
+        for (int i = 0; i < bufs; i++) {
+            mbar_init(full + 8 * i, kWgNT - 32);
+            mbar_init(freed + 8 * i, 1);
+        }
         fence_mbar_init();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
-    const uint32_t sbase = smem_u32(um_smem);
-
-    // This thread gathers pixel j = 8 warp + (lane & 7) of every stage, for the
-    // 8-row groups g = 4 i + (lane >> 3) of A and the channel groups
-    // kg = 4 i + (lane >> 3) of B.  Row group g: tap, first channel, and the
-    // element offset of its 8 channels from the tap's centre pixel.
-    const int j = warp * 8 + (lane & 7), gs = lane >> 3;
-    int toff[kWgMT * 4], tap_rs[kWgMT * 4];
-#pragma unroll
-    for (int i = 0; i < kWgMT * 4; i++) {
-        const int R = (t0 * 16 + 4 * i + gs) * 8;  // first row of the group
-        if (i < nt * 4 && R < rows) {
-            const int tap = R / d.C, c = R % d.C, r = tap / 3, sx = tap % 3;
-            toff[i] = (r * d.W + sx) * d.C + c;
-            tap_rs[i] = r | (sx << 2);
-        } else {
-            toff[i] = 0;
-            tap_rs[i] = -1;
-        }
-    }
-    const uint32_t jo = (uint32_t)((j >> 3) * 128 + (j & 7) * 16);
-
-    auto gather = [&](int s) {
-        const uint32_t a = sbase + (s % kUmStages) * stage_bytes;
-        const uint32_t b = a + ntg * kWgTile;
-        const int m = m_lo + s * kWgPix + j;
-        const bool mv = m < m_hi;
-        int y0 = 0, x0 = 0;
-        long long pbase = 0;
-        if (mv) {
-            const int q = m % d.Q, t = m / d.Q, p = t % d.P, n = t / d.P;
-            y0 = p * d.stride - 1;
-            x0 = q * d.stride - 1;
-            pbase = (((long long)n * d.H + y0) * d.W + x0) * d.C;
-        }
-#pragma unroll
-        for (int i = 0; i < kWgMT * 4; i++) {
-            if (i < nt * 4) {
-                const int rs = tap_rs[i];
-                const bool ok = mv && rs >= 0 && (unsigned)(y0 + (rs & 3)) < (unsigned)d.H &&
-                                (unsigned)(x0 + (rs >> 2)) < (unsigned)d.W;
-                cp_async16(a + (uint32_t)(4 * i + gs) * 512 + jo, ok ? x + pbase + toff[i] : x, ok);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < (KP / 8 + 3) / 4; i++) {
-            const int kg = 4 * i + gs;
-            if (kg < KP / 8) {
-                const bool ok = mv && kg * 8 < d.K;
-                cp_async16(b + (uint32_t)kg * 512 + jo, ok ? gb + (size_t)m * d.K + kg * 8 : gb, ok);
-            }
-        }
-    };
-
-    // one cp.async group per stage (empty past the last), so waiting until
-    // kWgAhead groups are pending means stage s has landed
     bool timed_out = false;
+
+    if (warp > 0) {
+        // a thread keeps its plane of x and its channels of g; lanes run over the
+        // planes of a pixel first: the shifted ones share lines
+        const int astep = (kWgNT - 32) / planes, pl = (tid - 32) % planes, apx = (tid - 32) / planes;
+        const int kc = pl / 3, sx = pl - 3 * kc;
+        constexpr int KG = KP / 8, BSTEP = (kWgNT - 32) / KG;
+        const int kg = (tid - 32) % KG, bpx = (tid - 32) / KG;
+        int buf = 0, ph = 1, abuf = 0;
 #pragma unroll 1
-    for (int s = 0; s < kWgAhead; s++) {
-        if (s < nst) gather(s);
-        cp_async_commit();
-    }
-#pragma unroll 1
-    for (int s = 0; s < nst; s++) {
-        const int sl = s + kWgAhead;
-        if (sl < nst) {
-            // buffer sl % 4 last held stage sl - 4 = s - 2, committed two stages ago
-            if (sl >= kUmStages && !timed_out) {
-                const int so = sl - kUmStages;
-                if (!mbar_wait_bounded(smem_u32(&mbar[so % kUmStages]), (so / kUmStages) & 1))
-                    timed_out = true;
+        for (int i = 0; i < nt; i++) {
+            if (i >= bufs && !mbar_wait_bounded(freed + 8 * buf, ph)) {
+                timed_out = true;
+                break;
             }
-            gather(sl);
-        }
-        cp_async_commit();
-        cp_async_wait<kWgAhead>();
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const int buf = s % kUmStages;
-            const uint32_t a = sbase + buf * stage_bytes, b = a + ntg * kWgTile;
-#pragma unroll 1
-            for (int t = 0; t < nt; t++) {
-#pragma unroll
-                for (int h = 0; h < kWgPix / 16; h++) {
-                    const uint64_t ad = umma_desc(a + t * kWgTile + h * 256, 128, 512);
-                    const uint64_t bd = umma_desc(b + h * 256, 128, 512);
-                    umma_bf16(tmem + (uint32_t)(t * KP), ad, bd, IDESC, (s > 0 || h > 0) ? 1u : 0u);
+            const int t = blockIdx.y + i * gridDim.y;
+            const int q0 = t % gx * 8, p0 = t / gx % gy * 16, n = t / (gx * gy);
+            const uint32_t a = sbase + (uint32_t)buf * stage, b = a + a_bytes;
+            const __nv_bfloat16 *xn = x + (size_t)n * d.H * d.W * d.C + (kc0 + kc) * 8;
+            if (apx < astep)
+#pragma unroll 4
+                for (int px = apx; px < T::RH * 8; px += astep) {
+                    const int yy = STRIDE * p0 - 1 + (px >> 3), xx = STRIDE * (q0 + (px & 7)) + sx - 1;
+                    const bool ok = (unsigned)yy < (unsigned)d.H && (unsigned)xx < (unsigned)d.W;
+                    cp_async16(a + (uint32_t)(pl * T::PXA + px) * 16, ok ? xn + ((size_t)yy * d.W + xx) * d.C : x, ok);
                 }
+            const __nv_bfloat16 *gn = gb + (size_t)n * d.P * d.Q * d.K + kg * 8;
+            if (bpx < BSTEP)
+#pragma unroll 4
+                for (int px = bpx; px < 128; px += BSTEP) {
+                    const int p = p0 + (px >> 3), q = q0 + (px & 7);
+                    const bool ok = p < d.P && q < d.Q && kg * 8 < d.K;
+                    cp_async16(b + (uint32_t)(kg * T::PXB + px) * 16, ok ? gn + ((size_t)p * d.Q + q) * d.K : gb, ok);
+                }
+            cp_async_commit();
+            // the tile bufs - 1 loads ago has landed
+            if (i >= bufs - 1) {
+                if (bufs == 3) cp_async_wait<2>();
+                else cp_async_wait<1>();
+                fence_async_smem();
+                mbar_arrive(full + 8 * abuf);
+                if (++abuf == bufs) abuf = 0;
             }
-            umma_commit(smem_u32(&mbar[buf]));
+            if (++buf == bufs) {
+                buf = 0;
+                ph ^= 1;
+            }
+        }
+        cp_async_wait<0>();
+        if (!timed_out) {
+            fence_async_smem();
+            for (int i = imax(0, nt - bufs + 1); i < nt; i++) {
+                mbar_arrive(full + 8 * abuf);
+                if (++abuf == bufs) abuf = 0;
+            }
+        }
+    } else {
+        const bool issuer = elect_one();
+        const uint64_t adesc = umma_desc(0, STRIDE * 128, T::PXA * 16), bdesc = umma_desc(0, 128, T::PXB * 16);
+        int buf = 0, ph = 0;
+#pragma unroll 1
+        for (int i = 0; i < nt; i++) {
+            if (!mbar_wait_bounded(full + 8 * buf, ph)) {
+                timed_out = true;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t a = sbase + (uint32_t)buf * stage;
+            const uint64_t ad = adesc + (a >> 4), bd = bdesc + ((a + a_bytes) >> 4);
+            if (issuer) {
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        umma_bf16(tmem + (uint32_t)(r * KP), ad + (uint32_t)(8 * r + 16 * STRIDE * j),
+                                  bd + (uint32_t)(16 * j), IDESC, j == 0 && i == 0 ? 0u : 1u);
+                umma_commit(freed + 8 * buf);
+            }
+            __syncwarp();
+            // the last commit tracks every MMA of this CTA
+            if (i == nt - 1 && !mbar_wait_bounded(freed + 8 * buf, ph)) timed_out = true;
+            if (++buf == bufs) {
+                buf = 0;
+                ph ^= 1;
+            }
         }
     }
-    if (nst > 0) {
-        const int sL = nst - 1;
-        if (!timed_out && !mbar_wait_bounded(smem_u32(&mbar[sL % kUmStages]), (sL / kUmStages) & 1))
-            timed_out = true;
-    }
-    cp_async_wait<0>();
     timed_out = __syncthreads_or(timed_out);
     if (timed_out && tid == 0) atomicOr(err, 1);
     tc_fence_after();
-    if (!timed_out && nst > 0) {
+    if (!timed_out && nt > 0) {
+        const int row = (warp & 3) * 32 + lane, pl = row >> 3;  // TMEM lane = row of D
+        const int c = (kc0 + pl / 3) * 8 + (row & 7), sx = pl % 3;
 #pragma unroll 1
-        for (int t = 0; t < nt; t++) {
-            const int R = (t0 + t) * kUmBM + warp * 32 + lane;  // TMEM lane = row of D
-            const bool rv = R < rows;
-            const int tap = rv ? R / d.C : 0, c = rv ? R % d.C : 0;
-#pragma unroll 1
-            for (int cc = 0; cc < KP; cc += 16) {
-                uint32_t r[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * KP + cc), r);
-                if (!rv) continue;
+        for (int h = warp >> 2; h < 3 * (KP / 16); h += 2) {
+            const int r = h / (KP / 16), cc = h % (KP / 16) * 16;
+            uint32_t v[16];
+            tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(r * KP + cc), v);
+            if (pl >= planes) continue;
 #pragma unroll
-                for (int e = 0; e < 16; e++)
-                    if (cc + e < d.K) atomicAdd(gw + ((size_t)(cc + e) * 9 + tap) * d.C + c, __uint_as_float(r[e]));
-            }
+            for (int e = 0; e < 16; e++)
+                if (cc + e < d.K)
+                    atomicAdd(gw + ((size_t)(cc + e) * 9 + 3 * r + sx) * d.C + c, __uint_as_float(v[e]));
         }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tcols)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS)
                      : "memory");
+}
+
+template <int KP, int STRIDE>
+void launch_wgrad(const ConvDims &d, const __nv_bfloat16 *gb, const __nv_bfloat16 *x, float *gw,
+                  int *err, cudaStream_t st) {
+    using T = WgTile<STRIDE>;
+    const int tiles = div_up(d.Q, 8) * div_up(d.P, 16) * d.N;
+    if (tiles <= 0) return;
+    const int mtiles = div_up(d.C / 8, kWgGroups), groups = div_up(d.C / 8, mtiles);
+    const int a = 3 * groups * T::PXA * 16, stage = a + KP / 8 * T::PXB * 16;
+    // the MMAs read 16 planes from the start of a buffer
+    const auto bytes = [&](int bufs) { return bufs * stage + imax(0, 16 * T::PXA * 16 - stage); };
+    const int tm = 512 / (int)tmem_cols<3 * KP>();  // CTAs an SM by tensor memory
+    const int bufs = bytes(3) <= kUmSmemMax / tm ? 3 : 2;
+    const int smem = bytes(bufs);
+    OF_CUDA(cudaFuncSetAttribute(k_conv_wgrad_mn<KP, STRIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // one wave of the CTAs that fit by shared and tensor memory
+    const int occ = imax(1, imin(227 * 1024 / (smem + 1024), tm));
+    const int splits = imin(tiles, imax(1, kNumSMs * occ / mtiles));
+    k_conv_wgrad_mn<KP, STRIDE><<<dim3(mtiles, splits), kWgNT, smem, st>>>(d, gb, x, gw, groups, bufs, err);
 }
 
 template <int KP>
 void launch_wgrad(const ConvDims &d, const __nv_bfloat16 *gb, const __nv_bfloat16 *x, float *gw,
                   int *err, cudaStream_t st) {
-    const int M = d.N * d.P * d.Q;
-    if (M <= 0) return;
-    const int tiles = div_up(9 * d.C, kUmBM);
-    const int groups = div_up(tiles, kWgMT);
-    const int ntg = div_up(tiles, groups);  // row tiles a CTA, balanced over the groups
-    const int smem = kUmStages * (ntg * kWgTile + KP * kWgPix * 2);
-    uint32_t tcols = 32;
-    while (tcols < (uint32_t)(ntg * KP)) tcols <<= 1;
-    OF_CUDA(cudaFuncSetAttribute(k_conv_wgrad_mn<KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    // CTAs an SM holds by shared memory and tensor memory; one wave of them
-    const int occ = imax(1, imin((227 * 1024) / (smem + 1024), (int)(512 / tcols)));
-    const int splits = imax(1, imin(div_up(M, kWgPix), div_up(kNumSMs * occ, groups)));
-    const int per = div_up(div_up(M, splits), kWgPix) * kWgPix;
-    k_conv_wgrad_mn<KP><<<dim3(groups, div_up(M, per)), kUmNT, smem, st>>>(d, gb, x, gw, ntg, per, tcols, err);
+    if (d.stride == 1) launch_wgrad<KP, 1>(d, gb, x, gw, err, st);
+    else launch_wgrad<KP, 2>(d, gb, x, gw, err, st);
 }
 
 // bf16 copy of the output gradient, zero where the layer's ReLU was inactive

@@ -44,3 +44,26 @@ def test_forward_and_backward_data(of, N, H, W, C, K, stride):
     of.conv3x3(1, N, H, W, C, K, stride, False, True, rep(gout), None, w.cuda(), gx)
     got = gx.cpu().numpy()
     assert all(_rel(got[i:i + m], gx_ref) < REL for i in range(0, N, m))
+
+
+@pytest.mark.parametrize("N,H,W,C,K,stride", [
+    (1, 1, 1, 16, 8, 1), (1, 16, 8, 32, 16, 1), (2, 17, 9, 48, 48, 1), (3, 31, 15, 80, 128, 1), (2, 50, 70, 96, 80, 1),
+    (1, 2, 2, 16, 32, 2), (2, 33, 17, 32, 96, 2), (1, 64, 31, 208, 112, 2), (40, 47, 33, 16, 24, 1),
+])
+def test_backward_weight(of, N, H, W, C, K, stride):
+    """Channel groups of every remainder (up to five a block), pixel tiles with
+    remainders, one tile and several a block, K padded to 16."""
+    import torch
+    from oracle import cnn_ref
+    g = torch.Generator().manual_seed(H * 100 + W + C + 1)
+    P, Q = cnn_ref.conv_out(H, stride), cnn_ref.conv_out(W, stride)
+    x = torch.randn((N, H, W, C), generator=g).bfloat16()
+    gout = torch.randn((N, P, Q, K), generator=g).bfloat16().float()
+    w = torch.zeros((K, 3, 3, C)).bfloat16()
+    gw_ref = cnn_ref.backward(x.float().numpy(), w.float().numpy(), gout.numpy(), stride, None)[1]
+    gw = torch.full((K, 3, 3, C), float("nan"), dtype=torch.float32, device="cuda")
+    gb = torch.empty(K, dtype=torch.float32, device="cuda")
+    of.conv3x3(2, N, H, W, C, K, stride, False, True, gout.cuda(), None, x.cuda(), gw, gbias=gb)
+    torch.cuda.synchronize()
+    # gw is [K][3][3][C]; float32 sums of N P Q exact products
+    assert _rel(gw.cpu().numpy(), gw_ref) < REL
