@@ -583,15 +583,30 @@ enum { kWarpFromU = 0, kWarpFromUz = 1, kWarpZero = 2 };
 
 // The first pass of each sample reads the column coefficients of its four
 // columns (k_cubic_pack) and evaluates them at ty; only the second pass runs
-// the whole cell.  6 blocks of 256 per SM: the gathers need the warps to hide
-// their latency.  Splitting the channels over three threads per pixel (all
-// eight gathers of a channel in flight, the samples combined in shared
-// memory) measured slower: 4.10 against 2.48 ms for the 25 warps of the
-// 1024x436 workload at 32 pairs.
+// the whole cell.  The waits for memory bound it (two in a row, the flow and then
+// the gathers; the conversions between float and double use 56 % of their unit):
+// 6 blocks of 256 per SM (5: 2.46 ms for the 25 warps of 32 pairs of 1024x436, 7:
+// 2.30), and the second wait is shortened by fetching the lines around the warp's
+// own pixels to L2 meanwhile (2.47 -> 2.19 ms).  Splitting the channels over three
+// threads per pixel measured slower (4.10 ms).
 constexpr int kWarpTW = 32, kWarpTH = 8;
+
+// One line a lane: the coefficients and the I0 samples of the warp's own pixels go
+// to L2 while the flow that says where to gather is still on its way.
+__device__ __forceinline__ void warp_prefetch(const float *I0, const WarpCoef &wc, size_t off, int nx, int y) {
+    const int lane = threadIdx.x, x0 = blockIdx.x * kWarpTW;
+    const int k = lane & 3, x = x0 + (lane < 16 ? 8 * k : 16 * (lane & 1));
+    if (lane >= 19 || x >= nx) return;
+    const size_t q = off + (size_t)y * nx + x;
+    const void *a = lane < 4 ? (const void *)(wc.cc0 + q) : lane < 8 ? (const void *)(wc.cc1 + q)
+                  : lane < 12 ? (const void *)(wc.cc2 + q) : lane < 16 ? (const void *)(wc.dv01 + q)
+                  : lane < 18 ? (const void *)(wc.dv2 + q) : (const void *)(I0 + (size_t)y * nx + x0);
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(a));
+}
+
 __global__ void __launch_bounds__(kWarpTW * kWarpTH, 6) k_warp(const float *__restrict__ pyr, size_t pyr_stride, WarpCoef wc,
                        float2 *W, float2 *U0, float2 *U1, const float2 *Uz, float2 *P, size_t plane,
-                       size_t stride, int nx, int ny, int mode, int first_warp,
+                       size_t stride, int nx, int ny, int mode, int first_warp, int ahead,
                        TvCtrl *ctrl, TbQueue *q, int *left) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -606,6 +621,7 @@ __global__ void __launch_bounds__(kWarpTW * kWarpTH, 6) k_warp(const float *__re
         q[b].ticket = 0;  // the persistent form's work queue, re-armed per stage
         if (b == 0) *left = gridDim.z;
     }
+    if (ahead && y < ny) warp_prefetch(pyr + (size_t)(2 * b) * pyr_stride, wc, (size_t)b * stride, nx, y);
     if (x >= nx || y >= ny) return;
     const int cur = ctrl[b].cur;
     const size_t off = (size_t)b * stride, p = (size_t)y * nx + x;
@@ -2362,12 +2378,17 @@ void TvPlan::record(cudaStream_t st) {
         dim3 ig(div_up(nx, kIterTW), div_up(ny, kIterTH), B);
         const int cfg = tb_cfg_[s];
         const dim3 wb(kWarpTW, kWarpTH), wg(div_up(nx, kWarpTW), div_up(ny, kWarpTH), B);
+        // 72 bytes of coefficients a pixel: more than the L2 keeps from one warp to
+        // the next.  25 warps of 32 pairs of 1024x436 take 2.47 ms without and 2.19
+        // with, of a pair of 1920x1080 436 and 412 us, 1024x768 (57 MB) 221 and 217,
+        // 960x540 (37 MB) 172 and 179, 640x480 133 and 142.
+        const int ahead = (size_t)nx * ny * B * 72 > ((size_t)48 << 20);
         for (int wi = 0; wi < sw_[s]; wi++) {
             const int mode = wi > 0 ? kWarpFromU
                                     : (s == s0_ ? (warm_ ? kWarpFromUz : kWarpZero) : kWarpFromUz);
             mark_begin(-1);
             k_warp<<<wg, wb, 0, st>>>(pyr + pyr_off_[s], lp, wc, W, U0, U1, Uz, P, plane, N0,
-                                       nx, ny, mode, wi == 0, ctrl, queue, left);
+                                       nx, ny, mode, wi == 0, ahead, ctrl, queue, left);
             mark_end();
             launches_ += 1;
             ia.stage = s * prm_.warps + wi;
