@@ -397,6 +397,147 @@ __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant
     }
 }
 
+// All sweeps of a warp of a small level in one launch: a cluster of blocks holds a
+// pair's level, a tile each, in the registers of k_hs_jacobi's sweeps.  Every K
+// sweeps the blocks lay the pixels they own in shared memory, meet at the cluster's
+// barrier and take their halos from the owners' (two buffers, so that one barrier
+// is enough).  A launch per 8 sweeps waits for its own start and its tile's data:
+// 152 sweeps of a level take (19 launches without the gaps between them, and here)
+//   40x30 103 and 68 us, 80x60 102 and 70, 160x120 109 and 87; 9 pairs of 160x120
+//   173 and 135, 16 pairs of 80x60 112 and 115, 37 pairs 176 and 178.
+// One block an SM instead of two saves the spills (160x120 83 us) and costs batches
+// more (9 pairs 166).  The barriers of the block and the cluster bound it.
+//
+// The guard is looked at once, at the end: where any block of the cluster broke
+// it, all of them run the warp again with IEEE divisions.
+template <typename T> struct HsRes {
+    float2 own[2][T::TH][T::TW];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(T::NT, 2) k_hs_res(const __grid_constant__ HsJacobiArgs a) {
+    constexpr int V = T::V, K = T::K, NW = T::NW;
+    static_assert(K % V == 0 && K % 2 == 0, "owned pixels are whole threads");
+    extern __shared__ __align__(128) char hs_dyn[];
+    HsRes<T> &sm = *reinterpret_cast<HsRes<T> *>(hs_dyn);
+    __shared__ float4 sRow[2][2][NW][32];
+    __shared__ int s_bad;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, w = a.w, h = a.h;
+    const HsAt t = hs_at<T>(a, blockIdx.x);
+    const int x = t.x, y0 = t.y0, blocks = a.tiles_x * a.tiles_y;
+    const bool in0 = x >= 0 && x < w, in1 = x + 1 >= 0 && x + 1 < w;
+    const bool own = lane >= K / 2 && lane < 32 - K / 2 && wid >= K / V && wid < NW - K / V;
+    HsState<V> s;
+    bool broken = false;
+    {
+        const float2 *D0 = a.D + (size_t)t.b * a.dstride, *D1 = D0 + a.plane;
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+            const bool iy = y0 + v >= 0 && y0 + v < h;
+            const size_t q = iy && in0 ? (size_t)(y0 + v) * w + x : 0;
+            const float4 d0 = hs_ld_two(D0, q, a.vec, iy && in0, iy && in0 && in1);
+            const float4 d1 = hs_ld_two(D1, q, a.vec, iy && in0, iy && in0 && in1);
+            s.ix[v][0] = d0.x; s.iy[v][0] = d0.y; s.iz[v][0] = d1.x; s.den[v][0] = iy && in0 ? d1.y : 1.0f;
+            s.ix[v][1] = d0.z; s.iy[v][1] = d0.w; s.iz[v][1] = d1.z; s.den[v][1] = iy && in0 && in1 ? d1.w : 1.0f;
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < V; v++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            s.rcp[v][c] = rcp_near_rn(s.den[v][c]);
+            broken |= !rcp_in_range(s.den[v][c]);
+        }
+    const bool interior = t.ox >= 1 && t.oy >= 1 && t.ox + T::RW <= w - 1 && t.oy + T::RH <= h - 1;
+    const bool plain = t.oy + T::RH <= h - 1 && (w & 1) == 0;
+    const HsEdge e{x == 0, x + 1 == w - 1, x == w - 1, h - 1 - y0};
+    const bool top = y0 == 0;
+    const auto taken = [] {};
+
+    auto exchange = [&](int buf) {
+        if (own) {
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                const bool iy = y0 + v < h;
+                if (!iy || !in0) s.a[v][0] = make_float2(0.f, 0.f);
+                if (!iy || !in1) s.a[v][1] = make_float2(0.f, 0.f);
+                *reinterpret_cast<float4 *>(&sm.own[buf][wid * V + v - K][2 * lane - K]) =
+                    make_float4(s.a[v][0].x, s.a[v][0].y, s.a[v][1].x, s.a[v][1].y);
+            }
+        }
+        cluster_barrier();
+        if (!own) {
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                const int y = y0 + v;
+                float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (in0 && y >= 0 && y < h) {  // zeros beyond an odd width are the owner's
+                    const int tx = x / T::TW, ty = y / T::TH;
+                    u = cluster_ld4(smem_u32(&sm.own[buf][y - ty * T::TH][x - tx * T::TW]), ty * a.tiles_x + tx);
+                }
+                s.a[v][0] = make_float2(u.x, u.y);
+                s.a[v][1] = make_float2(u.z, u.w);
+            }
+        }
+    };
+
+#pragma unroll 1
+    for (int exact = 0; exact < 2; exact++) {
+        unsigned key = ~0u;
+#pragma unroll
+        for (int v = 0; v < V; v++) s.a[v][0] = s.a[v][1] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int done = 0, buf = 0; done < a.sweeps; done += K, buf ^= 1) {
+            const int n = imin(K, a.sweeps - done);
+            if (exact) {
+#pragma unroll 1
+                for (int j = 0; j < n; j++) hs_step<T, 2, true>(s, j, sRow, top, e, key, taken);
+            } else if (n != K) {
+#pragma unroll 1
+                for (int j = 0; j < n; j++) hs_step<T, 2, false>(s, j, sRow, top, e, key, taken);
+            } else if (interior) {
+#pragma unroll 2
+                for (int j = 0; j < K; j++) hs_step<T, 0, false>(s, j, sRow, top, e, key, taken);
+            } else if (plain) {
+#pragma unroll 2
+                for (int j = 0; j < K; j++) hs_step<T, 1, false>(s, j, sRow, top, e, key, taken);
+            } else {
+#pragma unroll 2
+                for (int j = 0; j < K; j++) hs_step<T, 2, false>(s, j, sRow, top, e, key, taken);
+            }
+            if (done + K < a.sweeps) exchange(buf);
+        }
+        // whether any block of the cluster broke the guard (the barriers also end the
+        // reads of this block's shared memory)
+        const int bad = __syncthreads_or(!exact && (broken || key < kMarksteinKey));
+        if (threadIdx.x == 0) s_bad = bad;
+        cluster_barrier();
+        const int any = threadIdx.x < blocks ? cluster_ld1(smem_u32(&s_bad), threadIdx.x) : 0;
+        const bool again = __syncthreads_or(any != 0);
+        cluster_barrier();
+        if (!again) break;
+    }
+    if (!own || x >= w) return;
+    float2 *Out = (a.last ? a.U : a.out) + (size_t)t.b * a.stride;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        if (y0 + v >= h) break;
+        const size_t q = (size_t)(y0 + v) * w + x;
+        float2 r0 = s.a[v][0], r1 = s.a[v][1];
+        if (a.last) {
+            const float4 u = hs_ld_two(Out, q, a.vec, true, in1);
+            r0 = make_float2(u.x + r0.x, u.y + r0.y);
+            r1 = make_float2(u.z + r1.x, u.w + r1.y);
+        }
+        if (a.vec) {
+            *reinterpret_cast<float4 *>(Out + q) = make_float4(r0.x, r0.y, r1.x, r1.y);
+        } else {
+            Out[q] = r0;
+            if (in1) Out[q + 1] = r1;
+        }
+    }
+}
+
 // Flow prolongation (upscaleKernel.cuh:26-40 as a filtering upscale):
 // bilinear, clamp-to-edge, centre-aligned, component-wise scale.
 __device__ __forceinline__ float2 bilinear2(const float2 *__restrict__ src, int w, int h,
@@ -602,15 +743,6 @@ template <int C> static void hs_set_smem_attr() {
     OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<HsCfgTile<C>, kHsCfgs[C].mb>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, hs_smem<C>()));
 }
-static void hs_set_smem_attrs() {
-    hs_set_smem_attr<0>();
-    hs_set_smem_attr<1>();
-    hs_set_smem_attr<2>();
-    hs_set_smem_attr<3>();
-    hs_set_smem_attr<4>();
-    hs_set_smem_attr<5>();
-}
-
 static void hs_jacobi_cfg(int c, int B, cudaStream_t st, const HsJacobiArgs &a) {
     switch (c) {
         case 1: hs_jacobi_launch<1>(B, st, a); break;
@@ -622,10 +754,68 @@ static void hs_jacobi_cfg(int c, int B, cudaStream_t st, const HsJacobiArgs &a) 
     }
 }
 
-// All sweeps of one warp: from zero increments to the flow updated.
+// Resident levels: tiles of 48x16 with 8 sweeps between exchanges or, where those
+// are more than a cluster's 16 blocks, of 56x24 with 4.
+using HsRes8 = HsTile<2, 16, 8>;
+using HsRes4 = HsTile<2, 16, 4>;
+template <typename T> static bool hs_res_fits(int w, int h) { return div_up(w, T::TW) * div_up(h, T::TH) <= 16; }
+
+template <typename T> static void hs_res_launch(int B, cudaStream_t st, HsJacobiArgs a) {
+    a.tiles_x = div_up(a.w, T::TW);
+    a.tiles_y = div_up(a.h, T::TH);
+    a.tiles = a.tiles_x * a.tiles_y * B;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = a.tiles_x * a.tiles_y;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(a.tiles);
+    lc.blockDim = dim3(T::NT);
+    lc.dynamicSmemBytes = sizeof(HsRes<T>);
+    lc.stream = st;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    OF_CUDA(cudaLaunchKernelEx(&lc, k_hs_res<T>, a));
+}
+
+template <typename T> static void hs_res_attrs() {
+    OF_CUDA(cudaFuncSetAttribute(k_hs_res<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HsRes<T>)));
+    OF_CUDA(cudaFuncSetAttribute(k_hs_res<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+}
+
+static void hs_set_smem_attrs() {
+    hs_set_smem_attr<0>();
+    hs_set_smem_attr<1>();
+    hs_set_smem_attr<2>();
+    hs_set_smem_attr<3>();
+    hs_set_smem_attr<4>();
+    hs_set_smem_attr<5>();
+    hs_res_attrs<HsRes8>();
+    hs_res_attrs<HsRes4>();
+}
+
+// All sweeps of one warp: from zero increments to the flow updated.  The small
+// tiles run resident where a cluster holds the level.
 static void hs_sweeps(int cfg, int B, cudaStream_t st, const float2 *D, size_t plane, float2 *const dU[2],
                       float2 *U, size_t stride, int w, int h, int sweeps, bool update, int *err) {
     const int K = kHsCfgs[cfg].k;
+    if (cfg == 5 && sweeps > 0 && (hs_res_fits<HsRes8>(w, h) || hs_res_fits<HsRes4>(w, h))) {
+        HsJacobiArgs a;
+        memset(&a, 0, sizeof(a));
+        a.D = D;
+        a.plane = plane;
+        a.dstride = a.stride = stride;
+        a.out = dU[1];
+        a.U = U;
+        a.w = w;
+        a.h = h;
+        a.sweeps = sweeps;
+        a.last = update;
+        a.vec = (w & 1) == 0 && (stride & 1) == 0;
+        if (hs_res_fits<HsRes8>(w, h)) hs_res_launch<HsRes8>(B, st, a);
+        else hs_res_launch<HsRes4>(B, st, a);
+        return;
+    }
     for (int done = 0, cur = 0; done < sweeps; cur ^= 1) {
         const int k = imin(K, sweeps - done);
         HsJacobiArgs a;
@@ -651,8 +841,9 @@ static void hs_sweeps(int cfg, int B, cudaStream_t st, const float2 *D, size_t p
 // The configuration of a level; OFLOW_HS_CFG forces one (used to test and time
 // them), and a plan's tuning table comes before it.  A level whose 48x16 tiles
 // all fit on the GPU at once is bound by the launches' latency: small tiles of 8
-// sweeps (150 sweeps of a single 160x120, 80x60 or 40x30 level: 0.12 ms against
-// 0.16 with 48x48 tiles, 0.15 to 0.22 with 4 sweeps a launch).  Larger work takes
+// sweeps, resident where a cluster holds the level (150 sweeps of a single
+// 160x120, 80x60 or 40x30 level in launches: 0.12 ms against 0.16 with 48x48
+// tiles, 0.15 to 0.22 with 4 sweeps a launch).  Larger work takes
 // 48x48 tiles of 8 sweeps (64 pairs of 320x240, 200 sweeps: 2.7 ms against 3.1 to
 // 3.7).
 static int hs_pick(int w, int h, int B) {

@@ -67,6 +67,33 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
                  : "memory");
 }
 
+// All threads of the cluster meet; what they wrote to shared memory before is
+// visible to each other after.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// Loads from the shared memory of block `rank` of the cluster, at the address a
+// has in this block.
+__device__ __forceinline__ float4 cluster_ld4(uint32_t a, int rank) {
+    float4 v;
+    asm volatile(
+        "{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %4, %5;\n\t"
+        "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [r];\n\t}\n"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "r"(a), "r"(rank)
+        : "memory");
+    return v;
+}
+__device__ __forceinline__ int cluster_ld1(uint32_t a, int rank) {
+    int v;
+    asm volatile(
+        "{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.s32 %0, [r];\n\t}\n"
+        : "=r"(v)
+        : "r"(a), "r"(rank)
+        : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
 }

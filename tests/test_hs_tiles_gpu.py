@@ -34,6 +34,37 @@ def test_several_tiles_per_block(of, orc):
     assert all(np.array_equal(u, ou) and np.array_equal(v, ov) for u, v in res)
 
 
+@pytest.mark.parametrize("n", [1, 3])
+@pytest.mark.parametrize("sweeps", [1, 4, 7, 8, 9, 24])
+@pytest.mark.parametrize("w,h", [(1, 1), (48, 128), (49, 65), (192, 64), (193, 63), (224, 96), (113, 169), (57, 361),
+                                 (225, 97), (784, 10)])
+def test_resident_levels(of, orc, w, h, sweeps, n):
+    """Levels of one and of several blocks of a cluster, up to 16 of 48x16 (8
+    sweeps between exchanges) and of 56x24 (4), and the first ones beyond."""
+    from oflow import synth
+    qs = [synth.hs_pair(seed=w + h + k, w=w, h=h) for k in range(n)]
+    c = of.Context(0)
+    res = of.hs_batch([(q.I0, q.I1) for q in qs], of.HSParams(4.0, 1, 2, sweeps), c)
+    c.close()
+    for q, (u, v) in zip(qs, res):
+        ou, ov = orc.hs(q.I0, q.I1, 4.0, 1, 2, sweeps)
+        assert np.array_equal(u, ou) and np.array_equal(v, ov)
+
+
+@pytest.mark.parametrize("w,h", [(130, 70), (131, 45), (200, 90)])
+@pytest.mark.parametrize("scale,alpha", [(1e-32, 1.0), (1e4, 1.0), (0.0, 1e-14)])
+def test_resident_guard(of, orc, scale, alpha, w, h):
+    """One pair: the whole cluster runs the warp again with IEEE divisions."""
+    from oflow import synth
+    q = synth.hs_pair(seed=11, w=w, h=h)
+    a, b = (q.I0 * scale).astype(np.float32), (q.I1 * scale).astype(np.float32)
+    c = of.Context(0)
+    u, v = of.hs(a, b, of.HSParams(alpha, 1, 1, 19), c)
+    c.close()
+    ou, ov = orc.hs(a, b, alpha, 1, 1, 19)
+    assert np.array_equal(u, ou) and np.array_equal(v, ov)
+
+
 @pytest.mark.parametrize("w", [130, 131])
 @pytest.mark.parametrize("scale,alpha", [(1e-32, 1.0), (1e4, 1.0), (0.0, 1e-14)])
 def test_guard(of, orc, scale, alpha, w):
