@@ -126,7 +126,8 @@ template <int NT, int RW, int RH, typename F> __device__ __forceinline__ void fo
 // window sums and solve.  Pixels closer than the window radius to the border
 // get 0.  The five frames of a 1280x720 step used to be copied into the plan and
 // the flow out of it (31 of 96 us), and the sums ran one pixel a thread (65 us);
-// with eight pixels a thread the whole step takes 28 us.
+// with four pixels a thread the whole step takes 26.6 us (with eight 27.7, with
+// fewer blocks in flight).
 struct LkStep {
     const uint8_t *src[kLMaxT];
     long long pitch[kLMaxT];
@@ -188,10 +189,14 @@ __global__ void __launch_bounds__(kLTile *kLTile / (2 * PY)) k_lk_step(const __g
         }
 }
 
+// Rows a thread in launches that fill the GPU: two where the windows are wide and
+// the blocks' shared memory with them, else four, whose windows share more
+// (1920x1080, 9x9: 69.6 us with two, 77.0 with four; 5x5: 32.4 and 31.4).
 template <int C, int NS> static void lk_step_launch(const LkStep &a, cudaStream_t st) {
+    constexpr int PY = C > 2 ? 2 : 4;
     const dim3 g(div_up(a.nx, kLTile), div_up(a.ny, kLTile));
     if ((size_t)g.x * g.y > 4 * (size_t)kNumSMs)
-        k_lk_step<C, NS, 4><<<g, kLTile * kLTile / 8, 0, st>>>(a);
+        k_lk_step<C, NS, PY><<<g, kLTile * kLTile / (2 * PY), 0, st>>>(a);
     else
         k_lk_step<C, NS, 1><<<g, kLTile * kLTile / 2, 0, st>>>(a);
 }

@@ -360,16 +360,18 @@ __device__ __forceinline__ double gauss_sum(const float *c, int step, const Gaus
 // SRC 0: float planes at src; 1 / 2: uint8 / float frames through the frame
 // table (plane z = frame z of the table), converted to float on load.  A
 // uint8 frame is normalised through a 256-entry table of the same expression.
-// Tile kGaussTW x kGaussTH outputs, 256 threads as 32 x 8.
+// Tile kGaussTW x kGaussTH outputs, 256 threads as 32 x 8.  With the radius known,
+// four outputs a thread share their samples and inner regions skip the mirror, as
+// in k_gauss_dec2 (level 0 of 32 uint8 pairs of 1024x436: 154 -> 130 us).
 template <int SRC, int RT>
 __global__ void __launch_bounds__(kGaussNT) k_gauss(const float *__restrict__ src, float *dst,
                                                     int nx, int ny, size_t plane_stride,
                                                     GaussTaps taps, const TvCtrl *ctrl,
                                                     int normalize, const FrameRef *frames) {
     constexpr int MR = RT > 0 ? RT : kGaussMaxR;
-    constexpr int LW = kGaussTW + 2 * MR, LH = kGaussTH + 2 * MR;
-    __shared__ float sIn[LH * LW];
-    __shared__ float sRow[LH * kGaussTW];
+    constexpr int LW = (kGaussTW + 2 * MR + 3) / 4 * 4, LH = kGaussTH + 2 * MR;
+    __shared__ __align__(16) float sIn[LH * LW];
+    __shared__ __align__(16) float sRow[LH * kGaussTW];
     __shared__ float sLut[SRC == 1 ? 256 : 1];
     const int R = RT > 0 ? RT : taps.size - 1;
     const int z = blockIdx.z;
@@ -393,21 +395,54 @@ __global__ void __launch_bounds__(kGaussNT) k_gauss(const float *__restrict__ sr
         __syncthreads();
     }
     const int lw = kGaussTW + 2 * R, lh = kGaussTH + 2 * R;
-    auto fetch = [&](int ly, int lx) -> float {
-        const int my = gauss_mirror(y0 - R + ly, ny), mx = gauss_mirror(x0 - R + lx, nx);
-        if (my < 0 || my >= ny || mx < 0 || mx >= nx) return 0.0f;
+    auto value = [&](int my, int mx) -> float {
         if (SRC == 0) return __ldg(in + (size_t)my * nx + mx);
         if (SRC == 1) return sLut[__ldg(static_cast<const uint8_t *>(f.p) + (size_t)my * f.pitch + mx)];
         float v = __ldg(static_cast<const float *>(f.p) + (size_t)my * f.pitch + mx);
         if (apply) v = (float)(255.0 * (double)(v - mn) / (double)den);
         return v;
     };
-    if (RT > 0)
+    auto fetch = [&](int ly, int lx) -> float {
+        const int my = gauss_mirror(y0 - R + ly, ny), mx = gauss_mirror(x0 - R + lx, nx);
+        if (my < 0 || my >= ny || mx < 0 || mx >= nx) return 0.0f;
+        return value(my, mx);
+    };
+    if (RT > 0 && x0 >= R && y0 >= R && x0 - R + LW <= nx && y0 - R + LH <= ny)
+        load_region<kGaussNT, LW, LH>(sIn, [&](int ly, int lx) { return value(y0 - R + ly, x0 - R + lx); });
+    else if (RT > 0)
         load_region<kGaussNT, LW, LH>(sIn, fetch);
     else
         for (int ly = ty; ly < lh; ly += kGaussNT / 32)
             for (int lx = tx; lx < lw; lx += 32) sIn[ly * LW + lx] = fetch(ly, lx);
     __syncthreads();
+    if (RT > 0) {
+        constexpr int NV = 4 + 2 * MR, NQ = (NV + 3) / 4;  // samples of four outputs
+        static_assert(kGaussTH == 4 * (kGaussNT / 32) && kGaussTW - 4 + 4 * NQ <= LW, "four rows a thread");
+        for (int i = threadIdx.x; i < LH * (kGaussTW / 4); i += kGaussNT) {
+            const int ly = i / (kGaussTW / 4), q = i % (kGaussTW / 4);
+            float v[4 * NQ];
+#pragma unroll
+            for (int k = 0; k < NQ; k++)
+                *reinterpret_cast<float4 *>(v + 4 * k) = *reinterpret_cast<const float4 *>(sIn + ly * LW + 4 * (q + k));
+            *reinterpret_cast<float4 *>(sRow + ly * kGaussTW + 4 * q) =
+                make_float4((float)gauss_sum<RT>(v + MR, 1, taps, R), (float)gauss_sum<RT>(v + MR + 1, 1, taps, R),
+                            (float)gauss_sum<RT>(v + MR + 2, 1, taps, R), (float)gauss_sum<RT>(v + MR + 3, 1, taps, R));
+        }
+        __syncthreads();
+        for (int cx = tx; cx < kGaussTW; cx += 32) {
+            const int x = x0 + cx;
+            if (x >= nx) break;
+            float v[NV];
+#pragma unroll
+            for (int k = 0; k < NV; k++) v[k] = sRow[(4 * ty + k) * kGaussTW + cx];
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                const int y = y0 + 4 * ty + m;
+                if (y < ny) out[(size_t)y * nx + x] = (float)gauss_sum<RT>(v + MR + m, 1, taps, R);
+            }
+        }
+        return;
+    }
     for (int ly = ty; ly < lh; ly += kGaussNT / 32)
         for (int cx = tx; cx < kGaussTW; cx += 32)
             sRow[ly * kGaussTW + cx] = (float)gauss_sum<RT>(sIn + ly * LW + cx + R, 1, taps, R);
@@ -432,16 +467,20 @@ __global__ void __launch_bounds__(kGaussNT) k_gauss(const float *__restrict__ sr
 // and the column pass on even rows only, with the same taps, mirror, pairing
 // and double sums as k_gauss, so every output is bit-identical to blur then
 // resample.  Tile: kDecTW x kDecTH outputs, 256 threads as 32 x 8; gridDim.z
-// = planes.
+// = planes.  With the radius known a thread forms four neighbouring outputs of
+// either pass from the 17 samples they share (R = 5) in registers instead of
+// reading 11 for each, and regions inside the plane are read without mirroring
+// (the four coarser levels of 32 pairs of 1024x436: 135 -> 122 -> 105 us).  The
+// float-double conversions and the way in bound it.
 constexpr int kDecTW = 32, kDecTH = 32, kDecNT = 256, kDecMaxR = 8;
 template <int RT>
 __global__ void __launch_bounds__(kDecNT) k_gauss_dec2(const float *__restrict__ src, size_t src_stride,
                                                        int nx, int ny, float *dst, size_t dst_stride,
                                                        int nxx, int nyy, GaussTaps taps) {
     constexpr int MR = RT > 0 ? RT : kDecMaxR;
-    constexpr int LW = 2 * kDecTW - 1 + 2 * MR, LH = 2 * kDecTH - 1 + 2 * MR;
-    __shared__ float sIn[LH * LW];
-    __shared__ float sRow[LH * kDecTW];
+    constexpr int LW = (2 * kDecTW - 1 + 2 * MR + 3) / 4 * 4, LH = 2 * kDecTH - 1 + 2 * MR;
+    __shared__ __align__(16) float sIn[LH * LW];
+    __shared__ __align__(16) float sRow[LH * kDecTW];
     const int R = RT > 0 ? RT : taps.size - 1;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const float *in = src + (size_t)blockIdx.z * src_stride;
@@ -454,16 +493,43 @@ __global__ void __launch_bounds__(kDecNT) k_gauss_dec2(const float *__restrict__
         if (my < 0 || my >= ny || mx < 0 || mx >= nx) return 0.0f;
         return __ldg(in + (size_t)my * nx + mx);
     };
-    if (RT > 0)
+    if (RT > 0 && ix0 >= 0 && iy0 >= 0 && ix0 + LW <= nx && iy0 + LH <= ny) {
+        const float *o = in + (size_t)iy0 * nx + ix0;  // nothing to mirror
+        load_region<kDecNT, LW, LH>(sIn, [&](int ly, int lx) { return __ldg(o + ly * nx + lx); });
+    } else if (RT > 0)
         load_region<kDecNT, LW, LH>(sIn, fetch);
     else
         for (int ly = ty; ly < lh; ly += kDecNT / 32)
             for (int lx = tx; lx < lw; lx += 32) sIn[ly * LW + lx] = fetch(ly, lx);
     __syncthreads();
+    const int x = x0 + tx;
+    if (RT > 0) {
+        constexpr int NV = 7 + 2 * MR, NQ = (NV + 3) / 4;  // samples of four outputs
+        for (int i = threadIdx.x; i < LH * (kDecTW / 4); i += kDecNT) {
+            const int ly = i / (kDecTW / 4), q = i % (kDecTW / 4);
+            float v[4 * NQ];
+#pragma unroll
+            for (int k = 0; k < NQ; k++)
+                *reinterpret_cast<float4 *>(v + 4 * k) = *reinterpret_cast<const float4 *>(sIn + ly * LW + 8 * q + 4 * k);
+            *reinterpret_cast<float4 *>(sRow + ly * kDecTW + 4 * q) =
+                make_float4((float)gauss_sum<RT>(v + MR, 1, taps, R), (float)gauss_sum<RT>(v + MR + 2, 1, taps, R),
+                            (float)gauss_sum<RT>(v + MR + 4, 1, taps, R), (float)gauss_sum<RT>(v + MR + 6, 1, taps, R));
+        }
+        __syncthreads();
+        if (x >= nxx) return;
+        float v[NV];
+#pragma unroll
+        for (int k = 0; k < NV; k++) v[k] = sRow[(8 * ty + k) * kDecTW + tx];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const int y = y0 + 4 * ty + m;
+            if (y < nyy) out[(size_t)y * nxx + x] = (float)gauss_sum<RT>(v + MR + 2 * m, 1, taps, R);
+        }
+        return;
+    }
     for (int ly = ty; ly < lh; ly += kDecNT / 32)
         sRow[ly * kDecTW + tx] = (float)gauss_sum<RT>(sIn + ly * LW + 2 * tx + R, 1, taps, R);
     __syncthreads();
-    const int x = x0 + tx;
     if (x >= nxx) return;
     for (int cy = ty; cy < kDecTH; cy += kDecNT / 32) {
         const int y = y0 + cy;
