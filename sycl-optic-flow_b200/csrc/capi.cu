@@ -76,8 +76,7 @@ namespace {
 // A mixed batch: one plan per (solver, size, dtype, parameters) group and one
 // graph with a parallel branch per group.
 struct MixedBatch {
-    std::vector<std::string> key;
-    std::vector<std::vector<int>> members;  // job indices per group
+    std::vector<std::string> key;           // per group: its key and size (a call's own jobs say which they are)
     std::vector<std::unique_ptr<TvPlan>> tv;
     std::vector<std::unique_ptr<HsPlan>> hs;
     std::vector<int> kind, slot;            // per group: solver and index into tv/hs
@@ -591,7 +590,6 @@ oflow_status oflow_batch(oflow_ctx *ctx, int n, const oflow_job *jobs) {
         if (!mb) {
             std::unique_ptr<MixedBatch> m(new MixedBatch());
             m->key = comp;
-            m->members = members;
             for (size_t g = 0; g < gkeys.size(); g++) {
                 const oflow_job &j = jobs[members[g][0]];
                 const int B = (int)members[g].size();
@@ -632,8 +630,8 @@ oflow_status oflow_batch(oflow_ctx *ctx, int n, const oflow_job *jobs) {
         // device frames and flows in place through the plans' tables; host
         // ones through the plans' own buffers
         auto bind_group = [&](auto &pl, size_t g, cudaStream_t s) {
-            for (size_t b = 0; b < mb->members[g].size(); b++) {
-                const oflow_job &j = jobs[mb->members[g][b]];
+            for (size_t b = 0; b < members[g].size(); b++) {
+                const oflow_job &j = jobs[members[g][b]];
                 const oflow_image *im[2] = {&j.I0, &j.I1};
                 for (int k = 0; k < 2; k++) {
                     if (im[k]->location == OFLOW_DEVICE) {
@@ -657,8 +655,8 @@ oflow_status oflow_batch(oflow_ctx *ctx, int n, const oflow_job *jobs) {
         };
         bool device_only = true;
         auto unstage = [&](size_t g, cudaStream_t s) {
-            for (size_t b = 0; b < mb->members[g].size(); b++) {
-                const oflow_job &j = jobs[mb->members[g][b]];
+            for (size_t b = 0; b < members[g].size(); b++) {
+                const oflow_job &j = jobs[members[g][b]];
                 if (j.out.location != OFLOW_HOST) continue;  // written in place
                 const float *ou = mb->kind[g] == OFLOW_SOLVER_TVL1 ? mb->tv[mb->slot[g]]->out_u((int)b)
                                                                    : mb->hs[mb->slot[g]]->out_u((int)b);
