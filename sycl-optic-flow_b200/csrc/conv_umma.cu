@@ -18,7 +18,8 @@
 // tap x 8 kcs channels take them, so that a stage is one bulk copy; the copies
 // run as many stages ahead as there are buffers.  One thread issues the MMAs of
 // 128 x NP x 16 of a stage and commits them to the mbarrier that frees its buffer.
-// Taps come in order and channels in order within a tap, whatever the tile.
+// Taps come in order and channels in order within a tap, whatever the tile; where the
+// channels come in several regions (C above some 500), all taps of a region first.
 //
 //   stride 1    the region is the tile and one pixel around it
 //   stride 2    even and odd columns of a region row lie apart, so that a tap's
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
     constexpr uint32_t TCOLS = tmem_cols<T::NACC * NP>();
     constexpr uint32_t IDESC = umma_idesc_bf16(kUmBM, NP);
     extern __shared__ __align__(1024) uint8_t um_smem[];
-    __shared__ __align__(8) uint64_t mbar[2 * kUmMaxBufs + 1];  // landed, freed; the region has landed
+    __shared__ __align__(8) uint64_t mbar[2 * kUmMaxBufs + 2];  // landed, freed; the region has landed, is done with
     __shared__ uint32_t tmem_base;
 
     const int tid = threadIdx.x, lane = tid & 31;
@@ -195,7 +196,8 @@ __global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
     const int nst = 9 * (d.C / 8 / kcs), per_reg = 9 * (cr / 8 / kcs);
     // accumulators with a column inside the image
     const int nacc = MODE == kUmDilated ? 4 : imin(MT, div_up(d.Q - q0, 8));
-    const uint32_t full = smem_u32(mbar), freed = full + 8 * kUmMaxBufs, regbar = freed + 8 * kUmMaxBufs;
+    const uint32_t full = smem_u32(mbar), freed = full + 8 * kUmMaxBufs, regbar = freed + 8 * kUmMaxBufs,
+                   regdone = regbar + 8;
 
     // first input row and column of the region
     const int y0 = MODE == kUmStride1 ? p0 - 1 : MODE == kUmStride2 ? 2 * p0 - 1 : p0 / 2;
@@ -229,6 +231,7 @@ __global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
             mbar_init(freed + 8 * i, 1);
         }
         mbar_init(regbar, NT - 32);
+        mbar_init(regdone, 1);
         fence_mbar_init();
     }
     tc_fence_before();
@@ -265,29 +268,45 @@ __global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
         cp_async_wait<0>();
         fence_async_smem();
         mbar_arrive(regbar);
-        int buf = 0, ph = 0, left = per_reg, c0 = 0;  // stage s: its buffer is freed for the (ph + 1)-th time
-        // with several regions every thread follows the phases
-        if (tid == 32 || per_reg < nst)
+        // The next region replaces one whose MMAs are done.  Thread 32 knows that
+        // from the last stage's buffer; the others wait on a barrier that can't pass
+        // them (the next commit to it needs their next arrival), which the buffers'
+        // could: those are freed once a stage, and tell two phases apart.
+        auto next_region = [&](int c0) {
+            load_region(c0);
+            cp_async_commit();
+            cp_async_wait<0>();
+            fence_async_smem();
+            mbar_arrive(regbar);
+        };
+        if (tid == 32) {
+            int buf = 0, ph = 0, left = per_reg, c0 = 0;  // stage s: its buffer is freed for the (ph + 1)-th time
 #pragma unroll 1
             for (int s = 0; s < nst; s++) {
                 if (!mbar_wait_bounded(freed + 8 * buf, ph)) {
                     timed_out = true;
                     break;
                 }
-                if (tid == 32 && issued < nst) fetch();
-                if (--left == 0 && s + 1 < nst) {  // the region's MMAs are done: the next channels replace it
+                if (issued < nst) fetch();
+                if (--left == 0 && s + 1 < nst) {
                     left = per_reg;
-                    load_region(c0 += cr);
-                    cp_async_commit();
-                    cp_async_wait<0>();
-                    fence_async_smem();
-                    mbar_arrive(regbar);
+                    next_region(c0 += cr);
                 }
                 if (++buf == bufs) {
                     buf = 0;
                     ph ^= 1;
                 }
             }
+        } else {
+#pragma unroll 1
+            for (int c0 = cr, ph = 0; c0 < d.C; c0 += cr, ph ^= 1) {
+                if (!mbar_wait_bounded(regdone, ph)) {
+                    timed_out = true;
+                    break;
+                }
+                next_region(c0);
+            }
+        }
         if (timed_out && tid == 32)  // its own copies in flight
             for (int s = imax(0, issued - bufs); s < issued; s++)
                 mbar_wait_bounded(full + 8 * (s % bufs), (uint32_t)(s / bufs) & 1u);
@@ -332,6 +351,7 @@ __global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
                     default: um_issue<NP, T::NACC, DIL, PX, 14>(tmem, ad, bd, IDESC, t0, nacc, first); break;
                 }
                 umma_commit(freed + 8 * buf);
+                if (tap == 8 && kc0 + kcs == cr / 8 && s + 1 < nst) umma_commit(regdone);
             }
             __syncwarp();
             kc0 += kcs;
