@@ -1148,6 +1148,7 @@ oflow_status oflow_stream_create(oflow_ctx *ctx, const oflow_stream_desc *desc, 
         }
         s->slots.alloc(3 * (size_t)desc->lanes * s->frame_bytes());
         OF_CUDA(cudaMemset(s->slots.as<char>(), 0, s->slots.bytes()));
+        OF_CUDA(cudaStreamSynchronize(nullptr));  // the streams that use it don't wait for the default one
         OF_CUDA(cudaStreamCreateWithFlags(&s->copy, cudaStreamNonBlocking));
         OF_CUDA(cudaEventCreateWithFlags(&s->uploaded, cudaEventDisableTiming));
         for (cudaEvent_t &e : s->done) OF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

@@ -2307,6 +2307,7 @@ TvPlan::TvPlan(int w, int h, int B, int dtype, const oflow_tvl1_params &prm, boo
     if (const char *e = getenv("OFLOW_TB_PREDICT")) predict_ = atoi(e);
     // scales above a warm start's first scale never record a count
     OF_CUDA(cudaMemset(ar_.at<char>(o_iters_), 0, (size_t)B * iter_stride_ * 4));
+    OF_CUDA(cudaStreamSynchronize(nullptr));  // the caller's stream may not wait for the default one
 }
 
 void TvPlan::bind_frame(int b, int k, const void *p, int pitch) {

@@ -94,6 +94,7 @@ WarmNet::WarmNet(int w, int h, int B) : w_(w), h_(h), B_(B) {
     OF_CUDA(cudaMemset(ar_.at<char>(o_pb_), 0, np_ * 2));
     OF_CUDA(cudaMemset(ar_.at<char>(o_pkf_), 0, npk_ * 2));
     OF_CUDA(cudaMemset(ar_.at<char>(o_pkb_), 0, npk_ * 2));
+    OF_CUDA(cudaStreamSynchronize(nullptr));  // the caller's stream may not wait for the default one
 }
 
 void WarmNet::set_params(const float *host, cudaStream_t st) {
