@@ -466,6 +466,9 @@ int um_kcs(int C, int np) {
 }
 int um_bufs(int C, int np) { return imax(2, imin(kUmMaxBufs, 16 * 1024 / um_wstage(np, um_kcs(C, np)))); }
 
+// Dynamic shared memory of a CTA at most.  Kernels are allowed all of it at every
+// launch: the attribute belongs to the process, and one set to a launch's own need
+// could be lowered by another thread before the launch.
 constexpr int kUmSmemMax = 227 * 1024 - 1024;
 
 template <int MODE, int MT> int um_tiles(const ConvDims &d) {
@@ -485,7 +488,7 @@ template <int NP, int MODE, int MT> void launch_um(const UmCall &c) {
         while (nk % (cr / 8) != 0) cr -= 8 * kcs;
     }
     const int smem = um_smem<MODE, MT>(NP, c.d.C, cr);
-    OF_CUDA(cudaFuncSetAttribute(k_conv_fwd_umma<NP, MODE, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    OF_CUDA(cudaFuncSetAttribute(k_conv_fwd_umma<NP, MODE, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUmSmemMax));
     k_conv_fwd_umma<NP, MODE, MT><<<um_tiles<MODE, MT>(c.d), UmTile<MODE, MT>::NT, smem, c.st>>>(
         c.d, c.x, c.w, c.bias, c.y, c.flags, c.ldy, kcs, um_bufs(c.d.C, NP), cr, c.err);
 }
@@ -726,7 +729,7 @@ void launch_wgrad(const ConvDims &d, const __nv_bfloat16 *gb, const __nv_bfloat1
     const int tm = 512 / (int)tmem_cols<3 * KP>();  // CTAs an SM by tensor memory
     const int bufs = bytes(3) <= kUmSmemMax / tm ? 3 : 2;
     const int smem = bytes(bufs);
-    OF_CUDA(cudaFuncSetAttribute(k_conv_wgrad_mn<KP, STRIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    OF_CUDA(cudaFuncSetAttribute(k_conv_wgrad_mn<KP, STRIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUmSmemMax));
     // one wave of the CTAs that fit by shared and tensor memory
     const int occ = imax(1, imin(227 * 1024 / (smem + 1024), tm));
     const int splits = imin(tiles, imax(1, kNumSMs * occ / mtiles));
