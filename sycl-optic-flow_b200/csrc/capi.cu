@@ -1325,9 +1325,10 @@ oflow_status oflow_flow_to_color(oflow_ctx *ctx, int n, int width, int height,
     });
 }
 
-// Packed weights of one layer; false where the tensor-core kernels don't take it.
+// Packed weights of one layer; false where the tensor-core kernels don't take it
+// (the forward packing moves 16 bytes at a time, the backward one elements).
 static bool conv3x3_pack(const ConvDims &d, const void *w, __nv_bfloat16 *dst, bool backward, cudaStream_t st) {
-    if (d.C % 16 != 0 || (reinterpret_cast<uintptr_t>(w) & 15u) != 0) return false;
+    if (d.C % 16 != 0 || (!backward && (reinterpret_cast<uintptr_t>(w) & 15u) != 0)) return false;
     ConvPack p;
     p.add(static_cast<const __nv_bfloat16 *>(w), dst, d.K, d.C, backward);
     conv_pack_weights(p, st);
@@ -1346,14 +1347,16 @@ oflow_status oflow_conv3x3(int mode, int N, int H, int W, int C, int K, int stri
         if (mode == 0) {
             // the tcgen05 kernel; the shape must be one it takes
             OF_CHECK(bias != nullptr, "conv3x3: null bias");
-            DevBuf err(sizeof(int)), packed(conv_packed_size(K, C) * sizeof(__nv_bfloat16));
-            OF_CUDA(cudaMemsetAsync(err.as<int>(), 0, sizeof(int), st));
-            OF_CHECK(conv3x3_pack(d, b, packed.as<__nv_bfloat16>(), false, st) &&
-                         conv_forward_umma(d, static_cast<const __nv_bfloat16 *>(a), packed.as<__nv_bfloat16>(), bias,
-                                           out, out_f32 != 0, relu != 0, err.as<int>(), st),
+            DevBuf buf(256 + conv_packed_size(K, C) * sizeof(__nv_bfloat16));
+            int *err = buf.as<int>();
+            __nv_bfloat16 *packed = reinterpret_cast<__nv_bfloat16 *>(buf.as<char>() + 256);
+            OF_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
+            OF_CHECK(conv3x3_pack(d, b, packed, false, st) &&
+                         conv_forward_umma(d, static_cast<const __nv_bfloat16 *>(a), packed, bias, out, out_f32 != 0,
+                                           relu != 0, err, st),
                      "conv3x3: shape outside the tensor-core kernel (C % 16 == 0, K % 8 == 0, K <= 128)");
             int e = 0;
-            OF_CUDA(cudaMemcpyAsync(&e, err.as<int>(), sizeof(int), cudaMemcpyDeviceToHost, st));
+            OF_CUDA(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
             OF_CUDA(cudaStreamSynchronize(st));
             if (e) throw Error(OFLOW_ERR_TIMEOUT, "conv3x3: a bounded wait gave up");
         } else if (mode == 3) {
@@ -1363,17 +1366,19 @@ oflow_status oflow_conv3x3(int mode, int N, int H, int W, int C, int K, int stri
                          bias, out, out_f32 != 0, relu != 0, st);
         } else if (mode == 1) {
             // the tcgen05 kernel; the shape must be one it takes
-            DevBuf err(sizeof(int)), scratch(conv_backward_data_umma_scratch(d)),
-                packed(conv_packed_size(K, C) * sizeof(__nv_bfloat16));
-            OF_CUDA(cudaMemsetAsync(err.as<int>(), 0, sizeof(int), st));
-            OF_CHECK(conv3x3_pack(d, b, packed.as<__nv_bfloat16>(), true, st) &&
+            const size_t npacked = (conv_packed_size(K, C) * sizeof(__nv_bfloat16) + 255) / 256 * 256;
+            DevBuf buf(256 + npacked + conv_backward_data_umma_scratch(d));
+            int *err = buf.as<int>();
+            __nv_bfloat16 *packed = reinterpret_cast<__nv_bfloat16 *>(buf.as<char>() + 256);
+            OF_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
+            OF_CHECK(conv3x3_pack(d, b, packed, true, st) &&
                          conv_backward_data_umma(d, static_cast<const float *>(a),
-                                                 static_cast<const __nv_bfloat16 *>(y_act),
-                                                 packed.as<__nv_bfloat16>(), static_cast<float *>(out), false,
-                                                 scratch.as<void>(), err.as<int>(), st),
+                                                 static_cast<const __nv_bfloat16 *>(y_act), packed,
+                                                 static_cast<float *>(out), false, buf.as<char>() + 256 + npacked, err,
+                                                 st),
                      "conv3x3: shape outside the tensor-core kernel (C % 16 == 0, K % 8 == 0)");
             int e = 0;
-            OF_CUDA(cudaMemcpyAsync(&e, err.as<int>(), sizeof(int), cudaMemcpyDeviceToHost, st));
+            OF_CUDA(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
             OF_CUDA(cudaStreamSynchronize(st));
             if (e) throw Error(OFLOW_ERR_TIMEOUT, "conv3x3: a bounded wait gave up");
         } else if (mode == 4) {
