@@ -105,6 +105,19 @@ __host__ __device__ __forceinline__ float markstein(float p, float g, float y) {
     return OF_FMAF(-r, y, q0);
 }
 
+// p / g correctly rounded for every finite p but zeros, from y = RN(1/g) with g in
+// [2^-40, 2^24): Newton's step for the reciprocal and Markstein's correction of the
+// quotient, both in double, where neither p nor the quotient underflows.  That
+// leaves 2^-52 of the quotient; two 24-bit numbers' quotient is a rounding midpoint
+// of single precision (normal or not) or 2^-49 of itself away from any, so the last
+// rounding is that of p / g.
+__host__ __device__ __forceinline__ float div_in_double(float p, float g, float y) {
+    const double G = g, P = p, Y0 = y;
+    const double Y = fma(Y0, fma(-G, Y0, 1.0), Y0);
+    const double q = P * Y;
+    return (float)fma(fma(-q, G, P), Y, q);
+}
+
 // For a running minimum over numerators: every one is zero or above 2^-100 in
 // magnitude exactly when the minimum of markstein_key is at least kMarksteinKey.
 constexpr unsigned kMarksteinKey = 2u * 0x0d800000u;  // 2^-100

@@ -106,8 +106,15 @@ __global__ void __launch_bounds__(kDTW *kDTH) k_hs_warp_deriv(
 // The division by Ix^2+Iy^2+alpha is Markstein's correction from the
 // reciprocal, formed once per launch.  What that takes for granted (numerators
 // zero or above 2^-100, denominators in [2^-40, 2^24)) is kept as a running
-// minimum; a block that breaks it runs its tile again from the untouched input
-// with IEEE divisions.
+// minimum; a block that breaks it runs its tile again from the untouched input,
+// CAREFUL: looking at each numerator.  Where a part of the frames stands still the
+// increments fall off from what moves by about 1/4 a pixel, and there are such
+// numerators in every sweep; so the tile's next launch is careful at once
+// (HsJacobiArgs::hint) until a launch meets none.  64 pairs of 320x240 with one moving
+// disc each, 200 sweeps: 12.4 ms without the hint and with IEEE divisions for all of
+// a tile, 4.3 ms here, and 2.7 where everything moves.  (Looking at a warp's
+// numerators once a sweep, before its quotients, needs no second run; it costs
+// frames without any 15 %.)
 template <int V_, int NW_, int K_> struct HsTile {
     static constexpr int V = V_, NW = NW_, K = K_, NT = 32 * NW;
     static constexpr int RW = 64, RH = V * NW, TW = RW - 2 * K, TH = RH - 2 * K;
@@ -128,6 +135,7 @@ struct HsJacobiArgs {
     int vec;                  // two neighbouring pixels are 16-byte aligned
     int tiles_x, tiles_y, tiles;  // tiles: of all pairs
     int tma;                  // the maps below describe the level
+    int *hint;                // per tile: its last launch met a numerator or denominator out of range
     int *err;                 // set when a bounded wait gives up
     CUtensorMap m0, m1, mi;   // D's planes, the increments: (w, h, pair), 8-byte elements
 };
@@ -140,17 +148,29 @@ struct HsEdge {
     int bottom;             // the warp's row that is the last of the image (else out of its rows)
 };
 
+// p / den: Markstein's correction where it holds, in double where p is too small
+// for it, the IEEE division where den is out of range.
+__device__ __forceinline__ float hs_quotient(float p, float den, float rcp) {
+    float q = markstein(p, den, rcp);
+    if (markstein_key(p) < kMarksteinKey || !rcp_in_range(den))
+        q = rcp_in_range(den) ? div_in_double(p, den, rcp) : p / den;
+    return q;
+}
+
 // One sweep (solverKernel.cuh:41-153): neighbour mean of the increments
 // (clamped at the image border), frac = (Ix*su + Iy*sv + Iz) / den and the
 // update, in the reference's order.  above / below: the neighbouring warps'
-// rows.
+// rows; broken: a denominator of the thread is out of range.  CAREFUL: a warp
+// with a numerator out of range looks at each.
 // EDGE: 0 the region lies inside the image; 1 it meets its top, left or (at an
 // even width) right border; 2 any border.
-template <typename T, int EDGE, bool EXACT>
+template <typename T, int EDGE, bool CAREFUL>
 __device__ __forceinline__ void hs_sweep(HsState<T::V> &s, float4 above, float4 below, const HsEdge &e,
-                                         unsigned &key) {
+                                         bool broken, unsigned &key) {
     constexpr int V = T::V;
     float2 dn[2] = {make_float2(above.x, above.y), make_float2(above.z, above.w)};  // y - 1, before the sweep
+    float num[V][2];  // CAREFUL: the numerators
+    unsigned now = ~0u;
 #pragma unroll
     for (int v = 0; v < V; v++) {
         const float2 c0 = s.a[v][0], c1 = s.a[v][1];
@@ -179,20 +199,39 @@ __device__ __forceinline__ void hs_sweep(HsState<T::V> &s, float4 above, float4 
             const float su = (al.x + ar.x + au.x + ad.x) * 0.25f;
             const float sv = (al.y + ar.y + au.y + ad.y) * 0.25f;
             p[c] = s.ix[v][c] * su + s.iy[v][c] * sv + s.iz[v][c];
-            const float frac = EXACT ? p[c] / s.den[v][c] : markstein(p[c], s.den[v][c], s.rcp[v][c]);
-            s.a[v][c] = make_float2(su - s.ix[v][c] * frac, sv - s.iy[v][c] * frac);
+            if (CAREFUL) {
+                num[v][c] = p[c];
+                s.a[v][c] = make_float2(su, sv);
+            } else {
+                const float frac = markstein(p[c], s.den[v][c], s.rcp[v][c]);
+                s.a[v][c] = make_float2(su - s.ix[v][c] * frac, sv - s.iy[v][c] * frac);
+            }
         }
-        if (!EXACT) key = umin(umin(key, markstein_key(p[0])), markstein_key(p[1]));
+        unsigned &least = CAREFUL ? now : key;
+        least = umin(umin(least, markstein_key(p[0])), markstein_key(p[1]));
         dn[0] = c0;
         dn[1] = c1;
+    }
+    if (CAREFUL) {
+        const bool look = __any_sync(0xffffffffu, broken || now < kMarksteinKey);
+        key = umin(key, now);
+#pragma unroll
+        for (int v = 0; v < V; v++)
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const float2 m = s.a[v][c];
+                float frac = markstein(num[v][c], s.den[v][c], s.rcp[v][c]);
+                if (look) frac = hs_quotient(num[v][c], s.den[v][c], s.rcp[v][c]);
+                s.a[v][c] = make_float2(m.x - s.ix[v][c] * frac, m.y - s.iy[v][c] * frac);
+            }
     }
 }
 
 // Sweep j of a tile: the warps' first and last rows exchanged through
 // alternating buffers (one barrier a sweep), then the sweep.
-template <typename T, int EDGE, bool EXACT, typename F>
+template <typename T, int EDGE, bool CAREFUL, typename F>
 __device__ __forceinline__ void hs_step(HsState<T::V> &s, int j, float4 (*sRow)[2][T::NW][32], bool top,
-                                        const HsEdge &e, unsigned &key, F &&taken) {
+                                        const HsEdge &e, bool broken, unsigned &key, F &&taken) {
     constexpr int V = T::V, NW = T::NW;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float4(*row)[NW][32] = sRow[j & 1];
@@ -204,7 +243,7 @@ __device__ __forceinline__ void hs_step(HsState<T::V> &s, int j, float4 (*sRow)[
     float4 above = row[1][wid > 0 ? wid - 1 : 0][lane];
     const float4 below = row[0][wid + 1 < NW ? wid + 1 : wid][lane];
     if (EDGE && top) above = first;
-    hs_sweep<T, EDGE, EXACT>(s, above, below, e, key);
+    hs_sweep<T, EDGE, CAREFUL>(s, above, below, e, broken, key);
 }
 
 // Two neighbouring float2 at q; in0, in1: inside the level.
@@ -264,8 +303,8 @@ __device__ __forceinline__ void hs_fetch(const HsJacobiArgs &a, int tile, HsSmem
 // has taken its share into registers, `taken` runs.  first: increments start at 0
 // (flow.cu:168-171); last: add the increment to the flow (AddKernel,
 // addKernel.cuh:28-36) instead of storing it.  Returns whether the guard broke
-// (nothing is stored then).
-template <typename T, bool EXACT, typename F>
+// (nothing is stored then, unless CAREFUL).
+template <typename T, bool CAREFUL, typename F>
 __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const HsSmem<T> &sm,
                                         float4 (*sRow)[2][T::NW][32], F &&taken) {
     constexpr int V = T::V, K = T::K, NW = T::NW;
@@ -299,26 +338,27 @@ __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const H
     const bool interior = t.ox >= 1 && t.oy >= 1 && t.ox + T::RW <= w - 1 && t.oy + T::RH <= h - 1;
     const HsEdge e{x == 0, x + 1 == w - 1, x == w - 1, h - 1 - y0};
     const bool top = y0 == 0;
-    if (EXACT) {
+    if (CAREFUL) {
 #pragma unroll 1
-        for (int j = 0; j < a.sweeps; j++) hs_step<T, 2, true>(s, j, sRow, top, e, key, taken);
+        for (int j = 0; j < a.sweeps; j++) hs_step<T, 2, true>(s, j, sRow, top, e, broken, key, taken);
     } else if (a.sweeps != K) {
 #pragma unroll 1
-        for (int j = 0; j < a.sweeps; j++) hs_step<T, 2, false>(s, j, sRow, top, e, key, taken);
+        for (int j = 0; j < a.sweeps; j++) hs_step<T, 2, false>(s, j, sRow, top, e, broken, key, taken);
     } else if (interior) {
         // unrolled, so that old and new increments swap registers instead of being copied
 #pragma unroll 4
-        for (int j = 0; j < K; j++) hs_step<T, 0, false>(s, j, sRow, top, e, key, taken);
+        for (int j = 0; j < K; j++) hs_step<T, 0, false>(s, j, sRow, top, e, broken, key, taken);
     } else if (t.oy + T::RH <= h - 1 && (w & 1) == 0) {
 #pragma unroll 2
-        for (int j = 0; j < K; j++) hs_step<T, 1, false>(s, j, sRow, top, e, key, taken);
+        for (int j = 0; j < K; j++) hs_step<T, 1, false>(s, j, sRow, top, e, broken, key, taken);
     } else {
 #pragma unroll 2
-        for (int j = 0; j < K; j++) hs_step<T, 2, false>(s, j, sRow, top, e, key, taken);
+        for (int j = 0; j < K; j++) hs_step<T, 2, false>(s, j, sRow, top, e, broken, key, taken);
     }
     // (also: every warp has read the rows before the next tile writes them)
-    if (__syncthreads_or(!EXACT && (broken || key < kMarksteinKey))) return true;
-    if (lane < K / 2 || lane >= 32 - K / 2 || wid < K / V || wid >= NW - K / V || x >= w) return false;
+    const bool bad = __syncthreads_or(broken || key < kMarksteinKey);
+    if (!CAREFUL && bad) return true;
+    if (lane < K / 2 || lane >= 32 - K / 2 || wid < K / V || wid >= NW - K / V || x >= w) return bad;
     float2 *Out = (a.last ? a.U : a.out) + (size_t)t.b * a.stride;
 #pragma unroll
     for (int v = 0; v < V; v++) {
@@ -337,7 +377,7 @@ __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const H
             if (in1) Out[q + 1] = r1;
         }
     }
-    return false;
+    return bad;
 }
 
 // Resident blocks walk the tiles of all pairs; a tile's data is brought to
@@ -349,16 +389,21 @@ __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant
     HsSmem<T> &sm = *reinterpret_cast<HsSmem<T> *>(hs_dyn);
     __shared__ float4 sRow[2][2][T::NW][32];
     __shared__ __align__(8) unsigned long long s_bar;
-    const uint32_t bar = smem_u32(&s_bar);
+    __shared__ int s_hint;
+    const uint32_t bar = smem_u32(&s_bar), hint = smem_u32(&s_hint);
     uint32_t parity = 0;
-    if (a.tma && threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-        hs_fetch_tma<T>(a, blockIdx.x, sm, bar);
+    if (threadIdx.x == 0) {
+        if (a.tma) {
+            mbar_init(bar, 1);
+            fence_mbar_init();
+            hs_fetch_tma<T>(a, blockIdx.x, sm, bar);
+        }
+        cp_async4(hint, a.hint + blockIdx.x);
     }
     __syncthreads();  // the barrier is initialised before anyone waits on it
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
         const int next = tile + gridDim.x;
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
         if (a.tma) {
             const bool ok = mbar_wait_bounded(bar, parity);
             parity ^= 1u;
@@ -373,13 +418,19 @@ __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant
             hs_fetch<T>(a, tile, sm);
             __syncthreads();
         }
+        const bool careful = !a.first && s_hint != 0;  // (the first launch writes every tile's hint)
         const auto fetch_next = [&] {
-            if (a.tma && next < a.tiles && threadIdx.x == 0) {
-                fence_async_smem();  // the block's reads of this tile, then the copies of the next
-                hs_fetch_tma<T>(a, next, sm, bar);
+            if (next < a.tiles && threadIdx.x == 0) {
+                if (a.tma) {
+                    fence_async_smem();  // the block's reads of this tile, then the copies of the next
+                    hs_fetch_tma<T>(a, next, sm, bar);
+                }
+                cp_async4(hint, a.hint + next);  // (nobody waits for it before the tile's data)
             }
         };
-        if (hs_tile<T, false>(a, tile, sm, sRow, fetch_next)) {
+        bool bad = careful;
+        if (!careful && hs_tile<T, false>(a, tile, sm, sRow, fetch_next)) {
+            bad = true;
             // again from the untouched input, then the next tile's copies again
             if (a.tma && next < a.tiles) {
                 const bool ok = mbar_wait_bounded(bar, parity);
@@ -392,8 +443,9 @@ __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant
             }
             hs_fetch<T>(a, tile, sm);
             __syncthreads();
-            hs_tile<T, true>(a, tile, sm, sRow, fetch_next);
         }
+        if (bad) bad = hs_tile<T, true>(a, tile, sm, sRow, fetch_next);
+        if (threadIdx.x == 0 && (a.first || bad != careful)) a.hint[tile] = bad;
     }
 }
 
@@ -408,11 +460,106 @@ __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant
 // One block an SM instead of two saves the spills (160x120 83 us) and costs batches
 // more (9 pairs 166).  The barriers of the block and the cluster bound it.
 //
-// The guard is looked at once, at the end: where any block of the cluster broke
-// it, all of them run the warp again with IEEE divisions.
+// The guard is looked at once, at the end: where any block of the cluster broke it,
+// all of them run the warp again, CAREFUL.  150 sweeps of 160x120 take 102 us, and
+// 248 where a part of the frames stands still (start of one disc moving; 464 with an
+// IEEE division in every pixel of the second run); 9 pairs 172 and 405 us.  Looking
+// at the end of every exchange, and going on from there, takes 173 us where frames
+// stand still, but 106 and 184 where they don't.
 template <typename T> struct HsRes {
     float2 own[2][T::TH][T::TW];
 };
+
+// The thread's D, its reciprocals, and whether a denominator is out of range.
+template <typename T>
+__device__ __forceinline__ bool hs_res_load(const HsJacobiArgs &a, const HsAt &t, HsState<T::V> &s) {
+    constexpr int V = T::V;
+    const float2 *D0 = a.D + (size_t)t.b * a.dstride, *D1 = D0 + a.plane;
+    const int x = t.x, y0 = t.y0, w = a.w, h = a.h;
+    const bool in0 = x >= 0 && x < w, in1 = x + 1 >= 0 && x + 1 < w;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const bool iy = y0 + v >= 0 && y0 + v < h;
+        const size_t q = iy && in0 ? (size_t)(y0 + v) * w + x : 0;
+        const float4 d0 = hs_ld_two(D0, q, a.vec, iy && in0, iy && in0 && in1);
+        const float4 d1 = hs_ld_two(D1, q, a.vec, iy && in0, iy && in0 && in1);
+        s.ix[v][0] = d0.x; s.iy[v][0] = d0.y; s.iz[v][0] = d1.x; s.den[v][0] = iy && in0 ? d1.y : 1.0f;
+        s.ix[v][1] = d0.z; s.iy[v][1] = d0.w; s.iz[v][1] = d1.z; s.den[v][1] = iy && in0 && in1 ? d1.w : 1.0f;
+    }
+    bool broken = false;
+#pragma unroll
+    for (int v = 0; v < V; v++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            s.rcp[v][c] = rcp_near_rn(s.den[v][c]);
+            broken |= !rcp_in_range(s.den[v][c]);
+        }
+    return broken;
+}
+
+// The increments that the blocks laid in buffer buf: a thread's own pixels, or its
+// halo from the owners (zeros beyond an odd width are the owner's).
+template <typename T>
+__device__ __forceinline__ void hs_res_take(const HsJacobiArgs &a, const HsAt &t, const HsRes<T> &sm, int buf,
+                                            HsState<T::V> &s) {
+#pragma unroll
+    for (int v = 0; v < T::V; v++) {
+        const int x = t.x, y = t.y0 + v;
+        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (x >= 0 && x < a.w && y >= 0 && y < a.h) {
+            const int tx = x / T::TW, ty = y / T::TH;
+            u = cluster_ld4(smem_u32(&sm.own[buf][y - ty * T::TH][x - tx * T::TW]), ty * a.tiles_x + tx);
+        }
+        s.a[v][0] = make_float2(u.x, u.y);
+        s.a[v][1] = make_float2(u.z, u.w);
+    }
+}
+
+// Lays the thread's pixels in buffer buf (zeros outside the level).
+template <typename T>
+__device__ __forceinline__ void hs_res_lay(const HsJacobiArgs &a, const HsAt &t, HsRes<T> &sm, int buf,
+                                           HsState<T::V> &s) {
+    constexpr int V = T::V, K = T::K;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const bool iy = t.y0 + v < a.h;
+        if (!iy || t.x >= a.w) s.a[v][0] = make_float2(0.f, 0.f);
+        if (!iy || t.x + 1 >= a.w) s.a[v][1] = make_float2(0.f, 0.f);
+        *reinterpret_cast<float4 *>(&sm.own[buf][wid * V + v - K][2 * lane - K]) =
+            make_float4(s.a[v][0].x, s.a[v][0].y, s.a[v][1].x, s.a[v][1].y);
+    }
+}
+
+// Whether the thread's pixels are the block's own.
+template <typename T> __device__ __forceinline__ bool hs_own() {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    return lane >= T::K / 2 && lane < 32 - T::K / 2 && wid >= T::K / T::V && wid < T::NW - T::K / T::V;
+}
+
+// All sweeps again, CAREFUL.  Returns the buffer that holds the last increments.
+template <typename T>
+__device__ __forceinline__ int hs_res_careful(const HsJacobiArgs &a, HsRes<T> &sm, float4 (*sRow)[2][T::NW][32]) {
+    constexpr int K = T::K;
+    const HsAt t = hs_at<T>(a, blockIdx.x);
+    const HsEdge e{t.x == 0, t.x + 1 == a.w - 1, t.x == a.w - 1, a.h - 1 - t.y0};
+    HsState<T::V> s;
+    const bool broken = hs_res_load<T>(a, t, s);
+#pragma unroll
+    for (int v = 0; v < T::V; v++) s.a[v][0] = s.a[v][1] = make_float2(0.f, 0.f);
+    unsigned key = ~0u;
+    int buf = 0;
+#pragma unroll 1
+    for (int done = 0; done < a.sweeps; done += K, buf ^= 1) {
+        if (done > 0) hs_res_take<T>(a, t, sm, buf ^ 1, s);
+        const int n = imin(K, a.sweeps - done);
+#pragma unroll 1
+        for (int j = 0; j < n; j++) hs_step<T, 2, true>(s, j, sRow, t.y0 == 0, e, broken, key, [] {});
+        if (hs_own<T>()) hs_res_lay<T>(a, t, sm, buf, s);
+        cluster_barrier();
+    }
+    return buf ^ 1;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(T::NT, 2) k_hs_res(const __grid_constant__ HsJacobiArgs a) {
@@ -421,103 +568,57 @@ __global__ void __launch_bounds__(T::NT, 2) k_hs_res(const __grid_constant__ HsJ
     extern __shared__ __align__(128) char hs_dyn[];
     HsRes<T> &sm = *reinterpret_cast<HsRes<T> *>(hs_dyn);
     __shared__ float4 sRow[2][2][NW][32];
-    __shared__ int s_bad;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, w = a.w, h = a.h;
+    const int w = a.w, h = a.h;
     const HsAt t = hs_at<T>(a, blockIdx.x);
-    const int x = t.x, y0 = t.y0, blocks = a.tiles_x * a.tiles_y;
-    const bool in0 = x >= 0 && x < w, in1 = x + 1 >= 0 && x + 1 < w;
-    const bool own = lane >= K / 2 && lane < 32 - K / 2 && wid >= K / V && wid < NW - K / V;
+    const int x = t.x, y0 = t.y0;
+    const bool own = hs_own<T>();
     HsState<V> s;
-    bool broken = false;
-    {
-        const float2 *D0 = a.D + (size_t)t.b * a.dstride, *D1 = D0 + a.plane;
-#pragma unroll
-        for (int v = 0; v < V; v++) {
-            const bool iy = y0 + v >= 0 && y0 + v < h;
-            const size_t q = iy && in0 ? (size_t)(y0 + v) * w + x : 0;
-            const float4 d0 = hs_ld_two(D0, q, a.vec, iy && in0, iy && in0 && in1);
-            const float4 d1 = hs_ld_two(D1, q, a.vec, iy && in0, iy && in0 && in1);
-            s.ix[v][0] = d0.x; s.iy[v][0] = d0.y; s.iz[v][0] = d1.x; s.den[v][0] = iy && in0 ? d1.y : 1.0f;
-            s.ix[v][1] = d0.z; s.iy[v][1] = d0.w; s.iz[v][1] = d1.z; s.den[v][1] = iy && in0 && in1 ? d1.w : 1.0f;
-        }
-    }
-#pragma unroll
-    for (int v = 0; v < V; v++)
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-            s.rcp[v][c] = rcp_near_rn(s.den[v][c]);
-            broken |= !rcp_in_range(s.den[v][c]);
-        }
+    const bool broken = hs_res_load<T>(a, t, s);
     const bool interior = t.ox >= 1 && t.oy >= 1 && t.ox + T::RW <= w - 1 && t.oy + T::RH <= h - 1;
     const bool plain = t.oy + T::RH <= h - 1 && (w & 1) == 0;
     const HsEdge e{x == 0, x + 1 == w - 1, x == w - 1, h - 1 - y0};
     const bool top = y0 == 0;
     const auto taken = [] {};
 
-    auto exchange = [&](int buf) {
-        if (own) {
+    // whether a block of the cluster met anything out of range (told by the block itself
+    // before the last meeting)
+    __shared__ int s_bad;
+    if (threadIdx.x == 0) s_bad = 0;
+    unsigned key = broken ? 0u : ~0u;
 #pragma unroll
-            for (int v = 0; v < V; v++) {
-                const bool iy = y0 + v < h;
-                if (!iy || !in0) s.a[v][0] = make_float2(0.f, 0.f);
-                if (!iy || !in1) s.a[v][1] = make_float2(0.f, 0.f);
-                *reinterpret_cast<float4 *>(&sm.own[buf][wid * V + v - K][2 * lane - K]) =
-                    make_float4(s.a[v][0].x, s.a[v][0].y, s.a[v][1].x, s.a[v][1].y);
-            }
-        }
-        cluster_barrier();
-        if (!own) {
-#pragma unroll
-            for (int v = 0; v < V; v++) {
-                const int y = y0 + v;
-                float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (in0 && y >= 0 && y < h) {  // zeros beyond an odd width are the owner's
-                    const int tx = x / T::TW, ty = y / T::TH;
-                    u = cluster_ld4(smem_u32(&sm.own[buf][y - ty * T::TH][x - tx * T::TW]), ty * a.tiles_x + tx);
-                }
-                s.a[v][0] = make_float2(u.x, u.y);
-                s.a[v][1] = make_float2(u.z, u.w);
-            }
-        }
-    };
-
+    for (int v = 0; v < V; v++) s.a[v][0] = s.a[v][1] = make_float2(0.f, 0.f);
+    int buf = 0;
 #pragma unroll 1
-    for (int exact = 0; exact < 2; exact++) {
-        unsigned key = ~0u;
-#pragma unroll
-        for (int v = 0; v < V; v++) s.a[v][0] = s.a[v][1] = make_float2(0.f, 0.f);
+    for (int done = 0;; done += K, buf ^= 1) {
+        const int n = imin(K, a.sweeps - done);
+        if (n != K) {
 #pragma unroll 1
-        for (int done = 0, buf = 0; done < a.sweeps; done += K, buf ^= 1) {
-            const int n = imin(K, a.sweeps - done);
-            if (exact) {
-#pragma unroll 1
-                for (int j = 0; j < n; j++) hs_step<T, 2, true>(s, j, sRow, top, e, key, taken);
-            } else if (n != K) {
-#pragma unroll 1
-                for (int j = 0; j < n; j++) hs_step<T, 2, false>(s, j, sRow, top, e, key, taken);
-            } else if (interior) {
+            for (int j = 0; j < n; j++) hs_step<T, 2, false>(s, j, sRow, top, e, broken, key, taken);
+        } else if (interior) {
 #pragma unroll 2
-                for (int j = 0; j < K; j++) hs_step<T, 0, false>(s, j, sRow, top, e, key, taken);
-            } else if (plain) {
+            for (int j = 0; j < K; j++) hs_step<T, 0, false>(s, j, sRow, top, e, broken, key, taken);
+        } else if (plain) {
 #pragma unroll 2
-                for (int j = 0; j < K; j++) hs_step<T, 1, false>(s, j, sRow, top, e, key, taken);
-            } else {
+            for (int j = 0; j < K; j++) hs_step<T, 1, false>(s, j, sRow, top, e, broken, key, taken);
+        } else {
 #pragma unroll 2
-                for (int j = 0; j < K; j++) hs_step<T, 2, false>(s, j, sRow, top, e, key, taken);
-            }
-            if (done + K < a.sweeps) exchange(buf);
+            for (int j = 0; j < K; j++) hs_step<T, 2, false>(s, j, sRow, top, e, broken, key, taken);
         }
-        // whether any block of the cluster broke the guard (the barriers also end the
-        // reads of this block's shared memory)
-        const int bad = __syncthreads_or(!exact && (broken || key < kMarksteinKey));
-        if (threadIdx.x == 0) s_bad = bad;
+        if (done + K >= a.sweeps) break;
+        if (own) hs_res_lay<T>(a, t, sm, buf, s);
         cluster_barrier();
-        const int any = threadIdx.x < blocks ? cluster_ld1(smem_u32(&s_bad), threadIdx.x) : 0;
-        const bool again = __syncthreads_or(any != 0);
-        cluster_barrier();
-        if (!again) break;
+        if (!own) hs_res_take<T>(a, t, sm, buf, s);
     }
+    if (a.sweeps <= K) cluster_barrier();  // (every block runs before its memory is written)
+    if (key < kMarksteinKey)
+        for (int k = 0; k < a.tiles_x * a.tiles_y; k++) cluster_st1(smem_u32(&s_bad), k, 1);
+    cluster_barrier();
+    const bool bad = s_bad != 0;
+    if (bad) buf = hs_res_careful<T>(a, sm, sRow);
+    if (bad && own) hs_res_take<T>(a, t, sm, buf, s);
+    // (nobody reads another block's shared memory after the last meeting)
     if (!own || x >= w) return;
+    const bool in1 = x + 1 < w;
     float2 *Out = (a.last ? a.U : a.out) + (size_t)t.b * a.stride;
 #pragma unroll
     for (int v = 0; v < V; v++) {
@@ -797,7 +898,7 @@ static void hs_set_smem_attrs() {
 // All sweeps of one warp: from zero increments to the flow updated.  The small
 // tiles run resident where a cluster holds the level.
 static void hs_sweeps(int cfg, int B, cudaStream_t st, const float2 *D, size_t plane, float2 *const dU[2],
-                      float2 *U, size_t stride, int w, int h, int sweeps, bool update, int *err) {
+                      float2 *U, size_t stride, int w, int h, int sweeps, bool update, int *hint, int *err) {
     const int K = kHsCfgs[cfg].k;
     if (cfg == 5 && sweeps > 0 && (hs_res_fits<HsRes8>(w, h) || hs_res_fits<HsRes4>(w, h))) {
         HsJacobiArgs a;
@@ -826,6 +927,7 @@ static void hs_sweeps(int cfg, int B, cudaStream_t st, const float2 *D, size_t p
         a.in = dU[cur];
         a.out = dU[cur ^ 1];
         a.U = U;
+        a.hint = hint;
         a.w = w;
         a.h = h;
         a.sweeps = k;
@@ -883,6 +985,7 @@ HsPlan::HsPlan(int w, int h, int B, int dtype, const oflow_hs_params &prm, const
     o_Ua_ = ar_.reserve(B * N_ * 8);
     o_Ub_ = ar_.reserve(B * N_ * 8);
     o_out_ = ar_.reserve(2 * B * N_ * 4);
+    o_hint_ = ar_.reserve((size_t)B * div_up(w, 32) * div_up(h, 16) * 4);  // the smallest tiles are 32x32, 48x16
     o_ftab_ = ar_.reserve(sizeof(FrameRef) * 2 * B);
     o_otab_ = ar_.reserve(sizeof(OutRef) * B);
     ar_.commit();
@@ -945,7 +1048,7 @@ void HsPlan::record(cudaStream_t st) {
                                                              Ubuf[ub], N_, 0, prm_.alpha, D, B * N_, N_);
             // with no sweeps du = 0: the flow is unchanged
             hs_sweeps(jcfg_[l], B, st, D, B * N_, dU, Ubuf[ub], N_, lw, lh, prm_.nsolver, true,
-                      err_.device());
+                      ar_.at<int>(o_hint_), err_.device());
         }
         if (l != top) {
             const float sx = (float)W_[l + 1] / (float)lw;
@@ -986,7 +1089,8 @@ void HsPlan::autotune(cudaStream_t st, TuneTable *table, int reps) {
                 float ms_min = 1e30f;
                 for (int r = 0; r <= reps; r++) {  // the first round warms up
                     OF_CUDA(cudaEventRecord(e0, st));
-                    hs_sweeps(c, B_, st, D, B_ * N_, dU, U, N_, lw, lh, kSweeps, false, err_.device());
+                    hs_sweeps(c, B_, st, D, B_ * N_, dU, U, N_, lw, lh, kSweeps, false, ar_.at<int>(o_hint_),
+                              err_.device());
                     OF_CUDA(cudaEventRecord(e1, st));
                     OF_CUDA(cudaEventSynchronize(e1));
                     float ms = 0.0f;
@@ -1043,7 +1147,7 @@ size_t hs_scratch_bytes(int w, int h, int nlevels) {
     hs_carve(off, N * 8);     // dU1
     hs_carve(off, N * 8);     // Ua
     hs_carve(off, N * 8);     // Ub
-    hs_carve(off, 2 * N * 4); // u | v
+    hs_carve(off, 2 * N * 4); // u | v; before them the sweeps' hints (a tile has a pixel)
     return off;
 }
 
@@ -1096,7 +1200,7 @@ void hs_enqueue_into(void *scratch, const float *I0, const float *I1, int w, int
             k_hs_warp_deriv<<<dg, dim3(kDTW, kDTH), 0, st>>>(pyr + pyr_off[l], lp, lw, lh,
                                                              Ubuf[ub], N, 0, prm.alpha, D, N, N);
             hs_sweeps(hs_pick(lw, lh, 1), 1, st, D, N, dU, Ubuf[ub], N, lw, lh, prm.nsolver, true,
-                      nullptr);
+                      reinterpret_cast<int *>(out), nullptr);
         }
         if (l != top) {
             const float sx = (float)Wl[l + 1] / (float)lw;

@@ -52,7 +52,7 @@ class HsPlan {
     size_t N_ = 0;
     Arena ar_;
     size_t o_raw_ = 0, o_pyr_ = 0, o_D_ = 0, o_dU0_ = 0, o_dU1_ = 0, o_Ua_ = 0, o_Ub_ = 0,
-           o_out_ = 0;
+           o_out_ = 0, o_hint_ = 0;
     int jcfg_[16] = {};
     Graph graph_;
     HostFlag err_;

@@ -21,6 +21,10 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool o
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
 __device__ __forceinline__ unsigned long long globaltimer() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -92,6 +96,12 @@ __device__ __forceinline__ int cluster_ld1(uint32_t a, int rank) {
         : "r"(a), "r"(rank)
         : "memory");
     return v;
+}
+
+__device__ __forceinline__ void cluster_st1(uint32_t a, int rank, int v) {
+    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.s32 [r], %2;\n\t}\n" ::"r"(a),
+                 "r"(rank), "r"(v)
+                 : "memory");
 }
 
 __device__ __forceinline__ void fence_async_smem() {
