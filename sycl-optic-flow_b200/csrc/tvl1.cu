@@ -821,6 +821,11 @@ struct FastGuard {
     float den = 0.0f;
     __device__ __forceinline__ void add_den(float g) { asm("max.NaN.f32 %0, %0, %1;" : "+f"(den) : "f"(g)); }
     __device__ __forceinline__ void add_num(float n) { key = umin(key, markstein_key(n)); }
+    __device__ __forceinline__ void add(const FastGuard &o) {
+        key = umin(key, o.key);
+        near = umin(near, o.near);
+        add_den(o.den);
+    }
     __device__ __forceinline__ bool broken() const {
         return key < kMarksteinKey || near <= kHypotNear || !(den < kRcpHi);
     }
@@ -850,6 +855,28 @@ __device__ __forceinline__ float4 dual_update_fast(float4 po, float f1x, float f
     fg.key = umin(umin(fg.key, markstein_key(n3)), markstein_key(n4));
     return make_float4(markstein(n1, g1, r1), markstein(n2, g1, r1), markstein(n3, g2, r2),
                        markstein(n4, g2, r2));
+}
+
+// The same pixel by pixel: small numerators are divided in double, the rest of what
+// breaks the guard takes the forms with branches.
+__device__ __forceinline__ float th_coef_careful(float2 u, float4 wr, float l_t) {
+    const float grad = th_grad(wr), rho = th_rho(u, wr);
+    float q = markstein(-rho, grad, wr.w);
+    if (!(grad < kRcpHi)) q = -rho / grad;
+    else if (markstein_key(rho) < kMarksteinKey) q = grad < 1E-10f ? 0.0f : div_in_double(-rho, grad, wr.w);
+    return th_coef(rho, grad, q, l_t);
+}
+__device__ __forceinline__ float quot_careful(float n, float g, float r) {
+    return markstein_key(n) < kMarksteinKey ? div_in_double(n, g, r) : markstein(n, g, r);
+}
+__device__ __forceinline__ float4 dual_update_careful(float4 po, float f1x, float f1y, float f2x, float f2y,
+                                                      float taut) {
+    unsigned m1, m2;
+    const float g1 = 1.0f + taut * hypot_fast(f1x, f1y, m1), g2 = 1.0f + taut * hypot_fast(f2x, f2y, m2);
+    if (umin(m1, m2) <= kHypotNear || !(g1 < kRcpHi && g2 < kRcpHi)) return dual_update(po, f1x, f1y, f2x, f2y, taut);
+    const float r1 = rcp_near_rn(g1), r2 = rcp_near_rn(g2);
+    return make_float4(quot_careful(taut * f1x + po.x, g1, r1), quot_careful(taut * f1y + po.y, g1, r1),
+                       quot_careful(taut * f2x + po.z, g2, r2), quot_careful(taut * f2y + po.w, g2, r2));
 }
 
 struct IterArgs {
@@ -996,6 +1023,15 @@ __global__ void __launch_bounds__(NT) k_tvl1_iter(IterArgs a) {
 // tile saved 9 % of the arithmetic and cost as much in branches (10.2 ms);
 // waiting for the neighbouring warps' rows only, instead of block barriers,
 // 10.6 ms; the two columns as paired instructions (add/fma .f32x2) 12.2 ms.
+//
+// A tile whose guard broke is run a second time from its untouched input, CAREFUL:
+// a row of a warp at a time, and only its small numerators divided in double.
+// Where frames are equal outside something that moves there are such numerators
+// ahead of what spreads from it: 8 pairs of 320x240 with one disc each, one scale,
+// 5 warps of 300 iterations, take 17.9 ms and 13.0 where everything moves; with
+// IEEE divisions and square roots in all of a second run, 26.3 ms.  (Running the
+// tile the careful way at once where it broke in the block of iterations before:
+// 17.0 ms, but the registers that the choice takes cost 8 % where everything moves.)
 struct TbArgs {
     const float2 *W;
     float2 *U0, *U1;
@@ -1046,9 +1082,9 @@ template <int V> struct RtState {
 // the region compute values that no owned pixel sees within K iterations.
 // BORDER: the region touches the image border; the border forms of
 // mask.cpp:63-89 differ from the interior one by neighbours taken as zero and,
-// in the first and last column, by the order of the two additions.  EXACT: the
-// steps with all their branches, for a tile whose guard broke.
-template <typename T, bool BORDER, bool EXACT>
+// in the first and last column, by the order of the two additions.  CAREFUL: a
+// warp whose guard breaks in a row takes that row's pixels one by one.
+template <typename T, bool BORDER, bool CAREFUL>
 __device__ __forceinline__ void rt_iteration(RtState<T::V> &s, typename T::Smem &sm, int x, int y0,
                                              int nx, int ny, float l_t, float theta, float taut,
                                              FastGuard &fg, double &err) {
@@ -1064,6 +1100,19 @@ __device__ __forceinline__ void rt_iteration(RtState<T::V> &s, typename T::Smem 
         const float l3 = __shfl_up_sync(0xffffffffu, s.p[v][1].z, 1);
         const int y = y0 + v;
         const float4 wa = sm.w[2 * v][tid], wb = sm.w[2 * v + 1][tid];
+        float coef[2];
+        if (CAREFUL) {
+            FastGuard row;
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+                coef[c] = th_coef_fast(s.u[v][c], c ? make_float4(wa.z, wa.w, wb.z, wb.w) : make_float4(wa.x, wa.y, wb.x, wb.y),
+                                       l_t, row);
+            if (__any_sync(0xffffffffu, row.broken()))
+#pragma unroll
+                for (int c = 0; c < 2; c++)
+                    coef[c] = th_coef_careful(s.u[v][c], c ? make_float4(wa.z, wa.w, wb.z, wb.w) : make_float4(wa.x, wa.y, wb.x, wb.y), l_t);
+            fg.add(row);
+        }
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             const float4 pc = s.p[v][c];
@@ -1086,13 +1135,8 @@ __device__ __forceinline__ void rt_iteration(RtState<T::V> &s, typename T::Smem 
             }
             const float2 u = s.u[v][c];
             const float4 w = c ? make_float4(wa.z, wa.w, wb.z, wb.w) : make_float4(wa.x, wa.y, wb.x, wb.y);
-            float2 t;
-            if (EXACT) {
-                t = th_step(u, w, l_t);
-            } else {
-                const float k = th_coef_fast(u, w, l_t, fg);
-                t = make_float2(u.x + k * w.x, u.y + k * w.y);
-            }
+            const float k = CAREFUL ? coef[c] : th_coef_fast(u, w, l_t, fg);
+            const float2 t = make_float2(u.x + k * w.x, u.y + k * w.y);
             const float2 un = make_float2(t.x + theta * div1, t.y + theta * div2);
             s.u[v][c] = un;
             const float e1 = un.x - u.x, e2 = un.y - u.y;
@@ -1110,6 +1154,8 @@ __device__ __forceinline__ void rt_iteration(RtState<T::V> &s, typename T::Smem 
         const float rx = __shfl_down_sync(0xffffffffu, s.u[v][0].x, 1);
         const float ry = __shfl_down_sync(0xffffffffu, s.u[v][0].y, 1);
         const int y = y0 + v;
+        FastGuard row;
+        float4 f[2], pn[2];
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             const float2 uc = s.u[v][c];
@@ -1119,8 +1165,21 @@ __device__ __forceinline__ void rt_iteration(RtState<T::V> &s, typename T::Smem 
             float f1x = ur.x - uc.x, f2x = ur.y - uc.y, f1y = ud.x - uc.x, f2y = ud.y - uc.y;
             if (BORDER && x + c == nx - 1) f1x = f2x = 0.0f;
             if (BORDER && y == ny - 1) f1y = f2y = 0.0f;
-            s.p[v][c] = EXACT ? dual_update(s.p[v][c], f1x, f1y, f2x, f2y, taut)
-                              : dual_update_fast(s.p[v][c], f1x, f1y, f2x, f2y, taut, fg);
+            if (CAREFUL) {
+                f[c] = make_float4(f1x, f1y, f2x, f2y);
+                pn[c] = dual_update_fast(s.p[v][c], f1x, f1y, f2x, f2y, taut, row);
+            } else {
+                s.p[v][c] = dual_update_fast(s.p[v][c], f1x, f1y, f2x, f2y, taut, fg);
+            }
+        }
+        if (CAREFUL) {
+            const bool look = __any_sync(0xffffffffu, row.broken());
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                if (look) pn[c] = dual_update_careful(s.p[v][c], f[c].x, f[c].y, f[c].z, f[c].w, taut);
+                s.p[v][c] = pn[c];
+            }
+            fg.add(row);
         }
     }
     sm.pb[wid][lane] = make_float4(s.p[V - 1][0].y, s.p[V - 1][0].w, s.p[V - 1][1].y, s.p[V - 1][1].w);
@@ -1172,10 +1231,10 @@ struct TbStart {
 // blocks write the state), iterations, snapshot stores and the final store of
 // the owned tile.  Each thread leaves its squared change of iteration j in
 // err[j].  Returns whether the thread's guard broke: the tile is then run
-// again from its untouched input, EXACT.  `issued` runs once the loads are in
+// again from its untouched input, CAREFUL.  `issued` runs once the loads are in
 // flight.  The pair and tile come from shared memory and are read again where
 // needed, so that they do not occupy registers during the iterations.
-template <typename T, bool EXACT, typename F>
+template <typename T, bool CAREFUL, typename F>
 __device__ __forceinline__ bool rt_tile(const TbArgs &a, const volatile int *vb, const volatile int *vtile,
                                         int tiles_x, const TbStart &t, typename T::Smem &sm,
                                         double (*err)[T::NT], F &&issued) {
@@ -1233,22 +1292,22 @@ __device__ __forceinline__ bool rt_tile(const TbArgs &a, const volatile int *vb,
 #pragma unroll 1
     for (int j = 0; j < *(volatile const int *)&t.kk; j++) {
         double e = 0.0;
-        if (!EXACT && interior)
-            rt_iteration<T, false, false>(s, sm, x, y0, nx, ny, a.l_t, a.theta, a.taut, fg, e);
+        if (interior)
+            rt_iteration<T, false, CAREFUL>(s, sm, x, y0, nx, ny, a.l_t, a.theta, a.taut, fg, e);
         else
-            rt_iteration<T, true, EXACT>(s, sm, x, y0, nx, ny, a.l_t, a.theta, a.taut, fg, e);
+            rt_iteration<T, true, CAREFUL>(s, sm, x, y0, nx, ny, a.l_t, a.theta, a.taut, fg, e);
         err[j][tid] = lane >= K / 2 && lane < 32 - K / 2 && wid >= K / V && wid < T::NW - K / V ? e : 0.0;
         if (t.snaps && j + 1 < t.kk)  // the state a stop after iteration j+1 accepts
             store(s, (t.cur >= 2 && t.cur < 2 + (K - 1) ? 2 + (K - 1) : 2) + j);
     }
     store(s, t.cur == 0 ? 1 : 0);
-    return !EXACT && fg.broken();
+    return fg.broken();
 }
 
 template <typename T>
-static __device__ __noinline__ void rt_tile_exact(const TbArgs &a, const volatile int *vb,
-                                                  const volatile int *vtile, int tiles_x, const TbStart &t,
-                                                  typename T::Smem &sm, double (*err)[T::NT]) {
+static __device__ __noinline__ void rt_tile_careful(const TbArgs &a, const volatile int *vb,
+                                                    const volatile int *vtile, int tiles_x, const TbStart &t,
+                                                    typename T::Smem &sm, double (*err)[T::NT]) {
     rt_tile<T, true>(a, vb, vtile, tiles_x, t, sm, err, [] {});
 }
 
@@ -1425,7 +1484,7 @@ __global__ void __launch_bounds__(T::NT, MINB) k_tvl1_tb(const __grid_constant__
     __syncthreads();
     const int tiles_x = gridDim.x;
     if (__syncthreads_or(rt_tile<T, false>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err[0], [] {}))) {
-        rt_tile_exact<T>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err[0]);
+        rt_tile_careful<T>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err[0]);
         __syncthreads();
     }
     if (threadIdx.x < 32)
@@ -1535,7 +1594,7 @@ __global__ void __launch_bounds__(T::NT, MINB) k_tvl1_q(const __grid_constant__ 
         }
         __syncthreads();
         if (*v_b < 0) return;
-        const bool broken = rt_tile<T, false>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err[it], [&] {
+        const auto claim_ahead = [&] {
             if (threadIdx.x == 0) {
                 // not near the end of a block of iterations, where a tile
                 // claimed by a busy block would wait for it while others idle
@@ -1546,9 +1605,9 @@ __global__ void __launch_bounds__(T::NT, MINB) k_tvl1_q(const __grid_constant__ 
                 }
                 v_ahead[it] = ahead;
             }
-        });
-        if (__syncthreads_or(broken)) {
-            rt_tile_exact<T>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err[it]);
+        };
+        if (__syncthreads_or(rt_tile<T, false>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err[it], claim_ahead))) {
+            rt_tile_careful<T>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err[it]);
             __syncthreads();
         }
     }
