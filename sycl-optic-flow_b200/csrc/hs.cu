@@ -274,8 +274,9 @@ template <typename T> struct HsSmem {
     float2 d0[T::RH][T::RW], d1[T::RH][T::RW], in[T::RH][T::RW];
 };
 
-// Brings a tile's region into shared memory: by one thread's TMA boxes (zero
-// outside the level), completing on `bar`, or by every thread's loads.
+// Brings a tile's region into shared memory (zeros outside the level): by one
+// thread's TMA boxes, completing on `bar`, or by every thread's cp.async of two
+// pixels (one, where rows don't start on 16 bytes), waited for by wait_all.
 template <typename T>
 __device__ __forceinline__ void hs_fetch_tma(const HsJacobiArgs &a, int tile, HsSmem<T> &sm, uint32_t bar) {
     const HsAt t = hs_at<T>(a, tile);
@@ -288,14 +289,29 @@ template <typename T>
 __device__ __forceinline__ void hs_fetch(const HsJacobiArgs &a, int tile, HsSmem<T> &sm) {
     const HsAt t = hs_at<T>(a, tile);
     const float2 *D0 = a.D + (size_t)t.b * a.dstride, *D1 = D0 + a.plane, *In = a.in + (size_t)t.b * a.stride;
-    const float2 z = make_float2(0.f, 0.f);
-    for (int i = threadIdx.x; i < T::RH * T::RW; i += T::NT) {
-        const int rx = i % T::RW, ry = i / T::RW, x = t.ox + rx, y = t.oy + ry;
-        const bool in = x >= 0 && x < a.w && y >= 0 && y < a.h;
-        const size_t q = (size_t)y * a.w + x;
-        sm.d0[ry][rx] = in ? D0[q] : z;
-        sm.d1[ry][rx] = in ? D1[q] : z;
-        if (!a.first) sm.in[ry][rx] = in ? In[q] : z;
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int ry = threadIdx.x >> 5; ry < T::RH; ry += T::NW) {
+        const int y = t.oy + ry;
+        const bool iy = y >= 0 && y < a.h;
+        if (a.vec) {
+            const int rx = 2 * lane, x = t.ox + rx;
+            const bool in = iy && x >= 0 && x < a.w;
+            const size_t q = in ? (size_t)y * a.w + x : 0;
+            cp_async16(smem_u32(&sm.d0[ry][rx]), D0 + q, in);
+            cp_async16(smem_u32(&sm.d1[ry][rx]), D1 + q, in);
+            if (!a.first) cp_async16(smem_u32(&sm.in[ry][rx]), In + q, in);
+        } else {
+#pragma unroll
+            for (int rx = lane; rx < T::RW; rx += 32) {
+                const int x = t.ox + rx;
+                const bool in = iy && x >= 0 && x < a.w;
+                const size_t q = in ? (size_t)y * a.w + x : 0;
+                cp_async8(smem_u32(&sm.d0[ry][rx]), D0 + q, in);
+                cp_async8(smem_u32(&sm.d1[ry][rx]), D1 + q, in);
+                if (!a.first) cp_async8(smem_u32(&sm.in[ry][rx]), In + q, in);
+            }
+        }
     }
 }
 
@@ -381,9 +397,12 @@ __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const H
 }
 
 // Resident blocks walk the tiles of all pairs; a tile's data is brought to
-// shared memory (TMA, where the level's strides allow it) while the block's
-// previous tile is in the registers.
-template <typename T, int MINB>
+// shared memory (TMA, where the level's strides allow it and there is a flag for
+// its bounded wait) while the block's previous tile is in the registers.  Without
+// TMA the copies take every thread's instructions: 48 pairs of 321x241, 104 sweeps,
+// 1.55 ms (of 320x240 1.13); loading a tile between two barriers, with nothing else to
+// run on the SM meanwhile, 2.55.
+template <typename T, int MINB, bool TMA>
 __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant__ HsJacobiArgs a) {
     extern __shared__ __align__(128) char hs_dyn[];
     HsSmem<T> &sm = *reinterpret_cast<HsSmem<T> *>(hs_dyn);
@@ -393,18 +412,19 @@ __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant
     const uint32_t bar = smem_u32(&s_bar), hint = smem_u32(&s_hint);
     uint32_t parity = 0;
     if (threadIdx.x == 0) {
-        if (a.tma) {
+        if (TMA) {
             mbar_init(bar, 1);
             fence_mbar_init();
             hs_fetch_tma<T>(a, blockIdx.x, sm, bar);
         }
         cp_async4(hint, a.hint + blockIdx.x);
     }
+    if (!TMA) hs_fetch<T>(a, blockIdx.x, sm);
     __syncthreads();  // the barrier is initialised before anyone waits on it
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
         const int next = tile + gridDim.x;
         asm volatile("cp.async.wait_all;\n" ::: "memory");
-        if (a.tma) {
+        if (TMA) {
             const bool ok = mbar_wait_bounded(bar, parity);
             parity ^= 1u;
             if (__syncthreads_or(!ok)) {
@@ -415,24 +435,24 @@ __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant
                 return;
             }
         } else {
-            hs_fetch<T>(a, tile, sm);
             __syncthreads();
         }
         const bool careful = !a.first && s_hint != 0;  // (the first launch writes every tile's hint)
         const auto fetch_next = [&] {
-            if (next < a.tiles && threadIdx.x == 0) {
-                if (a.tma) {
-                    fence_async_smem();  // the block's reads of this tile, then the copies of the next
-                    hs_fetch_tma<T>(a, next, sm, bar);
-                }
-                cp_async4(hint, a.hint + next);  // (nobody waits for it before the tile's data)
+            if (next >= a.tiles) return;
+            if (!TMA) {
+                hs_fetch<T>(a, next, sm);
+            } else if (threadIdx.x == 0) {
+                fence_async_smem();  // the block's reads of this tile, then the copies of the next
+                hs_fetch_tma<T>(a, next, sm, bar);
             }
+            if (threadIdx.x == 0) cp_async4(hint, a.hint + next);  // (nobody waits for it before the tile's data)
         };
         bool bad = careful;
         if (!careful && hs_tile<T, false>(a, tile, sm, sRow, fetch_next)) {
             bad = true;
             // again from the untouched input, then the next tile's copies again
-            if (a.tma && next < a.tiles) {
+            if (TMA && next < a.tiles) {
                 const bool ok = mbar_wait_bounded(bar, parity);
                 parity ^= 1u;
                 if (__syncthreads_or(!ok)) {
@@ -441,7 +461,10 @@ __global__ void __launch_bounds__(T::NT, MINB) k_hs_jacobi(const __grid_constant
                     return;
                 }
             }
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            __syncthreads();
             hs_fetch<T>(a, tile, sm);
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
             __syncthreads();
         }
         if (bad) bad = hs_tile<T, true>(a, tile, sm, sRow, fetch_next);
@@ -837,11 +860,14 @@ template <int C> static void hs_jacobi_launch(int B, cudaStream_t st, const HsJa
     t.tiles_x = div_up(a.w, T::TW);
     t.tiles_y = div_up(a.h, T::TH);
     t.tiles = t.tiles_x * t.tiles_y * B;
-    k_hs_jacobi<T, kHsCfgs[C].mb><<<imin(t.tiles, kHsCfgs[C].mb * kNumSMs), T::NT, hs_smem<C>(), st>>>(t);
+    const auto k = a.tma ? k_hs_jacobi<T, kHsCfgs[C].mb, true> : k_hs_jacobi<T, kHsCfgs[C].mb, false>;
+    k<<<imin(t.tiles, kHsCfgs[C].mb * kNumSMs), T::NT, hs_smem<C>(), st>>>(t);
 }
 
 template <int C> static void hs_set_smem_attr() {
-    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<HsCfgTile<C>, kHsCfgs[C].mb>,
+    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<HsCfgTile<C>, kHsCfgs[C].mb, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, hs_smem<C>()));
+    OF_CUDA(cudaFuncSetAttribute(k_hs_jacobi<HsCfgTile<C>, kHsCfgs[C].mb, false>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, hs_smem<C>()));
 }
 static void hs_jacobi_cfg(int c, int B, cudaStream_t st, const HsJacobiArgs &a) {
