@@ -19,6 +19,9 @@
 #include <cudaTypedefs.h>
 
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 #include "common.cuh"
 #include "hs.hpp"
@@ -887,27 +890,87 @@ using HsRes8 = HsTile<2, 16, 8>;
 using HsRes4 = HsTile<2, 16, 4>;
 template <typename T> static bool hs_res_fits(int w, int h) { return div_up(w, T::TW) * div_up(h, T::TH) <= 16; }
 
+// Launch configuration of n blocks in clusters of C; at: its cluster attribute.
+template <typename T> static cudaLaunchConfig_t hs_res_config(int n, int C, cudaLaunchAttribute &at) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(n);
+    lc.blockDim = dim3(T::NT);
+    lc.dynamicSmemBytes = sizeof(HsRes<T>);
+    at = cudaLaunchAttribute{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    return lc;
+}
+
 template <typename T> static void hs_res_launch(int B, cudaStream_t st, HsJacobiArgs a) {
     a.tiles_x = div_up(a.w, T::TW);
     a.tiles_y = div_up(a.h, T::TH);
     a.tiles = a.tiles_x * a.tiles_y * B;
     cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = a.tiles_x * a.tiles_y;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(a.tiles);
-    lc.blockDim = dim3(T::NT);
-    lc.dynamicSmemBytes = sizeof(HsRes<T>);
+    cudaLaunchConfig_t lc = hs_res_config<T>(a.tiles, a.tiles_x * a.tiles_y, at);
     lc.stream = st;
-    lc.attrs = &at;
-    lc.numAttrs = 1;
     OF_CUDA(cudaLaunchKernelEx(&lc, k_hs_res<T>, a));
 }
 
+constexpr int kHsResAlone = 120 * 1024;  // shared memory that leaves a block its SM
+
 template <typename T> static void hs_res_attrs() {
-    OF_CUDA(cudaFuncSetAttribute(k_hs_res<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HsRes<T>)));
+    OF_CUDA(cudaFuncSetAttribute(k_hs_res<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHsResAlone));
     OF_CUDA(cudaFuncSetAttribute(k_hs_res<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+}
+
+// Clusters of C blocks that run at the same time, two blocks on an SM or (alone) one
+// (0: the device takes none).
+template <typename T> static int hs_res_active(int C, bool alone) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, int, bool>, int> seen;
+    int dev = 0;
+    OF_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(dev, C, alone);
+    const auto it = seen.find(key);
+    if (it != seen.end()) return it->second;
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t lc = hs_res_config<T>(C, C, at);
+    if (alone) lc.dynamicSmemBytes = kHsResAlone;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_hs_res<T>, &lc) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return seen[key] = n;
+}
+
+// Microseconds of K sweeps and an exchange: alone on the SMs, and two blocks an SM.
+template <typename T> static float hs_res_form_time(int w, int h, int B, int sweeps, float alone, float shared) {
+    const int C = div_up(w, T::TW) * div_up(h, T::TH), most = hs_res_active<T>(C, false);
+    if (most <= 0) return 1e30f;
+    const int waves = (B - 1) / most, rest = B - waves * most;
+    const float t = (float)waves * shared + (rest <= hs_res_active<T>(C, true) ? alone : shared);
+    return t * (float)div_up(sweeps, T::K);
+}
+// Microseconds of the sweeps of B pairs in resident levels (1e30: not possible).
+// OFLOW_HS_RES=0: as on a device that takes no clusters (used to test it).
+static float hs_res_time(int w, int h, int B, int sweeps) {
+    if (const char *e = getenv("OFLOW_HS_RES"))
+        if (!atoi(e)) return 1e30f;
+    if (hs_res_fits<HsRes8>(w, h)) return hs_res_form_time<HsRes8>(w, h, B, sweeps, 3.8f, 7.2f);
+    if (hs_res_fits<HsRes4>(w, h)) return hs_res_form_time<HsRes4>(w, h, B, sweeps, 2.3f, 4.0f);
+    return 1e30f;
+}
+
+// Microseconds of the sweeps in launches of a configuration, by TMA or without: what
+// a launch takes with one tile an SM, and what each further tile of the busiest SM
+// adds.  Fitted to 40x30 to 1280x720, 1 to 64 pairs, 52 to 200 sweeps.
+constexpr float kHsAlone[2][kHsNumCfgs] = {{6.8f, 4.4f, 9.3f, 4.05f, 13.9f, 6.55f}, {5.9f, 4.1f, 8.5f, 3.85f, 13.2f, 6.2f}};
+constexpr float kHsMore[2][kHsNumCfgs] = {{5.5f, 2.5f, 7.7f, 2.2f, 11.4f, 4.4f}, {4.1f, 1.9f, 6.25f, 1.75f, 10.0f, 3.45f}};
+static float hs_tiles_time(int c, int w, int h, int B, int sweeps, bool tma) {
+    const HsJCfg &f = kHsCfgs[c];
+    const long long tiles = (long long)div_up(w, 64 - 2 * f.k) * div_up(h, f.v * f.nw - 2 * f.k) * B;
+    return (float)div_up(sweeps, f.k) * (kHsAlone[tma][c] + (float)((tiles - 1) / kNumSMs) * kHsMore[tma][c]);
 }
 
 static void hs_set_smem_attrs() {
@@ -921,12 +984,13 @@ static void hs_set_smem_attrs() {
     hs_res_attrs<HsRes4>();
 }
 
-// All sweeps of one warp: from zero increments to the flow updated.  The small
-// tiles run resident where a cluster holds the level.
+// All sweeps of one warp: from zero increments to the flow updated.  Configuration 5
+// runs resident where a cluster holds the level and that is the faster way.
 static void hs_sweeps(int cfg, int B, cudaStream_t st, const float2 *D, size_t plane, float2 *const dU[2],
                       float2 *U, size_t stride, int w, int h, int sweeps, bool update, int *hint, int *err) {
     const int K = kHsCfgs[cfg].k;
-    if (cfg == 5 && sweeps > 0 && (hs_res_fits<HsRes8>(w, h) || hs_res_fits<HsRes4>(w, h))) {
+    const bool vec = (w & 1) == 0 && (stride & 1) == 0;  // and so by TMA, if there is a flag for its wait
+    if (cfg == 5 && sweeps > 0 && hs_res_time(w, h, B, sweeps) < hs_tiles_time(5, w, h, B, sweeps, vec && err)) {
         HsJacobiArgs a;
         memset(&a, 0, sizeof(a));
         a.D = D;
@@ -938,7 +1002,7 @@ static void hs_sweeps(int cfg, int B, cudaStream_t st, const float2 *D, size_t p
         a.h = h;
         a.sweeps = sweeps;
         a.last = update;
-        a.vec = (w & 1) == 0 && (stride & 1) == 0;
+        a.vec = vec;
         if (hs_res_fits<HsRes8>(w, h)) hs_res_launch<HsRes8>(B, st, a);
         else hs_res_launch<HsRes4>(B, st, a);
         return;
@@ -959,28 +1023,34 @@ static void hs_sweeps(int cfg, int B, cudaStream_t st, const float2 *D, size_t p
         a.sweeps = k;
         a.first = done == 0;
         a.last = update && done + k == sweeps;
-        a.vec = (w & 1) == 0 && (stride & 1) == 0;
+        a.vec = vec;
         hs_maps(a, cfg, B, err);
         hs_jacobi_cfg(cfg, B, st, a);
         done += k;
     }
 }
 
-// The configuration of a level; OFLOW_HS_CFG forces one (used to test and time
-// them), and a plan's tuning table comes before it.  A level whose 48x16 tiles
-// all fit on the GPU at once is bound by the launches' latency: small tiles of 8
-// sweeps, resident where a cluster holds the level (150 sweeps of a single
-// 160x120, 80x60 or 40x30 level in launches: 0.12 ms against 0.16 with 48x48
-// tiles, 0.15 to 0.22 with 4 sweeps a launch).  Larger work takes
-// 48x48 tiles of 8 sweeps (64 pairs of 320x240, 200 sweeps: 2.7 ms against 3.1 to
-// 3.7).
-static int hs_pick(int w, int h, int B) {
+// The configuration of a level, the one with the least estimated time; OFLOW_HS_CFG
+// forces one (used to test and time them), and a plan's tuning table comes before it.
+// 104 sweeps of B pairs, here and by two forms alone (resident or 48x16 tiles up to
+// 296 of them, else 48x48 tiles), both with tiles fetched ahead:
+//   101x99, 20 pairs 168 and 265 us; 145x97, 13: 143 and 254; 160x120, 13: 134 and 224;
+//   193x145, 8: 201 and 247; 337x170, 5: 199 and 243; 400x300, 1: 102 and 139
+static int hs_pick(int w, int h, int B, int sweeps, bool tma) {
     if (const char *e = getenv("OFLOW_HS_CFG")) {
         const int c = atoi(e);
         if (c >= 0 && c < kHsNumCfgs) return c;
     }
-    const long long small = (long long)div_up(w, 48) * div_up(h, 16) * B;
-    return small <= 2 * kNumSMs ? 5 : 2;
+    int best = 5;
+    float best_t = hs_res_time(w, h, B, sweeps);
+    for (int c = 0; c < kHsNumCfgs; c++) {
+        const float t = hs_tiles_time(c, w, h, B, sweeps, tma);
+        if (t < best_t) {
+            best_t = t;
+            best = c;
+        }
+    }
+    return best;
 }
 
 HsPlan::HsPlan(int w, int h, int B, int dtype, const oflow_hs_params &prm, const TuneTable *tuned)
@@ -1028,7 +1098,8 @@ HsPlan::HsPlan(int w, int h, int B, int dtype, const oflow_hs_params &prm, const
     for (int l = 0; l < L_; l++) {
         const auto it = tuned ? tuned->find(tune_key(W_[l], H_[l], B, kTuneHs)) : TuneTable::const_iterator();
         const bool ok = tuned && it != tuned->end() && it->second >= 0 && it->second < kHsNumCfgs;
-        jcfg_[l] = ok ? it->second : hs_pick(W_[l], H_[l], B);
+        jcfg_[l] = ok ? it->second
+                      : hs_pick(W_[l], H_[l], B, prm.nsolver, (W_[l] & 1) == 0 && (N_ & 1) == 0);
     }
 }
 
@@ -1225,7 +1296,7 @@ void hs_enqueue_into(void *scratch, const float *I0, const float *I1, int w, int
             dim3 dg(div_up(lw, kDTW), div_up(lh, kDTH), 1);
             k_hs_warp_deriv<<<dg, dim3(kDTW, kDTH), 0, st>>>(pyr + pyr_off[l], lp, lw, lh,
                                                              Ubuf[ub], N, 0, prm.alpha, D, N, N);
-            hs_sweeps(hs_pick(lw, lh, 1), 1, st, D, N, dU, Ubuf[ub], N, lw, lh, prm.nsolver, true,
+            hs_sweeps(hs_pick(lw, lh, 1, prm.nsolver, false), 1, st, D, N, dU, Ubuf[ub], N, lw, lh, prm.nsolver, true,
                       reinterpret_cast<int *>(out), nullptr);
         }
         if (l != top) {
