@@ -159,8 +159,10 @@ oflow_status oflow_tvl1_batch_profile(oflow_ctx *ctx, int n, const oflow_image *
  * 16 blocks (4 and 5 where the level fits).
  * cfg_per_scale (OFLOW_MAX_SCALES ints, may be NULL) receives the choice per
  * scale, -1 past the last scale.  The table lives in the context; it can be
- * saved to / loaded from a text file (lines: solver width height batch config)
- * keyed by the level size, so plans built later pick it up. */
+ * saved to / loaded from a text file (lines: solver width height batch config
+ * shape) keyed by the level size, so plans built later pick it up.  Lines whose
+ * shape is missing or not the one that the number stands for (tables saved when
+ * the numbers stood for other shapes) are read and left out. */
 oflow_status oflow_tvl1_autotune(oflow_ctx *ctx, int n, const oflow_image *I0,
                                  const oflow_image *I1, const oflow_tvl1_params *p,
                                  int *cfg_per_scale);

@@ -727,10 +727,13 @@ oflow_status oflow_ctx_save_tuning(oflow_ctx *ctx, const char *path) {
         OF_CHECK(ctx != nullptr && path != nullptr, "save tuning: null argument");
         FILE *f = fopen(path, "w");
         OF_CHECK(f != nullptr, std::string("save tuning: cannot open ") + path);
-        fprintf(f, "# oflow tuning table: solver level_width level_height batch config\n");
-        for (const auto &kv : ctx->tune)
-            fprintf(f, "%s %d %d %d %d\n", std::get<0>(kv.first) == kTuneHs ? "hs" : "tvl1",
-                    std::get<1>(kv.first), std::get<2>(kv.first), std::get<3>(kv.first), kv.second);
+        fprintf(f, "# oflow tuning table: solver level_width level_height batch config shape\n");
+        for (const auto &kv : ctx->tune) {
+            const bool hs = std::get<0>(kv.first) == kTuneHs;
+            fprintf(f, "%s %d %d %d %d %s\n", hs ? "hs" : "tvl1", std::get<1>(kv.first), std::get<2>(kv.first),
+                    std::get<3>(kv.first), kv.second,
+                    (hs ? hs_config_name(kv.second) : tvl1_config_name(kv.second)).c_str());
+        }
         fclose(f);
     });
 }
@@ -740,15 +743,18 @@ oflow_status oflow_ctx_load_tuning(oflow_ctx *ctx, const char *path) {
         OF_CHECK(ctx != nullptr && path != nullptr, "load tuning: null argument");
         FILE *f = fopen(path, "r");
         OF_CHECK(f != nullptr, std::string("load tuning: cannot open ") + path);
-        char line[256], solver[16];
+        char line[256], solver[16], shape[32];
         int w, h, B, c, bad = 0;
         while (fgets(line, sizeof line, f)) {
             if (line[0] == '#' || line[0] == '\n') continue;
-            if (sscanf(line, "%15s %d %d %d %d", solver, &w, &h, &B, &c) != 5 || c < 0) {
+            shape[0] = 0;
+            if (sscanf(line, "%15s %d %d %d %d %31s", solver, &w, &h, &B, &c, shape) < 5 || c < 0) {
                 bad = 1;
                 break;
             }
             const int kind = std::string(solver) == "hs" ? kTuneHs : kTuneTvl1;
+            // the number of a table without shapes, or with another, was the choice among others
+            if ((kind == kTuneHs ? hs_config_name(c) : tvl1_config_name(c)) != shape || !shape[0]) continue;
             ctx->tune[tune_key(w, h, B, kind)] = c;
         }
         fclose(f);

@@ -812,6 +812,12 @@ struct HsJCfg {
 };
 constexpr HsJCfg kHsCfgs[] = {{4, 16, 4, 1}, {4, 8, 4, 2}, {4, 16, 8, 1}, {2, 12, 4, 2}, {4, 16, 16, 1}, {2, 16, 8, 2}};
 constexpr int kHsNumCfgs = 6;
+std::string hs_config_name(int c) {  // owned tile and sweeps a launch
+    if (c < 0 || c >= kHsNumCfgs) return "";
+    const HsJCfg &f = kHsCfgs[c];
+    return std::to_string(64 - 2 * f.k) + "x" + std::to_string(f.v * f.nw - 2 * f.k) + "/" + std::to_string(f.k);
+}
+
 template <int C> using HsCfgTile = HsTile<kHsCfgs[C].v, kHsCfgs[C].nw, kHsCfgs[C].k>;
 
 template <int C> constexpr int hs_smem() { return (int)sizeof(HsSmem<HsCfgTile<C>>); }

@@ -67,6 +67,11 @@ inline bool cfg_tile(int c, int &tw, int &th) {
     }
     return false;
 }
+std::string tvl1_config_name(int c) {
+    int tw, th;
+    if (cfg_tile(c, tw, th)) return std::to_string(tw) + "x" + std::to_string(th);
+    return c == kLevelCfg ? "block" : c == kClusterCfg ? "cluster" : "";
+}
 // How a level of nx x ny is cut for k_tvl1_res: C blocks of wx x wy warps, a
 // thread with cpl columns of v rows.  false: it does not fit.
 struct ResCut {

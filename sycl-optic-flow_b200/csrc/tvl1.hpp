@@ -4,6 +4,7 @@
 #pragma once
 
 #include <map>
+#include <string>
 #include <tuple>
 
 #include "internal.hpp"
@@ -24,6 +25,11 @@ int tvl1_nscales(int w, int h, int nscales, float zfactor);
 using TuneKey = std::tuple<int, int, int, int>;
 using TuneTable = std::map<TuneKey, int>;
 enum { kTuneTvl1 = 1, kTuneHs = 2 };
+// What a configuration's number stands for in a saved table ("" for none): a
+// table saved by a build whose numbers stand for something else is not taken at
+// its numbers.
+std::string tvl1_config_name(int c);
+std::string hs_config_name(int c);
 inline TuneKey tune_key(int w, int h, int B, int solver = kTuneTvl1) {
     return TuneKey(solver, w, h, B);
 }
