@@ -182,6 +182,14 @@ oflow_status oflow_ctx_load_tuning(oflow_ctx *ctx, const char *path);
  *   which 1: the refined reciprocal equal to __frcp_rn, bit patterns [lo, hi)
  *   which 3: Markstein's quotient from the refined reciprocal equal to IEEE
  *            division, seeded pseudo-random operands, indices [lo, hi)
+ *   which 4: the square root behind the dual update's hypot within seed - 1 units
+ *            (seed 0: the 8 its rounding test allows for) of the last place of the IEEE
+ *            square root, and the estimate it starts from within 2^-20, for the
+ *            upper words of indices [lo, hi) (21 bits of mantissa and exponent
+ *            parity, then every second exponent from 2^-400 on: hi up to 330 << 21)
+ *   which 5: that hypot, where its rounding test passes it, equal to the square root
+ *            of the sum in double, rounded; seeded operands, on and next to
+ *            midpoints among them, indices [lo, hi)
  * (other values of which: OFLOW_ERR_BAD_ARG)
  * Synchronous on the default stream of the current device; *mismatches
  * receives the count (0 means the contract held on every operand). */

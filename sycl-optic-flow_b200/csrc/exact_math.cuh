@@ -37,7 +37,8 @@ __host__ __device__ __forceinline__ float hypot_ref(float a, float b) {
 // (rsqrt.approx; its relative error is below 2^-20 on every upper word, the
 // only one the unit reads, which leaves 2^-58 after the step) and Ziv's
 // rounding test.  The double result r is within kHypotUnits units of its last
-// place of the root, so it rounds to single precision as hypot_ref does unless
+// place of the root (measured: within 1, on every upper word of the sums' exponents
+// with three lower words each; oflow_selftest_math), so it rounds to single precision as hypot_ref does unless
 // it lies that close to the midpoint of two neighbouring floats (one sum in
 // 2^25).  `near` is the distance above the lower end of that interval, of the
 // 29 bits below a float's last, modulo 2^32: the result stands if it is above
@@ -45,14 +46,16 @@ __host__ __device__ __forceinline__ float hypot_ref(float a, float b) {
 // is far below a unit of any other; a root below 2^-100 may round differently
 // from hypot_ref's, which 1 + c*hypot does not show.  Infinities give NaN.
 constexpr unsigned kHypotUnits = 8, kHypotNear = 2 * 8 * kHypotUnits;
-__device__ __forceinline__ float hypot_fast(float a, float b, unsigned &near) {
-    const double da = a, db = b;
-    const double s = __fma_rn(da, da, __fma_rn(db, db, 0x1p-400));
-    double y;
+__device__ __forceinline__ double hypot_root(double s, double &y) {  // of s; y: the estimate
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
     const double h = __dmul_rn(s, y);
     const double e = __fma_rn(-h, y, 1.0);  // s y^2 = 1 - e
-    const double r = __fma_rn(__dmul_rn(h, e), __fma_rn(e, 0.375, 0.5), h);
+    return __fma_rn(__dmul_rn(h, e), __fma_rn(e, 0.375, 0.5), h);
+}
+__device__ __forceinline__ float hypot_fast(float a, float b, unsigned &near) {
+    const double da = a, db = b;
+    double y;
+    const double r = hypot_root(__fma_rn(da, da, __fma_rn(db, db, 0x1p-400)), y);
     near = (unsigned)__double2loint(r) * 8u + (8u * kHypotUnits - 0x80000000u);
     return (float)r;
 }
