@@ -315,7 +315,7 @@ __device__ __forceinline__ void lk_warp_pixels(const int (&rx)[M], const int (&r
                                                int RW, const float *__restrict__ I0, const float *__restrict__ I1,
                                                const float2 *__restrict__ G, const float2 *__restrict__ U, int nx,
                                                int ny, float *gx, float *gy, float *gt) {
-    int q[M], base[M];
+    unsigned q[M], base[M];  // (more pixels than these count don't fit the device's memory)
     bool in[M], easy[M];
     float2 u[M], g[M];
     float i0[M], xf[M], yf[M], v00[M], v10[M], v01[M], v11[M];
@@ -323,7 +323,7 @@ __device__ __forceinline__ void lk_warp_pixels(const int (&rx)[M], const int (&r
     for (int m = 0; m < M; m++) {
         const int x = x0 + rx[m], y = y0 + ry[m];
         in[m] = on[m] && x >= 0 && x < nx && y >= 0 && y < ny;
-        q[m] = in[m] ? y * nx + x : 0;
+        q[m] = in[m] ? (unsigned)y * (unsigned)nx + (unsigned)x : 0;
         u[m] = U[q[m]];
         xf[m] = (float)x;
         yf[m] = (float)y;
@@ -338,7 +338,7 @@ __device__ __forceinline__ void lk_warp_pixels(const int (&rx)[M], const int (&r
         xf[m] += u[m].x;
         yf[m] += u[m].y;
         easy[m] = xf[m] >= 0.0f && yf[m] >= 0.0f && xf[m] < (float)(nx - 1) && yf[m] < (float)(ny - 1);
-        base[m] = easy[m] ? (int)yf[m] * nx + (int)xf[m] : 0;  // (nonnegative: truncation is floor)
+        base[m] = easy[m] ? (unsigned)yf[m] * (unsigned)nx + (unsigned)xf[m] : 0;  // (nonnegative: truncation is floor)
         const float *p = I1 + base[m];
         v00[m] = __ldg(p);
         v10[m] = __ldg(p + 1);
