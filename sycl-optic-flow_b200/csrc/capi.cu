@@ -810,7 +810,9 @@ oflow_status oflow_hs_batch(oflow_ctx *ctx, int n, const oflow_image *I0,
             }
         }
         finish(ctx, device_only);
-        for (HsPlan *pl : ran) pl->check_device_error();
+        // (a batch of more sizes than are kept has dropped its first plans)
+        for (auto &q : ctx->hs)
+            if (std::find(ran.begin(), ran.end(), q.get()) != ran.end()) q->check_device_error();
     });
 }
 
