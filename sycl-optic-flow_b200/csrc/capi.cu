@@ -93,11 +93,10 @@ struct MixedBatch {
 // A TV-L1 batch with frames or flows in host memory may be solved in up to
 // this many chunks, each a plan of its own on a side stream, so that the
 // copies of one chunk overlap the solves of the others (OFLOW_HOST_CHUNKS).
-// By default it is one plan with its copies before and after: for 32 pairs of
-// 1024x436 that measured 1,155 pairs/s end to end against 1,143 with four
-// concurrent chunks (one launch per block of iterations) and 778-986 with the
-// chunks' solves one after another, each with the work queue (a small plan
-// pays the latency-bound coarse scales again).
+// By default it is one plan with its copies before and after, chosen when that
+// was the faster way; with the present kernels 32 pairs of 1024x436 from pinned
+// memory and back take 22.7 ms that way, 21.6 in two and 21.0 in four concurrent
+// chunks (one launch per block of iterations).
 constexpr int kHostChunks = 4;
 constexpr int kChunkMinPairs = 4;
 
@@ -208,9 +207,10 @@ TvPlan &side_plan(oflow_ctx *ctx, int c, int chunks, int w, int h, int B, int dt
     v.emplace_back(new TvPlan(w, h, B, dtype, p, false, &ctx->tune));
     // chunks share the GPU: one launch per block of iterations, interleaving
     // with the other chunks' kernels.  OFLOW_SIDE_QUEUE=n runs the work queue
-    // instead, each chunk's launches on 1/n of the resident slots; measured
-    // end to end: 1,118 pairs/s with n = 4 and 954 with n = 1, against 1,133
-    // (persistent blocks hold SMs the other chunks' kernels need).
+    // instead, each chunk's launches on 1/n of the resident slots: 32 pairs of
+    // 1024x436 in four chunks take 20.5 ms end to end with n = 4 and 23.0 with
+    // n = 1, where persistent blocks hold SMs the other chunks' kernels need
+    // (launches: 21.0).
     const char *e = getenv("OFLOW_SIDE_QUEUE");
     const int sq = e ? atoi(e) : 0;
     v.back()->use_queue(sq > 0);

@@ -60,11 +60,6 @@ namespace {
 
 constexpr int kUmBM = 128;       // rows of a tile (UMMA M)
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
-    const int n = valid ? 16 : 0;  // 0 bytes read: the destination is zero-filled
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n)
-                 : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
@@ -212,7 +207,7 @@ __global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
             const int ry = px / RW, rx = px % RW, yy = y0 + ry, xx = x0 + rx;
             const bool ok = (unsigned)yy < (unsigned)d.H && (unsigned)xx < (unsigned)d.W;
             const int pos = MODE == kUmStride2 ? ry * RW + (rx >> 1) + (rx & 1 ? 8 * MT + 1 : 0) : px;
-            cp_async16(sreg + (uint32_t)(kc * PX + pos) * 16,
+            cp_async16_l1(sreg + (uint32_t)(kc * PX + pos) * 16,
                        ok ? xn + ((size_t)yy * d.W + xx) * d.C + c0 + kc * 8 : x, ok);
         }
     };
@@ -628,7 +623,7 @@ __global__ void __launch_bounds__(kWgNT) k_conv_wgrad_mn(ConvDims d, const __nv_
                 for (int px = apx; px < T::RH * 8; px += astep) {
                     const int yy = STRIDE * p0 - 1 + (px >> 3), xx = STRIDE * (q0 + (px & 7)) + sx - 1;
                     const bool ok = (unsigned)yy < (unsigned)d.H && (unsigned)xx < (unsigned)d.W;
-                    cp_async16(a + (uint32_t)(pl * T::PXA + px) * 16, ok ? xn + ((size_t)yy * d.W + xx) * d.C : x, ok);
+                    cp_async16_l1(a + (uint32_t)(pl * T::PXA + px) * 16, ok ? xn + ((size_t)yy * d.W + xx) * d.C : x, ok);
                 }
             const __nv_bfloat16 *gn = gb + (size_t)n * d.P * d.Q * d.K + kg * 8;
             if (bpx < BSTEP)
@@ -636,7 +631,7 @@ __global__ void __launch_bounds__(kWgNT) k_conv_wgrad_mn(ConvDims d, const __nv_
                 for (int px = bpx; px < 128; px += BSTEP) {
                     const int p = p0 + (px >> 3), q = q0 + (px & 7);
                     const bool ok = p < d.P && q < d.Q && kg * 8 < d.K;
-                    cp_async16(b + (uint32_t)(kg * T::PXB + px) * 16, ok ? gn + ((size_t)p * d.Q + q) * d.K : gb, ok);
+                    cp_async16_l1(b + (uint32_t)(kg * T::PXB + px) * 16, ok ? gn + ((size_t)p * d.Q + q) * d.K : gb, ok);
                 }
             cp_async_commit();
             // the tile bufs - 1 loads ago has landed

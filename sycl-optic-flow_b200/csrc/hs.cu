@@ -249,14 +249,6 @@ __device__ __forceinline__ void hs_step(HsState<T::V> &s, int j, float4 (*sRow)[
     hs_sweep<T, EDGE, CAREFUL>(s, above, below, e, broken, key);
 }
 
-// Two neighbouring float2 at q; in0, in1: inside the level.
-__device__ __forceinline__ float4 hs_ld_two(const float2 *p, size_t q, int vec, bool in0, bool in1) {
-    if (vec) return in0 ? *reinterpret_cast<const float4 *>(p + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 z = make_float2(0.f, 0.f);
-    const float2 a = in0 ? p[q] : z, b = in1 ? p[q + 1] : z;
-    return make_float4(a.x, a.y, b.x, b.y);
-}
-
 // Pair, region origin and the thread's first pixel of a tile.
 struct HsAt {
     int b, ox, oy, x, y0;
@@ -385,7 +377,7 @@ __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const H
         const size_t q = (size_t)(y0 + v) * w + x;
         float2 r0 = s.a[v][0], r1 = s.a[v][1];
         if (a.last) {
-            const float4 u = hs_ld_two(Out, q, a.vec, true, in1);
+            const float4 u = ld_two(Out, q, a.vec, true, in1);
             r0 = make_float2(u.x + r0.x, u.y + r0.y);
             r1 = make_float2(u.z + r1.x, u.w + r1.y);
         }
@@ -507,8 +499,8 @@ __device__ __forceinline__ bool hs_res_load(const HsJacobiArgs &a, const HsAt &t
     for (int v = 0; v < V; v++) {
         const bool iy = y0 + v >= 0 && y0 + v < h;
         const size_t q = iy && in0 ? (size_t)(y0 + v) * w + x : 0;
-        const float4 d0 = hs_ld_two(D0, q, a.vec, iy && in0, iy && in0 && in1);
-        const float4 d1 = hs_ld_two(D1, q, a.vec, iy && in0, iy && in0 && in1);
+        const float4 d0 = ld_two(D0, q, a.vec, iy && in0, iy && in0 && in1);
+        const float4 d1 = ld_two(D1, q, a.vec, iy && in0, iy && in0 && in1);
         s.ix[v][0] = d0.x; s.iy[v][0] = d0.y; s.iz[v][0] = d1.x; s.den[v][0] = iy && in0 ? d1.y : 1.0f;
         s.ix[v][1] = d0.z; s.iy[v][1] = d0.w; s.iz[v][1] = d1.z; s.den[v][1] = iy && in0 && in1 ? d1.w : 1.0f;
     }
@@ -652,7 +644,7 @@ __global__ void __launch_bounds__(T::NT, 2) k_hs_res(const __grid_constant__ HsJ
         const size_t q = (size_t)(y0 + v) * w + x;
         float2 r0 = s.a[v][0], r1 = s.a[v][1];
         if (a.last) {
-            const float4 u = hs_ld_two(Out, q, a.vec, true, in1);
+            const float4 u = ld_two(Out, q, a.vec, true, in1);
             r0 = make_float2(u.x + r0.x, u.y + r0.y);
             r1 = make_float2(u.z + r1.x, u.w + r1.y);
         }

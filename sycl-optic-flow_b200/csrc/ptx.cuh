@@ -15,18 +15,32 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Asynchronous 16-byte copy to shared memory (waited for by cp.async.wait_all).
+// Asynchronous copies to shared memory (waited for by cp.async.wait_*); !ok: zero
+// fill, src is not read.  _l1: through L1, for lines that other blocks of the SM or
+// later copies read again.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool ok) {
-    const int n = ok ? 16 : 0;  // 0: zero fill, src is not read
+    const int n = ok ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
-
+__device__ __forceinline__ void cp_async16_l1(uint32_t dst, const void *src, bool ok) {
+    const int n = ok ? 16 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void *src, bool ok) {
     const int n = ok ? 8 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Two neighbouring float2 at q, past L1 (vec: 16-byte aligned); in0, in1: which are
+// inside the level.
+__device__ __forceinline__ float4 ld_two(const float2 *p, size_t q, int vec, bool in0, bool in1) {
+    if (vec) return in0 ? __ldcg(reinterpret_cast<const float4 *>(p + q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 z = make_float2(0.f, 0.f);
+    const float2 a = in0 ? __ldcg(p + q) : z, b = in1 ? __ldcg(p + q + 1) : z;
+    return make_float4(a.x, a.y, b.x, b.y);
 }
 
 __device__ __forceinline__ unsigned long long globaltimer() {
@@ -80,8 +94,8 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
-// Loads from the shared memory of block `rank` of the cluster, at the address a
-// has in this block.
+// A load from the shared memory of block `rank` of the cluster, and a store to it, at
+// the address a has in this block.
 __device__ __forceinline__ float4 cluster_ld4(uint32_t a, int rank) {
     float4 v;
     asm volatile(
@@ -92,16 +106,6 @@ __device__ __forceinline__ float4 cluster_ld4(uint32_t a, int rank) {
         : "memory");
     return v;
 }
-__device__ __forceinline__ int cluster_ld1(uint32_t a, int rank) {
-    int v;
-    asm volatile(
-        "{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.s32 %0, [r];\n\t}\n"
-        : "=r"(v)
-        : "r"(a), "r"(rank)
-        : "memory");
-    return v;
-}
-
 __device__ __forceinline__ void cluster_st1(uint32_t a, int rank, int v) {
     asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.s32 [r], %2;\n\t}\n" ::"r"(a),
                  "r"(rank), "r"(v)
@@ -129,15 +133,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(dst),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1,
-                                            int c2, int c3, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
         : "memory");
 }
 

@@ -152,8 +152,8 @@ struct TbQueue {
 // iterations (the ones a snapshot serves) is plausible.  Elsewhere a stop
 // inside a launch falls back to re-running its iterations.  A snapshot launch
 // costs about 12 % more than a plain one, a missed stop about one launch of
-// the pair; 1.3 measured best among 2.0 (extrapolating K iterations), 2.0
-// and 1.3 (K-1 iterations) on the 1024x436 workload.
+// the pair.  32 pairs of 1024x436 take 20.1 ms with 2.0 and 18.8 to 19.2 with
+// anything from 1.0 to 1.3, no less than runs of one differ.
 constexpr float kSnapMargin = 1.3f;
 
 struct NormRec {  // |x|, first index, signed value
@@ -188,10 +188,6 @@ template <typename F2> struct Quads {
     F2 *a, *b;
     __device__ __forceinline__ float4 get(size_t q) const {
         const float2 u = a[q], v = b[q];
-        return make_float4(u.x, u.y, v.x, v.y);
-    }
-    __device__ __forceinline__ float4 get_ro(size_t q) const {
-        const float2 u = __ldg(a + q), v = __ldg(b + q);
         return make_float4(u.x, u.y, v.x, v.y);
     }
     __device__ __forceinline__ void set(size_t q, float4 v) const {
@@ -1073,7 +1069,7 @@ template <int V_, int NW_> struct RtTile {
         float4 w[2 * V][NT];    // row v: (I1wx, I1wy) of both columns at [2v], (rho_c, 1/grad) at [2v + 1]
         float4 pb[NW][32];      // (p12, p22) of both columns of each warp's last row
         float4 ut[NW][32];      // u of both columns of each warp's first row
-        double err[2][K][NT];   // squared change per thread and iteration, of this tile and the last
+        double err[K][NT];      // squared change per thread and iteration
     };
 };
 
@@ -1218,14 +1214,6 @@ __device__ __forceinline__ void rt_store(const RtState<T::V> &s, float2 *__restr
     }
 }
 
-// Two neighbouring float2 at q, past L1; in0, in1: inside the level.
-__device__ __forceinline__ float4 ld_two(const float2 *p, size_t q, int vec, bool in0, bool in1) {
-    if (vec) return in0 ? __ldcg(reinterpret_cast<const float4 *>(p + q)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 z = make_float2(0.f, 0.f);
-    const float2 a = in0 ? __ldcg(p + q) : z, b = in1 ? __ldcg(p + q + 1) : z;
-    return make_float4(a.x, a.y, b.x, b.y);
-}
-
 // State of a pair at the start of a block of iterations.
 struct TbStart {
     int cur, n0, redo, kk;
@@ -1325,9 +1313,8 @@ static __device__ __noinline__ void rt_tile_careful(const TbArgs &a, const volat
 // result is that of one iteration per launch either way.  Partials are summed
 // in a fixed order, so the decision does not depend on block scheduling.
 // One warp does it, after a block barrier behind every thread's stores and
-// errors, while the block's other warps go on to the next tile: the sums, the
-// fence behind the tile's stores and the arrival would hold up the whole block
-// for about a quarter of a tile's time.
+// errors; in the queue form the same warp then takes the next tile, and the
+// block's others wait for that.
 template <typename T>
 __device__ __forceinline__ void tb_decide(const TbArgs &a, TvCtrl *ctrl, int b, int tile,
                                           int ntiles, const double (*err)[T::NT], const TbStart &t,
@@ -1444,8 +1431,8 @@ __device__ __forceinline__ TbStart tb_start(const TbArgs &a, const TvCtrl *ctrl)
             if (n >= 1.0f && n < (float)t.kk) {
                 t.kk = (int)n;
                 // predict 2: trust the prediction, no snapshots (an earlier
-                // stop re-runs its iterations); measured 1,234 against 1,225
-                // pairs/s with snapshots, 1,176 with full blocks
+                // stop re-runs its iterations); 32 pairs of 1024x436 take
+                // 19.2 ms, 19.7 with snapshots and 20.2 with full blocks
                 if (a.predict == 2) t.snaps = false;
             }
         }
@@ -1488,12 +1475,12 @@ __global__ void __launch_bounds__(T::NT, MINB) k_tvl1_tb(const __grid_constant__
     }
     __syncthreads();
     const int tiles_x = gridDim.x;
-    if (__syncthreads_or(rt_tile<T, false>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err[0], [] {}))) {
-        rt_tile_careful<T>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err[0]);
+    if (__syncthreads_or(rt_tile<T, false>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err, [] {}))) {
+        rt_tile_careful<T>(a, &s_b, &s_tile, tiles_x, s_t, sm, sm.err);
         __syncthreads();
     }
     if (threadIdx.x < 32)
-        tb_decide<T>(a, ctrl, s_b, s_tile, gridDim.x * gridDim.y, sm.err[0], s_t, nullptr, nullptr);
+        tb_decide<T>(a, ctrl, s_b, s_tile, gridDim.x * gridDim.y, sm.err, s_t, nullptr, nullptr);
 }
 
 // One warp: the next tile of any pair that has one to hand out, or -1 when
@@ -1579,7 +1566,7 @@ __global__ void __launch_bounds__(T::NT, MINB) k_tvl1_q(const __grid_constant__ 
             // behind them, then one thread's device-scope fence before it
             // arrives (the pattern of a grid-wide barrier).
             const int prev = v_tile[it ^ 1];
-            if (prev >= 0) tb_decide<T>(a, a.ctrl + *v_b, *v_b, prev, ntiles, sm.err[it ^ 1], s_t, q, left);
+            if (prev >= 0) tb_decide<T>(a, a.ctrl + *v_b, *v_b, prev, ntiles, sm.err, s_t, q, left);
         }
         if (v_ahead[it ^ 1] < 0) {
             if (threadIdx.x < 32) {
@@ -1611,8 +1598,8 @@ __global__ void __launch_bounds__(T::NT, MINB) k_tvl1_q(const __grid_constant__ 
                 v_ahead[it] = ahead;
             }
         };
-        if (__syncthreads_or(rt_tile<T, false>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err[it], claim_ahead))) {
-            rt_tile_careful<T>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err[it]);
+        if (__syncthreads_or(rt_tile<T, false>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err, claim_ahead))) {
+            rt_tile_careful<T>(a, v_b, v_tile + it, tiles_x, s_t, sm, sm.err);
             __syncthreads();
         }
     }
@@ -2236,8 +2223,9 @@ static dim3 tb_grid(int cfg, int nx, int ny, int B) {
 // Microseconds measured on single pairs of 160x117 to 1280x720 (kTbAlone) and on
 // 32 pairs of 1024x436 (kTbMore); a large tile wastes less on its halo, small
 // ones use more SMs.  OFLOW_TB_CFG forces one configuration (used to test and
-// time them).  In the launch form (OFLOW_TB_QUEUE=0) levels above kTiledPx run
-// tiled.
+// time them).  With OFLOW_TB_QUEUE=0 levels above kTiledPx run tiled (plans that
+// share the GPU with others take the launch form after their configurations are
+// chosen, and keep resident levels).
 constexpr long long kTiledPx = 9216;
 constexpr float kTbAlone[kTbNumCfgs] = {24.0f, 21.0f, 17.5f, 16.0f};
 constexpr float kTbMore[kTbNumCfgs] = {12.0f, 7.6f, 6.8f, 4.5f};

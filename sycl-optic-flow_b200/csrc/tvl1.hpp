@@ -194,7 +194,6 @@ class TvPlan {
     size_t o_raw_ = 0, o_T_ = 0, o_pyr_ = 0, o_cc_ = 0, o_U0_ = 0, o_Uz_ = 0, o_P0_ = 0,
            o_out_ = 0, o_ctrl_ = 0, o_part_ = 0, o_recs_ = 0, o_iters_ = 0, o_energy_ = 0;
     float2 *ubuf(int k) const;  // state buffer k of u (all pairs)
-    float4 *pbuf(int k) const;  // state buffer k of p
     Graph graph_;
     int graph_launches_ = 0;
     std::vector<FrameRef> frames_;  // [B][2], host copy of the device table
