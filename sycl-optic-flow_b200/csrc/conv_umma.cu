@@ -264,44 +264,38 @@ __global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
         fence_async_smem();
         mbar_arrive(regbar);
         // The next region replaces one whose MMAs are done.  Thread 32 knows that
-        // from the last stage's buffer; the others wait on a barrier that can't pass
-        // them (the next commit to it needs their next arrival), which the buffers'
-        // could: those are freed once a stage, and tell two phases apart.
-        auto next_region = [&](int c0) {
-            load_region(c0);
-            cp_async_commit();
-            cp_async_wait<0>();
-            fence_async_smem();
-            mbar_arrive(regbar);
-        };
-        if (tid == 32) {
-            int buf = 0, ph = 0, left = per_reg, c0 = 0;  // stage s: its buffer is freed for the (ph + 1)-th time
+        // from the last stage's buffer and tells the others, on a barrier that can't
+        // pass them (thread 32's next arrival needs theirs on regbar), which the
+        // buffers' could: those are freed once a stage, and tell two phases apart.
+        int buf = 0, ph = 0, left = per_reg, c0 = 0;  // stage s: its buffer is freed for the (ph + 1)-th time
+        if (tid == 32 || per_reg < nst)
 #pragma unroll 1
-            for (int s = 0; s < nst; s++) {
-                if (!mbar_wait_bounded(freed + 8 * buf, ph)) {
+            for (int s = 0, rph = 0; s < nst; s++) {
+                if (tid == 32 && !mbar_wait_bounded(freed + 8 * buf, ph)) {
                     timed_out = true;
                     break;
                 }
-                if (issued < nst) fetch();
-                if (--left == 0 && s + 1 < nst) {
+                if (tid == 32 && issued < nst) fetch();
+                if (--left == 0 && s + 1 < nst) {  // the next channels
+                    if (tid == 32) {
+                        mbar_arrive(regdone);
+                    } else if (!mbar_wait_bounded(regdone, rph)) {
+                        timed_out = true;
+                        break;
+                    }
+                    rph ^= 1;
                     left = per_reg;
-                    next_region(c0 += cr);
+                    load_region(c0 += cr);
+                    cp_async_commit();
+                    cp_async_wait<0>();
+                    fence_async_smem();
+                    mbar_arrive(regbar);
                 }
                 if (++buf == bufs) {
                     buf = 0;
                     ph ^= 1;
                 }
             }
-        } else {
-#pragma unroll 1
-            for (int c0 = cr, ph = 0; c0 < d.C; c0 += cr, ph ^= 1) {
-                if (!mbar_wait_bounded(regdone, ph)) {
-                    timed_out = true;
-                    break;
-                }
-                next_region(c0);
-            }
-        }
         if (timed_out && tid == 32)  // its own copies in flight
             for (int s = imax(0, issued - bufs); s < issued; s++)
                 mbar_wait_bounded(full + 8 * (s % bufs), (uint32_t)(s / bufs) & 1u);
@@ -346,7 +340,6 @@ __global__ void __launch_bounds__(UmTile<MODE, MT>::NT)
                     default: um_issue<NP, T::NACC, DIL, PX, 14>(tmem, ad, bd, IDESC, t0, nacc, first); break;
                 }
                 umma_commit(freed + 8 * buf);
-                if (tap == 8 && kc0 + kcs == cr / 8 && s + 1 < nst) umma_commit(regdone);
             }
             __syncwarp();
             kc0 += kcs;
