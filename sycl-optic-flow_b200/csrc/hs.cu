@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kDTW *kDTH) k_hs_warp_deriv(
 // numerators in every sweep; so the tile's next launch is careful at once
 // (HsJacobiArgs::hint) until a launch meets none.  64 pairs of 320x240 with one moving
 // disc each, 200 sweeps: 12.4 ms without the hint and with IEEE divisions for all of
-// a tile, 4.3 ms here, and 2.7 where everything moves.  (Looking at a warp's
+// a tile, 4.3 ms here, and 2.6 where everything moves.  (Looking at a warp's
 // numerators once a sweep, before its quotients, needs no second run; it costs
 // frames without any 15 %.)
 template <int V_, int NW_, int K_> struct HsTile {
@@ -318,7 +318,7 @@ __device__ __forceinline__ void hs_fetch(const HsJacobiArgs &a, int tile, HsSmem
 template <typename T, bool CAREFUL, typename F>
 __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const HsSmem<T> &sm,
                                         float4 (*sRow)[2][T::NW][32], F &&taken) {
-    constexpr int V = T::V, K = T::K, NW = T::NW;
+    constexpr int V = T::V, K = T::K, NW = T::NW, U = K < 8 ? K : 8;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, w = a.w, h = a.h;
     const HsAt t = hs_at<T>(a, tile);
     const int x = t.x, y0 = t.y0;
@@ -357,10 +357,11 @@ __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const H
         for (int j = 0; j < a.sweeps; j++) hs_step<T, 2, false>(s, j, sRow, top, e, broken, key, taken);
     } else if (interior) {
         // unrolled, so that old and new increments swap registers instead of being copied
-#pragma unroll 4
+        // (64 pairs of 320x240, 200 sweeps: 2.61 ms, with 4 and 2 sweeps here and below 2.70)
+#pragma unroll U
         for (int j = 0; j < K; j++) hs_step<T, 0, false>(s, j, sRow, top, e, broken, key, taken);
     } else if (t.oy + T::RH <= h - 1 && (w & 1) == 0) {
-#pragma unroll 2
+#pragma unroll U
         for (int j = 0; j < K; j++) hs_step<T, 1, false>(s, j, sRow, top, e, broken, key, taken);
     } else {
 #pragma unroll 2
