@@ -1029,7 +1029,7 @@ __global__ void __launch_bounds__(NT) k_tvl1_iter(IterArgs a) {
 // a row of a warp at a time, and only its small numerators divided in double.
 // Where frames are equal outside something that moves there are such numerators
 // ahead of what spreads from it: 8 pairs of 320x240 with one disc each, one scale,
-// 5 warps of 300 iterations, take 17.9 ms and 13.0 where everything moves; with
+// 5 warps of 300 iterations, take 17.4 ms and 12.8 where everything moves; with
 // IEEE divisions and square roots in all of a second run, 26.3 ms.  (Running the
 // tile the careful way at once where it broke in the block of iterations before:
 // 17.0 ms, but the registers that the choice takes cost 8 % where everything moves.)
@@ -1285,7 +1285,7 @@ __device__ __forceinline__ bool rt_tile(const TbArgs &a, const volatile int *vb,
 #pragma unroll 1
     for (int j = 0; j < *(volatile const int *)&t.kk; j++) {
         double e = 0.0;
-        if (interior)
+        if (!CAREFUL && interior)
             rt_iteration<T, false, CAREFUL>(s, sm, x, y0, nx, ny, a.l_t, a.theta, a.taut, fg, e);
         else
             rt_iteration<T, true, CAREFUL>(s, sm, x, y0, nx, ny, a.l_t, a.theta, a.taut, fg, e);
