@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(kDTW *kDTH) k_hs_warp_deriv(
 //
 // The division by Ix^2+Iy^2+alpha is Markstein's correction from the
 // reciprocal, formed once per launch.  What that takes for granted (numerators
-// zero or above 2^-100, denominators in [2^-40, 2^24)) is kept as a running
+// zero or above 2^-100, denominators in [2^-40, 2^24); or, for frames of 16 bits,
+// above 2^-76 and in [2^24, 2^48)) is kept as a running
 // minimum; a block that breaks it runs its tile again from the untouched input,
 // CAREFUL: looking at each numerator.  Where a part of the frames stands still the
 // increments fall off from what moves by about 1/4 a pixel, and there are such
@@ -151,13 +152,31 @@ struct HsEdge {
     int bottom;             // the warp's row that is the last of the image (else out of its rows)
 };
 
+// Denominators whose reciprocal rcp_near_rn rounds correctly (the device tests check
+// every float of the range), and the least key of a numerator whose quotient by one
+// below den markstein forms: either way quotients stay above 2^-124.
+constexpr float kHsDenHi = 0x1p48f;
+constexpr unsigned kMarksteinKeyFar = 2u * 0x19800000u;  // 2^-76
+__device__ __forceinline__ bool hs_den_in_range(float den) { return den >= kRcpLo && den < kHsDenHi; }
+__device__ __forceinline__ unsigned hs_least_key(float den) {
+    return den < kRcpHi ? kMarksteinKey : kMarksteinKeyFar;
+}
+
 // p / den: Markstein's correction where it holds, in double where p is too small
 // for it, the IEEE division where den is out of range.
 __device__ __forceinline__ float hs_quotient(float p, float den, float rcp) {
     float q = markstein(p, den, rcp);
-    if (markstein_key(p) < kMarksteinKey || !rcp_in_range(den))
-        q = rcp_in_range(den) ? div_in_double(p, den, rcp) : p / den;
+    if (markstein_key(p) < hs_least_key(den) || !hs_den_in_range(den))
+        q = hs_den_in_range(den) ? div_in_double(p, den, rcp) : p / den;
     return q;
+}
+
+// The largest of the thread's denominators.
+template <int V> __device__ __forceinline__ float hs_den_most(const HsState<V> &s) {
+    float m = s.den[0][0];
+#pragma unroll
+    for (int v = 0; v < V; v++) m = fmaxf(m, fmaxf(s.den[v][0], s.den[v][1]));
+    return m;
 }
 
 // One sweep (solverKernel.cuh:41-153): neighbour mean of the increments
@@ -216,7 +235,7 @@ __device__ __forceinline__ void hs_sweep(HsState<T::V> &s, float4 above, float4 
         dn[1] = c1;
     }
     if (CAREFUL) {
-        const bool look = __any_sync(0xffffffffu, broken || now < kMarksteinKey);
+        const bool look = __any_sync(0xffffffffu, broken || now < hs_least_key(hs_den_most(s)));
         key = umin(key, now);
 #pragma unroll
         for (int v = 0; v < V; v++)
@@ -344,7 +363,7 @@ __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const H
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             s.rcp[v][c] = rcp_near_rn(s.den[v][c]);
-            broken |= !rcp_in_range(s.den[v][c]);
+            broken |= !hs_den_in_range(s.den[v][c]);
         }
     const bool interior = t.ox >= 1 && t.oy >= 1 && t.ox + T::RW <= w - 1 && t.oy + T::RH <= h - 1;
     const HsEdge e{x == 0, x + 1 == w - 1, x == w - 1, h - 1 - y0};
@@ -368,7 +387,7 @@ __device__ __forceinline__ bool hs_tile(const HsJacobiArgs &a, int tile, const H
         for (int j = 0; j < K; j++) hs_step<T, 2, false>(s, j, sRow, top, e, broken, key, taken);
     }
     // (also: every warp has read the rows before the next tile writes them)
-    const bool bad = __syncthreads_or(broken || key < kMarksteinKey);
+    const bool bad = __syncthreads_or(broken || key < hs_least_key(hs_den_most(s)));
     if (!CAREFUL && bad) return true;
     if (lane < K / 2 || lane >= 32 - K / 2 || wid < K / V || wid >= NW - K / V || x >= w) return bad;
     float2 *Out = (a.last ? a.U : a.out) + (size_t)t.b * a.stride;
@@ -511,7 +530,7 @@ __device__ __forceinline__ bool hs_res_load(const HsJacobiArgs &a, const HsAt &t
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             s.rcp[v][c] = rcp_near_rn(s.den[v][c]);
-            broken |= !rcp_in_range(s.den[v][c]);
+            broken |= !hs_den_in_range(s.den[v][c]);
         }
     return broken;
 }
@@ -603,7 +622,7 @@ __global__ void __launch_bounds__(T::NT, 2) k_hs_res(const __grid_constant__ HsJ
     // before the last meeting)
     __shared__ int s_bad;
     if (threadIdx.x == 0) s_bad = 0;
-    unsigned key = broken ? 0u : ~0u;
+    unsigned key = ~0u;
 #pragma unroll
     for (int v = 0; v < V; v++) s.a[v][0] = s.a[v][1] = make_float2(0.f, 0.f);
     int buf = 0;
@@ -629,7 +648,7 @@ __global__ void __launch_bounds__(T::NT, 2) k_hs_res(const __grid_constant__ HsJ
         if (!own) hs_res_take<T>(a, t, sm, buf, s);
     }
     if (a.sweeps <= K) cluster_barrier();  // (every block runs before its memory is written)
-    if (key < kMarksteinKey)
+    if (broken || key < hs_least_key(hs_den_most(s)))
         for (int k = 0; k < a.tiles_x * a.tiles_y; k++) cluster_st1(smem_u32(&s_bad), k, 1);
     cluster_barrier();
     const bool bad = s_bad != 0;
